@@ -74,6 +74,15 @@ __device__ __forceinline__ U32x8 ld_nc_256(const void* p) {
   return r;
 }
 
+// One value that the kernel before this one on the stream may have written, read after pdl_wait().  __ldg promises the
+// compiler that the value does not change while the kernel runs and may be moved in front of the wait: under a
+// programmatic launch that read what was there before (seen as a wrong global scale in some CTAs of the NVFP4 GEMM).
+__device__ __forceinline__ float ld_dependent(const float* p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ uint4 ld_nc_128(const void* p) {
   uint4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"

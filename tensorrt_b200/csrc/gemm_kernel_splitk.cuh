@@ -254,8 +254,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
       pdl_wait();  // the activation scales come from the kernel before this one
       if (wrow < p.M) {
-        if constexpr (NVF4) xs = __fmul_rn(__ldg(p.a_scales), __ldg(p.b_scales));
-        else xs = __ldg(p.a_scales + static_cast<int64_t>(wrow) * p.a_scale_stride);
+        if constexpr (NVF4) xs = __fmul_rn(ld_dependent(p.a_scales), ld_dependent(p.b_scales));
+        else xs = ld_dependent(p.a_scales + static_cast<int64_t>(wrow) * p.a_scale_stride);
       }
       wscale[wrow] = ws;
       wbias[wrow] = wb;

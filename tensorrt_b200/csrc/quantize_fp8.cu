@@ -83,9 +83,9 @@ fp8_rows_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t
   if constexpr (AMAX_MODE == 0) {
     a = block_max<kRowThreads>(local, red);
   } else if constexpr (AMAX_MODE == 1) {
-    a = __ldg(amax);
+    a = ld_dependent(amax);
   } else {
-    a = __ldg(amax + row);
+    a = ld_dependent(amax + row);
   }
   const float scale = fp8_scale_from_amax(a);
   if (threadIdx.x == 0 && scales != nullptr && (AMAX_MODE != 1 || row == 0)) scales[AMAX_MODE == 1 ? 0 : row] = scale;
