@@ -353,6 +353,72 @@ def add_rms_norm_fp8_quantize(h: torch.Tensor, delta: torch.Tensor | None, weigh
     return h_out, codes, scales
 
 
+def _nvfp4_out(shape, rows, cols, device):
+    """(packed codes, swizzled block scales, global scale) of an NVFP4 operand [rows, cols], uninitialised."""
+    return (torch.empty(*shape[:-1], cols // 2, dtype=torch.uint8, device=device),
+            torch.empty(nvfp4_scale_bytes(rows, cols), dtype=torch.uint8, device=device), torch.empty((), dtype=torch.float32, device=device))
+
+
+def _scalar_amax(amax_t, device):
+    return amax_t.to(device=device, dtype=torch.float32).reshape(1)
+
+
+def add_rms_norm_nvfp4_quantize(h: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, amax_t: torch.Tensor, eps: float = 1e-5):
+    """-> (h + delta (h itself when delta is None), NVFP4 operand of rms_norm(h + delta) under the calibrated
+    tensor amax): the same bits as `add`, `rms_norm`, `nvfp4_quantize`, in one pass.  At most 16384 columns."""
+    _need_cuda(h, delta, weight, amax_t)
+    _bf16(h, weight)
+    h = h.contiguous()
+    rows, cols = _rows_cols(h)
+    if cols % 16:
+        raise ValueError(f"last dimension ({cols}) must be a multiple of the block size 16")
+    h_out = h
+    if delta is not None:
+        _bf16(delta)
+        delta = delta.contiguous()
+        h_out = torch.empty_like(h)
+    a = _scalar_amax(amax_t, h.device)
+    codes, scales, g = _nvfp4_out(h.shape, rows, cols, h.device)
+    with torch.cuda.device(h.device):
+        check(load().b200q_add_rms_norm_nvfp4_quantize(h.data_ptr(), _ptr(delta), weight.data_ptr(), h_out.data_ptr(), a.data_ptr(),
+                                                       codes.data_ptr(), scales.data_ptr(), g.data_ptr(), rows, cols, eps, _stream(h)),
+              "b200q_add_rms_norm_nvfp4_quantize")
+    return h_out, (codes, scales, g)
+
+
+def silu_mul_nvfp4_quantize(gate_up: torch.Tensor, amax_t: torch.Tensor):
+    """[.., 2F] (gate columns first) -> NVFP4 operand of silu(gate) * up under a calibrated tensor amax: the same bits
+    as `silu_mul` and `nvfp4_quantize`, the bf16 activation is never written.  F a multiple of 16."""
+    _need_cuda(gate_up, amax_t)
+    _bf16(gate_up)
+    gate_up = gate_up.contiguous()
+    rows, two_f = _rows_cols(gate_up)
+    f = two_f // 2
+    if two_f % 32:
+        raise ValueError(f"the activation width ({two_f / 2:g}) must be a multiple of the block size 16")
+    a = _scalar_amax(amax_t, gate_up.device)
+    codes, scales, g = _nvfp4_out(gate_up.shape, rows, f, gate_up.device)
+    with torch.cuda.device(gate_up.device):
+        check(load().b200q_silu_mul_nvfp4_quantize(gate_up.data_ptr(), a.data_ptr(), codes.data_ptr(), scales.data_ptr(), g.data_ptr(), rows, f,
+                                                   _stream(gate_up)), "b200q_silu_mul_nvfp4_quantize")
+    return codes, scales, g
+
+
+def expand_heads_nvfp4_quantize(src: torch.Tensor, col0: int, heads_out: int, rep: int, head_dim: int, amax_t: torch.Tensor):
+    """`expand_heads` followed by `nvfp4_quantize` under a calibrated tensor amax, in one pass, the same bits."""
+    _need_cuda(src, amax_t)
+    _bf16(src)
+    src = src.contiguous()
+    rows, width = _rows_cols(src)
+    a = _scalar_amax(amax_t, src.device)
+    codes, scales, g = _nvfp4_out((*src.shape[:-1], 0), rows, heads_out * head_dim, src.device)
+    with torch.cuda.device(src.device):
+        check(load().b200q_expand_heads_nvfp4_quantize(src.data_ptr(), width, col0, a.data_ptr(), codes.data_ptr(), scales.data_ptr(),
+                                                       g.data_ptr(), rows, heads_out, rep, head_dim, _stream(src)),
+              "b200q_expand_heads_nvfp4_quantize")
+    return codes, scales, g
+
+
 def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
     """[.., 2F] (gate columns first) -> [.., F] = silu(gate) * up."""
     _need_cuda(gate_up)

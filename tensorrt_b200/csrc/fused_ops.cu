@@ -4,7 +4,7 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "common.cuh"
+#include "nvfp4_block.cuh"
 #include "tcgen05.cuh"
 
 namespace b200q {
@@ -25,6 +25,27 @@ __device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
+}
+
+// Eight normalised values per thread (bf16-rounded), one group g of 8 per lane, the two halves of a 16-element block
+// in neighbouring lanes -> NVFP4 codes and swizzled block scales of row `row`.  All 32 lanes take part; lanes whose g
+// lies beyond the row pass zeros.  The warp's first g is a multiple of 8, so that 8 lanes hold one scale word.
+__device__ __forceinline__ void store_nvfp4_group(const float* v, int g, int groups, int64_t row, int64_t cols, const GlobalScale& gs,
+                                                  const Nvfp4Out& o) {
+  float a = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) a = fmaxf(a, fabsf(v[j]));
+  a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 1));
+  uint32_t codes, sb = 0u;
+  if (g < groups) {
+    sb = quantize_half_block(v, a, gs, codes);
+    *reinterpret_cast<uint32_t*>(o.codes + row * (cols >> 1) + static_cast<int64_t>(g) * 4) = codes;
+  }
+  uint32_t w = (g & 1) == 0 ? sb << (8 * ((g >> 1) & 3)) : 0u;
+  w |= __shfl_xor_sync(0xffffffffu, w, 2);
+  w |= __shfl_xor_sync(0xffffffffu, w, 4);
+  if ((g & 7) == 0 && g < groups)
+    *reinterpret_cast<uint32_t*>(o.sf + ((row >> 7) * o.col_tiles + (g >> 3)) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4) = w;
 }
 
 // y = x * rsqrt(mean(x^2) + eps) * w, fp32 math, bf16 in/out; one CTA per row, the row stays
@@ -92,20 +113,29 @@ rms_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // other, with 1.75 bytes of traffic per element and step instead of 3.25.
 // PARTS > 1: a cluster of PARTS CTAs shares one token (few tokens: a decode step); the slices'
 // sums of squares and maxima meet through distributed shared memory, summed in rank order.
-template <int ITEMS, int PARTS>
+// NVF4: the normalised row leaves as NVFP4 codes and block scales under a calibrated tensor amax (`nv`) instead of
+// per-token FP8; no row maximum is needed.  CTAs of the rows that only pad the last 128-row scale tile clear theirs.
+template <int ITEMS, int PARTS, bool NVF4>
 __global__ void __launch_bounds__(kThreads)
 add_norm_quant_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out, uint8_t* __restrict__ codes,
-                      float* __restrict__ scales, int64_t cols, float eps) {
+                      float* __restrict__ scales, int64_t rows, int64_t cols, float eps, const Nvfp4Out nv) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[kThreads / 32];
   __shared__ float part_val[2];
   const int64_t row = blockIdx.x / PARTS;
+  if constexpr (NVF4) {
+    if (row >= rows) {                       // whole clusters: no CTA of this token waits for another
+      if (blockIdx.x % PARTS == 0) zero_scale_row(nv.sf, row, nv.col_tiles);
+      return;
+    }
+  }
   const int part = PARTS > 1 ? static_cast<int>(blockIdx.x % PARTS) : 0;   // == rank in the cluster
   const int groups = static_cast<int>(cols >> 3);
-  const int per_part = (groups + PARTS - 1) / PARTS;
-  const int g_begin = part * per_part, g_end = min(groups, g_begin + per_part);
+  int per_part = (groups + PARTS - 1) / PARTS;
+  if constexpr (NVF4) per_part = (per_part + 7) / 8 * 8;   // whole scale words
+  const int g_begin = min(groups, part * per_part), g_end = min(groups, g_begin + per_part);
   // few-token form: the norm weights are requested together with the row, ahead of the first
   // reduction; many-token form: loaded after it (fewer live registers, more CTAs per SM)
   constexpr bool kEarlyW = PARTS > 1;
@@ -156,6 +186,14 @@ add_norm_quant_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* 
       }
     }
   }
+  if constexpr (NVF4) {
+    const GlobalScale gs(ld_dependent(nv.amax));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nv.gout != nullptr) *nv.gout = gs.g;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) store_nvfp4_group(v[i], g_begin + threadIdx.x + i * kThreads, g_end, row, cols, gs, nv);
+    if constexpr (PARTS > 1) cluster_barrier();  // nobody leaves while a peer may still read its shared memory
+    return;
+  }
   // block max (values are >= 0): reuse the sum scratch
   amax = warp_max(amax);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
@@ -197,11 +235,12 @@ add_norm_quant_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* 
 constexpr int kStreamStagesMax = 8;
 constexpr int kStreamRingBytes = 96 * 1024;
 
-template <int ITEMS, bool HAS_DELTA>
+template <int ITEMS, bool HAS_DELTA, bool NVF4>
 __global__ void __launch_bounds__(kThreads, 2)
 add_norm_quant_stream_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
                              const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out, uint8_t* __restrict__ codes,
-                             float* __restrict__ scales, int rows, int cols, float eps, int stages, int* __restrict__ status) {
+                             float* __restrict__ scales, int rows, int cols, float eps, int stages, int* __restrict__ status,
+                             const Nvfp4Out nv) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(128) unsigned char ring[];
@@ -233,6 +272,11 @@ add_norm_quant_stream_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfl
   for (int i = 0; i < ITEMS; ++i) {
     const int g = threadIdx.x + i * kThreads;
     wp[i] = g < groups ? ld_nc_128(w + (int64_t)g * 8) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  const GlobalScale gs(NVF4 ? ld_dependent(nv.amax) : 1.0f);
+  if constexpr (NVF4) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nv.gout != nullptr) *nv.gout = gs.g;
+    for (int64_t row = rows + blockIdx.x; row < (rows + 127) / 128 * 128; row += step) zero_scale_row(nv.sf, row, nv.col_tiles);
   }
   int k = 0;
   for (int64_t row = blockIdx.x; row < rows; row += step, ++k) {
@@ -285,6 +329,11 @@ add_norm_quant_stream_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfl
           amax = fmaxf(amax, fabsf(v[i][j]));
         }
       }
+    }
+    if constexpr (NVF4) {
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i) store_nvfp4_group(v[i], threadIdx.x + i * kThreads, groups, row, cols, gs, nv);
+      continue;
     }
     amax = warp_max(amax);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
@@ -618,6 +667,89 @@ int grid_for(int64_t work_items) {
   return static_cast<int>(ctas < 1 ? 1 : (ctas > cap ? cap : ctas));
 }
 
+// Launch of the add + RMSNorm + quantize kernels (checked arguments).  NVF4: result into `nv`, else per-token FP8.
+template <bool NVF4>
+int launch_add_norm_quant(const void* h, const void* delta, const void* weight, void* h_out, uint8_t* codes_out, float* scales_out,
+                          int64_t rows, int64_t cols, float eps, const Nvfp4Out& nv, cudaStream_t st) {
+  const auto* hp = static_cast<const __nv_bfloat16*>(h);
+  const auto* dp = static_cast<const __nv_bfloat16*>(delta);
+  const auto* wp = static_cast<const __nv_bfloat16*>(weight);
+  auto* op = static_cast<__nv_bfloat16*>(h_out);
+  const int64_t groups = cols >> 3;
+  int parts = 1;   // few tokens: split every row over a cluster so that the launch covers more SMs
+  while (parts < 8 && rows * parts < 2 * sm_count() && groups / (parts * 2) >= kThreads / 2) parts *= 2;
+  int64_t per_part = (groups + parts - 1) / parts;
+  if (NVF4) per_part = (per_part + 7) / 8 * 8;
+  const int items = static_cast<int>((per_part + kThreads - 1) / kThreads);
+  const int64_t grid_rows = NVF4 ? (rows + 127) / 128 * 128 : rows;
+  // many tokens: persistent CTAs fed through a shared-memory ring of rows
+  const int64_t stage_bytes = cols * 2 * (delta != nullptr ? 2 : 1);
+  if (parts == 1 && items <= 4 && rows >= 8 * sm_count() && kStreamRingBytes / stage_bytes >= 2) {
+    int stages = static_cast<int>(kStreamRingBytes / stage_bytes);
+    if (stages > kStreamStagesMax) stages = kStreamStagesMax;
+    int* status = gemm::device_status_word();
+    if (status == nullptr) return B200Q_ERR_CUDA;
+    const size_t smem = static_cast<size_t>(stages) * static_cast<size_t>(stage_bytes);
+    const dim3 grid(static_cast<unsigned>(2 * sm_count()));
+    const int r32 = static_cast<int>(rows), c32 = static_cast<int>(cols);
+#define B200Q_ANQS(I, D)                                                                                                     \
+  do {                                                                                                                        \
+    cudaFuncSetAttribute(add_norm_quant_stream_kernel<I, D, NVF4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamRingBytes); \
+    launch_pdl(add_norm_quant_stream_kernel<I, D, NVF4>, grid, dim3(kThreads), smem, st, hp, dp, wp, op, codes_out, scales_out,     \
+               r32, c32, eps, stages, status, nv);                                                                                \
+  } while (0)
+    if (delta != nullptr) {
+      if (items <= 1) B200Q_ANQS(1, true);
+      else if (items <= 2) B200Q_ANQS(2, true);
+      else B200Q_ANQS(4, true);
+    } else {
+      if (items <= 1) B200Q_ANQS(1, false);
+      else if (items <= 2) B200Q_ANQS(2, false);
+      else B200Q_ANQS(4, false);
+    }
+#undef B200Q_ANQS
+    return check_launch();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid_rows * parts));
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(parts);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+#define B200Q_ANQ(I, P) cudaLaunchKernelEx(&cfg, add_norm_quant_kernel<I, P, NVF4>, hp, dp, wp, op, codes_out, scales_out, rows, cols, eps, nv)
+  if (parts == 1) {
+    if (items <= 1) B200Q_ANQ(1, 1);
+    else if (items <= 2) B200Q_ANQ(2, 1);
+    else if (items <= 4) B200Q_ANQ(4, 1);
+    else B200Q_ANQ(8, 1);
+  } else if (parts == 2) {
+    if (items <= 1) B200Q_ANQ(1, 2);
+    else if (items <= 2) B200Q_ANQ(2, 2);
+    else B200Q_ANQ(4, 2);
+  } else if (parts == 4) {
+    if (items <= 1) B200Q_ANQ(1, 4);
+    else B200Q_ANQ(2, 4);
+  } else {
+    B200Q_ANQ(1, 8);
+  }
+#undef B200Q_ANQ
+  return check_launch();
+}
+
+int check_add_norm(const void* h, const void* delta, const void* weight, const void* h_out) {
+  if (h == nullptr || weight == nullptr) return B200Q_ERR_INVALID;
+  if (delta != nullptr && h_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(h, 16) || !aligned(weight, 16) || (delta != nullptr && (!aligned(delta, 16) || !aligned(h_out, 16)))) return B200Q_ERR_ALIGN;
+  return B200Q_OK;
+}
+
 }  // namespace
 
 // Dynamic per-token FP8 quantize of many long bf16 rows through the ring-fed persistent kernel
@@ -680,79 +812,24 @@ int b200q_add_rms_norm_fp8_quantize(const void* h, const void* delta, const void
                                     float* scales_out, int64_t rows, int64_t cols, float eps, b200q_stream_t stream) {
   if (rows < 0 || cols < 0 || cols % 16 != 0 || rows > 0x7fffffffLL || cols > kThreads * 8 * 8) return B200Q_ERR_INVALID;
   if (rows == 0 || cols == 0) return B200Q_OK;
-  if (h == nullptr || weight == nullptr || codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
-  if (delta != nullptr && h_out == nullptr) return B200Q_ERR_INVALID;
-  if (!aligned(h, 16) || !aligned(weight, 16) || !aligned(codes_out, 8) || (delta != nullptr && (!aligned(delta, 16) || !aligned(h_out, 16))))
-    return B200Q_ERR_ALIGN;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (int rc = check_add_norm(h, delta, weight, h_out)) return rc;
+  if (!aligned(codes_out, 8)) return B200Q_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const auto* hp = static_cast<const __nv_bfloat16*>(h);
-  const auto* dp = static_cast<const __nv_bfloat16*>(delta);
-  const auto* wp = static_cast<const __nv_bfloat16*>(weight);
-  auto* op = static_cast<__nv_bfloat16*>(h_out);
-  const int64_t groups = cols >> 3;
-  int parts = 1;   // few tokens: split every row over a cluster so that the launch covers more SMs
-  while (parts < 8 && rows * parts < 2 * sm_count() && groups / (parts * 2) >= kThreads / 2) parts *= 2;
-  const int items = static_cast<int>(((groups + parts - 1) / parts + kThreads - 1) / kThreads);
-  // many tokens: persistent CTAs fed through a shared-memory ring of rows
-  const int64_t stage_bytes = cols * 2 * (delta != nullptr ? 2 : 1);
-  if (parts == 1 && items <= 4 && rows >= 8 * sm_count() && kStreamRingBytes / stage_bytes >= 2) {
-    int stages = static_cast<int>(kStreamRingBytes / stage_bytes);
-    if (stages > kStreamStagesMax) stages = kStreamStagesMax;
-    int* status = gemm::device_status_word();
-    if (status == nullptr) return B200Q_ERR_CUDA;
-    const size_t smem = static_cast<size_t>(stages) * static_cast<size_t>(stage_bytes);
-    const dim3 grid(static_cast<unsigned>(2 * sm_count()));
-    const int r32 = static_cast<int>(rows), c32 = static_cast<int>(cols);
-#define B200Q_ANQS(I, D)                                                                                                     \
-  do {                                                                                                                        \
-    cudaFuncSetAttribute(add_norm_quant_stream_kernel<I, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamRingBytes); \
-    launch_pdl(add_norm_quant_stream_kernel<I, D>, grid, dim3(kThreads), smem, st, hp, dp, wp, op, codes_out, scales_out,     \
-               r32, c32, eps, stages, status);                                                                                \
-  } while (0)
-    if (delta != nullptr) {
-      if (items <= 1) B200Q_ANQS(1, true);
-      else if (items <= 2) B200Q_ANQS(2, true);
-      else B200Q_ANQS(4, true);
-    } else {
-      if (items <= 1) B200Q_ANQS(1, false);
-      else if (items <= 2) B200Q_ANQS(2, false);
-      else B200Q_ANQS(4, false);
-    }
-#undef B200Q_ANQS
-    return check_launch();
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(rows * parts));
-  cfg.blockDim = dim3(kThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(parts);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-#define B200Q_ANQ(I, P) cudaLaunchKernelEx(&cfg, add_norm_quant_kernel<I, P>, hp, dp, wp, op, codes_out, scales_out, cols, eps)
-  if (parts == 1) {
-    if (items <= 1) B200Q_ANQ(1, 1);
-    else if (items <= 2) B200Q_ANQ(2, 1);
-    else if (items <= 4) B200Q_ANQ(4, 1);
-    else B200Q_ANQ(8, 1);
-  } else if (parts == 2) {
-    if (items <= 1) B200Q_ANQ(1, 2);
-    else if (items <= 2) B200Q_ANQ(2, 2);
-    else B200Q_ANQ(4, 2);
-  } else if (parts == 4) {
-    if (items <= 1) B200Q_ANQ(1, 4);
-    else B200Q_ANQ(2, 4);
-  } else {
-    B200Q_ANQ(1, 8);
-  }
-#undef B200Q_ANQ
-  return check_launch();
+  return launch_add_norm_quant<false>(h, delta, weight, h_out, codes_out, scales_out, rows, cols, eps, Nvfp4Out{}, static_cast<cudaStream_t>(stream));
+}
+
+int b200q_add_rms_norm_nvfp4_quantize(const void* h, const void* delta, const void* weight, void* h_out, const float* amax,
+                                      uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out, int64_t rows, int64_t cols,
+                                      float eps, b200q_stream_t stream) {
+  if (rows < 0 || cols < 0 || cols % 16 != 0 || rows > 0x7fffff80LL || cols > kThreads * 8 * 8) return B200Q_ERR_INVALID;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  if (amax == nullptr || codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (int rc = check_add_norm(h, delta, weight, h_out)) return rc;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  const Nvfp4Out nv{amax, codes_out, scales_out, global_scale_out, static_cast<uint32_t>((cols / 16 + 3) / 4)};
+  return launch_add_norm_quant<true>(h, delta, weight, h_out, nullptr, nullptr, rows, cols, eps, nv, static_cast<cudaStream_t>(stream));
 }
 
 int b200q_silu_mul(const void* gate_up, void* out, int64_t rows, int64_t f, b200q_stream_t stream) {

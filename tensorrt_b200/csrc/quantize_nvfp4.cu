@@ -18,7 +18,7 @@
 //   s_blk  = e4m3_rne(min((amax_blk / 6) / global, 448));  d = fp32(s_blk) * global
 //   code   = e2m1_rne_sat(x_fp32 / d); all codes of a block with s_blk == 0 are 0
 //   x_hat  = e2m1 * d, rounded (RNE) to the input dtype.
-#include "common.cuh"
+#include "nvfp4_block.cuh"
 
 namespace b200q {
 namespace {
@@ -85,109 +85,54 @@ struct Block16<float> {
   }
 };
 
-// byte offset of the 4-byte scale word holding scale columns [4*(c/4), 4*(c/4)+4) of row r
-__device__ __forceinline__ int64_t swizzled_word_offset(int64_t r, int64_t c, int64_t col_tiles) {
-  const int64_t tile = (r >> 7) * col_tiles + (c >> 2);
-  return tile * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4;
-}
-
-// eight fp32 -> eight E2M1 nibbles in one word (RNE, saturating), element 0 in the lowest nibble
-__device__ __forceinline__ uint32_t pack8_e2m1(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
-  uint32_t r;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(r)
-      : "f"(a0), "f"(a1), "f"(a2), "f"(a3), "f"(a4), "f"(a5), "f"(a6), "f"(a7));
-  return r;
-}
-
-constexpr float kRcp6 = 0.16666667163372039794921875f;   // RN(1/6)
-constexpr float kRcp448 = 0.002232142956927418708801269531f;  // RN(1/448)
-
-// Per-launch constants of the scale computation: global scale, its reciprocal, and whether
-// the shared-divisor sequence may be used for divisions by it.
-struct GlobalScale {
-  float g, yg;
-  bool fast;
-  __device__ __forceinline__ explicit GlobalScale(float amax) {
-    // (amax / 6) / 448 as exact IEEE quotients; the shared-divisor sequence is exact for a
-    // numerator in the normal range away from its ends, anything else takes true divisions
-    const uint32_t e = (__float_as_uint(amax) >> 23) & 0xffu;
-    if (e >= 64u && e <= 190u) {
-      g = b200q_div_by_shared(b200q_div_by_shared(amax, kE2M1Max, kRcp6), kE4M3Max, kRcp448);
-    } else {
-      g = nvfp4_global_from_amax(amax);
-    }
-    yg = b200q_rcp_rn(g);
-    fast = b200q_div_fast_ok(g);
-  }
+// Where a block's 16 values come from.
+//   Src::kPlain     row-major [rows, cols]
+//   Src::kSiluMul   silu(gate) * up of a [rows, 2 cols] gate/up projection (gate columns first), rounded to bf16 as
+//                   silu_mul_kernel stores it: the activation in front of the down projection is never written
+//   Src::kExpand    column c of the output is column src_col0 + (c / hd / rep) * hd + c % hd of a row of src_stride
+//                   elements (every kv head repeated `rep` times): the expanded tensor is never written
+enum class Src { kPlain, kSiluMul, kExpand };
+struct ExpandMap {
+  int64_t src_stride, src_col0;
+  uint32_t head_dim, rep;
 };
-
-
-// Quantize one block held in f[16]: returns the 8-bit scale, writes 16 codes as two words and
-// the effective divisor d = fp32(scale) * global.
-__device__ __forceinline__ uint32_t quantize_block(const float* f, const GlobalScale& gs, uint32_t& c_lo, uint32_t& c_hi,
-                                                   float& d_out) {
-  float m[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m[i] = fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1]));
-  const float a = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
-  // s = (a / 6) / g, both as exact IEEE quotients
-  float s;
-  if (gs.fast) {
-    s = b200q_div_by_shared(b200q_div_by_shared(a, kE2M1Max, kRcp6), gs.g, gs.yg);
-  } else {
-    s = __fdiv_rn(__fdiv_rn(a, kE2M1Max), gs.g);
-  }
-  const bool clamped = s > kE4M3Max;
-  const uint32_t sb = f32x2_to_e4m3x2(s, 0.0f) & 0xffu;  // saturates to 448
-  const float d = __fmul_rn(e4m3_to_f32(sb), gs.g);
-  d_out = d;
-  if (sb != 0u && !clamped && b200q_div_fast_ok(d)) {
-    // common case: |x| <= 6.5 d, so the quotient can neither overflow nor need a clamp
-    const float y = b200q_rcp_rn(d);
-    float q[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] = b200q_div_by_shared(f[i], d, y);
-    c_lo = pack8_e2m1(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-    c_hi = pack8_e2m1(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
-  } else if (sb != 0u) {
-    // stored scale saturated at 448 (amax input below the data) or an extreme divisor:
-    // true division on a numerator clamped to 8 d, which still saturates to +-6
-    const float lim = __fmul_rn(d, 8.0f);
-    float q[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] = with_sign_of(__fdiv_rn(fminf(fabsf(f[i]), lim), d), f[i]);
-    c_lo = pack8_e2m1(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-    c_hi = pack8_e2m1(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
-  } else {
-    c_lo = 0u;
-    c_hi = 0u;
-  }
-  return sb;
-}
 
 // FAKE = false: codes + swizzled scales.  FAKE = true: dequantized values in T.
 // Grid: x = row, y = chunk of the row.  A warp covers U spans of 32 consecutive blocks
 // (512 elements each); all U 256-bit loads of a lane are issued before any arithmetic.
-template <typename T, bool FAKE, int U>
+// Rows from `rows` to the end of the last 128-row scale tile (FAKE = false) only clear their scale words.
+template <typename T, bool FAKE, int U, Src SRC>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_quantize_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ codes,
-                      uint8_t* __restrict__ sf, T* __restrict__ fake, float* __restrict__ gout, uint32_t cols,
-                      uint32_t blocks_per_row, uint32_t col_tiles) {
+                      uint8_t* __restrict__ sf, T* __restrict__ fake, float* __restrict__ gout, uint32_t rows, uint32_t cols,
+                      uint32_t blocks_per_row, uint32_t col_tiles, const ExpandMap map) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t row = blockIdx.x;
+  if constexpr (!FAKE) {
+    if (blockIdx.x >= rows) {
+      if (blockIdx.y == 0) zero_scale_row(sf, row, col_tiles);
+      return;
+    }
+  }
   const uint32_t blk0 = ((blockIdx.y * (blockDim.x >> 5) + warp) * U) * 32u + lane;
-  const T* xr = x + row * cols;
-  typename Block16<T>::Raw raw[U];
+  const T* xr = SRC == Src::kSiluMul ? x + row * 2 * cols : (SRC == Src::kExpand ? x + row * map.src_stride + map.src_col0 : x + row * cols);
+  typename Block16<T>::Raw raw[U], up[SRC == Src::kSiluMul ? U : 1];
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (blk0 + u * 32u < blocks_per_row) raw[u] = Block16<T>::load_raw(xr + (blk0 + u * 32u) * 16u);
-  const GlobalScale gs(__ldg(amax));
+  for (int u = 0; u < U; ++u) {
+    const uint32_t blk = blk0 + u * 32u;
+    if (blk < blocks_per_row) {
+      uint32_t col = blk * 16u;
+      if constexpr (SRC == Src::kExpand) {
+        const uint32_t head = col / map.head_dim;
+        col = (head / map.rep) * map.head_dim + (col - head * map.head_dim);
+      }
+      raw[u] = Block16<T>::load_raw(xr + col);
+      if constexpr (SRC == Src::kSiluMul) up[u] = Block16<T>::load_raw(xr + cols + col);
+    }
+  }
+  const GlobalScale gs(ld_dependent(amax));
   if (gout != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *gout = gs.g;
   uint8_t* code_row = codes + row * (cols >> 1);
   uint8_t* sf_row = sf + ((row >> 7) * col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
@@ -200,6 +145,12 @@ nvfp4_quantize_kernel(const T* __restrict__ x, const float* __restrict__ amax, u
     if (live) {
       float f[16];
       Block16<T>::widen(raw[u], f);
+      if constexpr (SRC == Src::kSiluMul) {
+        float b[16];
+        Block16<T>::widen(up[u], b);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = __bfloat162float(__float2bfloat16_rn(silu_mul_f32(f[i], b[i])));
+      }
       sb = quantize_block(f, gs, c_lo, c_hi, d);
     }
     if constexpr (!FAKE) {
@@ -249,10 +200,10 @@ nvfp4_dequantize_kernel(const uint8_t* __restrict__ codes, const uint8_t* __rest
   }
 }
 
-template <typename T, bool FAKE>
+template <typename T, bool FAKE, Src SRC = Src::kPlain>
 int launch(const void* x, const float* amax, uint8_t* codes, uint8_t* sf, void* fake, float* gout, int64_t rows,
-           int64_t cols, cudaStream_t st) {
-  constexpr int U = sizeof(T) == 4 ? 2 : 4;  // 128 bytes of loads in flight per lane
+           int64_t cols, cudaStream_t st, const ExpandMap& map = ExpandMap{}) {
+  constexpr int U = sizeof(T) == 4 || SRC == Src::kSiluMul ? 2 : 4;  // 128 bytes of loads in flight per lane
   const uint32_t blocks_per_row = static_cast<uint32_t>(cols >> 4);
   const uint32_t spans_per_row = (blocks_per_row + 31u) >> 5;
   const uint32_t warps_needed = (spans_per_row + U - 1) / U;
@@ -260,10 +211,17 @@ int launch(const void* x, const float* amax, uint8_t* codes, uint8_t* sf, void* 
   const uint32_t warps = warps_needed < 8u ? warps_needed : 8u;
   const uint32_t chunks = (warps_needed + warps - 1) / warps;
   if (chunks > 65535u) return B200Q_ERR_INVALID;
-  dim3 grid(static_cast<unsigned>(rows), chunks), block(warps * 32u);
-  nvfp4_quantize_kernel<T, FAKE, U><<<grid, block, 0, st>>>(static_cast<const T*>(x), amax, codes, sf, static_cast<T*>(fake),
-                                                             gout, static_cast<uint32_t>(cols), blocks_per_row,
-                                                             (blocks_per_row + 3u) >> 2);
+  // real quantize: the padding rows of the last 128-row scale tile are CTAs of the same launch (a memset in front of
+  // it cost a launch of its own)
+  int64_t grid_rows = FAKE ? rows : (rows + 127) / 128 * 128;
+  if (grid_rows > 0x7fffffffLL) {   // beyond the grid limit: clear the last tile in front
+    const int64_t ct = (cols / 16 + 3) / 4;
+    if (cudaMemsetAsync(sf + (rows / 128) * ct * 512, 0, static_cast<size_t>(ct * 512), st) != cudaSuccess) return B200Q_ERR_CUDA;
+    grid_rows = rows;
+  }
+  dim3 grid(static_cast<unsigned>(grid_rows), chunks), block(warps * 32u);
+  launch_pdl(nvfp4_quantize_kernel<T, FAKE, U, SRC>, grid, block, 0, st, static_cast<const T*>(x), amax, codes, sf, static_cast<T*>(fake),
+             gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), blocks_per_row, (blocks_per_row + 3u) >> 2, map);
   return check_launch();
 }
 
@@ -299,18 +257,39 @@ int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, c
   if (int rc = check_arch()) return rc;
   if (rows == 0 || cols == 0) return B200Q_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // rows that only exist as padding of the last 128-row tile are never visited by the
-  // kernel: clear the last row tile first so the padding reads as zero.
-  if (rows % 128 != 0) {
-    const int64_t ct = (cols / 16 + 3) / 4;
-    const int64_t last = (rows / 128) * ct * 512;
-    if (cudaMemsetAsync(scales_out + last, 0, static_cast<size_t>(ct * 512), st) != cudaSuccess) return B200Q_ERR_CUDA;
-  }
   switch (dtype) {
     case B200Q_BF16: return launch<__nv_bfloat16, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
     case B200Q_F16: return launch<__half, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
     default: return launch<float, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
   }
+}
+
+int b200q_silu_mul_nvfp4_quantize(const void* gate_up, const float* amax, uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out,
+                                  int64_t rows, int64_t f, b200q_stream_t stream) {
+  if (int rc = validate(gate_up, B200Q_BF16, rows, f, amax)) return rc;
+  if (rows == 0 || f == 0) return B200Q_OK;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  return launch<__nv_bfloat16, false, Src::kSiluMul>(gate_up, amax, codes_out, scales_out, nullptr, global_scale_out, rows, f,
+                                                     static_cast<cudaStream_t>(stream));
+}
+
+int b200q_expand_heads_nvfp4_quantize(const void* src, int64_t src_stride, int64_t src_col0, const float* amax, uint8_t* codes_out,
+                                      uint8_t* scales_out, float* global_scale_out, int64_t rows, int heads_out, int rep, int head_dim,
+                                      b200q_stream_t stream) {
+  if (heads_out <= 0 || rep <= 0 || head_dim <= 0 || head_dim % 16 != 0 || heads_out % rep != 0 || src_stride < 0 || src_col0 < 0 ||
+      src_stride % 16 != 0 || src_col0 % 16 != 0)
+    return B200Q_ERR_INVALID;
+  const int64_t cols = static_cast<int64_t>(heads_out) * head_dim;
+  if (int rc = validate(src, B200Q_BF16, rows, cols, amax)) return rc;
+  if (rows == 0) return B200Q_OK;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  return launch<__nv_bfloat16, false, Src::kExpand>(src, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols,
+                                                    static_cast<cudaStream_t>(stream),
+                                                    ExpandMap{src_stride, src_col0, static_cast<uint32_t>(head_dim), static_cast<uint32_t>(rep)});
 }
 
 int b200q_nvfp4_fake_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, void* out,

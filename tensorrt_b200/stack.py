@@ -147,12 +147,26 @@ class CudaBackend:
             return None
         return capi.silu_mul_fp8_quantize(gate_up)
 
+    # NVFP4 with a calibrated tensor amax of the linear that follows: the producer quantizes as well (one kernel, the
+    # bf16 tensor is never written), or None when the shape does not fit
+    def silu_mul_quantize_static(self, gate_up: torch.Tensor, amax):
+        if self.mode != "nvfp4" or gate_up.shape[-1] % 32:
+            return None
+        return capi.silu_mul_nvfp4_quantize(gate_up, amax)
+
+    def expand_heads_quantize_static(self, src, col0, heads_out, rep, head_dim, amax):
+        if self.mode != "nvfp4" or head_dim % 16 or src.shape[-1] % 16 or col0 % 16:
+            return None
+        return capi.expand_heads_nvfp4_quantize(src, col0, heads_out, rep, head_dim, amax)
+
     def add_norm_quantize(self, h: torch.Tensor, delta, weight: torch.Tensor, eps: float, amax=None):
-        """(h + delta, quantized rms_norm(h + delta)).  FP8: one fused kernel; NVFP4: add, norm and
-        block quantize as separate kernels (the block quantize needs the tensor amax)."""
+        """(h + delta, quantized rms_norm(h + delta)).  FP8, and NVFP4 with a calibrated amax: one fused kernel;
+        NVFP4 without: add, norm and block quantize as separate kernels (the block quantize needs the tensor amax)."""
         if self.mode == "fp8":
             h_new, codes, scales = capi.add_rms_norm_fp8_quantize(h, delta, weight, eps)
             return h_new, (codes, scales)
+        if amax is not None and h.shape[-1] <= 16384:
+            return capi.add_rms_norm_nvfp4_quantize(h, delta, weight, amax, eps)
         h_new = h if delta is None else capi.add(h, delta)
         x = capi.rms_norm(h_new, weight, eps)
         return h_new, self.quantize(x, amax)
@@ -319,7 +333,16 @@ class DecoderLayer:
             xq = be.expand_heads_quantize(qkv, col0, heads, rep, cfg.head_dim)    # quantized input of the O projection in one pass
             if xq is not None:
                 return xq
-        return be.expand_heads(qkv, col0, heads, rep, cfg.head_dim)
+        amax = self._static_amax("o", "expand_heads_quantize_static")
+        xq = None if amax is None else be.expand_heads_quantize_static(qkv, col0, heads, rep, cfg.head_dim, amax)
+        return be.expand_heads(qkv, col0, heads, rep, cfg.head_dim) if xq is None else xq
+
+    def _static_amax(self, name: str, method: str):
+        """Calibrated amax of linear input `name` when the backend can quantize while it produces that input.  One rank
+        only: the swizzled scales of a quantized operand cannot be sliced by token as the multi-rank forms do."""
+        if self.calibrating or self.world != 1 or not hasattr(self.backend, method):
+            return None
+        return self.amax.get(name)
 
     def _ffn_act(self, xq):
         """gate/up linear + silu(gate) * up -> input of the down projection (quantized when the
@@ -331,6 +354,9 @@ class DecoderLayer:
                 return act
         gu = be.matmul(xq, self.wgu)
         act = be.silu_mul_quantize(gu) if hasattr(be, "silu_mul_quantize") and not self.calibrating else None
+        if act is None:
+            amax = self._static_amax("down", "silu_mul_quantize_static")
+            act = None if amax is None else be.silu_mul_quantize_static(gu, amax)
         return be.silu_mul(gu) if act is None else act
 
     def forward(self, h: torch.Tensor, delta=None):

@@ -1,0 +1,66 @@
+"""Kernels that quantize to NVFP4 what they produce (residual add + RMSNorm, silu(gate) * up, repeated kv heads) under a
+calibrated amax: codes, swizzled scales (padding rows included) and global scale equal the separate kernels' bit for
+bit, at row counts around 128-row scale tiles and at the edges of their launch shapes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(got, ref):
+    for a, b in zip(got, ref):
+        assert a.shape == b.shape and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("with_delta", [True, False])
+@pytest.mark.parametrize("rows,cols", [(1, 16), (3, 272), (5, 4096), (64, 8192), (127, 2064), (128, 2048), (300, 4096), (1184, 4096),
+                                       (1300, 2080), (1190, 8192), (2, 16384), (400, 16384)])
+def test_add_rms_norm(b200, rows, cols, with_delta):
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    h, d = (torch.randn(rows, cols, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=g)).bfloat16()
+    delta = d if with_delta else None
+    h_ref = capi.add(h, d) if with_delta else h
+    x = capi.rms_norm(h_ref, w)
+    for amax in (capi.amax(x), capi.amax(x) * 0.25, torch.zeros((), device="cuda")):
+        h_new, got = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)
+        assert torch.equal(h_new, h_ref)
+        _same(got, capi.nvfp4_quantize(x, amax))
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,f", [(1, 16), (3, 528), (128, 1040), (130, 14336), (33, 28672)])
+def test_silu_mul(b200, rows, f):
+    capi = b200.capi
+    gu = torch.randn(rows, 2 * f, device="cuda", generator=torch.Generator(device="cuda").manual_seed(f)).bfloat16() * 3
+    act = capi.silu_mul(gu)
+    for amax in (capi.amax(act), capi.amax(act) * 0.3):
+        _same(capi.silu_mul_nvfp4_quantize(gu, amax), capi.nvfp4_quantize(act, amax))
+
+
+@pytest.mark.parametrize("rows,n_q,n_kv,d", [(1, 2, 1, 16), (5, 8, 2, 48), (129, 32, 8, 128), (64, 16, 8, 64)])
+def test_expand_heads(b200, rows, n_q, n_kv, d):
+    capi = b200.capi
+    qkv = torch.randn(rows, (n_q + 2 * n_kv) * d, device="cuda", generator=torch.Generator(device="cuda").manual_seed(d)).bfloat16()
+    col0, rep = (n_q + n_kv) * d, n_q // n_kv
+    wide = capi.expand_heads(qkv, col0, n_q, rep, d)
+    amax = capi.amax(wide)
+    _same(capi.expand_heads_nvfp4_quantize(qkv, col0, n_q, rep, d, amax), capi.nvfp4_quantize(wide, amax))
+
+
+@pytest.mark.parametrize("rows", [1, 16, 127, 128, 129, 300])
+def test_padding_rows_of_the_scale_tile_are_cleared(b200, rows):
+    from tensorrt_b200 import _lib
+
+    cols = 80
+    x = torch.randn(rows, cols, device="cuda").bfloat16()
+    amax = x.abs().max().float().reshape(1)
+    codes, ref, g = b200.capi.nvfp4_quantize(x, amax)
+    sf = torch.full_like(ref, 0xAA)
+    assert _lib.load().b200q_nvfp4_quantize(x.data_ptr(), 2, rows, cols, amax.data_ptr(), codes.data_ptr(), sf.data_ptr(), g.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream) == 0
+    tiles = sf.view(-1, (cols // 16 + 3) // 4, 32, 4, 4)                # [row tile, column tile, row % 32, row // 32 % 4, 4 scales]
+    by_row = tiles.permute(0, 3, 2, 1, 4).reshape(-1, tiles.shape[1] * 4)
+    assert int(by_row[rows:].max() if by_row.shape[0] > rows else 0) == 0
+    assert int(by_row[:rows, cols // 16:].max()) == 0 and bool((by_row[:rows, :cols // 16] != 0xAA).all())
