@@ -261,11 +261,13 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
 // the smallest power of two that reaches that many CTAs wins, larger clusters only add
 // reduction cost.  With at most 32 tokens the partial tiles are small enough that two CTAs per SM
 // pay (one's prologue and cluster reduction under the other's weight stream: 10-25 % faster at
-// 16 tokens, neutral at 64, slower at 128), so the target there is one and a half CTAs per SM.
+// 16 tokens, neutral at 64, slower at 128), so the target there is one and a half CTAs per SM, as long
+// as all CTAs are resident at once: 80 tiles x 4 = 320 CTAs on 296 places cost a second round (10240 x 8192
+// at 1 / 16 tokens: FP8 23.0 / 24.4 us against 17.4 / 18.4 with 2 CTAs per tile, NVFP4 16.2 / 17.6 against 12.4 / 13.2).
 inline int smallm_splits(int n_tiles, int k_tiles, int sms, int tokens) {
   const int want = tokens <= 32 ? (sms * 3) / 2 : (sms * 3) / 4;
   int s = 1;
-  while (s < 8 && n_tiles * s < want && s * 2 <= k_tiles) s <<= 1;
+  while (s < 8 && n_tiles * s < want && n_tiles * s * 2 <= 2 * sms && s * 2 <= k_tiles) s <<= 1;
   return s;
 }
 
