@@ -275,9 +275,33 @@ bool valid_tile_n(int bn);    // values b200q_cfg::tile_n accepts
 int sf_copier_enabled();     // environment variable B200Q_SF_COPIER (default in gemm_fp8.cu)
 int forced_smallm_stages();  // from the environment variable B200Q_SMALLM_STAGES (0 when unset)
 
-// Tile width: 256 when that still gives every SM a tile, else 128.  `cfg->tile_n` (128 / 256)
-// overrides the choice (used by tests to cover both instantiations); 512 forces the CTA-pair
-// kernel (256 x 256 tiles), which is otherwise used when there are at least sm_count/2 such tiles.
+// Kernel of a problem with more than 128 rows: 512 = CTA pair with 256 x 256 tiles, 256 / 128 = one CTA with 128 x 256 /
+// 128 x 128 tiles.  A launch takes as long as its rounds: tiles over SMs (SM pairs), rounded up, times the time of one
+// tile, in units of a pair's 256 x 256 tile.  Large problems (many rounds) go to the pair kernels; a problem just above
+// a whole number of rounds, or with few rows, to the finer tiles (333 x 10240 x 8192 FP8: 80 pair tiles on 74 pairs are
+// two rounds, 48.0 us; 120 tiles of 128 x 256 are one, 32.6).  A single round of the small tile is not half of the big one's:
+// both wait for the same K loop.  The percentages are from a sweep of the three kernels over 14 row counts (129 to 4096)
+// and seven weight shapes in each format: the rule takes the fastest kernel or one within 1.6 % of it at all 196
+// points.  The choice by tile counts before it was 10 % slower on average and 2.0 times at worst (NVFP4 4096 x
+// 14336 at 600 to 1000 rows: 48 to 64 pair tiles, 57 to 59 us on 128 x 128 tiles, 29.0 to 29.5 on pairs).  The reduce-scatter epilogue keeps the choice by tile counts that
+// its NVLink overlap was measured with.
+constexpr int kTile256Fp8 = 110, kTile128Fp8 = 85, kTile256Nv = 145, kTile128Nv = 110;   // per cent of a pair tile
+inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
+  const int64_t pair = static_cast<int64_t>((M + kPairM - 1) / kPairM) * ((N + kPairN - 1) / kPairN);
+  const int64_t t256 = static_cast<int64_t>((M + kBM - 1) / kBM) * ((N + 255) / 256);
+  const int64_t t128 = static_cast<int64_t>((M + kBM - 1) / kBM) * ((N + 127) / 128);
+  if (rs) {
+    if (!nvf4 && pair >= sms / 2) return 512;
+    return t256 >= sms ? 256 : 128;
+  }
+  const auto cost = [](int64_t tiles, int units, int each) { return (tiles + units - 1) / units * each; };
+  const int64_t c512 = cost(pair, sms / 2, 100), c256 = cost(t256, sms, nvf4 ? kTile256Nv : kTile256Fp8),
+                c128 = cost(t128, sms, nvf4 ? kTile128Nv : kTile128Fp8);
+  if (c512 <= c256 && c512 <= c128) return 512;
+  return c256 <= c128 ? 256 : 128;
+}
+
+// `cfg->tile_n` (128 / 256 / 512) overrides the choice of `large_tile` (used by tests to cover the instantiations).
 // M <= 128 goes to the small-M kernel unless a tile width is forced.
 template <bool NVF4>
 int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const b200q_cfg* cfg, const RsTargets* rs = nullptr) {
@@ -296,22 +320,16 @@ int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const 
     if (splits >= 1 && splits <= k_tiles) return launch_smallm<NVF4>(a, b, p, st, splits, forced_smallm_stages());
   }
   if (bn >= 1000) bn = 0;
-  const int64_t pair_tiles = static_cast<int64_t>((p.M + kPairM - 1) / kPairM) * ((p.N + kPairN - 1) / kPairN);
-  // CTA-pair kernels (256 x 256 tiles) whenever they fill the SM pairs: measured 2.9 vs 2.75 PFLOP/s
-  // for FP8 and 4.8 vs 3.4 for NVFP4 at 8192^3 against the single-CTA 128 x 256 tile.  The NVFP4 pair
-  // kernel with the scale warps writes local output only; the reduce-scatter epilogue keeps the
+  if (bn == 0) bn = large_tile(p.M, p.N, sm_count(), NVF4, rs != nullptr);
+  // The NVFP4 pair kernel with the scale warps writes local output only; the reduce-scatter epilogue keeps the
   // generic kernels.
-  if (bn == 512 || (bn == 0 && pair_tiles >= sm_count() / 2)) {
+  if (bn == 512) {
     if constexpr (NVF4) {
       if (rs == nullptr) return launch_nvf4_pair(a, b, p, st);
-      if (bn == 512) return launch_pair<NVF4>(a, b, p, st, rs);
+      return launch_pair<NVF4>(a, b, p, st, rs);
     } else {
       return launch_pair<NVF4>(a, b, p, st, rs);
     }
-  }
-  if (bn != 128 && bn != 256) {
-    const int64_t tiles256 = static_cast<int64_t>((p.M + kBM - 1) / kBM) * ((p.N + 255) / 256);
-    bn = (tiles256 >= sm_count()) ? 256 : 128;
   }
   return bn == 256 ? launch_tile<NVF4, 256>(a, b, p, st, rs) : launch_tile<NVF4, 128>(a, b, p, st, rs);
 }
