@@ -355,6 +355,25 @@ int b200q_fp8_sdpa(const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t
                    const float* k_scale, const float* v_scale, void* out, int out_dtype, int64_t B, int64_t Hq,
                    int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D, float softmax_scale, int causal,
                    b200q_stream_t stream);
+/* The same with the result at caller-given strides (elements, multiples of 8: batch, head, query row; the head
+ * dimension is contiguous): a token-major [tokens, Hq * D] buffer is written in place. */
+int b200q_fp8_sdpa_strided(const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* vt_codes, const float* q_scale,
+                           const float* k_scale, const float* v_scale, void* out, const int64_t* out_strides, int out_dtype,
+                           int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D,
+                           float softmax_scale, int causal, b200q_stream_t stream);
+/* The three operands of b200q_fp8_sdpa in one launch: q [B, Hq, Sq, D], k and v [B, Hkv, Sk, D] of one dtype with a
+ * per-tensor amax each -> q_codes and k_codes (contiguous), vt_codes (transposed per head, zero beyond Sk) and the
+ * scales amax / 448 (zero -> 1) of q, k, v in scales[0..2].  strides: batch, head, row of q, then of k, then of v, in
+ * elements, each a multiple of 16 bytes (D contiguous, 16-byte aligned pointers).  The same codes as
+ * b200q_fp8_quantize and b200q_fp8_quantize_transpose.  Sk = 0: k, v and their outputs may be NULL. */
+int b200q_fp8_attention_quantize(const void* q, const void* k, const void* v, int dtype, const int64_t* strides,
+                                 const float* amax_q, const float* amax_k, const float* amax_v, uint8_t* q_codes,
+                                 uint8_t* k_codes, uint8_t* vt_codes, float* scales, int64_t B, int64_t Hq, int64_t Hkv,
+                                 int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D, b200q_stream_t stream);
+/* abs-max of three column ranges of x [rows, c1 + c2 + c3] (dtype, row-major): amax_out[0..2], fp32, exact.  The Q, K
+ * and V slices of a QKV projection in one pass.  c1, c2, c3 >= 0, multiples of 16; x 32-byte aligned. */
+int b200q_amax_columns(const void* x, int dtype, int64_t rows, int64_t c1, int64_t c2, int64_t c3, float* amax_out,
+                       b200q_stream_t stream);
 
 /* ------------------------------------------------------------------ glue of the decoder linear stack
  * The benchmark workloads wrap the quantized linears in a Llama-shaped decoder layer

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import contextlib
 import contextvars
+import ctypes
 
 import torch
 
@@ -296,6 +297,10 @@ def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, 
     _, Hkv, Sk, _ = k.shape
     if Hq % Hkv or D % 16 or D > 128:
         raise ValueError(f"need Hq % Hkv == 0 and a head dimension that is a multiple of 16 up to 128, got Hq={Hq}, Hkv={Hkv}, D={D}")
+    out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    if k.dtype == q.dtype and v.dtype == q.dtype:
+        return _fp8_sdpa_into(out, q, k, v, amax_q, amax_k, amax_v, is_causal, scale)
+    # mixed input types: one quantize launch each
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     dev = q.device
     amaxes = [a.to(device=dev, dtype=torch.float32).reshape(1) for a in (amax_q, amax_k, amax_v)]
@@ -304,7 +309,6 @@ def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, 
     stride = (Sk + 15) // 16 * 16
     vt = torch.empty(B, Hkv, D, max(stride, 16), dtype=torch.uint8, device=dev)
     vs = torch.empty(1, dtype=torch.float32, device=dev)
-    out = torch.empty_like(q)
     lib = load()
     with torch.cuda.device(dev):
         check(lib.b200q_fp8_quantize_transpose(v.data_ptr(), _dt(v), B * Hkv, Sk, D, amaxes[2].data_ptr(), vt.data_ptr(), max(stride, 16),
@@ -314,6 +318,76 @@ def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, 
         check(lib.b200q_fp8_sdpa(qc.data_ptr(), kc.data_ptr(), vt.data_ptr(), qs.data_ptr(), ks.data_ptr(), vs.data_ptr(), out.data_ptr(),
                                  _dt(q), B, Hq, Hkv, Sq, Sk, max(stride, 16), D, float(scale if scale is not None else 1.0 / math.sqrt(D)),
                                  1 if is_causal else 0, _stream(q)), "b200q_fp8_sdpa")
+    return out
+
+
+def _strided_16(t: torch.Tensor) -> torch.Tensor:
+    """t [B, H, S, D] itself when the attention quantize kernel can read it where it lies (D contiguous, rows, heads
+    and batches a multiple of 16 bytes apart, 16-byte aligned), else a contiguous copy."""
+    unit = 16 // t.element_size()
+    if t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(s % unit == 0 for s in _outer_strides(t)):
+        return t
+    return t.contiguous()
+
+
+def _outer_strides(t: torch.Tensor):
+    """Strides of batch, head and row; 0 where there is one only (torch leaves any value there)."""
+    return [s if n > 1 else 0 for s, n in zip(t.stride()[:3], t.shape[:3])]
+
+
+def _fp8_sdpa_into(out: torch.Tensor, q, k, v, amax_q, amax_k, amax_v, is_causal: bool, scale) -> torch.Tensor:
+    """`fp8_sdpa` of checked inputs of one dtype into `out` (q's shape and dtype; any strides with D contiguous and
+    the others multiples of 8 elements, 32-byte aligned): one launch that quantizes Q, K and V, one of attention."""
+    import math
+
+    q, k, v = _strided_16(q), _strided_16(k), _strided_16(v)
+    B, Hq, Sq, D = q.shape
+    _, Hkv, Sk, _ = k.shape
+    dev, dt = q.device, _dt(q)
+    aq, ak, av = (a.to(device=dev, dtype=torch.float32).reshape(1) for a in (amax_q, amax_k, amax_v))
+    vt_stride = max((Sk + 15) // 16 * 16, 16)
+    nq, nk, nv = q.numel(), k.numel(), B * Hkv * D * vt_stride
+    # one workspace: Q codes, K codes, transposed V codes (each a multiple of 16 bytes), three scales
+    ws = torch.empty(nq + nk + nv + 16, dtype=torch.uint8, device=dev)
+    base = ws.data_ptr()
+    scales = base + nq + nk + nv
+    strides = (ctypes.c_int64 * 9)(*_outer_strides(q), *_outer_strides(k), *_outer_strides(v))
+    out_strides = (ctypes.c_int64 * 3)(*_outer_strides(out))
+    lib = load()
+    with torch.cuda.device(dev):
+        st = _stream(q)
+        check(lib.b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr(), ak.data_ptr(), av.data_ptr(),
+                                               base, base + nq, base + nq + nk, scales, B, Hq, Hkv, Sq, Sk, vt_stride, D, st),
+              "b200q_fp8_attention_quantize")
+        check(lib.b200q_fp8_sdpa_strided(base, base + nq, base + nq + nk, scales, scales + 4, scales + 8, out.data_ptr(), out_strides, dt, B, Hq,
+                                         Hkv, Sq, Sk, vt_stride, D, float(scale if scale is not None else 1.0 / math.sqrt(D)),
+                                         1 if is_causal else 0, st), "b200q_fp8_sdpa")
+    return out
+
+
+def fp8_sdpa_packed(qkv: torch.Tensor, batch: int, n_q: int, n_kv: int, head_dim: int, is_causal: bool = True) -> torch.Tensor:
+    """FP8 attention on a token-major QKV projection: qkv [batch * S, (n_q + 2 n_kv) * head_dim] (query heads, key
+    heads, value heads) -> [batch * S, n_q * head_dim].  Q, K, V are quantized per tensor at their measured abs-max;
+    read and written in place of head-major copies.  The same bits as `fp8_sdpa` on those copies."""
+    _need_cuda(qkv)
+    qkv = qkv.contiguous()
+    if qkv.data_ptr() % 32:
+        qkv = qkv.clone()
+    tokens = qkv.shape[0]
+    qw, kvw, s = n_q * head_dim, n_kv * head_dim, tokens // max(batch, 1)
+    if qkv.shape[1] != qw + 2 * kvw or s * batch != tokens:
+        raise ValueError(f"expected [batch * S, {qw + 2 * kvw}], got {tuple(qkv.shape)} for batch {batch}")
+    if tokens == 0:
+        return qkv.new_empty(0, qw)
+    amaxes = torch.empty(3, dtype=torch.float32, device=qkv.device)
+    with torch.cuda.device(qkv.device):
+        check(load().b200q_amax_columns(qkv.data_ptr(), _dt(qkv), tokens, qw, kvw, kvw, amaxes.data_ptr(), _stream(qkv)), "b200q_amax_columns")
+    out = torch.empty(tokens, qw, dtype=qkv.dtype, device=qkv.device)
+    heads = lambda t, n: t.view(batch, s, n, head_dim).transpose(1, 2)  # noqa: E731
+    rows = qkv.view(batch, s, -1)
+    _fp8_sdpa_into(heads(out, n_q), *(rows[:, :, c:c + n * head_dim].unflatten(2, (n, head_dim)).transpose(1, 2)
+                                      for c, n in ((0, n_q), (qw, n_kv), (qw + kvw, n_kv))),
+                   amaxes[0], amaxes[1], amaxes[2], is_causal, None)
     return out
 
 

@@ -57,7 +57,8 @@ struct AttParams {
   const float* q_scale;     // per-tensor scales (device scalars)
   const float* k_scale;
   const float* v_scale;
-  void* out;                // [B, Hq, Sq, D]
+  void* out;                // [B, Hq, Sq, D] at these strides (elements, multiples of 8; D contiguous)
+  int64_t out_sb, out_sh, out_ss;
   int out_dtype;
   int Hq, Hkv, Sq, Sk, D;
   float softmax_scale;
@@ -379,7 +380,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (ok && q0 + q * 32 < p.Sq) {
       ptx::tc_fence_after();
       const float oscale = n_tiles > 0 ? __ldg(p.v_scale) / kE4M3Max : 0.0f;
-      const int64_t row_off = (static_cast<int64_t>(bh) * p.Sq + qi) * p.D;
+      const int64_t row_off = b * p.out_sb + h * p.out_sh + qi * p.out_ss;
 #pragma unroll 1
       for (int c = 2 * ch; c < 2 * ch + 2; ++c) {
         if (c * 32 >= p.D) break;
@@ -414,47 +415,137 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
 }
 
-// x [heads, S, D] -> E4M3 codes transposed per head [heads, D, s_stride] (keys contiguous), zero beyond S.
-template <typename T>
+// ---------------------------------------------------------------- Q, K, V -> operands
+// One launch quantizes Q and K to E4M3 codes [B, H, S, D] and V to codes transposed per head [B, H, D, vt_stride]
+// (keys contiguous, zero beyond S).  The inputs may be strided (D contiguous): a token-major [tokens, heads * D] slice
+// of a QKV projection is read where it lies.  HBM-bound (3 bytes per 16-bit element); a CTA takes 128 rows of one
+// head, 16 elements per thread and step with four steps of loads in flight.  Before, Q and K went through the
+// row kernels, one CTA per row of D elements: at [4, 32, 2048, 128] 262144 CTAs of which 16 threads had work.
+struct QkvPart {
+  const void* x;
+  int64_t sb, sh, ss;        // strides of batch, head, row in elements
+  const float* amax;
+  uint8_t* out;
+  float* scale_out;
+  int H, S;
+  int tiles;                 // tiles of 128 rows per head
+};
+struct QkvParts {
+  QkvPart part[3];
+  int first[3];              // first CTA of each part
+  int D;
+  int64_t vt_stride;
+};
+
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256)
-fp8_quantize_transpose_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ out, int S, int D,
-                              int64_t s_stride, float* __restrict__ scale_out) {
-  __shared__ uint8_t tile[64][128 + 16];
-  const int head = blockIdx.y;
-  const int k0 = blockIdx.x * 64;
-  const float scale = fp8_scale_from_amax(__ldg(amax));
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && scale_out != nullptr) *scale_out = scale;
+fp8_attention_quantize_kernel(const __grid_constant__ QkvParts p) {
+  __shared__ uint32_t tile[kTile * 32];           // V: 128 keys x 128 bytes
+  const int cta = static_cast<int>(blockIdx.x);
+  const int which = cta >= p.first[2] ? 2 : (cta >= p.first[1] ? 1 : 0);
+  const QkvPart& part = p.part[which];
+  if (cta == 0 && threadIdx.x < 3 && p.part[threadIdx.x].scale_out != nullptr)
+    *p.part[threadIdx.x].scale_out = fp8_scale_from_amax(__ldg(p.part[threadIdx.x].amax));
+  const int local = cta - p.first[which];
+  const int head = local / part.tiles;            // b * H + h
+  const int r0 = (local - head * part.tiles) * kTile;
+  const int b = head / part.H, h = head - b * part.H;
+  const T* x = static_cast<const T*>(part.x) + b * part.sb + h * part.sh;
+  const float scale = fp8_scale_from_amax(__ldg(part.amax));
   const float y = b200q_rcp_rn(scale);
   const bool fast = b200q_div_fast_ok(scale);
-  const float lim = __fmul_rn(scale, 512.0f);   // |x| >= 512 * scale saturates to 448 anyway
-  const int groups = D >> 3;
-  for (int t = threadIdx.x; t < 64 * groups; t += 256) {
-    const int kk = t / groups, g = t - kk * groups;
-    uint2 packed = make_uint2(0u, 0u);
-    if (k0 + kk < S) {
-      float v[8], qv[8];
-      Elem<T>::load8(x + (static_cast<int64_t>(head) * S + k0 + kk) * D + g * 8, v);
+  const float lim = __fmul_rn(scale, 512.0f);     // |x| >= 512 * scale saturates to 448 anyway
+  const int pieces = p.D >> 4;                    // 16-element pieces of a row
+  constexpr int U = sizeof(T) == 4 ? 2 : 4;
+  const int rows = min(kTile, part.S - r0);       // V: rows beyond S up to the tile's end are zero codes
+  for (int t0 = threadIdx.x; t0 < kTile * pieces; t0 += 256 * U) {
+    Raw16<T, WIDE> raw[U];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) qv[i] = fast ? div_path<kDivClamped>(v[i], scale, y, lim) : div_path<kDivTrue>(v[i], scale, y, lim);
-      packed.x = f32x2_to_e4m3x2(qv[0], qv[1]) | (f32x2_to_e4m3x2(qv[2], qv[3]) << 16);
-      packed.y = f32x2_to_e4m3x2(qv[4], qv[5]) | (f32x2_to_e4m3x2(qv[6], qv[7]) << 16);
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * 256, row = t / pieces, g = t - row * pieces;
+      if (row < rows) raw[u].load(x + static_cast<int64_t>(r0 + row) * part.ss + g * 16);
     }
-    *reinterpret_cast<uint2*>(&tile[kk][g * 8]) = packed;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * 256, row = t / pieces, g = t - row * pieces;
+      uint4 c = make_uint4(0u, 0u, 0u, 0u);
+      if (row < rows) {
+        float v[16];
+        raw[u].widen(v);
+        uint32_t* w = &c.x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float q[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            q[e] = fast ? div_path<kDivClamped>(v[4 * i + e], scale, y, lim) : div_path<kDivTrue>(v[4 * i + e], scale, y, lim);
+          w[i] = f32x2_to_e4m3x2(q[0], q[1]) | (f32x2_to_e4m3x2(q[2], q[3]) << 16);
+        }
+        if (which != 2)
+          *reinterpret_cast<uint4*>(part.out + (static_cast<int64_t>(head) * part.S + r0 + row) * p.D + g * 16) = c;
+      }
+      // 16-byte pieces of a key row are swizzled by the key's group of 16, so that the transposing reads below
+      // (8 key groups x 4 words) hit 32 different banks
+      if (which == 2 && row < kTile) *reinterpret_cast<uint4*>(&tile[row * 32 + ((g ^ ((row >> 4) & 7)) << 2)]) = c;
+    }
   }
+  if (which != 2) return;
   __syncthreads();
-  // every (d, 16-key piece) is one 16-byte store
-  for (int t = threadIdx.x; t < D * 4; t += 256) {
-    const int d = t >> 2, part = t & 3;
-    if (k0 + part * 16 >= s_stride) continue;
-    uint32_t w[4];
+  // item: 4 columns (one word) of 16 keys, transposed in 4 x 4 byte blocks -> four 16-byte stores
+  for (int t = threadIdx.x; t < pieces * 4 * 8; t += 256) {
+    const int kg = t & 7, d4 = t >> 3;
+    if (r0 + kg * 16 >= p.vt_stride) continue;
+    uint32_t o[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      w[i] = 0u;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) w[i] |= static_cast<uint32_t>(tile[part * 16 + i * 4 + e][d]) << (8 * e);
+      const uint32_t* src = &tile[(kg * 16 + i * 4) * 32 + (d4 ^ (kg << 2))];
+      const uint32_t k0 = src[0], k1 = src[32], k2 = src[64], k3 = src[96];
+      const uint32_t a01 = __byte_perm(k0, k1, 0x5140), a23 = __byte_perm(k2, k3, 0x5140);
+      const uint32_t b01 = __byte_perm(k0, k1, 0x7362), b23 = __byte_perm(k2, k3, 0x7362);
+      o[0][i] = __byte_perm(a01, a23, 0x5410);
+      o[1][i] = __byte_perm(a01, a23, 0x7632);
+      o[2][i] = __byte_perm(b01, b23, 0x5410);
+      o[3][i] = __byte_perm(b01, b23, 0x7632);
     }
-    *reinterpret_cast<uint4*>(out + (static_cast<int64_t>(head) * D + d) * s_stride + k0 + part * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    uint8_t* dst = part.out + (static_cast<int64_t>(head) * p.D + d4 * 4) * p.vt_stride + r0 + kg * 16;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + i * p.vt_stride) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
   }
+}
+
+// `first` and the grid of the parts filled in; 0 CTAs = nothing to do.
+int launch_attention_quantize(QkvParts& p, int B, int dtype, cudaStream_t st) {
+  int64_t ctas = 0;
+  for (int i = 0; i < 3; ++i) {
+    p.first[i] = static_cast<int>(ctas);
+    // V: the zero columns between S and the row stride are written too
+    const int64_t extent = i < 2 ? p.part[i].S : (p.part[i].S > 0 ? p.vt_stride : 0);
+    p.part[i].tiles = static_cast<int>((extent + kTile - 1) / kTile);
+    ctas += static_cast<int64_t>(p.part[i].tiles) * p.part[i].H * B;
+    if (ctas > 0x7fffffffLL) return B200Q_ERR_INVALID;
+  }
+  if (ctas == 0) return B200Q_OK;
+  // 256-bit loads when every row starts on a 32-byte boundary
+  const int64_t unit = dtype == B200Q_F32 ? 8 : 16;
+  bool wide = true;
+  for (int i = 0; i < 3; ++i) {
+    const QkvPart& a = p.part[i];
+    wide = wide && (a.tiles == 0 || (aligned(a.x, 32) && a.sb % unit == 0 && a.sh % unit == 0 && a.ss % unit == 0));
+  }
+  const dim3 grid(static_cast<unsigned>(ctas));
+#define B200Q_AQ(T)                                                                  \
+  do {                                                                               \
+    if (wide) fp8_attention_quantize_kernel<T, true><<<grid, 256, 0, st>>>(p);       \
+    else fp8_attention_quantize_kernel<T, false><<<grid, 256, 0, st>>>(p);           \
+  } while (0)
+  switch (dtype) {
+    case B200Q_BF16: B200Q_AQ(__nv_bfloat16); break;
+    case B200Q_F16: B200Q_AQ(__half); break;
+    case B200Q_F32: B200Q_AQ(float); break;
+    default: return B200Q_ERR_INVALID;
+  }
+#undef B200Q_AQ
+  return check_launch();
 }
 
 // [inner bytes, rows, heads] byte tensor -> boxes of 128 x 128 x 1, 128-byte swizzle, zero fill out of bounds
@@ -484,21 +575,68 @@ int b200q_fp8_quantize_transpose(const void* x, int dtype, int64_t heads, int64_
   if (x == nullptr || amax == nullptr || out_t == nullptr) return B200Q_ERR_INVALID;
   if (!aligned(x, 16) || !aligned(out_t, 16) || (dtype == B200Q_F32 && !aligned(x, 32))) return B200Q_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
-  const dim3 grid(static_cast<unsigned>((s_stride + 63) / 64), static_cast<unsigned>(heads));
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int s = static_cast<int>(S), d = static_cast<int>(D);
-  switch (dtype) {
-    case B200Q_BF16: fp8_quantize_transpose_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), amax, out_t, s, d, s_stride, scale_out); break;
-    case B200Q_F16: fp8_quantize_transpose_kernel<<<grid, 256, 0, st>>>(static_cast<const __half*>(x), amax, out_t, s, d, s_stride, scale_out); break;
-    case B200Q_F32: fp8_quantize_transpose_kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(x), amax, out_t, s, d, s_stride, scale_out); break;
-    default: return B200Q_ERR_INVALID;
+  if (dtype != B200Q_BF16 && dtype != B200Q_F16 && dtype != B200Q_F32) return B200Q_ERR_INVALID;
+  if (s_stride > 0x7fffff00LL) return B200Q_ERR_INVALID;
+  QkvParts p{};
+  p.D = static_cast<int>(D);
+  p.vt_stride = s_stride;
+  p.part[0].H = p.part[1].H = 1;
+  p.part[2] = QkvPart{x, S * D, 0, D, amax, out_t, scale_out, 1, static_cast<int>(S), 0};
+  return launch_attention_quantize(p, static_cast<int>(heads), dtype, static_cast<cudaStream_t>(stream));
+}
+
+// Host-side check of one strided input of b200q_fp8_attention_quantize.
+static int check_strided(const void* x, const int64_t* strides, int dtype) {
+  const int64_t unit = dtype == B200Q_F32 ? 4 : 8;     // elements in 16 bytes
+  if (x == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(x, 16)) return B200Q_ERR_ALIGN;
+  for (int i = 0; i < 3; ++i)
+    if (strides[i] < 0 || strides[i] % unit != 0) return B200Q_ERR_ALIGN;
+  return B200Q_OK;
+}
+
+int b200q_fp8_attention_quantize(const void* q, const void* k, const void* v, int dtype, const int64_t* strides, const float* amax_q,
+                                 const float* amax_k, const float* amax_v, uint8_t* q_codes, uint8_t* k_codes, uint8_t* vt_codes,
+                                 float* scales, int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D,
+                                 b200q_stream_t stream) {
+  if (B < 0 || Hq <= 0 || Hkv <= 0 || Sq < 0 || Sk < 0 || D <= 0 || D > 128 || D % 16 != 0) return B200Q_ERR_INVALID;
+  if (vt_stride < Sk || vt_stride % 16 != 0 || vt_stride > 0x7fffff00LL || B > 0x7fffffffLL || Hq > 0x7fffffffLL || Hkv > 0x7fffffffLL || Sq > 0x7fffff00LL || Sk > 0x7fffff00LL)
+    return B200Q_ERR_INVALID;
+  if (dtype != B200Q_BF16 && dtype != B200Q_F16 && dtype != B200Q_F32) return B200Q_ERR_INVALID;
+  if (B == 0 || (Sq == 0 && Sk == 0)) return B200Q_OK;
+  if (strides == nullptr || amax_q == nullptr || amax_k == nullptr || amax_v == nullptr || scales == nullptr) return B200Q_ERR_INVALID;
+  if (Sq > 0) {
+    if (int rc = check_strided(q, strides, dtype)) return rc;
+    if (q_codes == nullptr) return B200Q_ERR_INVALID;
   }
-  return check_launch();
+  if (Sk > 0) {
+    if (int rc = check_strided(k, strides + 3, dtype)) return rc;
+    if (int rc = check_strided(v, strides + 6, dtype)) return rc;
+    if (k_codes == nullptr || vt_codes == nullptr) return B200Q_ERR_INVALID;
+  }
+  if (!aligned(q_codes, 16) || !aligned(k_codes, 16) || !aligned(vt_codes, 16)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  QkvParts p{};
+  p.D = static_cast<int>(D);
+  p.vt_stride = vt_stride;
+  p.part[0] = QkvPart{q, strides[0], strides[1], strides[2], amax_q, q_codes, scales, static_cast<int>(Hq), static_cast<int>(Sq), 0};
+  p.part[1] = QkvPart{k, strides[3], strides[4], strides[5], amax_k, k_codes, scales + 1, static_cast<int>(Hkv), static_cast<int>(Sk), 0};
+  p.part[2] = QkvPart{v, strides[6], strides[7], strides[8], amax_v, vt_codes, scales + 2, static_cast<int>(Hkv), static_cast<int>(Sk), 0};
+  return launch_attention_quantize(p, static_cast<int>(B), dtype, static_cast<cudaStream_t>(stream));
 }
 
 int b200q_fp8_sdpa(const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* vt_codes, const float* q_scale, const float* k_scale,
                    const float* v_scale, void* out, int out_dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk,
                    int64_t vt_stride, int64_t D, float softmax_scale, int causal, b200q_stream_t stream) {
+  const int64_t strides[3] = {Hq * Sq * D, Sq * D, D};
+  return b200q_fp8_sdpa_strided(q_codes, k_codes, vt_codes, q_scale, k_scale, v_scale, out, strides, out_dtype, B, Hq, Hkv, Sq, Sk, vt_stride,
+                                D, softmax_scale, causal, stream);
+}
+
+int b200q_fp8_sdpa_strided(const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* vt_codes, const float* q_scale,
+                           const float* k_scale, const float* v_scale, void* out, const int64_t* out_strides, int out_dtype, int64_t B,
+                           int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D, float softmax_scale, int causal,
+                           b200q_stream_t stream) {
   if (B < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || Sq < 0 || Sk < 0 || D <= 0 || D > 128 || D % 16 != 0) return B200Q_ERR_INVALID;
   if (vt_stride < Sk || vt_stride % 16 != 0 || B * Hq > 65535 || Sq > 0x7fffffffLL || Sk > 0x7fffffffLL) return B200Q_ERR_INVALID;
   if (out_dtype != B200Q_BF16 && out_dtype != B200Q_F16 && out_dtype != B200Q_F32) return B200Q_ERR_INVALID;
@@ -507,8 +645,14 @@ int b200q_fp8_sdpa(const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t
   if (q_codes == nullptr || out == nullptr || q_scale == nullptr || k_scale == nullptr || v_scale == nullptr) return B200Q_ERR_INVALID;
   if (Sk > 0 && (k_codes == nullptr || vt_codes == nullptr)) return B200Q_ERR_INVALID;
   if (!aligned(q_codes, 16) || !aligned(k_codes, 16) || !aligned(vt_codes, 16) || !aligned(out, 32)) return B200Q_ERR_ALIGN;
+  if (out_strides == nullptr) return B200Q_ERR_INVALID;
+  for (int i = 0; i < 3; ++i)
+    if (out_strides[i] < 0 || out_strides[i] % 8 != 0) return B200Q_ERR_ALIGN;   // 8-element stores
   if (int rc = check_arch()) return rc;
   AttParams p{};
+  p.out_sb = out_strides[0];
+  p.out_sh = out_strides[1];
+  p.out_ss = out_strides[2];
   p.status = gemm::device_status_word();
   if (p.status == nullptr) return B200Q_ERR_CUDA;
   static bool configured[64] = {};

@@ -166,6 +166,35 @@ struct Elem<float> {
   }
 };
 
+// 16 consecutive elements as they come from memory, so that several loads can be in flight before any arithmetic.
+// WIDE: 256-bit loads (32-byte aligned), else 128-bit ones (16-byte aligned).
+template <typename T, bool WIDE>
+struct Raw16 {
+  static constexpr int kLoads = static_cast<int>(sizeof(T)) / 2;   // 32-byte pieces
+  U32x8 w[kLoads];
+  __device__ __forceinline__ void load(const T* p) {
+    const char* c = reinterpret_cast<const char*>(p);
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i) {
+      if constexpr (WIDE) {
+        w[i] = ld_nc_256(c + 32 * i);
+      } else {
+        const uint4 a = ld_nc_128(c + 32 * i), b = ld_nc_128(c + 32 * i + 16);
+        w[i] = U32x8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+      }
+    }
+  }
+  __device__ __forceinline__ void widen(float* f) const {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(w[0].v[i]), f[8 + i] = __uint_as_float(w[kLoads - 1].v[i]);
+    } else {
+      Elem<T>::unpack(make_uint4(w[0].v[0], w[0].v[1], w[0].v[2], w[0].v[3]), f);
+      Elem<T>::unpack(make_uint4(w[0].v[4], w[0].v[5], w[0].v[6], w[0].v[7]), f + 8);
+    }
+  }
+};
+
 // ---------------------------------------------------------------- number formats
 // two fp32 -> two E4M3 bytes (RNE, saturate to +-448); low byte = a.
 __device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float a, float b) {

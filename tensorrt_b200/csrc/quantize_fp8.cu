@@ -304,6 +304,51 @@ amax_kernel(const T* __restrict__ x, int64_t n, float* __restrict__ out, float* 
   }
 }
 
+// Abs-max of three column ranges of a row-major matrix in one pass (Q, K, V of a QKV projection).  A thread walks
+// 16-element chunks (whole chunks lie in one range), keeps one running maximum per range and takes part in one
+// reduction per range at the end.  Values are >= 0, so their bit patterns order like unsigned integers; out is zero
+// before the launch.  HBM-bound: 2 bytes per 16-bit element, four chunks in flight per thread.
+template <typename T>
+__global__ void __launch_bounds__(kAmaxThreads)
+amax_columns_kernel(const T* __restrict__ x, int64_t chunks, uint32_t per_row, uint32_t first2, uint32_t first3,
+                    unsigned int* __restrict__ out) {
+  __shared__ float red[kAmaxThreads / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  float m[3] = {0.0f, 0.0f, 0.0f};
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kAmaxThreads;
+  constexpr int kLoads = 16 / ChunkMax<T>::kElems;    // 32-byte loads per chunk
+  constexpr int U = 4 / kLoads;
+  for (int64_t c0 = blockIdx.x * static_cast<int64_t>(kAmaxThreads) + threadIdx.x; c0 < chunks; c0 += U * stride) {
+    U32x8 r[U][kLoads];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + u * stride < chunks) {
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) r[u][i] = ld_nc_256(x + (c0 + u * stride) * 16 + i * ChunkMax<T>::kElems);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t c = c0 + u * stride;
+      if (c < chunks) {
+        ChunkMax<T> acc;
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) acc.add(r[u][i]);
+        const float a = acc.get();
+        const uint32_t col = static_cast<uint32_t>(c % per_row);
+        m[0] = fmaxf(m[0], col < first2 ? a : 0.0f);
+        m[1] = fmaxf(m[1], col >= first2 && col < first3 ? a : 0.0f);
+        m[2] = fmaxf(m[2], col >= first3 ? a : 0.0f);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float v = block_max<kAmaxThreads>(m[i], red);
+    if (threadIdx.x == 0 && v > 0.0f) atomicMax(out + i, __float_as_uint(v));
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
 row_amax_kernel(const T* __restrict__ x, float* __restrict__ out, int64_t rows, int64_t cols) {
@@ -419,6 +464,32 @@ int b200q_amax(const void* x, int dtype, int64_t n, float* amax_out, void* works
   unsigned int* ticket = static_cast<unsigned int*>(workspace);
   float* partials = static_cast<float*>(workspace) + 64;
   return launch_amax(x, dtype, n, amax_out, partials, ticket, static_cast<cudaStream_t>(stream));
+}
+
+int b200q_amax_columns(const void* x, int dtype, int64_t rows, int64_t c1, int64_t c2, int64_t c3, float* amax_out, b200q_stream_t stream) {
+  if (rows < 0 || c1 < 0 || c2 < 0 || c3 < 0 || (c1 | c2 | c3) % 16 != 0 || amax_out == nullptr) return B200Q_ERR_INVALID;
+  if (dtype != B200Q_F32 && dtype != B200Q_F16 && dtype != B200Q_BF16) return B200Q_ERR_INVALID;
+  const int64_t per_row = (c1 + c2 + c3) / 16;
+  if (per_row > 0x7fffffffLL) return B200Q_ERR_INVALID;
+  if (!aligned(amax_out, 4)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(amax_out, 0, 3 * sizeof(float), st) != cudaSuccess) return B200Q_ERR_CUDA;
+  const int64_t chunks = rows * per_row;
+  if (chunks == 0) return B200Q_OK;
+  if (x == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(x, 32)) return B200Q_ERR_ALIGN;
+  int64_t blocks = (chunks + kAmaxThreads * 4 - 1) / (kAmaxThreads * 4);
+  if (blocks > sm_count() * 8) blocks = sm_count() * 8;
+  const dim3 grid(static_cast<unsigned>(blocks)), block(kAmaxThreads);
+  const uint32_t pr = static_cast<uint32_t>(per_row), f2 = static_cast<uint32_t>(c1 / 16), f3 = static_cast<uint32_t>((c1 + c2) / 16);
+  unsigned int* out = reinterpret_cast<unsigned int*>(amax_out);
+  switch (dtype) {
+    case B200Q_BF16: launch_pdl(amax_columns_kernel<__nv_bfloat16>, grid, block, 0, st, static_cast<const __nv_bfloat16*>(x), chunks, pr, f2, f3, out); break;
+    case B200Q_F16: launch_pdl(amax_columns_kernel<__half>, grid, block, 0, st, static_cast<const __half*>(x), chunks, pr, f2, f3, out); break;
+    default: launch_pdl(amax_columns_kernel<float>, grid, block, 0, st, static_cast<const float*>(x), chunks, pr, f2, f3, out); break;
+  }
+  return check_launch();
 }
 
 int b200q_row_amax(const void* x, int dtype, int64_t rows, int64_t cols, float* amax_out, b200q_stream_t stream) {

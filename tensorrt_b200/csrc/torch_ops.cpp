@@ -446,23 +446,20 @@ Tensor fp8_sdpa_cuda(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in,
   Tensor out = at::empty_like(q);
   if (out.numel() == 0) return out;
   auto bytes = q.options().dtype(at::kByte);
-  auto f32 = q.options().dtype(at::kFloat);
   Tensor aq = as_f32_cuda(amax_q, q).reshape({1}), ak = as_f32_cuda(amax_k, q).reshape({1}), av = as_f32_cuda(amax_v, q).reshape({1});
   Tensor qc = at::empty(q.sizes(), bytes), kc = at::empty(k.sizes(), bytes);
-  Tensor sq = at::empty({1}, f32), sk = at::ones({1}, f32), sv = at::ones({1}, f32);
+  Tensor scales = at::empty({3}, q.options().dtype(at::kFloat));
   const int64_t stride = std::max<int64_t>((Sk + 15) / 16 * 16, 16);
   Tensor vt = at::empty({B, Hkv, D, stride}, bytes);
-  check_status(b200q_fp8_quantize(q.data_ptr(), dt, B * Hq * Sq, D, aq.data_ptr<float>(), 1, qc.data_ptr<uint8_t>(), sq.data_ptr<float>(),
-                                  current_stream()), "b200q_fp8_quantize");
-  if (Sk > 0) {
-    check_status(b200q_fp8_quantize(k.data_ptr(), dt, B * Hkv * Sk, D, ak.data_ptr<float>(), 1, kc.data_ptr<uint8_t>(), sk.data_ptr<float>(),
-                                    current_stream()), "b200q_fp8_quantize");
-    check_status(b200q_fp8_quantize_transpose(v.data_ptr(), dt, B * Hkv, Sk, D, av.data_ptr<float>(), vt.data_ptr<uint8_t>(), stride,
-                                              sv.data_ptr<float>(), current_stream()), "b200q_fp8_quantize_transpose");
-  }
+  const int64_t strides[9] = {Hq * Sq * D, Sq * D, D, Hkv * Sk * D, Sk * D, D, Hkv * Sk * D, Sk * D, D};
+  float* sp = scales.data_ptr<float>();
+  check_status(b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr<float>(), ak.data_ptr<float>(),
+                                            av.data_ptr<float>(), qc.data_ptr<uint8_t>(), kc.data_ptr<uint8_t>(), vt.data_ptr<uint8_t>(), sp, B,
+                                            Hq, Hkv, Sq, Sk, stride, D, current_stream()),
+               "b200q_fp8_attention_quantize");
   const float sm = scale > 0.0 ? static_cast<float>(scale) : 1.0f / std::sqrt(static_cast<float>(D));
-  check_status(b200q_fp8_sdpa(qc.data_ptr<uint8_t>(), kc.data_ptr<uint8_t>(), vt.data_ptr<uint8_t>(), sq.data_ptr<float>(), sk.data_ptr<float>(),
-                              sv.data_ptr<float>(), out.data_ptr(), dt, B, Hq, Hkv, Sq, Sk, stride, D, sm, is_causal ? 1 : 0, current_stream()),
+  check_status(b200q_fp8_sdpa(qc.data_ptr<uint8_t>(), kc.data_ptr<uint8_t>(), vt.data_ptr<uint8_t>(), sp, sp + 1, sp + 2, out.data_ptr(), dt, B,
+                              Hq, Hkv, Sq, Sk, stride, D, sm, is_causal ? 1 : 0, current_stream()),
                "b200q_fp8_sdpa");
   return out;
 }

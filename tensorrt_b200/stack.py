@@ -177,11 +177,7 @@ class CudaBackend:
         t = qkv.shape[0]
         if seq_len <= 0 or t % seq_len:
             raise ValueError(f"{t} tokens are not whole sequences of {seq_len}")
-        b, qw, kvw = t // seq_len, n_q * head_dim, n_kv * head_dim
-        heads = lambda x, n: x.reshape(b, seq_len, n, head_dim).permute(0, 2, 1, 3).contiguous()  # noqa: E731
-        q, k, v = heads(qkv[:, :qw], n_q), heads(qkv[:, qw:qw + kvw], n_kv), heads(qkv[:, qw + kvw:], n_kv)
-        out = capi.fp8_sdpa(q, k, v, capi.amax(q), capi.amax(k), capi.amax(v), True)
-        return out.permute(0, 2, 1, 3).reshape(t, qw)
+        return capi.fp8_sdpa_packed(qkv, t // seq_len, n_q, n_kv, head_dim, True)
 
     def measure_norm_amax(self, h, delta, weight, eps):
         if self.mode != "nvfp4":
