@@ -128,6 +128,14 @@ size_t b200q_nvfp4_scale_bytes(int64_t rows, int64_t cols);
 int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax,
                          uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out,
                          b200q_stream_t stream);
+/* b200q_nvfp4_quantize under the tensor's own abs-max, measured here: the same result as b200q_amax followed by
+ * b200q_nvfp4_quantize.  One launch for small tensors, which need no workspace (.._workspace_bytes() is 0); for
+ * others the workspace of b200q_amax, whose first 16 bytes are zero before the first use and whose first 8 are zero
+ * again afterwards. */
+size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols);
+int b200q_nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out,
+                                 uint8_t* scales_out, float* global_scale_out, void* workspace, size_t workspace_bytes,
+                                 b200q_stream_t stream);
 
 /* Eager semantics of `tensorrt::dynamic_block_quantize_op(input, 16, amax, 4, 2, 8, 4)`:
  * quantize then double-dequantize, x_hat = e2m1 * (e4m3 * global), back to the input dtype

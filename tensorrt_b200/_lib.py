@@ -30,6 +30,8 @@ SIGNATURES = {
     "b200q_fp8_dequantize": (_c.c_int, [_p, _p, _i64, _i64, _i64, _p, _c.c_int, _p]),
     "b200q_nvfp4_scale_bytes": (_c.c_size_t, [_i64, _i64]),
     "b200q_nvfp4_quantize": (_c.c_int, [_p, _c.c_int, _i64, _i64, _p, _p, _p, _p, _p]),
+    "b200q_nvfp4_quantize_dynamic_workspace_bytes": (_c.c_size_t, [_i64, _i64]),
+    "b200q_nvfp4_quantize_dynamic": (_c.c_int, [_p, _c.c_int, _i64, _i64, _p, _p, _p, _p, _c.c_size_t, _p]),
     "b200q_nvfp4_fake_quantize": (_c.c_int, [_p, _c.c_int, _i64, _i64, _p, _p, _p]),
     "b200q_nvfp4_dequantize": (_c.c_int, [_p, _p, _p, _i64, _i64, _p, _c.c_int, _p]),
     "b200q_fp8_gemm": (_c.c_int, [_p, _p, _i64, _p, _p, _i64, _p, _p, _i64, _i64, _i64, _p, _p]),

@@ -58,9 +58,9 @@ def amax_workspace(device) -> torch.Tensor:
 def amax(x: torch.Tensor) -> torch.Tensor:
     _need_cuda(x)
     x = x.contiguous()
-    out = torch.zeros((), dtype=torch.float32, device=x.device)
     if x.numel() == 0:
-        return out
+        return torch.zeros((), dtype=torch.float32, device=x.device)
+    out = torch.empty((), dtype=torch.float32, device=x.device)
     ws = amax_workspace(x.device)
     with torch.cuda.device(x.device):
         check(load().b200q_amax(x.data_ptr(), _dt(x), x.numel(), out.data_ptr(), ws.data_ptr(), ws.numel(), _stream(x)),
@@ -129,6 +129,12 @@ def nvfp4_scale_bytes(rows: int, cols: int) -> int:
     return load().b200q_nvfp4_scale_bytes(rows, cols)
 
 
+def _nvfp4_out(shape, rows, cols, device):
+    """(packed codes, swizzled block scales, global scale) of an NVFP4 operand [rows, cols], uninitialised."""
+    return (torch.empty(*shape[:-1], cols // 2, dtype=torch.uint8, device=device),
+            torch.empty(nvfp4_scale_bytes(rows, cols), dtype=torch.uint8, device=device), torch.empty((), dtype=torch.float32, device=device))
+
+
 def nvfp4_quantize(x: torch.Tensor, amax_t: torch.Tensor):
     """-> (packed codes uint8 [.., cols/2], swizzled E4M3 block scales uint8 [bytes], global scale fp32 0-dim)."""
     _need_cuda(x, amax_t)
@@ -143,6 +149,21 @@ def nvfp4_quantize(x: torch.Tensor, amax_t: torch.Tensor):
     with torch.cuda.device(x.device):
         check(load().b200q_nvfp4_quantize(x.data_ptr(), _dt(x), rows, cols, a.data_ptr(), codes.data_ptr(),
                                           scales.data_ptr(), g.data_ptr(), _stream(x)), "b200q_nvfp4_quantize")
+    return codes, scales, g
+
+
+def nvfp4_quantize_dynamic(x: torch.Tensor):
+    """`nvfp4_quantize(x, amax(x))`, the abs-max measured on the way (one launch for small tensors)."""
+    _need_cuda(x)
+    x = x.contiguous()
+    rows, cols = _rows_cols(x)
+    if cols % 16:
+        raise ValueError(f"last dimension ({cols}) must be a multiple of the block size 16")
+    codes, scales, g = _nvfp4_out(x.shape, rows, cols, x.device)
+    ws = amax_workspace(x.device)
+    with torch.cuda.device(x.device):
+        check(load().b200q_nvfp4_quantize_dynamic(x.data_ptr(), _dt(x), rows, cols, codes.data_ptr(), scales.data_ptr(), g.data_ptr(),
+                                                  ws.data_ptr(), ws.numel(), _stream(x)), "b200q_nvfp4_quantize_dynamic")
     return codes, scales, g
 
 
@@ -425,12 +446,6 @@ def add_rms_norm_fp8_quantize(h: torch.Tensor, delta: torch.Tensor | None, weigh
         check(load().b200q_add_rms_norm_fp8_quantize(h.data_ptr(), _ptr(delta), weight.data_ptr(), h_out.data_ptr(), codes.data_ptr(),
                                                      scales.data_ptr(), rows, cols, eps, _stream(h)), "b200q_add_rms_norm_fp8_quantize")
     return h_out, codes, scales
-
-
-def _nvfp4_out(shape, rows, cols, device):
-    """(packed codes, swizzled block scales, global scale) of an NVFP4 operand [rows, cols], uninitialised."""
-    return (torch.empty(*shape[:-1], cols // 2, dtype=torch.uint8, device=device),
-            torch.empty(nvfp4_scale_bytes(rows, cols), dtype=torch.uint8, device=device), torch.empty((), dtype=torch.float32, device=device))
 
 
 def _scalar_amax(amax_t, device):

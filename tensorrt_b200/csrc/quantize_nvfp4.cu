@@ -175,6 +175,72 @@ nvfp4_quantize_kernel(const T* __restrict__ x, const float* __restrict__ amax, u
   }
 }
 
+// Quantize of a small tensor under its own abs-max, measured in the same launch: every CTA reads the whole tensor (at
+// most kDynamicMaxElems elements, from L2 after the first) for the maximum and quantizes its share.  A decode step's
+// activation is a few hundred KB at most: three launches in a row (a cleared result, the abs-max, the quantize) cost
+// more than reading it 16 times over.  A thread owns one block; rows take a multiple of four blocks (one scale word),
+// the rows that pad the last 128-row scale tile only clear their words.
+constexpr int64_t kDynamicMaxElems = 1 << 17;
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+nvfp4_quantize_dynamic_kernel(const T* __restrict__ x, uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, float* __restrict__ gout,
+                              uint32_t rows, uint32_t cols, uint32_t blocks_per_row, uint32_t col_tiles, uint32_t units) {
+  __shared__ float red[kThreads / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t unit = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t row = unit / (col_tiles * 4u), blk = unit - row * (col_tiles * 4u);
+  const bool live = row < rows && blk < blocks_per_row;
+  float amax = 0.0f;
+  if ((blockIdx.x * kThreads) / (col_tiles * 4u) < rows) {    // the CTA has blocks of its own
+    constexpr int U = sizeof(T) == 4 ? 4 : 8;                 // 256 bytes of loads in flight per lane
+    const uint32_t total = rows * blocks_per_row;
+    for (uint32_t b0 = threadIdx.x; b0 < total; b0 += U * kThreads) {
+      typename Block16<T>::Raw raw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + u * kThreads < total) raw[u] = Block16<T>::load_raw(x + static_cast<int64_t>(b0 + u * kThreads) * 16);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + u * kThreads < total) {
+          float f[16];
+          Block16<T>::widen(raw[u], f);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
+        }
+    }
+    amax = warp_max(amax);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+    __syncthreads();
+    amax = warp_max((threadIdx.x & 31) < kThreads / 32 ? red[threadIdx.x & 31] : 0.0f);
+  }
+  const GlobalScale gs(amax);
+  if (unit == 0 && gout != nullptr) *gout = gs.g;
+  uint32_t sb = 0u;
+  if (live) {
+    float f[16], d;
+    uint32_t c_lo, c_hi;
+    Block16<T>::widen(Block16<T>::load_raw(x + (static_cast<int64_t>(row) * blocks_per_row + blk) * 16), f);
+    sb = quantize_block(f, gs, c_lo, c_hi, d);
+    *reinterpret_cast<uint2*>(codes + (static_cast<int64_t>(row) * blocks_per_row + blk) * 8) = make_uint2(c_lo, c_hi);
+  }
+  uint32_t w = sb << (8u * (threadIdx.x & 3u));
+  w |= __shfl_xor_sync(0xffffffffu, w, 1);
+  w |= __shfl_xor_sync(0xffffffffu, w, 2);
+  if ((threadIdx.x & 3u) == 0u && unit < units)
+    *reinterpret_cast<uint32_t*>(sf + ((row >> 7) * col_tiles + (blk >> 2)) * 512u + (row & 31u) * 16u + ((row >> 5) & 3u) * 4u) = w;
+}
+
+template <typename T>
+int launch_dynamic(const void* x, uint8_t* codes, uint8_t* sf, float* gout, int64_t rows, int64_t cols, cudaStream_t st) {
+  const uint32_t bpr = static_cast<uint32_t>(cols >> 4), col_tiles = (bpr + 3u) >> 2;
+  const uint32_t units = static_cast<uint32_t>((rows + 127) / 128 * 128) * col_tiles * 4u;   // rows <= 8192, bpr <= 8192: < 2^26
+  launch_pdl(nvfp4_quantize_dynamic_kernel<T>, dim3((units + kThreads - 1) / kThreads), dim3(kThreads), 0, st, static_cast<const T*>(x), codes,
+             sf, gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), bpr, col_tiles, units);
+  return check_launch();
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_dequantize_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ sf, const float* __restrict__ gptr,
@@ -262,6 +328,32 @@ int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, c
     case B200Q_F16: return launch<__half, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
     default: return launch<float, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
   }
+}
+
+size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols) {
+  return rows <= 0 || cols <= 0 || rows <= kDynamicMaxElems / cols ? 0 : b200q_amax_workspace_bytes();
+}
+
+int b200q_nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
+                                 float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream) {
+  if (int rc = validate(x, dtype, rows, cols, reinterpret_cast<const float*>(x))) return rc;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  const size_t need = b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols);
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need)) return B200Q_ERR_WORKSPACE;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (need == 0) {
+    switch (dtype) {
+      case B200Q_BF16: return launch_dynamic<__nv_bfloat16>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
+      case B200Q_F16: return launch_dynamic<__half>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
+      default: return launch_dynamic<float>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
+    }
+  }
+  float* amax = static_cast<float*>(workspace) + 2;      // behind the two words that the abs-max kernel keeps
+  if (int rc = b200q_amax(x, dtype, rows * cols, amax, workspace, workspace_bytes, stream)) return rc;
+  return b200q_nvfp4_quantize(x, dtype, rows, cols, amax, codes_out, scales_out, global_scale_out, stream);
 }
 
 int b200q_silu_mul_nvfp4_quantize(const void* gate_up, const float* amax, uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out,

@@ -24,9 +24,7 @@ def fp8_linear(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor, b
 def nvfp4_linear(x: torch.Tensor, w_codes, w_scales, w_global, bias=None,
                  x_amax: torch.Tensor | None = None) -> torch.Tensor:
     """NVFP4 W4A4.  `x_amax` is the activation tensor amax (static calibration); None = measured per call."""
-    if x_amax is None:
-        x_amax = capi.amax(x)
-    x_codes, x_scales, x_global = capi.nvfp4_quantize(x, x_amax)
+    x_codes, x_scales, x_global = capi.nvfp4_quantize_dynamic(x) if x_amax is None else capi.nvfp4_quantize(x, x_amax)
     return capi.nvfp4_gemm(x_codes, x_scales, x_global, w_codes, w_scales, w_global, bias)
 
 

@@ -114,7 +114,7 @@ class CudaBackend:
         NVFP4, None = measured on this input; FP8 activations are scaled per token in the kernel."""
         if self.mode == "fp8":
             return capi.fp8_quantize(x, None)
-        return capi.nvfp4_quantize(x, capi.amax(x) if amax is None else amax)
+        return capi.nvfp4_quantize_dynamic(x) if amax is None else capi.nvfp4_quantize(x, amax)
 
     def matmul(self, xq, qw) -> torch.Tensor:
         if self.mode == "fp8":
