@@ -3,7 +3,9 @@
 `libb200q.so`      — CUDA kernels + the C ABI declared in include/b200q.h (nvcc, sm_100a only).
 `libb200q_torch.so` — the torch.library shim registering the `tensorrt::` ops on top of it (g++).
 
-Both are written next to this file so they travel with the source tree; nothing is
+`libb200q_python.so` — the Python modules' whole calls as native functions (g++, csrc/python_calls.cpp).
+
+All are written next to this file so they travel with the source tree; nothing is
 installed into site-packages and no JIT cache is used.
 """
 from __future__ import annotations
@@ -20,6 +22,7 @@ CSRC = PKG / "csrc"
 ROOT = PKG.parent
 LIB = PKG / "libb200q.so"
 TORCH_LIB = PKG / "libb200q_torch.so"
+PYTHON_LIB = PKG / "libb200q_python.so"
 
 CUDA_SOURCES = ["runtime.cu", "quantize_fp8.cu", "quantize_nvfp4.cu", "gemm_fp8.cu", "gemm_nvfp4.cu",
                 "fused_ops.cu", "p2p_allreduce.cu", "attention_fp8.cu", "comm_context.cu"]
@@ -113,20 +116,28 @@ def _build_cuda(force: bool, verbose: bool) -> Path:
 def build_torch_shim(force: bool = False) -> Path:
     """Compile the torch.library shim (C++17, no CUDA code) against libb200q.so."""
     with _BuildLock():
-        return _build_torch_shim(force)
+        return _build_torch_extension(CSRC / "torch_ops.cpp", TORCH_LIB, "torch", [], [], force)
 
 
-def _build_torch_shim(force: bool) -> Path:
+def build_python_calls(force: bool = False) -> Path:
+    """Compile the native calls of the Python modules (C++17, CPython API) against libb200q.so."""
+    import sysconfig
+
+    with _BuildLock():
+        return _build_torch_extension(CSRC / "python_calls.cpp", PYTHON_LIB, "python", ["-isystem", sysconfig.get_paths()["include"]],
+                                      ["-ltorch_python"], force)
+
+
+def _build_torch_extension(src: Path, lib: Path, name: str, includes: list, libs: list, force: bool) -> Path:
     import torch
     from torch.utils import cpp_extension
 
-    src = CSRC / "torch_ops.cpp"
     stamp = _stamp([src, ROOT / "include" / "b200q.h"], torch.__version__)
-    stamp_file = PKG / "build" / "torch.stamp"
-    if not force and TORCH_LIB.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
-        return TORCH_LIB
+    stamp_file = PKG / "build" / f"{name}.stamp"
+    if not force and lib.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+        return lib
     (PKG / "build").mkdir(exist_ok=True)
-    inc = []
+    inc = list(includes)
     for p in cpp_extension.include_paths():
         inc += ["-isystem", p]
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -134,20 +145,21 @@ def _build_torch_shim(force: bool) -> Path:
     torch_lib = Path(torch.__file__).parent / "lib"
     cxx11 = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={cxx11}",
-           "-I", str(ROOT / "include"), *inc, str(src), "-o", str(TORCH_LIB),
-           f"-L{PKG}", "-lb200q", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda",
+           "-I", str(ROOT / "include"), *inc, str(src), "-o", str(lib),
+           f"-L{PKG}", "-lb200q", f"-L{torch_lib}", *libs, "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda",
            f"-L{cuda_home}/lib64", "-lcudart",
            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-    _run(cmd, PKG / "build" / "torch_ops.log")
+    _run(cmd, PKG / "build" / f"{src.stem}.log")
     stamp_file.write_text(stamp)
-    return TORCH_LIB
+    return lib
 
 
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cuda(force, verbose)
     build_torch_shim(force)
+    build_python_calls(force)
 
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print(LIB, TORCH_LIB)
+    print(LIB, TORCH_LIB, PYTHON_LIB)

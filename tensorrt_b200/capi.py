@@ -11,6 +11,7 @@ import ctypes
 
 import torch
 
+from . import _native
 from ._lib import cfg_ref, check, load
 
 _DTYPE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
@@ -210,6 +211,11 @@ def gemm_config(tile_n: int | None = None, static_weights: bool | None = None):
         _gemm_cfg.reset(token)
 
 
+def gemm_defaults():
+    """(tile_n, static_weights) in force here."""
+    return _gemm_cfg.get()
+
+
 def _cfg(tile_n, static_weights):
     cur = _gemm_cfg.get()
     return cfg_ref(cur[0] if tile_n is None else tile_n, cur[1] if static_weights is None else static_weights)
@@ -311,6 +317,9 @@ def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, 
     with the fixed scale 1/448, both contractions run on FP8 tensor cores; result in q's dtype."""
     import math
 
+    y = _native.fp8_sdpa(q, k, v, amax_q, amax_k, amax_v, is_causal, scale)
+    if y is not None:
+        return y
     _need_cuda(q, k, v)
     if q.dim() != 4 or k.dim() != 4 or v.dim() != 4 or k.shape != v.shape or q.shape[0] != k.shape[0] or q.shape[3] != k.shape[3]:
         raise ValueError(f"expected q [B, Hq, Sq, D] and k, v [B, Hkv, Sk, D], got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")

@@ -11,12 +11,15 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from . import capi
+from . import _native, capi
 
 
 def fp8_linear(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor, bias=None,
                x_amax: torch.Tensor | None = None) -> torch.Tensor:
     """Per-token (dynamic, or `x_amax` static) FP8 activations x per-channel/per-tensor FP8 weights."""
+    y = _native.fp8_linear(x, w_codes, w_scales, bias, x_amax, *capi.gemm_defaults())
+    if y is not None:
+        return y
     x_codes, x_scales = capi.fp8_quantize(x, x_amax)
     return capi.fp8_gemm(x_codes, x_scales, w_codes, w_scales, bias)
 
@@ -24,6 +27,9 @@ def fp8_linear(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor, b
 def nvfp4_linear(x: torch.Tensor, w_codes, w_scales, w_global, bias=None,
                  x_amax: torch.Tensor | None = None) -> torch.Tensor:
     """NVFP4 W4A4.  `x_amax` is the activation tensor amax (static calibration); None = measured per call."""
+    y = _native.nvfp4_linear(x, w_codes, w_scales, w_global, bias, x_amax, *capi.gemm_defaults())
+    if y is not None:
+        return y
     x_codes, x_scales, x_global = capi.nvfp4_quantize_dynamic(x) if x_amax is None else capi.nvfp4_quantize(x, x_amax)
     return capi.nvfp4_gemm(x_codes, x_scales, x_global, w_codes, w_scales, w_global, bias)
 
@@ -84,6 +90,10 @@ class Fp8GatedMlp(nn.Module):
         return cls(torch.cat([parts[0][0], parts[1][0]]).contiguous(), gu_scales.contiguous(), parts[2][0], parts[2][1], input_amax, act_amax)
 
     def forward(self, x):
+        y = _native.fp8_gated_mlp(x, self.gu_codes, self.gu_scales, self.down_codes, self.down_scales, self.input_amax, self.act_amax,
+                                  *capi.gemm_defaults())
+        if y is not None:
+            return y
         xq = capi.fp8_quantize(x, self.input_amax)
         tokens = xq[0].numel() // xq[0].shape[-1]
         if tokens >= 256 and self.act_amax is not None and self.act_amax.numel() == 1:
