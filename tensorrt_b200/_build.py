@@ -132,7 +132,7 @@ def _build_torch_extension(src: Path, lib: Path, name: str, includes: list, libs
     import torch
     from torch.utils import cpp_extension
 
-    stamp = _stamp([src, ROOT / "include" / "b200q.h"], torch.__version__)
+    stamp = _stamp([src, CSRC / "internal.h", ROOT / "include" / "b200q.h"], torch.__version__)
     stamp_file = PKG / "build" / f"{name}.stamp"
     if not force and lib.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
         return lib

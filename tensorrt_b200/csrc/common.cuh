@@ -32,6 +32,16 @@ bool pdl_enabled();  // environment variable B200Q_PDL, default on
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Both for a kernel that quantizes an activation.  `late`: the dependents are let go only once everything before this
+// kernel has completed.  A GEMM launched right behind it may then treat its weights as complete from its first
+// instruction (b200q_cfg::static_weights) whatever produced them, and requests its first ring of weight tiles while this
+// kernel runs.  Otherwise dependents may start at once, under the tail of the kernel before this one.
+__device__ __forceinline__ void pdl_enter(bool late) {
+  if (!late) pdl_launch_dependents();
+  pdl_wait();
+  if (late) pdl_launch_dependents();
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -4,6 +4,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "internal.h"
 #include "nvfp4_block.cuh"
 #include "tcgen05.cuh"
 
@@ -390,9 +391,8 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict_
 // maxima meet through distributed shared memory.
 template <int ITEMS, int PARTS>
 __global__ void __launch_bounds__(kThreads)
-silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ codes, float* __restrict__ scales, int64_t f) {
-  pdl_launch_dependents();
-  pdl_wait();
+silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ codes, float* __restrict__ scales, int64_t f, bool late) {
+  pdl_enter(late);
   __shared__ float red[kThreads / 32];
   __shared__ float part_max;
   const int64_t row = blockIdx.x / PARTS;
@@ -783,6 +783,80 @@ int launch_fp8_rows_stream(const __nv_bfloat16* x, uint8_t* codes, float* scales
 #undef B200Q_ROWS_STREAM
   return check_launch();
 }
+
+int silu_mul_fp8_quantize(const void* gate_up, uint8_t* codes_out, float* scales_out, int64_t rows, int64_t f,
+                                b200q_stream_t stream, bool late) {
+  if (rows < 0 || f < 0 || f % 8 != 0 || rows > 0x7fffffffLL || f > kThreads * 8 * 16) return B200Q_ERR_INVALID;
+  if (rows == 0 || f == 0) return B200Q_OK;
+  if (gate_up == nullptr || codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(gate_up, 16) || !aligned(codes_out, 8)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const auto* gp = static_cast<const __nv_bfloat16*>(gate_up);
+  const int64_t groups = f >> 3;
+  // many tokens, rows of at least one chunk: persistent CTAs fed through a shared-memory ring
+  if (rows >= 8 * sm_count() && groups >= kSiluChunkGroups) {
+    int* status = gemm::device_status_word();
+    if (status == nullptr) return B200Q_ERR_CUDA;
+    const int nch = static_cast<int>((groups + kSiluChunkGroups - 1) / kSiluChunkGroups);
+    const size_t smem = static_cast<size_t>(kSiluStages) * 2 * kSiluChunkBytes;
+    const dim3 grid(static_cast<unsigned>(2 * sm_count()));
+    const int r32 = static_cast<int>(rows), f32 = static_cast<int>(f);
+#define B200Q_SILUS(C)                                                                                              \
+  do {                                                                                                               \
+    cudaFuncSetAttribute(silu_mul_quant_stream_kernel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
+    launch_pdl(silu_mul_quant_stream_kernel<C, true>, grid, dim3(kThreads), smem, st, gp, codes_out, scales_out, r32, f32, status);   \
+  } while (0)
+    if (nch <= 2) B200Q_SILUS(2);
+    else if (nch <= 4) B200Q_SILUS(4);
+    else B200Q_SILUS(8);
+#undef B200Q_SILUS
+    return check_launch();
+  }
+  // few tokens: split every row over a cluster so that the launch covers the SMs
+  int parts = 1;
+  while (parts < 8 && rows * parts < 2 * sm_count() && groups / (parts * 2) >= kThreads / 2) parts *= 2;
+  // long rows: 16 groups per thread cost 92 registers (two CTAs per SM) and the kernel turns
+  // compute-bound on the exponentials; two CTAs per row at 8 groups per thread double the warps per SM
+  if (parts == 1 && groups > 8 * kThreads) parts = 2;
+  const int items = static_cast<int>(((groups + parts - 1) / parts + kThreads - 1) / kThreads);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows * parts));
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(parts);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+#define B200Q_SILU(I, P) cudaLaunchKernelEx(&cfg, silu_mul_quant_kernel<I, P>, gp, codes_out, scales_out, f, late)
+  if (parts == 1) {
+    if (items <= 1) B200Q_SILU(1, 1);
+    else if (items <= 2) B200Q_SILU(2, 1);
+    else if (items <= 4) B200Q_SILU(4, 1);
+    else if (items <= 8) B200Q_SILU(8, 1);
+    else B200Q_SILU(16, 1);
+  } else if (parts == 2) {
+    if (items <= 1) B200Q_SILU(1, 2);
+    else if (items <= 2) B200Q_SILU(2, 2);
+    else if (items <= 4) B200Q_SILU(4, 2);
+    else B200Q_SILU(8, 2);
+  } else if (parts == 4) {
+    if (items <= 1) B200Q_SILU(1, 4);
+    else if (items <= 2) B200Q_SILU(2, 4);
+    else B200Q_SILU(4, 4);
+  } else {
+    if (items <= 1) B200Q_SILU(1, 8);
+    else B200Q_SILU(2, 8);
+  }
+#undef B200Q_SILU
+  return check_launch();
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -845,75 +919,7 @@ int b200q_silu_mul(const void* gate_up, void* out, int64_t rows, int64_t f, b200
 
 int b200q_silu_mul_fp8_quantize(const void* gate_up, uint8_t* codes_out, float* scales_out, int64_t rows, int64_t f,
                                 b200q_stream_t stream) {
-  if (rows < 0 || f < 0 || f % 8 != 0 || rows > 0x7fffffffLL || f > kThreads * 8 * 16) return B200Q_ERR_INVALID;
-  if (rows == 0 || f == 0) return B200Q_OK;
-  if (gate_up == nullptr || codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
-  if (!aligned(gate_up, 16) || !aligned(codes_out, 8)) return B200Q_ERR_ALIGN;
-  if (int rc = check_arch()) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const auto* gp = static_cast<const __nv_bfloat16*>(gate_up);
-  const int64_t groups = f >> 3;
-  // many tokens, rows of at least one chunk: persistent CTAs fed through a shared-memory ring
-  if (rows >= 8 * sm_count() && groups >= kSiluChunkGroups) {
-    int* status = gemm::device_status_word();
-    if (status == nullptr) return B200Q_ERR_CUDA;
-    const int nch = static_cast<int>((groups + kSiluChunkGroups - 1) / kSiluChunkGroups);
-    const size_t smem = static_cast<size_t>(kSiluStages) * 2 * kSiluChunkBytes;
-    const dim3 grid(static_cast<unsigned>(2 * sm_count()));
-    const int r32 = static_cast<int>(rows), f32 = static_cast<int>(f);
-#define B200Q_SILUS(C)                                                                                              \
-  do {                                                                                                               \
-    cudaFuncSetAttribute(silu_mul_quant_stream_kernel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
-    launch_pdl(silu_mul_quant_stream_kernel<C, true>, grid, dim3(kThreads), smem, st, gp, codes_out, scales_out, r32, f32, status);   \
-  } while (0)
-    if (nch <= 2) B200Q_SILUS(2);
-    else if (nch <= 4) B200Q_SILUS(4);
-    else B200Q_SILUS(8);
-#undef B200Q_SILUS
-    return check_launch();
-  }
-  // few tokens: split every row over a cluster so that the launch covers the SMs
-  int parts = 1;
-  while (parts < 8 && rows * parts < 2 * sm_count() && groups / (parts * 2) >= kThreads / 2) parts *= 2;
-  // long rows: 16 groups per thread cost 92 registers (two CTAs per SM) and the kernel turns
-  // compute-bound on the exponentials; two CTAs per row at 8 groups per thread double the warps per SM
-  if (parts == 1 && groups > 8 * kThreads) parts = 2;
-  const int items = static_cast<int>(((groups + parts - 1) / parts + kThreads - 1) / kThreads);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(rows * parts));
-  cfg.blockDim = dim3(kThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(parts);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-#define B200Q_SILU(I, P) cudaLaunchKernelEx(&cfg, silu_mul_quant_kernel<I, P>, gp, codes_out, scales_out, f)
-  if (parts == 1) {
-    if (items <= 1) B200Q_SILU(1, 1);
-    else if (items <= 2) B200Q_SILU(2, 1);
-    else if (items <= 4) B200Q_SILU(4, 1);
-    else if (items <= 8) B200Q_SILU(8, 1);
-    else B200Q_SILU(16, 1);
-  } else if (parts == 2) {
-    if (items <= 1) B200Q_SILU(1, 2);
-    else if (items <= 2) B200Q_SILU(2, 2);
-    else if (items <= 4) B200Q_SILU(4, 2);
-    else B200Q_SILU(8, 2);
-  } else if (parts == 4) {
-    if (items <= 1) B200Q_SILU(1, 4);
-    else if (items <= 2) B200Q_SILU(2, 4);
-    else B200Q_SILU(4, 4);
-  } else {
-    if (items <= 1) B200Q_SILU(1, 8);
-    else B200Q_SILU(2, 8);
-  }
-#undef B200Q_SILU
-  return check_launch();
+  return silu_mul_fp8_quantize(gate_up, codes_out, scales_out, rows, f, stream, false);
 }
 
 int b200q_add(const void* a, const void* b, void* out, int64_t n, b200q_stream_t stream) {

@@ -4,6 +4,10 @@
 // Python (argument checks, two to six tensors, a ctypes call per kernel) take longer than that on the host.  The
 // functions here issue the same b200q_* calls on the current stream with the scratch of a call in one allocation.
 //
+// Every GEMM here stands directly behind a kernel that quantizes its activation and lets its dependents go late
+// (common.cuh::pdl_enter), so it may request weight tiles before that kernel ends: static_weights without a promise
+// from the caller.
+//
 // They take the plain case only (strided CUDA tensors of the exact Python type, matching sizes, fp32 scales, no
 // dispatch or function mode active) and return None for anything else, before anything is launched: the caller then
 // takes the general path in capi.py, which converts, or raises the error that belongs to the input.
@@ -22,6 +26,7 @@
 #include <optional>
 
 #include "b200q.h"
+#include "internal.h"
 
 namespace {
 
@@ -101,7 +106,7 @@ std::optional<Tensor> fp8_linear(const Tensor& x_in, const Tensor& w, const Tens
   auto* scales = reinterpret_cast<float*>(codes + up16(M * K));
   Tensor out = bf16_like(x, N);
   const auto st = current_stream();
-  if (b200q_fp8_quantize(x.data_ptr(), dt, M, K, f32(amax), n, codes, scales, st) != B200Q_OK) return std::nullopt;
+  if (b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(amax), n, codes, scales, st, true) != B200Q_OK) return std::nullopt;
   if (b200q_fp8_gemm(codes, scales, n_scales, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),
                      bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, st, &cfg) != B200Q_OK)
     return std::nullopt;
@@ -134,11 +139,11 @@ std::optional<Tensor> nvfp4_linear(const Tensor& x_in, const Tensor& w, const Te
   const auto st = current_stream();
   int rc;
   if (amax != nullptr) {
-    rc = b200q_nvfp4_quantize(x.data_ptr(), dt, M, K, f32(amax), codes, sf, g, st);
+    rc = b200q::nvfp4_quantize(x.data_ptr(), dt, M, K, f32(amax), codes, sf, g, st, true);
   } else {
     // the two words that the abs-max of a large tensor counts in start at zero
     if (ws_bytes > 0 && cudaMemsetAsync(workspace, 0, 16, static_cast<cudaStream_t>(st)) != cudaSuccess) return std::nullopt;
-    rc = b200q_nvfp4_quantize_dynamic(x.data_ptr(), dt, M, K, codes, sf, g, workspace, static_cast<size_t>(ws_bytes), st);
+    rc = b200q::nvfp4_quantize_dynamic(x.data_ptr(), dt, M, K, codes, sf, g, workspace, static_cast<size_t>(ws_bytes), st, true);
   }
   if (rc != B200Q_OK) return std::nullopt;
   if (b200q_nvfp4_gemm(codes, sf, g, static_cast<const uint8_t*>(w.data_ptr()), static_cast<const uint8_t*>(wsf.data_ptr()), f32(&wg),
@@ -178,22 +183,22 @@ std::optional<Tensor> fp8_gated_mlp(const Tensor& x_in, const Tensor& gu, const 
   uint8_t* m1 = base + o_mid;
   const auto* guc = static_cast<const uint8_t*>(gu.data_ptr());
   Tensor out = bf16_like(x, H);
-  if (b200q_fp8_quantize(x.data_ptr(), dt, M, K, f32(in_amax), n_in, xc, xs, st) != B200Q_OK) return std::nullopt;
+  if (b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(in_amax), n_in, xc, xs, st, true) != B200Q_OK) return std::nullopt;
   int rc;
   if (fused_quant) {
     rc = b200q_fp8_gemm_silu_mul_quantize(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, f32(act_amax), ac, as, M, 2 * F, K, st, nullptr);
   } else if (fused) {
     rc = b200q_fp8_gemm_silu_mul(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, nullptr);
-    if (rc == B200Q_OK) rc = b200q_fp8_quantize(m1, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st);
+    if (rc == B200Q_OK) rc = b200q::fp8_quantize(m1, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true);
   } else {
     rc = b200q_fp8_gemm(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, &cfg);
     if (rc == B200Q_OK) {
       if (n_act) {
         uint8_t* act = m1 + M * F * 4;
         rc = b200q_silu_mul(m1, act, M, F, st);
-        if (rc == B200Q_OK) rc = b200q_fp8_quantize(act, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st);
+        if (rc == B200Q_OK) rc = b200q::fp8_quantize(act, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true);
       } else {
-        rc = b200q_silu_mul_fp8_quantize(m1, ac, as, M, F, st);
+        rc = b200q::silu_mul_fp8_quantize(m1, ac, as, M, F, st, true);
       }
     }
   }
@@ -256,23 +261,21 @@ PyObject* finish(F&& fn) {
   return THPVariable_Wrap(std::move(*out));
 }
 
-// (tile_n, static_weights) of capi.gemm_config
-bool read_cfg(PyObject* tile_n, PyObject* static_weights, b200q_cfg& cfg) {
+// tile_n of capi.gemm_config
+bool read_cfg(PyObject* tile_n, b200q_cfg& cfg) {
   cfg = b200q_cfg{};
   const long t = PyLong_AsLong(tile_n);
   if (t == -1 && PyErr_Occurred()) return false;
-  const int s = PyObject_IsTrue(static_weights);
-  if (s < 0) return false;
   cfg.tile_n = static_cast<int32_t>(t);
-  cfg.static_weights = s;
+  cfg.static_weights = 1;     // holds behind a late quantize kernel
   return true;
 }
 
 PyObject* py_fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   b200q_cfg cfg;
-  TORCH_CHECK_VALUE(n == 7, "fp8_linear: 7 arguments expected");
-  if (!read_cfg(a[5], a[6], cfg)) return nullptr;
+  TORCH_CHECK_VALUE(n == 6, "fp8_linear: 6 arguments expected");
+  if (!read_cfg(a[5], cfg)) return nullptr;
   bool ok = plain(a[0]) && plain(a[1]) && plain(a[2]) && !modes_active();
   const Tensor *bias = optional_arg(a[3], ok), *amax = optional_arg(a[4], ok);
   if (!ok) Py_RETURN_NONE;
@@ -283,8 +286,8 @@ PyObject* py_fp8_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_nvfp4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   b200q_cfg cfg;
-  TORCH_CHECK_VALUE(n == 8, "nvfp4_linear: 8 arguments expected");
-  if (!read_cfg(a[6], a[7], cfg)) return nullptr;
+  TORCH_CHECK_VALUE(n == 7, "nvfp4_linear: 7 arguments expected");
+  if (!read_cfg(a[6], cfg)) return nullptr;
   bool ok = plain(a[0]) && plain(a[1]) && plain(a[2]) && plain(a[3]) && !modes_active();
   const Tensor *bias = optional_arg(a[4], ok), *amax = optional_arg(a[5], ok);
   if (!ok) Py_RETURN_NONE;
@@ -297,8 +300,8 @@ PyObject* py_nvfp4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_fp8_gated_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   b200q_cfg cfg;
-  TORCH_CHECK_VALUE(n == 9, "fp8_gated_mlp: 9 arguments expected");
-  if (!read_cfg(a[7], a[8], cfg)) return nullptr;
+  TORCH_CHECK_VALUE(n == 8, "fp8_gated_mlp: 8 arguments expected");
+  if (!read_cfg(a[7], cfg)) return nullptr;
   bool ok = plain(a[0]) && plain(a[1]) && plain(a[2]) && plain(a[3]) && plain(a[4]) && !modes_active();
   const Tensor *in_amax = optional_arg(a[5], ok), *act_amax = optional_arg(a[6], ok);
   if (!ok) Py_RETURN_NONE;
@@ -334,11 +337,11 @@ PyObject* py_fp8_sdpa(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyMethodDef methods[] = {
     {"fp8_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fp8_linear)), METH_FASTCALL,
-     "x, w_codes, w_scales, bias, x_amax, tile_n, static_weights -> bf16 tensor, or None: take the general path"},
+     "x, w_codes, w_scales, bias, x_amax, tile_n -> bf16 tensor, or None: take the general path"},
     {"nvfp4_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_nvfp4_linear)), METH_FASTCALL,
-     "x, w_codes, w_scales, w_global, bias, x_amax, tile_n, static_weights -> bf16 tensor or None"},
+     "x, w_codes, w_scales, w_global, bias, x_amax, tile_n -> bf16 tensor or None"},
     {"fp8_gated_mlp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fp8_gated_mlp)), METH_FASTCALL,
-     "x, gu_codes, gu_scales, down_codes, down_scales, input_amax, act_amax, tile_n, static_weights -> bf16 tensor or None"},
+     "x, gu_codes, gu_scales, down_codes, down_scales, input_amax, act_amax, tile_n -> bf16 tensor or None"},
     {"fp8_sdpa", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fp8_sdpa)), METH_FASTCALL,
      "q, k, v, amax_q, amax_k, amax_v, is_causal, scale -> tensor like q or None"},
     {nullptr, nullptr, 0, nullptr}};

@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "internal.h"
 
 namespace b200q {
 
@@ -43,9 +44,8 @@ enum class Out { Codes, Fake };
 template <typename T, int ITEMS, int AMAX_MODE, Out OUT>
 __global__ void __launch_bounds__(kRowThreads)
 fp8_rows_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ codes,
-                T* __restrict__ fake, float* __restrict__ scales, int64_t rows, int64_t cols) {
-  pdl_launch_dependents();
-  pdl_wait();
+                T* __restrict__ fake, float* __restrict__ scales, int64_t rows, int64_t cols, bool late) {
+  pdl_enter(late);
   __shared__ float red[kRowThreads / 32];
   const int64_t row = blockIdx.x;
   const T* xr = x + row * cols;
@@ -139,11 +139,11 @@ fp8_rows_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t
 
 template <typename T, int AMAX_MODE, Out OUT>
 int launch_rows_items(const T* x, const float* amax, uint8_t* codes, T* fake, float* scales, int64_t rows,
-                      int64_t cols, cudaStream_t st) {
+                      int64_t cols, cudaStream_t st, bool late) {
   const int64_t groups = cols >> 3;
   const int items = static_cast<int>((groups + kRowThreads - 1) / kRowThreads);
   dim3 grid(static_cast<unsigned>(rows)), block(kRowThreads);
-#define B200Q_ROWS(I) launch_pdl(fp8_rows_kernel<T, I, AMAX_MODE, OUT>, grid, block, 0, st, x, amax, codes, fake, scales, rows, cols)
+#define B200Q_ROWS(I) launch_pdl(fp8_rows_kernel<T, I, AMAX_MODE, OUT>, grid, block, 0, st, x, amax, codes, fake, scales, rows, cols, late)
   if (items <= 1) B200Q_ROWS(1);
   else if (items <= 2) B200Q_ROWS(2);
   else if (items <= 4) B200Q_ROWS(4);
@@ -155,7 +155,7 @@ int launch_rows_items(const T* x, const float* amax, uint8_t* codes, T* fake, fl
 
 template <typename T, Out OUT>
 int launch_rows(const void* x, const float* amax, int64_t amax_numel, uint8_t* codes, void* fake, float* scales,
-                int64_t rows, int64_t cols, cudaStream_t st) {
+                int64_t rows, int64_t cols, cudaStream_t st, bool late = false) {
   const T* xt = static_cast<const T*>(x);
   T* ft = static_cast<T*>(fake);
   if (amax_numel == 0) {
@@ -164,10 +164,10 @@ int launch_rows(const void* x, const float* amax, int64_t amax_numel, uint8_t* c
       const int rc = launch_fp8_rows_stream(xt, codes, scales, rows, cols, st);
       if (rc != 1) return rc;
     }
-    return launch_rows_items<T, 0, OUT>(xt, amax, codes, ft, scales, rows, cols, st);
+    return launch_rows_items<T, 0, OUT>(xt, amax, codes, ft, scales, rows, cols, st, late);
   }
-  if (amax_numel == 1) return launch_rows_items<T, 1, OUT>(xt, amax, codes, ft, scales, rows, cols, st);
-  return launch_rows_items<T, 2, OUT>(xt, amax, codes, ft, scales, rows, cols, st);
+  if (amax_numel == 1) return launch_rows_items<T, 1, OUT>(xt, amax, codes, ft, scales, rows, cols, st, late);
+  return launch_rows_items<T, 2, OUT>(xt, amax, codes, ft, scales, rows, cols, st, late);
 }
 
 int validate_rows(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, int64_t amax_numel,
@@ -446,6 +446,20 @@ int launch_amax_static(const void* x, int dtype, int64_t n, float* out, float* p
 }
 }  // namespace
 
+int fp8_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, int64_t amax_numel,
+                       uint8_t* codes_out, float* scales_out, b200q_stream_t stream, bool late) {
+  if (int rc = validate_rows(x, dtype, rows, cols, amax, amax_numel, codes_out, 16)) return rc;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  if (amax_numel != 1 && scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case B200Q_BF16: return launch_rows<__nv_bfloat16, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st, late);
+    case B200Q_F16: return launch_rows<__half, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st, late);
+    default: return launch_rows<float, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st, late);
+  }
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -511,16 +525,7 @@ int b200q_row_amax(const void* x, int dtype, int64_t rows, int64_t cols, float* 
 
 int b200q_fp8_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, int64_t amax_numel,
                        uint8_t* codes_out, float* scales_out, b200q_stream_t stream) {
-  if (int rc = validate_rows(x, dtype, rows, cols, amax, amax_numel, codes_out, 16)) return rc;
-  if (rows == 0 || cols == 0) return B200Q_OK;
-  if (amax_numel != 1 && scales_out == nullptr) return B200Q_ERR_INVALID;
-  if (int rc = check_arch()) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (dtype) {
-    case B200Q_BF16: return launch_rows<__nv_bfloat16, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st);
-    case B200Q_F16: return launch_rows<__half, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st);
-    default: return launch_rows<float, Out::Codes>(x, amax, amax_numel, codes_out, nullptr, scales_out, rows, cols, st);
-  }
+  return fp8_quantize(x, dtype, rows, cols, amax, amax_numel, codes_out, scales_out, stream, false);
 }
 
 int b200q_fp8_fake_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax,

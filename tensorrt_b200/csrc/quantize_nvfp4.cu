@@ -18,6 +18,7 @@
 //   s_blk  = e4m3_rne(min((amax_blk / 6) / global, 448));  d = fp32(s_blk) * global
 //   code   = e2m1_rne_sat(x_fp32 / d); all codes of a block with s_blk == 0 are 0
 //   x_hat  = e2m1 * d, rounded (RNE) to the input dtype.
+#include "internal.h"
 #include "nvfp4_block.cuh"
 
 namespace b200q {
@@ -105,9 +106,8 @@ template <typename T, bool FAKE, int U, Src SRC>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_quantize_kernel(const T* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ codes,
                       uint8_t* __restrict__ sf, T* __restrict__ fake, float* __restrict__ gout, uint32_t rows, uint32_t cols,
-                      uint32_t blocks_per_row, uint32_t col_tiles, const ExpandMap map) {
-  pdl_launch_dependents();
-  pdl_wait();
+                      uint32_t blocks_per_row, uint32_t col_tiles, const ExpandMap map, bool late) {
+  pdl_enter(late);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t row = blockIdx.x;
   if constexpr (!FAKE) {
@@ -185,10 +185,9 @@ constexpr int64_t kDynamicMaxElems = 1 << 17;
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_quantize_dynamic_kernel(const T* __restrict__ x, uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, float* __restrict__ gout,
-                              uint32_t rows, uint32_t cols, uint32_t blocks_per_row, uint32_t col_tiles, uint32_t units) {
+                              uint32_t rows, uint32_t cols, uint32_t blocks_per_row, uint32_t col_tiles, uint32_t units, bool late) {
   __shared__ float red[kThreads / 32];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_enter(late);
   const uint32_t unit = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t row = unit / (col_tiles * 4u), blk = unit - row * (col_tiles * 4u);
   const bool live = row < rows && blk < blocks_per_row;
@@ -233,11 +232,11 @@ nvfp4_quantize_dynamic_kernel(const T* __restrict__ x, uint8_t* __restrict__ cod
 }
 
 template <typename T>
-int launch_dynamic(const void* x, uint8_t* codes, uint8_t* sf, float* gout, int64_t rows, int64_t cols, cudaStream_t st) {
+int launch_dynamic(const void* x, uint8_t* codes, uint8_t* sf, float* gout, int64_t rows, int64_t cols, cudaStream_t st, bool late) {
   const uint32_t bpr = static_cast<uint32_t>(cols >> 4), col_tiles = (bpr + 3u) >> 2;
   const uint32_t units = static_cast<uint32_t>((rows + 127) / 128 * 128) * col_tiles * 4u;   // rows <= 8192, bpr <= 8192: < 2^26
   launch_pdl(nvfp4_quantize_dynamic_kernel<T>, dim3((units + kThreads - 1) / kThreads), dim3(kThreads), 0, st, static_cast<const T*>(x), codes,
-             sf, gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), bpr, col_tiles, units);
+             sf, gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), bpr, col_tiles, units, late);
   return check_launch();
 }
 
@@ -268,7 +267,7 @@ nvfp4_dequantize_kernel(const uint8_t* __restrict__ codes, const uint8_t* __rest
 
 template <typename T, bool FAKE, Src SRC = Src::kPlain>
 int launch(const void* x, const float* amax, uint8_t* codes, uint8_t* sf, void* fake, float* gout, int64_t rows,
-           int64_t cols, cudaStream_t st, const ExpandMap& map = ExpandMap{}) {
+           int64_t cols, cudaStream_t st, const ExpandMap& map = ExpandMap{}, bool late = false) {
   constexpr int U = sizeof(T) == 4 || SRC == Src::kSiluMul ? 2 : 4;  // 128 bytes of loads in flight per lane
   const uint32_t blocks_per_row = static_cast<uint32_t>(cols >> 4);
   const uint32_t spans_per_row = (blocks_per_row + 31u) >> 5;
@@ -287,7 +286,7 @@ int launch(const void* x, const float* amax, uint8_t* codes, uint8_t* sf, void* 
   }
   dim3 grid(static_cast<unsigned>(grid_rows), chunks), block(warps * 32u);
   launch_pdl(nvfp4_quantize_kernel<T, FAKE, U, SRC>, grid, block, 0, st, static_cast<const T*>(x), amax, codes, sf, static_cast<T*>(fake),
-             gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), blocks_per_row, (blocks_per_row + 3u) >> 2, map);
+             gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), blocks_per_row, (blocks_per_row + 3u) >> 2, map, late);
   return check_launch();
 }
 
@@ -302,6 +301,44 @@ int validate(const void* x, int dtype, int64_t rows, int64_t cols, const float* 
 }
 
 }  // namespace
+int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, uint8_t* codes_out,
+                         uint8_t* scales_out, float* global_scale_out, b200q_stream_t stream, bool late) {
+  if (int rc = validate(x, dtype, rows, cols, amax)) return rc;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case B200Q_BF16: return launch<__nv_bfloat16, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st, ExpandMap{}, late);
+    case B200Q_F16: return launch<__half, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st, ExpandMap{}, late);
+    default: return launch<float, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st, ExpandMap{}, late);
+  }
+}
+
+int nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
+                                 float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream, bool late) {
+  if (int rc = validate(x, dtype, rows, cols, reinterpret_cast<const float*>(x))) return rc;
+  if (rows == 0 || cols == 0) return B200Q_OK;
+  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
+  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
+  const size_t need = b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols);
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need)) return B200Q_ERR_WORKSPACE;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (need == 0) {
+    switch (dtype) {
+      case B200Q_BF16: return launch_dynamic<__nv_bfloat16>(x, codes_out, scales_out, global_scale_out, rows, cols, st, late);
+      case B200Q_F16: return launch_dynamic<__half>(x, codes_out, scales_out, global_scale_out, rows, cols, st, late);
+      default: return launch_dynamic<float>(x, codes_out, scales_out, global_scale_out, rows, cols, st, late);
+    }
+  }
+  float* amax = static_cast<float*>(workspace) + 2;      // behind the two words that the abs-max kernel keeps
+  if (int rc = b200q_amax(x, dtype, rows * cols, amax, workspace, workspace_bytes, stream)) return rc;
+  return nvfp4_quantize(x, dtype, rows, cols, amax, codes_out, scales_out, global_scale_out, stream, late);
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -316,18 +353,7 @@ size_t b200q_nvfp4_scale_bytes(int64_t rows, int64_t cols) {
 
 int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, uint8_t* codes_out,
                          uint8_t* scales_out, float* global_scale_out, b200q_stream_t stream) {
-  if (int rc = validate(x, dtype, rows, cols, amax)) return rc;
-  if (rows == 0 || cols == 0) return B200Q_OK;
-  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
-  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
-  if (int rc = check_arch()) return rc;
-  if (rows == 0 || cols == 0) return B200Q_OK;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (dtype) {
-    case B200Q_BF16: return launch<__nv_bfloat16, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
-    case B200Q_F16: return launch<__half, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
-    default: return launch<float, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st);
-  }
+  return nvfp4_quantize(x, dtype, rows, cols, amax, codes_out, scales_out, global_scale_out, stream, false);
 }
 
 size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols) {
@@ -336,24 +362,7 @@ size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols) 
 
 int b200q_nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
                                  float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream) {
-  if (int rc = validate(x, dtype, rows, cols, reinterpret_cast<const float*>(x))) return rc;
-  if (rows == 0 || cols == 0) return B200Q_OK;
-  if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
-  if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
-  const size_t need = b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols);
-  if (need > 0 && (workspace == nullptr || workspace_bytes < need)) return B200Q_ERR_WORKSPACE;
-  if (int rc = check_arch()) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (need == 0) {
-    switch (dtype) {
-      case B200Q_BF16: return launch_dynamic<__nv_bfloat16>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
-      case B200Q_F16: return launch_dynamic<__half>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
-      default: return launch_dynamic<float>(x, codes_out, scales_out, global_scale_out, rows, cols, st);
-    }
-  }
-  float* amax = static_cast<float*>(workspace) + 2;      // behind the two words that the abs-max kernel keeps
-  if (int rc = b200q_amax(x, dtype, rows * cols, amax, workspace, workspace_bytes, stream)) return rc;
-  return b200q_nvfp4_quantize(x, dtype, rows, cols, amax, codes_out, scales_out, global_scale_out, stream);
+  return nvfp4_quantize_dynamic(x, dtype, rows, cols, codes_out, scales_out, global_scale_out, workspace, workspace_bytes, stream, false);
 }
 
 int b200q_silu_mul_nvfp4_quantize(const void* gate_up, const float* amax, uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out,

@@ -17,7 +17,7 @@ from . import _native, capi
 def fp8_linear(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor, bias=None,
                x_amax: torch.Tensor | None = None) -> torch.Tensor:
     """Per-token (dynamic, or `x_amax` static) FP8 activations x per-channel/per-tensor FP8 weights."""
-    y = _native.fp8_linear(x, w_codes, w_scales, bias, x_amax, *capi.gemm_defaults())
+    y = _native.fp8_linear(x, w_codes, w_scales, bias, x_amax, capi.gemm_defaults()[0])
     if y is not None:
         return y
     x_codes, x_scales = capi.fp8_quantize(x, x_amax)
@@ -27,7 +27,7 @@ def fp8_linear(x: torch.Tensor, w_codes: torch.Tensor, w_scales: torch.Tensor, b
 def nvfp4_linear(x: torch.Tensor, w_codes, w_scales, w_global, bias=None,
                  x_amax: torch.Tensor | None = None) -> torch.Tensor:
     """NVFP4 W4A4.  `x_amax` is the activation tensor amax (static calibration); None = measured per call."""
-    y = _native.nvfp4_linear(x, w_codes, w_scales, w_global, bias, x_amax, *capi.gemm_defaults())
+    y = _native.nvfp4_linear(x, w_codes, w_scales, w_global, bias, x_amax, capi.gemm_defaults()[0])
     if y is not None:
         return y
     x_codes, x_scales, x_global = capi.nvfp4_quantize_dynamic(x) if x_amax is None else capi.nvfp4_quantize(x, x_amax)
@@ -91,7 +91,7 @@ class Fp8GatedMlp(nn.Module):
 
     def forward(self, x):
         y = _native.fp8_gated_mlp(x, self.gu_codes, self.gu_scales, self.down_codes, self.down_scales, self.input_amax, self.act_amax,
-                                  *capi.gemm_defaults())
+                                  capi.gemm_defaults()[0])
         if y is not None:
             return y
         xq = capi.fp8_quantize(x, self.input_amax)
