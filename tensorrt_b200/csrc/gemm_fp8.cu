@@ -4,6 +4,7 @@
 #include <mutex>
 
 #include "gemm_host.cuh"
+#include "internal.h"
 
 namespace b200q {
 namespace gemm {
@@ -58,6 +59,42 @@ int forced_smallm_stages() {
 }
 
 }  // namespace gemm
+}  // namespace b200q
+
+namespace b200q {
+
+// One launch for tokens few enough that every CTA can find their abs-max itself: at most 16 tokens and 65536 elements
+// (128 KB of 16-bit values read from L2 per CTA, about 1 us; the separate quantize launch costs 2 us on the device and
+// as much on the host).
+int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,
+                     int64_t w_scales_numel, const void* bias, void* out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream) {
+  if (M <= 0 || M > 16 || N <= 0 || K <= 0 || M * K > 65536 || K % 16 != 0 || N > 0x7fffffffLL) return 1;
+  if (!aligned(x, 16) || !aligned(w, 16) || !aligned(out, 16)) return 1;
+  if (int rc = check_arch()) return rc;
+  gemm::Params p{};
+  p.status = gemm::device_status_word();
+  if (p.status == nullptr) return B200Q_ERR_CUDA;
+  p.x = x;
+  p.x_amax = amax;
+  p.x_amax_numel = static_cast<int>(amax_numel);
+  p.b_scales = w_scales;
+  p.b_scale_stride = w_scales_numel == 1 ? 0 : 1;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.M = static_cast<int>(M);
+  p.N = static_cast<int>(N);
+  p.k_bytes = static_cast<int>(K);
+  const int k_tiles = (p.k_bytes + gemm::kBKBytes - 1) / gemm::kBKBytes;
+  const int splits = gemm::smallm_splits((p.N + gemm::kSmallWRows - 1) / gemm::kSmallWRows, k_tiles, sm_count(), p.M);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (dtype) {
+    case B200Q_BF16: return gemm::launch_smallm_own_x<__nv_bfloat16>(w, p, st, splits);
+    case B200Q_F16: return gemm::launch_smallm_own_x<__half>(w, p, st, splits);
+    case B200Q_F32: return gemm::launch_smallm_own_x<float>(w, p, st, splits);
+    default: return 1;
+  }
+}
+
 }  // namespace b200q
 
 using namespace b200q;

@@ -256,6 +256,51 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
   return B200Q_OK;
 }
 
+// The small-M kernel that quantizes its activation (FP8, M <= 16; p.x, p.x_amax set).  Returns 1 when the problem does
+// not qualify.
+template <typename XT>
+int launch_smallm_own_x(const uint8_t* b, Params p, cudaStream_t st, int splits) {
+  using C = SmallCfg<false>;
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(gemm_smallm_kernel<false, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess)
+      return B200Q_ERR_CUDA;
+    configured[dev] = true;
+  }
+  const int tiles = (p.N + kSmallWRows - 1) / kSmallWRows;
+  const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
+  const int per = (k_tiles + splits - 1) / splits;
+  const int fixed = 1024 + kSmallTailBytes + per * 2048;
+  const int budget = tiles * splits > sm_count() ? kSmallHalfSmem : kSmemLimit;
+  int stages = (budget - fixed) / C::kWBytes;
+  if (stages > kSmallMaxStages) stages = kSmallMaxStages;
+  if (stages > per) stages = per < 2 ? 2 : per;
+  if (stages < 2) return 1;
+  CUtensorMap tw;
+  if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(fixed + stages * C::kWBytes);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<false, XT>, tw, tw, p, splits, stages, 16) != cudaSuccess) {
+    cudaGetLastError();
+    return B200Q_ERR_CUDA;
+  }
+  return B200Q_OK;
+}
+
 // Cluster size of the small-M kernel.  Measured: one SM pulls about 60 bytes per nanosecond
 // through TMA whatever the ring depth, so about 110 streaming SMs are needed to saturate HBM;
 // the smallest power of two that reaches that many CTAs wins, larger clusters only add

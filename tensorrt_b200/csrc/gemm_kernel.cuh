@@ -90,6 +90,9 @@ struct Params {
   int static_weights;      // small-M kernel under programmatic dependent launch: 1 = B (weights, their scales, bias) was
                            // written before the preceding kernel on the stream started, so it may be read before
                            // waiting for that kernel; 0 = wait first
+  const void* x;           // small-M kernel that quantizes its activation: x [M, k_bytes] and its amax (x_amax_numel values:
+  const float* x_amax;     // 0 = per-token abs-max measured by the kernel, 1 = per tensor, M = per token)
+  int x_amax_numel;
   int silu_f;              // FP8 CTA-pair kernel, > 0: B holds F gate rows then F up rows (N = 2 F); the epilogue
                            // writes out[M, F] = silu(gate) * up, each linear output rounded to bf16 first
   const float* act_amax;   // quantizing form of the above: static per-tensor abs-max of the activation; `out` then

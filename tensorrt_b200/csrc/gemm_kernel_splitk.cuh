@@ -13,7 +13,14 @@
 //     a cluster barrier CTA r sums the tokens it owns over all S partials with 16-byte
 //     ld.shared::cluster loads, applies the dequantization scales and the bias and stores
 //     bf16 rows.  No global workspace, no atomics, fixed summation order.
+//
+// XT != void (FP8, M <= 16, short rows): the kernel also quantizes the activation.  Four warps read x, find every
+// token's abs-max (each CTA for itself: the rows are a few KB in L2) and write the codes of the CTA's K slice
+// into shared memory in the operand layout while the weight ring fills.  One launch instead of two; codes, scales
+// and sums are those of the quantize kernel followed by the plain form.
 #pragma once
+
+#include <type_traits>
 
 #include "gemm_kernel.cuh"
 
@@ -97,23 +104,90 @@ __device__ __forceinline__ void small_reduce_store(uint32_t partial_u32, int t0,
   }
 }
 
+// FP8 codes of K tiles [kt0, kt1) of x [M, k] into `xs` ([K tile][16 rows][128 bytes], 128-byte swizzle, rows M..15 zero)
+// and the scale of every token into `xscale`; by 128 threads (t), barrier 1.
+template <typename T>
+__device__ __forceinline__ void small_quantize_x(const Params& p, uint8_t* xs, float* xscale, int kt0, int kt1, int t) {
+  const T* x = static_cast<const T*>(p.x);
+  const int k = p.k_bytes, warp = t >> 5, lane = t & 31;
+  const int pieces = k >> 4;                                   // 16-element pieces of a row (k % 16 == 0)
+  for (int tok = warp; tok < p.M; tok += 4) {                  // a warp takes whole tokens
+    float a = 0.0f;
+    if (p.x_amax_numel == 0) {
+      const T* row = x + static_cast<int64_t>(tok) * k;
+      for (int g0 = lane; g0 < pieces; g0 += 32 * 4) {
+        Raw16<T, false> raw[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (g0 + u * 32 < pieces) raw[u].load(row + (g0 + u * 32) * 16);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (g0 + u * 32 < pieces) {
+            float v[16];
+            raw[u].widen(v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) a = fmaxf(a, fabsf(v[i]));
+          }
+      }
+      a = warp_max(a);
+    } else {
+      a = ld_dependent(p.x_amax + (p.x_amax_numel == 1 ? 0 : tok));
+    }
+    if (lane == 0) xscale[tok] = fp8_scale_from_amax(a);
+  }
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  const int items = (kt1 - kt0) * 16 * 8;                      // 16-byte pieces of the operand tiles
+  for (int i = t; i < items; i += 128) {
+    const int kt = i >> 7, row = (i >> 3) & 15, piece = i & 7;
+    const int g = (kt0 + kt) * 8 + piece;
+    uint4 c = make_uint4(0u, 0u, 0u, 0u);
+    if (row < p.M && g < pieces) {
+      const float scale = xscale[row], y = b200q_rcp_rn(scale), lim = __fmul_rn(scale, 512.0f);
+      const bool fast = b200q_div_fast_ok(scale);
+      Raw16<T, false> raw;
+      raw.load(x + static_cast<int64_t>(row) * k + g * 16);
+      float v[16];
+      raw.widen(v);
+      uint32_t* w = &c.x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float q[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float f = v[4 * j + e];
+          q[e] = !fast ? div_path<kDivTrue>(f, scale, y, lim)
+                       : (p.x_amax_numel == 0 ? div_path<kDivFast>(f, scale, y, lim) : div_path<kDivClamped>(f, scale, y, lim));
+        }
+        w[j] = f32x2_to_e4m3x2(q[0], q[1]) | (f32x2_to_e4m3x2(q[2], q[3]) << 16);
+      }
+    }
+    *reinterpret_cast<uint4*>(xs + kt * 2048 + row * 128 + ((piece ^ (row & 7)) * 16)) = c;
+  }
+  ptx::fence_proxy_async();                                    // the tensor core reads the tiles through the async proxy
+}
+
 // tmap_w: weights [N, k_bytes], box 128 rows; tmap_x: activations [M, k_bytes], box `bt` rows
 // (bt = M rounded up to 16).  `splits` = cluster size, `stages` = depth of the operand ring.
-template <bool NVF4>
+template <bool NVF4, typename XT = void>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const Params p,
                    const int splits, const int stages, const int bt) {
   using C = SmallCfg<NVF4>;
+  constexpr bool kOwnX = !std::is_void<XT>::value;       // the kernel quantizes the activation itself
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int stage_bytes = C::stage_bytes(bt);
-  const int x_bytes = bt * kBKBytes;
-  uint8_t* tail = smem + stages * stage_bytes;
+  const int x_bytes = kOwnX ? 0 : bt * kBKBytes;         // activation bytes of a ring stage
+  const int stage_bytes = kOwnX ? C::kWBytes : C::stage_bytes(bt);
+  const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
+  const int per = (k_tiles + splits - 1) / splits;
+  uint8_t* own_x = smem + stages * stage_bytes;          // kOwnX: [per][16 rows][128 bytes] codes of this CTA's K slice
+  uint8_t* tail = own_x + (kOwnX ? per * 2048 : 0);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(tail);
   uint64_t* empty_bar = full_bar + kSmallMaxStages;
   uint64_t* acc_full = empty_bar + kSmallMaxStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tail + 256);
   volatile int* failed = reinterpret_cast<volatile int*>(tail + 260);
+  uint64_t* x_full = reinterpret_cast<uint64_t*>(tail + 272);     // kOwnX: the codes are in shared memory (4 warps)
   uint64_t* sft_full = reinterpret_cast<uint64_t*>(tail + 384);   // NVFP4: a stage's scales are in tensor memory (4 warps)
   float* wscale = reinterpret_cast<float*>(tail + 512);   // [128] dequantization scale of each weight row
   float* wbias = wscale + 128;                            // [128]
@@ -123,8 +197,6 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int rank = static_cast<int>(ptx::cluster_ctarank());
   const int nb = blockIdx.x / splits;                     // one cluster per tile of 128 weight rows
   const int n_base = nb * kSmallWRows;
-  const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
-  const int per = (k_tiles + splits - 1) / splits;
   const int kt0 = min(rank * per, k_tiles), kt1 = min(kt0 + per, k_tiles);
   const uint32_t tmem_cols = static_cast<uint32_t>(C::tmem_cols(stages));
 
@@ -135,10 +207,11 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       ptx::mbar_init(sft_full + s, 4);
     }
     ptx::mbar_init(acc_full, 1);
+    if constexpr (kOwnX) ptx::mbar_init(x_full, 4);
     *failed = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&tmap_w);
-    ptx::prefetch_tmap(&tmap_x);
+    if constexpr (!kOwnX) ptx::prefetch_tmap(&tmap_x);
   }
   if (warp == 1) {
     ptx::tmem_alloc<1>(tmem_holder, tmem_cols);
@@ -169,6 +242,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       if constexpr (NVF4) ptx::bulk_load(sw + C::kWBytes + x_bytes, sfw_src + kt * 2048, sfb, full_bar + stage);
     };
     auto issue_x = [&](int kt, int stage) {
+      if constexpr (kOwnX) return;
       uint8_t* sx = smem + stage * stage_bytes + C::kWBytes;
       ptx::tma_load_2d(sx, &tmap_x, full_bar + stage, kt * kBKBytes, 0);
       if constexpr (NVF4) ptx::bulk_load(sx + x_bytes + 2048, sfx_src + kt * 2048, sf_bytes_of(kt), full_bar + stage);
@@ -203,7 +277,14 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int kt = kt0; kt < kt1; ++kt) {
+    if constexpr (kOwnX) {
+      if (kt1 > kt0 && !ptx::mbar_wait(x_full, 0)) {
+        raise_timeout(p.status, 35);
+        *failed = 1;
+        ok = false;
+      }
+    }
+    for (int kt = kt0; kt < kt1 && ok; ++kt) {
       if (!ptx::mbar_wait(full_bar + stage, phase)) {
         raise_timeout(p.status, 32);
         *failed = 1;
@@ -212,7 +293,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
       ptx::tc_fence_after();
       const uint32_t sw = smem_u + stage * stage_bytes;
-      const uint32_t w_lo = ptx::desc_lo_sw128(sw), x_lo = w_lo + (C::kWBytes >> 4);
+      const uint32_t w_lo = ptx::desc_lo_sw128(sw);
+      const uint32_t x_lo = kOwnX ? ptx::desc_lo_sw128(ptx::smem_u32(own_x) + (kt - kt0) * 2048) : w_lo + (C::kWBytes >> 4);
       const uint32_t tmem_sfw = tmem_base + 128 + stage * C::kSfCols, tmem_sfx = tmem_sfw + 16;
       int kblocks = 4;
       if constexpr (NVF4) {
@@ -253,13 +335,18 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (p.bias != nullptr) wb = __bfloat162float(p.bias[n]);
       }
       pdl_wait();  // the activation scales come from the kernel before this one
-      if (wrow < p.M) {
+      if (wrow < p.M && !kOwnX) {
         if constexpr (NVF4) xs = __fmul_rn(ld_dependent(p.a_scales), ld_dependent(p.b_scales));
         else xs = ld_dependent(p.a_scales + static_cast<int64_t>(wrow) * p.a_scale_stride);
       }
       wscale[wrow] = ws;
       wbias[wrow] = wb;
-      xscale[wrow] = xs;
+      if constexpr (!kOwnX) xscale[wrow] = xs;
+    }
+    if constexpr (kOwnX) {
+      small_quantize_x<XT>(p, own_x, xscale, kt0, kt1, threadIdx.x - 64);
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(x_full);
     }
     if constexpr (NVF4) {
       // main loop: shared memory -> tensor memory for the scale tiles of every stage.  Lane l of each

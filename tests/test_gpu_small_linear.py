@@ -1,0 +1,25 @@
+"""FP8 linear of a few tokens in one launch (the GEMM quantizes its activation): the same bits as the quantize kernel
+followed by the GEMM, for every way of scaling, at the edges of its range (tokens, row length, K slices of a cluster,
+ragged N and K) and just outside it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (1, 128, 16), (1, 130, 144), (2, 1000, 2064), (7, 257, 1040), (16, 4096, 4096), (16, 8192, 4112),
+                                   (15, 384, 4368), (9, 512, 7280), (1, 1024, 28672), (2, 28672, 32768), (1, 136, 65536), (17, 256, 1024)])
+def test_same_bits_as_two_launches(b200, m, n, k, dtype):
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n + k)
+    x = torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    w, ws = capi.fp8_quantize((torch.randn(n, k, device="cuda", generator=g) * 0.02).bfloat16(), None)
+    bias = torch.randn(n, device="cuda", generator=g).bfloat16()
+    per_token = x.abs().amax(dim=1).float() * 0.5                          # some elements saturate
+    for amax, b in ((None, None), (x.abs().max().float(), bias), (per_token, bias), (torch.zeros((), device="cuda"), None)):
+        xq, xs = capi.fp8_quantize(x, amax)
+        ref = capi.fp8_gemm(xq, xs, w, ws, b)
+        assert torch.equal(b200.fp8_linear(x, w, ws, b, amax), ref)
+    assert torch.equal(b200.fp8_linear(torch.zeros_like(x), w, ws), torch.zeros(m, n, device="cuda", dtype=torch.bfloat16))
+    assert capi.device_status() == 0
