@@ -420,7 +420,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 // (keys contiguous, zero beyond S).  The inputs may be strided (D contiguous): a token-major [tokens, heads * D] slice
 // of a QKV projection is read where it lies.  HBM-bound (3 bytes per 16-bit element); a CTA takes 128 rows of one
 // head, 16 elements per thread and step with four steps of loads in flight.  Before, Q and K went through the
-// row kernels, one CTA per row of D elements: at [4, 32, 2048, 128] 262144 CTAs of which 16 threads had work.
+// row kernels, one CTA per row of D elements (at [4, 32, 2048, 128] 262144 CTAs of which 16 threads had work), and V through a
+// byte-wise transpose: 355 us for the three operands of [4, 32 / 8, 2048, 128] bf16, 42 us here (3.6 TB/s).
 struct QkvPart {
   const void* x;
   int64_t sb, sh, ss;        // strides of batch, head, row in elements

@@ -92,6 +92,8 @@ struct Block16<float> {
 //                   silu_mul_kernel stores it: the activation in front of the down projection is never written
 //   Src::kExpand    column c of the output is column src_col0 + (c / hd / rep) * hd + c % hd of a row of src_stride
 //                   elements (every kv head repeated `rep` times): the expanded tensor is never written
+// Measured at [8192, 14336] bf16: kSiluMul 146 us (3.7 TB/s; issue slots: about 17 instructions an element) against 114 for
+// silu_mul_kernel and 55 for the plain form behind it.
 enum class Src { kPlain, kSiluMul, kExpand };
 struct ExpandMap {
   int64_t src_stride, src_col0;
