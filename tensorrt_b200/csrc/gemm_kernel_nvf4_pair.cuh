@@ -290,7 +290,8 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int half = (warp - 8) >> 2;       // which 128 of the 256 accumulator columns
     uint32_t acc_phase = 0;
     const float gscale = __fmul_rn(__ldg(p.a_scales), __ldg(p.b_scales));
-    const bool vec32 = (p.N % 16) == 0, vec16 = (p.N % 8) == 0;
+    // 32-byte stores need rows and base on 32-byte boundaries; the entry point asks for a 16-byte aligned output only
+    const bool vec32 = (p.N % 16) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0, vec16 = (p.N % 8) == 0;
     for (int t = pair; t < num_tiles; t += num_pairs) {
       int mb, nb;
       tile_coord(t, mb, nb);

@@ -21,3 +21,17 @@ def test_choice(b200, m, n, k):
     for gemm, ops in ((capi.fp8_gemm, fp8), (capi.nvfp4_gemm, nv)):
         assert o.rel_l2(gemm(*ops, bias).float(), gemm(*ops, bias, tile_n=128).float()) <= 2.0 ** -9
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n", [(300, 4096), (600, 4104), (129, 1001)])
+def test_output_on_a_16_byte_boundary(b200, m, n):
+    """`out` may start on any 16-byte boundary, whichever kernel is chosen."""
+    capi, k = b200.capi, 256
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    fp8 = (*capi.fp8_quantize(x), *capi.fp8_quantize(w))
+    nv = (*capi.nvfp4_quantize(x, capi.amax(x)), *capi.nvfp4_quantize(w, capi.amax(w)))
+    for gemm, ops in ((capi.fp8_gemm, fp8), (capi.nvfp4_gemm, nv)):
+        out = torch.empty(m * n + 8, device="cuda", dtype=torch.bfloat16)[8:].view(m, n)
+        assert out.data_ptr() % 32 == 16
+        gemm(*ops, out=out)
+        assert torch.equal(out, gemm(*ops))
