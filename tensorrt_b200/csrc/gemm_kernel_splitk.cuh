@@ -331,7 +331,9 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       float ws = 1.0f, wb = 0.0f, xs = 0.0f;
       if (!p.static_weights) pdl_wait();
       if (n < p.N) {
-        if constexpr (!NVF4) ws = __ldg(p.b_scales + static_cast<int64_t>(n) * p.b_scale_stride);
+        // without the promise they may come from the kernel before this one (the one-launch form never has it): loads
+        // that the compiler keeps behind the wait above (the bias is a plain load, held by the wait's memory clobber)
+        if constexpr (!NVF4) ws = ld_dependent(p.b_scales + static_cast<int64_t>(n) * p.b_scale_stride);
         if (p.bias != nullptr) wb = __bfloat162float(p.bias[n]);
       }
       pdl_wait();  // the activation scales come from the kernel before this one

@@ -79,6 +79,38 @@ def test_weights_written_just_before_the_call(b200):
             assert torch.equal(y, refs[i & 1])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("m", [1, 2, 7, 16, 40])
+def test_scales_and_bias_written_just_before_the_call(b200, m, dtype):
+    """The same for the weight scales alone (the weights doubled: equal codes, other scales), for the bias, and for every
+    part of an NVFP4 weight; m <= 16 FP8 tokens are one launch directly behind the writing kernel."""
+    from tensorrt_b200 import _lib
+
+    capi, lib, n, k = b200.capi, _lib.load(), 4096, 2048
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.02).bfloat16()
+    ws, x = [w, w * 2], torch.randn(m, k, device="cuda", generator=g).to(dtype)
+    zero, biases = torch.zeros(n, device="cuda").bfloat16(), [torch.randn(n, device="cuda", generator=g).bfloat16() for _ in range(2)]
+    bias, st = biases[0].clone(), torch.cuda.current_stream().cuda_stream
+    (codes, scales), (nc, ns, ng) = capi.fp8_quantize(w, None), capi.nvfp4_quantize(w, capi.amax(w))
+    amax = [capi.amax(t).reshape(1) for t in ws]
+    quant = [(capi.fp8_quantize(t, None), capi.nvfp4_quantize(t, a)) for t, a in zip(ws, amax)]
+    assert torch.equal(quant[0][0][0], quant[1][0][0]) and not torch.equal(quant[0][0][1], quant[1][0][1])
+    refs = []
+    for (f8, nv), b in zip(quant, biases):
+        refs.append((_fp8_steps(capi, x, *f8, b, None), capi.nvfp4_gemm(*capi.nvfp4_quantize(x, capi.amax(x)), *nv, b)))
+    torch.cuda.synchronize()
+    for i in range(10):
+        f8_ref, nv_ref = refs[i & 1]
+        assert lib.b200q_fp8_quantize(ws[i & 1].data_ptr(), 2, n, k, None, 0, codes.data_ptr(), scales.data_ptr(), st) == 0
+        y_scales = b200.fp8_linear(x, codes, scales, biases[i & 1])
+        capi.add(biases[i & 1], zero, out=bias)
+        y_bias = b200.fp8_linear(x, codes, scales, bias)
+        assert lib.b200q_nvfp4_quantize(ws[i & 1].data_ptr(), 2, n, k, amax[i & 1].data_ptr(), nc.data_ptr(), ns.data_ptr(), ng.data_ptr(), st) == 0
+        y_nv = b200.nvfp4_linear(x, nc, ns, ng, biases[i & 1])
+        assert torch.equal(y_scales, f8_ref) and torch.equal(y_bias, f8_ref) and torch.equal(y_nv, nv_ref)
+
+
 def test_sdpa(b200):
     from tensorrt_b200 import _native
 

@@ -322,3 +322,17 @@ def test_validation_of_the_fused_gate_up_gemm_without_a_device(b200):
     assert g(p, p, 1, p, p, 1, None, None, p, p, 256, 256, 64, None, None) == -1     # the static amax is required
     assert g(p, p, 1, p, p, 1, None, p, None, p, 256, 256, 64, None, None) == -1     # so is the code buffer
     assert g(p, p, 1, p, p, 1, None, p, p, None, 256, 384, 64, None, None) == -1     # F not a multiple of 128
+
+
+def test_kernels_that_wait_for_their_predecessor_read_nothing_through_ldg():
+    """A kernel that may start under the one before it (griddepcontrol.wait) must keep its reads behind the wait.  `__ldg`
+    says that a value never changes while the kernel runs, so the compiler may move it in front of the wait."""
+    import re
+
+    from tensorrt_b200 import _build
+
+    for path in sorted(_build.CSRC.glob("*.cu*")):
+        head, *kernels = re.sub(r"//[^\n]*", "", path.read_text()).split("__global__")
+        waiting = [body for body in kernels if "pdl_wait()" in body or "pdl_enter(" in body]
+        if waiting and path.name != "common.cuh":
+            assert not [c for c in (head, *waiting) if "__ldg(" in c], path.name
