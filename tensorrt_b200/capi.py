@@ -154,17 +154,20 @@ def nvfp4_quantize(x: torch.Tensor, amax_t: torch.Tensor):
 
 
 def nvfp4_quantize_dynamic(x: torch.Tensor):
-    """`nvfp4_quantize(x, amax(x))`, the abs-max measured on the way (one launch for small tensors)."""
+    """`nvfp4_quantize(x, amax(x))`; small tensors in one launch.  Larger ones take two, with the abs-max between them in a
+    tensor of this call's own: the workspace that `amax` shares with the other threads of a stream holds nothing of a call
+    from one launch to the next."""
     _need_cuda(x)
     x = x.contiguous()
     rows, cols = _rows_cols(x)
     if cols % 16:
         raise ValueError(f"last dimension ({cols}) must be a multiple of the block size 16")
+    if load().b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols):
+        return nvfp4_quantize(x, amax(x))
     codes, scales, g = _nvfp4_out(x.shape, rows, cols, x.device)
-    ws = amax_workspace(x.device)
     with torch.cuda.device(x.device):
-        check(load().b200q_nvfp4_quantize_dynamic(x.data_ptr(), _dt(x), rows, cols, codes.data_ptr(), scales.data_ptr(), g.data_ptr(),
-                                                  ws.data_ptr(), ws.numel(), _stream(x)), "b200q_nvfp4_quantize_dynamic")
+        check(load().b200q_nvfp4_quantize_dynamic(x.data_ptr(), _dt(x), rows, cols, codes.data_ptr(), scales.data_ptr(), g.data_ptr(), None, 0,
+                                                  _stream(x)), "b200q_nvfp4_quantize_dynamic")
     return codes, scales, g
 
 

@@ -336,3 +336,49 @@ def test_kernels_that_wait_for_their_predecessor_read_nothing_through_ldg():
         waiting = [body for body in kernels if "pdl_wait()" in body or "pdl_enter(" in body]
         if waiting and path.name != "common.cuh":
             assert not [c for c in (head, *waiting) if "__ldg(" in c], path.name
+
+
+def test_measured_nvfp4_range_survives_a_call_of_another_thread_in_between(b200, monkeypatch):
+    """Two calls on one stream, the second issued by another thread between the two launches of the first (a library
+    that only records stands in for the device): each is quantized under its own abs-max, wherever that is kept."""
+    import contextlib
+
+    import torch
+
+    from tensorrt_b200 import _lib, capi
+
+    real, memory, seen, between = _lib.load(), {}, [], []
+
+    class Recorder:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def measure(self, x, where):
+            memory[where] = x
+            if between:
+                between.pop()()
+
+        def b200q_amax(self, x, dt, n, out, ws, ws_bytes, st):
+            self.measure(x, out)
+            return 0
+
+        def b200q_nvfp4_quantize(self, x, dt, rows, cols, amax, *rest):
+            seen.append((x, memory[amax]))
+            return 0
+
+        def b200q_nvfp4_quantize_dynamic(self, x, dt, rows, cols, codes, scales, g, ws, ws_bytes, st):
+            if real.b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols):
+                self.measure(x, ws + 8)
+                seen.append((x, memory[ws + 8]))
+            return 0
+
+    shared = torch.zeros(real.b200q_amax_workspace_bytes(), dtype=torch.uint8)
+    monkeypatch.setattr(capi, "load", lambda lib=Recorder(): lib)
+    monkeypatch.setattr(capi, "_need_cuda", lambda *ts: None)
+    monkeypatch.setattr(capi, "_stream", lambda x: 0)
+    monkeypatch.setattr(capi, "amax_workspace", lambda device: shared)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    a, b = torch.zeros(64, 4096), torch.zeros(64, 4096)
+    between.append(lambda: capi.nvfp4_quantize_dynamic(b))
+    capi.nvfp4_quantize_dynamic(a)
+    assert sorted(x for x, _ in seen) == sorted((a.data_ptr(), b.data_ptr())) and all(x == measured for x, measured in seen)
