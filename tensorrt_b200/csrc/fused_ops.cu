@@ -33,13 +33,14 @@ __device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
 // lies beyond the row pass zeros.  The warp's first g is a multiple of 8, so that 8 lanes hold one scale word.
 __device__ __forceinline__ void store_nvfp4_group(const float* v, int g, int groups, int64_t row, int64_t cols, const GlobalScale& gs,
                                                   const Nvfp4Out& o) {
-  float a = 0.0f;
+  float a = fabsf(v[0]);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) a = fmaxf(a, fabsf(v[j]));
+  for (int j = 1; j < 8; ++j) a = fmaxf(a, fabsf(v[j]));
   a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 1));
   uint32_t codes, sb = 0u;
   if (g < groups) {
-    sb = quantize_half_block(v, a, gs, codes);
+    float d;
+    sb = quantize_values<8>(v, a, gs, &codes, d);
     *reinterpret_cast<uint32_t*>(o.codes + row * (cols >> 1) + static_cast<int64_t>(g) * 4) = codes;
   }
   uint32_t w = (g & 1) == 0 ? sb << (8 * ((g >> 1) & 3)) : 0u;

@@ -52,14 +52,11 @@ struct GlobalScale {
 };
 
 
-// Quantize one block held in f[16]: returns the 8-bit scale, writes 16 codes as two words and
-// the effective divisor d = fp32(scale) * global.
-__device__ __forceinline__ uint32_t quantize_block(const float* f, const GlobalScale& gs, uint32_t& c_lo, uint32_t& c_hi,
-                                                   float& d_out) {
-  float m[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m[i] = fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1]));
-  const float a = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
+// Codes of N values (8 or 16) of a block whose abs-max is `a`: returns the 8-bit scale, writes the codes as N / 8 words and
+// the effective divisor d = fp32(scale) * global.  `a` is NaN when every value of the block is, and only then; its scale is
+// then NaN too (0x7f).  So the maximum has to be folded from the values themselves: fmaxf from a zero drops it.
+template <int N>
+__device__ __forceinline__ uint32_t quantize_values(const float* f, float a, const GlobalScale& gs, uint32_t* codes, float& d_out) {
   // s = (a / 6) / g, both as exact IEEE quotients
   float s;
   if (gs.fast) {
@@ -71,56 +68,39 @@ __device__ __forceinline__ uint32_t quantize_block(const float* f, const GlobalS
   const uint32_t sb = f32x2_to_e4m3x2(s, 0.0f) & 0xffu;  // saturates to 448
   const float d = __fmul_rn(e4m3_to_f32(sb), gs.g);
   d_out = d;
+  float q[N];
   if (sb != 0u && !clamped && b200q_div_fast_ok(d)) {
     // common case: |x| <= 6.5 d, so the quotient can neither overflow nor need a clamp
     const float y = b200q_rcp_rn(d);
-    float q[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] = b200q_div_by_shared(f[i], d, y);
-    c_lo = pack8_e2m1(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-    c_hi = pack8_e2m1(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+    for (int i = 0; i < N; ++i) q[i] = b200q_div_by_shared(f[i], d, y);
   } else if (sb != 0u) {
     // stored scale saturated at 448 (amax input below the data) or an extreme divisor:
     // true division on a numerator clamped to 8 d, which still saturates to +-6
     const float lim = __fmul_rn(d, 8.0f);
-    float q[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] = with_sign_of(__fdiv_rn(fminf(fabsf(f[i]), lim), d), f[i]);
-    c_lo = pack8_e2m1(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-    c_hi = pack8_e2m1(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+    for (int i = 0; i < N; ++i) q[i] = with_sign_of(__fdiv_rn(fminf(fabsf(f[i]), lim), d), f[i]);
   } else {
-    c_lo = 0u;
-    c_hi = 0u;
+#pragma unroll
+    for (int i = 0; i < N / 8; ++i) codes[i] = 0u;
+    return sb;
   }
+#pragma unroll
+  for (int i = 0; i < N; i += 8) codes[i / 8] = pack8_e2m1(q[i], q[i + 1], q[i + 2], q[i + 3], q[i + 4], q[i + 5], q[i + 6], q[i + 7]);
   return sb;
 }
 
-// The same for a thread that holds half of a block (8 elements) and knows the block's abs-max `a`: returns the 8-bit
-// scale and the eight codes of its half.  Same expressions, hence the same bits, as quantize_block.
-__device__ __forceinline__ uint32_t quantize_half_block(const float* f, float a, const GlobalScale& gs, uint32_t& codes) {
-  float s;
-  if (gs.fast) {
-    s = b200q_div_by_shared(b200q_div_by_shared(a, kE2M1Max, kRcp6), gs.g, gs.yg);
-  } else {
-    s = __fdiv_rn(__fdiv_rn(a, kE2M1Max), gs.g);
-  }
-  const bool clamped = s > kE4M3Max;
-  const uint32_t sb = f32x2_to_e4m3x2(s, 0.0f) & 0xffu;
-  const float d = __fmul_rn(e4m3_to_f32(sb), gs.g);
-  float q[8];
-  if (sb != 0u && !clamped && b200q_div_fast_ok(d)) {
-    const float y = b200q_rcp_rn(d);
+// Quantize one block held in f[16].
+__device__ __forceinline__ uint32_t quantize_block(const float* f, const GlobalScale& gs, uint32_t& c_lo, uint32_t& c_hi,
+                                                   float& d_out) {
+  float m[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = b200q_div_by_shared(f[i], d, y);
-  } else if (sb != 0u) {
-    const float lim = __fmul_rn(d, 8.0f);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = with_sign_of(__fdiv_rn(fminf(fabsf(f[i]), lim), d), f[i]);
-  } else {
-    codes = 0u;
-    return sb;
-  }
-  codes = pack8_e2m1(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
+  for (int i = 0; i < 8; ++i) m[i] = fmaxf(fabsf(f[2 * i]), fabsf(f[2 * i + 1]));
+  const float a = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
+  uint32_t codes[2];
+  const uint32_t sb = quantize_values<16>(f, a, gs, codes, d_out);
+  c_lo = codes[0];
+  c_hi = codes[1];
   return sb;
 }
 

@@ -30,6 +30,28 @@ def test_add_rms_norm(b200, rows, cols, with_delta):
     assert capi.device_status() == 0
 
 
+def _scales_by_row(sf, cols):
+    """Swizzled scales -> [rows padded to 128, columns padded to 64 / 16]."""
+    tiles = sf.view(-1, (cols // 16 + 3) // 4, 32, 4, 4)                # [row tile, column tile, row % 32, row // 32 % 4, 4 scales]
+    return tiles.permute(0, 3, 2, 1, 4).reshape(-1, tiles.shape[1] * 4)
+
+
+@pytest.mark.parametrize("rows,cols", [(3, 272), (5, 4096), (300, 4096), (1300, 2080)])      # one CTA, a cluster a row, many rows, the ring
+def test_add_rms_norm_of_rows_that_are_not_finite(b200, rows, cols):
+    """A NaN makes its whole row NaN, an infinity makes its row zeros with one NaN: as the separate kernels store them."""
+    capi = b200.capi
+    h, d = (torch.randn(rows, cols, device="cuda").bfloat16() for _ in range(2))
+    h[0, cols // 2], h[1, 5], d[2, cols - 1] = float("nan"), float("inf"), float("nan")
+    w = torch.ones(cols, device="cuda").bfloat16()
+    x = capi.rms_norm(capi.add(h, d), w)
+    amax = torch.tensor(4.0, device="cuda")
+    _, (codes, sf, _) = capi.add_rms_norm_nvfp4_quantize(h, d, w, amax)
+    ref_codes, ref_sf, _ = capi.nvfp4_quantize(x, amax)
+    sf, ref_sf = _scales_by_row(sf, cols), _scales_by_row(ref_sf, cols)
+    assert torch.equal(codes[:3], ref_codes[:3]) and torch.equal(sf[:3], ref_sf[:3])
+    assert int(sf[0, :cols // 16].min()) == int(sf[2, :cols // 16].min()) == 0x7F and int(sf[1].max()) == 0
+
+
 @pytest.mark.parametrize("rows,f", [(1, 16), (3, 528), (128, 1040), (130, 14336), (33, 28672)])
 def test_silu_mul(b200, rows, f):
     capi = b200.capi
@@ -60,7 +82,6 @@ def test_padding_rows_of_the_scale_tile_are_cleared(b200, rows):
     sf = torch.full_like(ref, 0xAA)
     assert _lib.load().b200q_nvfp4_quantize(x.data_ptr(), 2, rows, cols, amax.data_ptr(), codes.data_ptr(), sf.data_ptr(), g.data_ptr(),
                                             torch.cuda.current_stream().cuda_stream) == 0
-    tiles = sf.view(-1, (cols // 16 + 3) // 4, 32, 4, 4)                # [row tile, column tile, row % 32, row // 32 % 4, 4 scales]
-    by_row = tiles.permute(0, 3, 2, 1, 4).reshape(-1, tiles.shape[1] * 4)
+    by_row = _scales_by_row(sf, cols)
     assert int(by_row[rows:].max() if by_row.shape[0] > rows else 0) == 0
     assert int(by_row[:rows, cols // 16:].max()) == 0 and bool((by_row[:rows, :cols // 16] != 0xAA).all())
