@@ -10,7 +10,8 @@
 //
 // They take the plain case only (strided CUDA tensors of the exact Python type, matching sizes, fp32 scales, no
 // dispatch or function mode active) and return None for anything else, before anything is launched: the caller then
-// takes the general path in capi.py, which converts, or raises the error that belongs to the input.
+// takes the general path in capi.py, which converts, or raises the error that belongs to the input.  From the first
+// launch on, and for a failure of the device or the driver, a status raises the error that capi.py raises for it.
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/TensorSubclassLikeUtils.h>
@@ -88,6 +89,23 @@ struct Operand {   // FP8 operand: codes and scales inside a scratch buffer
   int64_t n_scales;
 };
 
+// A status that ends the call: raised by `finish` as the B200QError of _lib.check.
+struct CallError {
+  int status;
+  const char* what;
+};
+
+void must(int status, const char* what) {
+  if (status != B200Q_OK) throw CallError{status, what};
+}
+
+// Status of the first launch of a call: false = the arguments were refused, nothing has run.
+bool taken(int status, const char* what) {
+  if (status == B200Q_ERR_INVALID || status == B200Q_ERR_ALIGN) return false;
+  must(status, what);
+  return true;
+}
+
 // ---------------------------------------------------------------- fp8_linear
 std::optional<Tensor> fp8_linear(const Tensor& x_in, const Tensor& w, const Tensor& ws, const Tensor* bias, const Tensor* amax,
                                  const b200q_cfg& cfg) {
@@ -105,18 +123,20 @@ std::optional<Tensor> fp8_linear(const Tensor& x_in, const Tensor& w, const Tens
     Tensor out = bf16_like(x, N);
     const int rc = b200q::fp8_linear_small(x.data_ptr(), dt, f32(amax), n, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),
                                            bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, current_stream());
-    if (rc == B200Q_OK) return out;
-    if (rc != 1) return std::nullopt;
+    if (rc != 1) {
+      must(rc, "b200q_fp8_gemm");
+      return out;
+    }
   }
   Tensor scratch = at::empty({up16(M * K) + 4 * n_scales}, x.options().dtype(at::kByte));
   auto* codes = static_cast<uint8_t*>(scratch.data_ptr());
   auto* scales = reinterpret_cast<float*>(codes + up16(M * K));
   Tensor out = bf16_like(x, N);
   const auto st = current_stream();
-  if (b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(amax), n, codes, scales, st, true) != B200Q_OK) return std::nullopt;
-  if (b200q_fp8_gemm(codes, scales, n_scales, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),
-                     bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, st, &cfg) != B200Q_OK)
-    return std::nullopt;
+  if (!taken(b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(amax), n, codes, scales, st, true), "b200q_fp8_quantize")) return std::nullopt;
+  must(b200q_fp8_gemm(codes, scales, n_scales, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),
+                      bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, st, &cfg),
+       "b200q_fp8_gemm");
   return out;
 }
 
@@ -134,6 +154,7 @@ std::optional<Tensor> nvfp4_linear(const Tensor& x_in, const Tensor& w, const Te
   if (amax != nullptr && !f32_of(*amax, 1, 1, dev)) return std::nullopt;
   c10::cuda::CUDAGuard guard(dev);
   const Tensor x = x_in.contiguous();
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 != 0) return std::nullopt;
   const int64_t M = x.numel() / K, sf_bytes = static_cast<int64_t>(b200q_nvfp4_scale_bytes(M, K));
   const int64_t ws_bytes = amax == nullptr ? static_cast<int64_t>(b200q_nvfp4_quantize_dynamic_workspace_bytes(M, K)) : 0;
   const int64_t code_bytes = up16(M * K / 2);
@@ -149,13 +170,13 @@ std::optional<Tensor> nvfp4_linear(const Tensor& x_in, const Tensor& w, const Te
     rc = b200q::nvfp4_quantize(x.data_ptr(), dt, M, K, f32(amax), codes, sf, g, st, true);
   } else {
     // the two words that the abs-max of a large tensor counts in start at zero
-    if (ws_bytes > 0 && cudaMemsetAsync(workspace, 0, 16, static_cast<cudaStream_t>(st)) != cudaSuccess) return std::nullopt;
+    if (ws_bytes > 0 && cudaMemsetAsync(workspace, 0, 16, static_cast<cudaStream_t>(st)) != cudaSuccess) must(B200Q_ERR_CUDA, "b200q_amax");
     rc = b200q::nvfp4_quantize_dynamic(x.data_ptr(), dt, M, K, codes, sf, g, workspace, static_cast<size_t>(ws_bytes), st, true);
   }
-  if (rc != B200Q_OK) return std::nullopt;
-  if (b200q_nvfp4_gemm(codes, sf, g, static_cast<const uint8_t*>(w.data_ptr()), static_cast<const uint8_t*>(wsf.data_ptr()), f32(&wg),
-                       bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, st, &cfg) != B200Q_OK)
-    return std::nullopt;
+  if (!taken(rc, "b200q_nvfp4_quantize")) return std::nullopt;
+  must(b200q_nvfp4_gemm(codes, sf, g, static_cast<const uint8_t*>(w.data_ptr()), static_cast<const uint8_t*>(wsf.data_ptr()), f32(&wg),
+                        bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, st, &cfg),
+       "b200q_nvfp4_gemm");
   return out;
 }
 
@@ -190,29 +211,27 @@ std::optional<Tensor> fp8_gated_mlp(const Tensor& x_in, const Tensor& gu, const 
   uint8_t* m1 = base + o_mid;
   const auto* guc = static_cast<const uint8_t*>(gu.data_ptr());
   Tensor out = bf16_like(x, H);
-  if (b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(in_amax), n_in, xc, xs, st, true) != B200Q_OK) return std::nullopt;
-  int rc;
+  if (!taken(b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(in_amax), n_in, xc, xs, st, true), "b200q_fp8_quantize")) return std::nullopt;
   if (fused_quant) {
-    rc = b200q_fp8_gemm_silu_mul_quantize(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, f32(act_amax), ac, as, M, 2 * F, K, st, nullptr);
+    must(b200q_fp8_gemm_silu_mul_quantize(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, f32(act_amax), ac, as, M, 2 * F, K, st, nullptr),
+         "b200q_fp8_gemm_silu_mul_quantize");
   } else if (fused) {
-    rc = b200q_fp8_gemm_silu_mul(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, nullptr);
-    if (rc == B200Q_OK) rc = b200q::fp8_quantize(m1, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true);
+    must(b200q_fp8_gemm_silu_mul(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, nullptr),
+         "b200q_fp8_gemm_silu_mul");
+    must(b200q::fp8_quantize(m1, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true), "b200q_fp8_quantize");
   } else {
-    rc = b200q_fp8_gemm(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, &cfg);
-    if (rc == B200Q_OK) {
-      if (n_act) {
-        uint8_t* act = m1 + M * F * 4;
-        rc = b200q_silu_mul(m1, act, M, F, st);
-        if (rc == B200Q_OK) rc = b200q::fp8_quantize(act, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true);
-      } else {
-        rc = b200q::silu_mul_fp8_quantize(m1, ac, as, M, F, st, true);
-      }
+    must(b200q_fp8_gemm(xc, xs, in_scales, guc, f32(&gus), gus.numel(), nullptr, m1, M, 2 * F, K, st, &cfg), "b200q_fp8_gemm");
+    if (n_act) {
+      uint8_t* act = m1 + M * F * 4;
+      must(b200q_silu_mul(m1, act, M, F, st), "b200q_silu_mul");
+      must(b200q::fp8_quantize(act, B200Q_BF16, M, F, f32(act_amax), n_act, ac, as, st, true), "b200q_fp8_quantize");
+    } else {
+      must(b200q::silu_mul_fp8_quantize(m1, ac, as, M, F, st, true), "b200q_silu_mul_fp8_quantize");
     }
   }
-  if (rc != B200Q_OK) return std::nullopt;
-  if (b200q_fp8_gemm(ac, as, act_scales, static_cast<const uint8_t*>(dn.data_ptr()), f32(&dns), dns.numel(), nullptr, out.data_ptr(), M, H, F, st,
-                     &cfg) != B200Q_OK)
-    return std::nullopt;
+  must(b200q_fp8_gemm(ac, as, act_scales, static_cast<const uint8_t*>(dn.data_ptr()), f32(&dns), dns.numel(), nullptr, out.data_ptr(), M, H, F, st,
+                      &cfg),
+       "b200q_fp8_gemm");
   return out;
 }
 
@@ -246,12 +265,13 @@ std::optional<Tensor> fp8_sdpa(const Tensor& q, const Tensor& k, const Tensor& v
   uint8_t *kc = qc + nq, *vc = kc + nk;
   auto* scales = reinterpret_cast<float*>(vc + nv);
   const auto st = current_stream();
-  if (b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, f32(&aq), f32(&ak), f32(&av), qc, kc, vc, scales, B, Hq,
-                                   Hkv, Sq, Sk, vt_stride, D, st) != B200Q_OK)
+  if (!taken(b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, f32(&aq), f32(&ak), f32(&av), qc, kc, vc, scales, B,
+                                          Hq, Hkv, Sq, Sk, vt_stride, D, st),
+             "b200q_fp8_attention_quantize"))
     return std::nullopt;
-  if (b200q_fp8_sdpa(qc, kc, vc, scales, scales + 1, scales + 2, out.data_ptr(), dt, B, Hq, Hkv, Sq, Sk, vt_stride, D, static_cast<float>(scale),
-                     causal ? 1 : 0, st) != B200Q_OK)
-    return std::nullopt;
+  must(b200q_fp8_sdpa(qc, kc, vc, scales, scales + 1, scales + 2, out.data_ptr(), dt, B, Hq, Hkv, Sq, Sk, vt_stride, D, static_cast<float>(scale),
+                      causal ? 1 : 0, st),
+       "b200q_fp8_sdpa");
   return out;
 }
 
@@ -260,9 +280,11 @@ std::optional<Tensor> fp8_sdpa(const Tensor& q, const Tensor& k, const Tensor& v
 template <typename F>
 PyObject* finish(F&& fn) {
   std::optional<Tensor> out;
-  {
+  try {
     pybind11::gil_scoped_release no_gil;
     out = fn();
+  } catch (const CallError& e) {
+    pybind11::module_::import("tensorrt_b200._lib").attr("check")(e.status, e.what);
   }
   if (!out.has_value()) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(*out));

@@ -152,3 +152,26 @@ def test_other_inputs_take_the_general_path(b200):
         b200.fp8_linear(x.double(), w, ws)
     with pytest.raises(RuntimeError):
         b200.fp8_linear(x.cpu(), w, ws)
+
+
+def test_a_status_behind_the_first_launch_is_raised(b200):
+    """A call whose later step is refused has already launched its quantize: it raises what the general path raises for it
+    and does not go through that path from the start.  A call whose first step is refused returns None."""
+    from tensorrt_b200 import _native
+
+    def off8(t):                                                                                     # the same values, 8 bytes off
+        return torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")[8:].view(t.shape).copy_(t)
+
+    (w, ws), (nw, nws, ng) = _codes(b200, 256, 128)
+    down, ds = _codes(b200, 128, 128)[0]
+    for m in (1, 40):
+        x = torch.randn(m, 128, device="cuda").bfloat16()
+        for call in (lambda: _native.fp8_linear(x, off8(w), ws, None, None, 0), lambda: _native.nvfp4_linear(x, off8(nw), nws, ng, None, None, 0),
+                     lambda: _native.fp8_gated_mlp(x, w, ws, off8(down), ds, None, None, 0), lambda: _native.fp8_linear(x, w, ws, None, None, 77)):
+            with pytest.raises(b200.B200QError):
+                call()
+        shifted = torch.empty(m * 128 + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, 128).copy_(x)
+        assert _native.fp8_linear(shifted, w, ws, None, None, 0) is None and _native.nvfp4_linear(shifted, nw, nws, ng, None, None, 0) is None
+    q, a = torch.randn(1, 2, 8, 16, device="cuda").bfloat16(), torch.ones(1, device="cuda")
+    with pytest.raises(b200.B200QError):
+        _native.fp8_sdpa(q, q, q, a, a, a, False, -1.0)
