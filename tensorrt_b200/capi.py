@@ -313,6 +313,11 @@ def nvfp4_gemm(a_codes, a_scales, a_global, b_codes, b_scales, b_global, bias=No
     return out
 
 
+def _need_heads(Hq: int, Hkv: int, D: int) -> None:
+    if Hkv <= 0 or Hq % Hkv or D <= 0 or D % 16 or D > 128:
+        raise ValueError(f"need Hq % Hkv == 0 and a head dimension that is a multiple of 16 up to 128, got Hq={Hq}, Hkv={Hkv}, D={D}")
+
+
 def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, amax_v, is_causal: bool = False,
              scale: float | None = None) -> torch.Tensor:
     """FP8 attention on q [B, Hq, Sq, D], k / v [B, Hkv, Sk, D] (bf16 / fp16 / fp32) with per-tensor amax
@@ -328,8 +333,7 @@ def fp8_sdpa(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, amax_q, amax_k, 
         raise ValueError(f"expected q [B, Hq, Sq, D] and k, v [B, Hkv, Sk, D], got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
     B, Hq, Sq, D = q.shape
     _, Hkv, Sk, _ = k.shape
-    if Hq % Hkv or D % 16 or D > 128:
-        raise ValueError(f"need Hq % Hkv == 0 and a head dimension that is a multiple of 16 up to 128, got Hq={Hq}, Hkv={Hkv}, D={D}")
+    _need_heads(Hq, Hkv, D)
     out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
     if k.dtype == q.dtype and v.dtype == q.dtype:
         return _fp8_sdpa_into(out, q, k, v, amax_q, amax_k, amax_v, is_causal, scale)
@@ -403,6 +407,7 @@ def fp8_sdpa_packed(qkv: torch.Tensor, batch: int, n_q: int, n_kv: int, head_dim
     heads, value heads) -> [batch * S, n_q * head_dim].  Q, K, V are quantized per tensor at their measured abs-max;
     read and written in place of head-major copies.  The same bits as `fp8_sdpa` on those copies."""
     _need_cuda(qkv)
+    _need_heads(n_q, n_kv, head_dim)
     qkv = qkv.contiguous()
     if qkv.data_ptr() % 32:
         qkv = qkv.clone()

@@ -343,8 +343,6 @@ def test_measured_nvfp4_range_survives_a_call_of_another_thread_in_between(b200,
     that only records stands in for the device): each is quantized under its own abs-max, wherever that is kept."""
     import contextlib
 
-    import torch
-
     from tensorrt_b200 import _lib, capi
 
     real, memory, seen, between = _lib.load(), {}, [], []
@@ -382,3 +380,13 @@ def test_measured_nvfp4_range_survives_a_call_of_another_thread_in_between(b200,
     between.append(lambda: capi.nvfp4_quantize_dynamic(b))
     capi.nvfp4_quantize_dynamic(a)
     assert sorted(x for x, _ in seen) == sorted((a.data_ptr(), b.data_ptr())) and all(x == measured for x, measured in seen)
+
+
+@pytest.mark.parametrize("n_q,n_kv,head_dim", [(3, 2, 64), (4, 2, 24), (4, 2, 256), (4, 0, 64)])
+def test_packed_attention_names_a_head_layout_that_it_does_not_take(b200, monkeypatch, n_q, n_kv, head_dim):
+    """The error of `fp8_sdpa`, before anything is launched (no device needed)."""
+    from tensorrt_b200 import capi
+
+    monkeypatch.setattr(capi, "_need_cuda", lambda *ts: None)
+    with pytest.raises(ValueError, match="head dimension"):
+        capi.fp8_sdpa_packed(torch.zeros(8, (n_q + 2 * n_kv) * head_dim, dtype=torch.bfloat16), 1, n_q, n_kv, head_dim)
