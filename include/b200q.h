@@ -414,7 +414,7 @@ int b200q_silu_mul_fp8_quantize(const void* gate_up, uint8_t* codes_out, float* 
  * (padding rows zero) and global scale as rms_norm of h + delta / silu_mul / expand_heads followed by
  * b200q_nvfp4_quantize, without the bf16 tensor in between.  bf16 in.  add_rms_norm: cols % 16 == 0, cols <= 16384;
  * silu_mul: f % 16 == 0, gate_up 32-byte aligned; expand_heads: head_dim, src_stride, src_col0 multiples of 16, src
- * 32-byte aligned.  global_scale_out may be NULL. */
+ * 32-byte aligned, the slice src_col0 + heads_out / rep * head_dim within src_stride.  global_scale_out may be NULL. */
 int b200q_add_rms_norm_nvfp4_quantize(const void* h, const void* delta, const void* weight, void* h_out, const float* amax,
                                       uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out, int64_t rows,
                                       int64_t cols, float eps, b200q_stream_t stream);

@@ -510,12 +510,19 @@ def silu_mul_nvfp4_quantize(gate_up: torch.Tensor, amax_t: torch.Tensor):
     return codes, scales, g
 
 
+def _need_columns(width: int, col0: int, heads_out: int, rep: int, head_dim: int) -> None:
+    """The kv slice that the head expansions read lies inside a row (the kernels do not check it)."""
+    if rep > 0 and (col0 < 0 or col0 + heads_out // rep * head_dim > width):
+        raise ValueError(f"columns {col0} to {col0} + {heads_out} / {rep} * {head_dim} do not lie in a row of {width}")
+
+
 def expand_heads_nvfp4_quantize(src: torch.Tensor, col0: int, heads_out: int, rep: int, head_dim: int, amax_t: torch.Tensor):
     """`expand_heads` followed by `nvfp4_quantize` under a calibrated tensor amax, in one pass, the same bits."""
     _need_cuda(src, amax_t)
     _bf16(src)
     src = src.contiguous()
     rows, width = _rows_cols(src)
+    _need_columns(width, col0, heads_out, rep, head_dim)
     a = _scalar_amax(amax_t, src.device)
     codes, scales, g = _nvfp4_out((*src.shape[:-1], 0), rows, heads_out * head_dim, src.device)
     with torch.cuda.device(src.device):
@@ -568,6 +575,7 @@ def expand_heads(src: torch.Tensor, col0: int, heads_out: int, rep: int, head_di
     _bf16(src)
     src = src.contiguous()
     rows, width = _rows_cols(src)
+    _need_columns(width, col0, heads_out, rep, head_dim)
     out = torch.empty(*src.shape[:-1], heads_out * head_dim, dtype=torch.bfloat16, device=src.device)
     with torch.cuda.device(src.device):
         check(load().b200q_expand_heads(src.data_ptr(), width, col0, out.data_ptr(), rows, heads_out, rep, head_dim, _stream(src)),
@@ -582,6 +590,7 @@ def expand_heads_fp8_quantize(src: torch.Tensor, col0: int, heads_out: int, rep:
     _bf16(src)
     src = src.contiguous()
     rows, width = _rows_cols(src)
+    _need_columns(width, col0, heads_out, rep, head_dim)
     codes = torch.empty(*src.shape[:-1], heads_out * head_dim, dtype=torch.uint8, device=src.device)
     scales = torch.empty(rows, dtype=torch.float32, device=src.device)
     with torch.cuda.device(src.device):

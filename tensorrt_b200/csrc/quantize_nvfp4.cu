@@ -385,6 +385,7 @@ int b200q_expand_heads_nvfp4_quantize(const void* src, int64_t src_stride, int64
       src_stride % 16 != 0 || src_col0 % 16 != 0)
     return B200Q_ERR_INVALID;
   const int64_t cols = static_cast<int64_t>(heads_out) * head_dim;
+  if (rows > 1 && src_col0 + cols / rep > src_stride) return B200Q_ERR_INVALID;      // beyond the row
   if (int rc = validate(src, B200Q_BF16, rows, cols, amax)) return rc;
   if (rows == 0) return B200Q_OK;
   if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;

@@ -390,3 +390,17 @@ def test_packed_attention_names_a_head_layout_that_it_does_not_take(b200, monkey
     monkeypatch.setattr(capi, "_need_cuda", lambda *ts: None)
     with pytest.raises(ValueError, match="head dimension"):
         capi.fp8_sdpa_packed(torch.zeros(8, (n_q + 2 * n_kv) * head_dim, dtype=torch.bfloat16), 1, n_q, n_kv, head_dim)
+
+
+def test_head_expansion_stays_inside_a_row(b200, monkeypatch):
+    """A slice that ends behind its row is refused before anything is launched (no device needed)."""
+    from tensorrt_b200 import _lib, capi
+
+    monkeypatch.setattr(capi, "_need_cuda", lambda *ts: None)
+    src, amax = torch.zeros(4, 256, dtype=torch.bfloat16), torch.ones(1)
+    for args in ((208, 8, 2, 16), (256, 2, 2, 16), (-16, 2, 1, 16)):
+        for call in (capi.expand_heads, capi.expand_heads_fp8_quantize, lambda *a: capi.expand_heads_nvfp4_quantize(*a, amax)):
+            with pytest.raises(ValueError):
+                call(src, *args)
+    p = (ctypes.addressof(ctypes.create_string_buffer(8192)) + 255) & ~255
+    assert _lib.load().b200q_expand_heads_nvfp4_quantize(p, 256, 208, p, p, p, p, 4, 8, 2, 16, None) == -1
