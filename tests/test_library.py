@@ -400,7 +400,7 @@ def test_head_expansion_stays_inside_a_row(b200, monkeypatch):
     src, amax = torch.zeros(4, 256, dtype=torch.bfloat16), torch.ones(1)
     for args in ((208, 8, 2, 16), (256, 2, 2, 16), (-16, 2, 1, 16)):
         for call in (capi.expand_heads, capi.expand_heads_fp8_quantize, lambda *a: capi.expand_heads_nvfp4_quantize(*a, amax)):
-            with pytest.raises(ValueError):
+            with pytest.raises(ValueError, match="do not lie in a row of 256"):
                 call(src, *args)
     p = (ctypes.addressof(ctypes.create_string_buffer(8192)) + 255) & ~255
     assert _lib.load().b200q_expand_heads_nvfp4_quantize(p, 256, 208, p, p, p, p, 4, 8, 2, 16, None) == -1
