@@ -125,14 +125,15 @@ def build_python_calls(force: bool = False) -> Path:
 
     with _BuildLock():
         return _build_torch_extension(CSRC / "python_calls.cpp", PYTHON_LIB, "python", ["-isystem", sysconfig.get_paths()["include"]],
-                                      ["-ltorch_python"], force)
+                                      ["-ltorch_python"], force, abi=sys.implementation.cache_tag)
 
 
-def _build_torch_extension(src: Path, lib: Path, name: str, includes: list, libs: list, force: bool) -> Path:
+def _build_torch_extension(src: Path, lib: Path, name: str, includes: list, libs: list, force: bool, abi: str = "") -> Path:
+    """`abi`: the interpreter, where the library is a CPython extension: another one builds it again."""
     import torch
     from torch.utils import cpp_extension
 
-    stamp = _stamp([src, CSRC / "internal.h", ROOT / "include" / "b200q.h"], torch.__version__)
+    stamp = _stamp([src, CSRC / "internal.h", ROOT / "include" / "b200q.h"], torch.__version__ + abi)
     stamp_file = PKG / "build" / f"{name}.stamp"
     if not force and lib.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
         return lib

@@ -404,3 +404,25 @@ def test_head_expansion_stays_inside_a_row(b200, monkeypatch):
                 call(src, *args)
     p = (ctypes.addressof(ctypes.create_string_buffer(8192)) + 255) & ~255
     assert _lib.load().b200q_expand_heads_nvfp4_quantize(p, 256, 208, p, p, p, p, 4, 8, 2, 16, None) == -1
+
+
+def test_python_extension_is_built_again_for_another_interpreter(b200, monkeypatch):
+    """The stamp beside libb200q_python.so names the interpreter that it was built for; the torch shim does not depend on it."""
+    import sys
+    import types
+
+    from tensorrt_b200 import _build
+
+    class Compiled(Exception):
+        pass
+
+    def run(cmd, log_path=None):
+        raise Compiled
+
+    _build.build_python_calls()
+    monkeypatch.setattr(_build, "_run", run)
+    assert _build.build_python_calls() == _build.PYTHON_LIB
+    monkeypatch.setattr(_build.sys, "implementation", types.SimpleNamespace(**{**vars(sys.implementation), "cache_tag": "cpython-999"}))
+    assert _build.build_torch_shim() == _build.TORCH_LIB
+    with pytest.raises(Compiled):
+        _build.build_python_calls()
