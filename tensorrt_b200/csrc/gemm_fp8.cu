@@ -63,12 +63,24 @@ int forced_smallm_stages() {
 
 namespace b200q {
 
-// One launch for tokens few enough that every CTA can find their abs-max itself: at most 16 tokens and 65536 elements
-// (128 KB of 16-bit values read from L2 per CTA, about 1 us; the separate quantize launch costs 2 us on the device and
-// as much on the host).
+// One launch where every CTA can quantize its slice of the activation while its weights arrive: at most 16 KB of
+// activation (read by every CTA for the abs-max), at most kOwnXTiles K tiles per CTA, at most kOwnXSlice tokens x K tiles,
+// and 16 tiles of weight rows.  Measured against the quantize launch and the GEMM behind it at 1 to 16 tokens, N 1024 to
+// 28672, K 1024 to 65536, bf16, fp16 and fp32, weights rotating through more than L2 where they are that large: at the 152
+// points inside it takes 0.89 of their device time on average (0.57 at N = 2048, where the eight-CTA clusters of the plain
+// GEMM take two rounds; 0.92 elsewhere; at most 1.04 or 0.3 us more, 4 fp32 tokens of 4096 x 1024) and 0.86 of the time of
+// an eager call, which a launch less decides.  Outside, with the same kernel: 4 x 10240 x 4096 16.0 us against 13.3, 1 x
+// 10240 x 8192 27.0 against 19.5, 16 x 4096 x 4096 14.7 against 9.4 (the quantizer's work in every CTA), 1 x 1024 x 1024
+// 5.3 against 4.9 (too few CTAs to gain).
 int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,
                      int64_t w_scales_numel, const void* bias, void* out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream) {
-  if (M <= 0 || M > 16 || N <= 0 || K <= 0 || M * K > 65536 || K % 16 != 0 || N > 0x7fffffffLL) return 1;
+  const int64_t width = dtype == B200Q_F32 ? 4 : 2;
+  if (M <= 0 || M > gemm::kOwnXSlice || K <= 0 || K > 16384 || M * K * width > 16384 || K % 16 != 0 || N > 0x7fffffffLL) return 1;
+  const int tiles = static_cast<int>((N + gemm::kSmallWRows - 1) / gemm::kSmallWRows);
+  const int k_tiles = static_cast<int>((K + gemm::kBKBytes - 1) / gemm::kBKBytes);
+  if (tiles < 16) return 1;
+  const int splits = gemm::smallm_splits(tiles, k_tiles, sm_count(), static_cast<int>(M)), per_cta = (k_tiles + splits - 1) / splits;
+  if (per_cta > gemm::kOwnXTiles || per_cta * M > gemm::kOwnXSlice) return 1;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(out, 16)) return 1;
   if (int rc = check_arch()) return rc;
   gemm::Params p{};
@@ -84,13 +96,11 @@ int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_n
   p.M = static_cast<int>(M);
   p.N = static_cast<int>(N);
   p.k_bytes = static_cast<int>(K);
-  const int k_tiles = (p.k_bytes + gemm::kBKBytes - 1) / gemm::kBKBytes;
-  const int splits = gemm::smallm_splits((p.N + gemm::kSmallWRows - 1) / gemm::kSmallWRows, k_tiles, sm_count(), p.M);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case B200Q_BF16: return gemm::launch_smallm_own_x<__nv_bfloat16>(w, p, st, splits);
-    case B200Q_F16: return gemm::launch_smallm_own_x<__half>(w, p, st, splits);
-    case B200Q_F32: return gemm::launch_smallm_own_x<float>(w, p, st, splits);
+    case B200Q_BF16: return gemm::launch_smallm_own_x<__nv_bfloat16>(w, p, st, splits, per_cta);
+    case B200Q_F16: return gemm::launch_smallm_own_x<__half>(w, p, st, splits, per_cta);
+    case B200Q_F32: return gemm::launch_smallm_own_x<float>(w, p, st, splits, per_cta);
     default: return 1;
   }
 }

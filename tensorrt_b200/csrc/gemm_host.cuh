@@ -202,6 +202,43 @@ inline int launch_nvf4_pair(const uint8_t* a, const uint8_t* b, Params p, cudaSt
   return B200Q_OK;
 }
 
+// Dynamic shared memory that `kernel` may be launched with, set once per device (`configured`: one flag per device).
+template <typename Kernel>
+int allow_smem(Kernel* kernel, int bytes, bool* configured) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return B200Q_ERR_CUDA;
+    configured[dev] = true;
+  }
+  return B200Q_OK;
+}
+
+// One launch of a small-M kernel: `tiles` clusters of `splits` CTAs.
+template <typename Kernel>
+int launch_clusters(Kernel* kernel, int tiles, int splits, int smem_bytes, cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tx,
+                    const Params& p, int stages, int bt) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see common.cuh: pdl_wait in the kernel
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, tw, tx, p, splits, stages, bt) != cudaSuccess) {
+    cudaGetLastError();
+    return B200Q_ERR_CUDA;
+  }
+  return B200Q_OK;
+}
+
 // Small-M kernel (M <= 128): operands swapped, one cluster of `splits` CTAs per tile of 128
 // weight rows.  Up to one CTA per SM the operand ring takes all of shared memory; beyond that
 // the ring is sized so that two CTAs share an SM, which lets one CTA's prologue and cluster
@@ -211,13 +248,7 @@ template <bool NVF4>
 int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, int splits, int stages) {
   using C = SmallCfg<NVF4>;
   static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
-  if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gemm_smallm_kernel<NVF4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess)
-      return B200Q_ERR_CUDA;
-    configured[dev] = true;
-  }
+  if (int rc = allow_smem(gemm_smallm_kernel<NVF4>, kSmemLimit, configured)) return rc;
   const int bt = ((p.M + 15) / 16) * 16;
   const int tiles = (p.N + kSmallWRows - 1) / kSmallWRows;
   const int most = C::max_stages(bt, kSmemLimit);
@@ -235,70 +266,21 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
   CUtensorMap tw, tx;
   if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
   if (int rc = make_operand_map(&tx, a, p.M, p.k_bytes, bt)) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(C::smem_bytes(bt, stages));
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see common.cuh: pdl_wait in the kernel
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<NVF4>, tw, tx, p, splits, stages, bt) != cudaSuccess) {
-    cudaGetLastError();
-    return B200Q_ERR_CUDA;
-  }
-  return B200Q_OK;
+  return launch_clusters(gemm_smallm_kernel<NVF4>, tiles, splits, C::smem_bytes(bt, stages), st, tw, tx, p, stages, bt);
 }
 
-// The small-M kernel that quantizes its activation (FP8, M <= 16; p.x, p.x_amax set).  Returns 1 when the problem does
-// not qualify.
+// The small-M kernel that quantizes its activation (FP8; p.x, p.x_amax set; limits kOwnXTiles, kOwnXSlice).
 template <typename XT>
-int launch_smallm_own_x(const uint8_t* b, Params p, cudaStream_t st, int splits) {
-  using C = SmallCfg<false>;
+int launch_smallm_own_x(const uint8_t* b, const Params& p, cudaStream_t st, int splits, int tiles_per_cta) {
+  const int stages = tiles_per_cta < 2 ? 2 : tiles_per_cta;      // the whole K slice at once
+  constexpr int kMostBytes = 1024 + kSmallTailBytes + kOwnXTiles * (SmallCfg<false>::kWBytes + 2048);
+  static_assert(kMostBytes <= kSmallHalfSmem, "two CTAs share an SM");
+  const int bytes = 1024 + kSmallTailBytes + stages * SmallCfg<false>::kWBytes + tiles_per_cta * 2048;
   static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
-  if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gemm_smallm_kernel<false, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess)
-      return B200Q_ERR_CUDA;
-    configured[dev] = true;
-  }
-  const int tiles = (p.N + kSmallWRows - 1) / kSmallWRows;
-  const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
-  const int per = (k_tiles + splits - 1) / splits;
-  const int fixed = 1024 + kSmallTailBytes + per * 2048;
-  const int budget = tiles * splits > sm_count() ? kSmallHalfSmem : kSmemLimit;
-  int stages = (budget - fixed) / C::kWBytes;
-  if (stages > kSmallMaxStages) stages = kSmallMaxStages;
-  if (stages > per) stages = per < 2 ? 2 : per;
-  if (stages < 2) return 1;
+  if (int rc = allow_smem(gemm_smallm_kernel<false, XT>, kMostBytes, configured)) return rc;
   CUtensorMap tw;
   if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(fixed + stages * C::kWBytes);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<false, XT>, tw, tw, p, splits, stages, 16) != cudaSuccess) {
-    cudaGetLastError();
-    return B200Q_ERR_CUDA;
-  }
-  return B200Q_OK;
+  return launch_clusters(gemm_smallm_kernel<false, XT>, (p.N + kSmallWRows - 1) / kSmallWRows, splits, bytes, st, tw, tw, p, stages, 16);
 }
 
 // Cluster size of the small-M kernel.  Measured: one SM pulls about 60 bytes per nanosecond

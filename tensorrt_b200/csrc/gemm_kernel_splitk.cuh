@@ -14,9 +14,9 @@
 //     ld.shared::cluster loads, applies the dequantization scales and the bias and stores
 //     bf16 rows.  No global workspace, no atomics, fixed summation order.
 //
-// XT != void (FP8, M <= 16, short rows): the kernel also quantizes the activation.  Four warps read x, find every
-// token's abs-max (each CTA for itself: the rows are a few KB in L2) and write the codes of the CTA's K slice
-// into shared memory in the operand layout while the weight ring fills.  One launch instead of two; codes, scales
+// XT != void (FP8, a few tokens of short rows: see fp8_linear_small): the kernel also quantizes the activation.  Four
+// warps read x, find every token's abs-max (each CTA for itself: at most 16 KB from L2) and write the codes of the CTA's
+// K slice into shared memory in the operand layout while the weight ring fills.  One launch instead of two; codes, scales
 // and sums are those of the quantize kernel followed by the plain form.
 #pragma once
 
@@ -104,48 +104,73 @@ __device__ __forceinline__ void small_reduce_store(uint32_t partial_u32, int t0,
   }
 }
 
-// FP8 codes of K tiles [kt0, kt1) of x [M, k] into `xs` ([K tile][16 rows][128 bytes], 128-byte swizzle, rows M..15 zero)
-// and the scale of every token into `xscale`; by 128 threads (t), barrier 1.
+// Limits of the kernel that quantizes its activation: all of a CTA's K tiles stand in the ring at once, and its slice of
+// the activation is at most half a 16-element piece per thread.
+constexpr int kOwnXTiles = 4;        // K tiles per CTA
+constexpr int kOwnXSlice = 8;        // tokens x K tiles per CTA (8 pieces each)
+
+// The two parts of the activation quantizer, by 128 threads (t), barrier 1.
+// Before the activation may be read: rows M..15 of the operand tiles `xs` ([K tile][16 rows][128 bytes]) are zeroed, and
+// so are the words that the abs-maxima of the tokens meet in (xscale[16..], as bit patterns: values >= 0, never NaN).
+__device__ __forceinline__ void small_clear_x(const Params& p, uint8_t* xs, float* xscale, int tiles, int t) {
+  const int pad = (16 - p.M) * 8;                              // 16-byte pieces of a tile's unused rows
+  for (int i = t; i < tiles * pad; i += 128) {
+    const int kt = i / pad;
+    *reinterpret_cast<uint4*>(xs + kt * 2048 + p.M * 128 + (i - kt * pad) * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (t < kOwnXSlice) xscale[16 + t] = 0.0f;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+
+// FP8 codes of K tiles [kt0, kt1) of x [M, k] into rows 0..M-1 of `xs` (128-byte swizzle) and the scale of every token
+// into xscale[0..M).  The chain in front of the first MMA decides here: one L2 round trip (a thread requests its piece of
+// the slice and, with all threads on every token, its pieces of the rows before it uses any), a maximum, a store.  With a
+// warp per token and one load in flight per thread in a second pass it was 10.7 us at 1 x 4096 x 4096 and 7.3 at
+// 1 x 4096 x 2048 (weights from HBM, in a graph), now 8.1 and 6.8; the two launches take 8.4 to 8.7 and 6.7 to 7.2.
 template <typename T>
 __device__ __forceinline__ void small_quantize_x(const Params& p, uint8_t* xs, float* xscale, int kt0, int kt1, int t) {
+  constexpr int U = 4;                                         // pieces of a row in flight per thread
   const T* x = static_cast<const T*>(p.x);
-  const int k = p.k_bytes, warp = t >> 5, lane = t & 31;
-  const int pieces = k >> 4;                                   // 16-element pieces of a row (k % 16 == 0)
-  for (int tok = warp; tok < p.M; tok += 4) {                  // a warp takes whole tokens
+  const int k = p.k_bytes, pieces = k >> 4;                    // 16-element pieces of a row (k % 16 == 0)
+  const int per_row = (kt1 - kt0) * 8;
+  const bool mine = t < per_row * p.M;                         // at most 8 * kOwnXSlice pieces
+  const int row = mine ? t / per_row : 0, r = t - row * per_row, g = kt0 * 8 + r;
+  Raw16<T, false> raw;
+  if (mine && g < pieces) raw.load(x + static_cast<int64_t>(row) * k + g * 16);
+  if (p.x_amax_numel == 0) {
+    const int width = p.M <= 1 ? 128 : (p.M <= 2 ? 64 : (p.M <= 4 ? 32 : 16));   // threads of a token
+    const int tok = t / width;
     float a = 0.0f;
-    if (p.x_amax_numel == 0) {
-      const T* row = x + static_cast<int64_t>(tok) * k;
-      for (int g0 = lane; g0 < pieces; g0 += 32 * 4) {
-        Raw16<T, false> raw[4];
+    if (tok < p.M) {
+      const T* xr = x + static_cast<int64_t>(tok) * k;
+      for (int g0 = t - tok * width; g0 < pieces; g0 += width * U) {
+        Raw16<T, false> part[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (g0 + u * 32 < pieces) raw[u].load(row + (g0 + u * 32) * 16);
+        for (int u = 0; u < U; ++u)
+          if (g0 + u * width < pieces) part[u].load(xr + (g0 + u * width) * 16);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (g0 + u * 32 < pieces) {
+        for (int u = 0; u < U; ++u)
+          if (g0 + u * width < pieces) {
             float v[16];
-            raw[u].widen(v);
+            part[u].widen(v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) a = fmaxf(a, fabsf(v[i]));
           }
       }
-      a = warp_max(a);
-    } else {
-      a = ld_dependent(p.x_amax + (p.x_amax_numel == 1 ? 0 : tok));
     }
-    if (lane == 0) xscale[tok] = fp8_scale_from_amax(a);
+    const int lanes = width < 32 ? width : 32;                 // of this warp on the same token
+    for (int o = lanes >> 1; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if ((t & (lanes - 1)) == 0 && tok < p.M) atomicMax(reinterpret_cast<unsigned int*>(xscale + 16 + tok), __float_as_uint(a));
+  } else if (t < p.M) {
+    xscale[16 + t] = ld_dependent(p.x_amax + (p.x_amax_numel == 1 ? 0 : t));
   }
   asm volatile("bar.sync 1, 128;" ::: "memory");
-  const int items = (kt1 - kt0) * 16 * 8;                      // 16-byte pieces of the operand tiles
-  for (int i = t; i < items; i += 128) {
-    const int kt = i >> 7, row = (i >> 3) & 15, piece = i & 7;
-    const int g = (kt0 + kt) * 8 + piece;
+  if (t < p.M) xscale[t] = fp8_scale_from_amax(xscale[16 + t]);   // for the epilogue
+  if (mine) {
     uint4 c = make_uint4(0u, 0u, 0u, 0u);
-    if (row < p.M && g < pieces) {
-      const float scale = xscale[row], y = b200q_rcp_rn(scale), lim = __fmul_rn(scale, 512.0f);
+    if (g < pieces) {
+      const float scale = fp8_scale_from_amax(xscale[16 + row]), y = b200q_rcp_rn(scale), lim = __fmul_rn(scale, 512.0f);
       const bool fast = b200q_div_fast_ok(scale);
-      Raw16<T, false> raw;
-      raw.load(x + static_cast<int64_t>(row) * k + g * 16);
       float v[16];
       raw.widen(v);
       uint32_t* w = &c.x;
@@ -161,7 +186,7 @@ __device__ __forceinline__ void small_quantize_x(const Params& p, uint8_t* xs, f
         w[j] = f32x2_to_e4m3x2(q[0], q[1]) | (f32x2_to_e4m3x2(q[2], q[3]) << 16);
       }
     }
-    *reinterpret_cast<uint4*>(xs + kt * 2048 + row * 128 + ((piece ^ (row & 7)) * 16)) = c;
+    *reinterpret_cast<uint4*>(xs + (r >> 3) * 2048 + row * 128 + (((r & 7) ^ (row & 7)) * 16)) = c;
   }
   ptx::fence_proxy_async();                                    // the tensor core reads the tiles through the async proxy
 }
@@ -329,6 +354,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     {
       const int n = n_base + wrow;
       float ws = 1.0f, wb = 0.0f, xs = 0.0f;
+      if constexpr (kOwnX) small_clear_x(p, own_x, xscale, kt1 - kt0, threadIdx.x - 64);
       if (!p.static_weights) pdl_wait();
       if (n < p.N) {
         // without the promise they may come from the kernel before this one (the one-launch form never has it): loads
@@ -341,14 +367,14 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if constexpr (NVF4) xs = __fmul_rn(ld_dependent(p.a_scales), ld_dependent(p.b_scales));
         else xs = ld_dependent(p.a_scales + static_cast<int64_t>(wrow) * p.a_scale_stride);
       }
+      if constexpr (kOwnX) {     // in front of the stores below, which wait for the scales' loads
+        small_quantize_x<XT>(p, own_x, xscale, kt0, kt1, threadIdx.x - 64);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(x_full);
+      }
       wscale[wrow] = ws;
       wbias[wrow] = wb;
       if constexpr (!kOwnX) xscale[wrow] = xs;
-    }
-    if constexpr (kOwnX) {
-      small_quantize_x<XT>(p, own_x, xscale, kt0, kt1, threadIdx.x - 64);
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(x_full);
     }
     if constexpr (NVF4) {
       // main loop: shared memory -> tensor memory for the scale tiles of every stage.  Lane l of each

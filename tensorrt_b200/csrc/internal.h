@@ -15,7 +15,8 @@ int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const f
                    float* global_scale_out, b200q_stream_t stream, bool late);
 int nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
                            float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream, bool late);
-// bf16 out [M, N] = fp8(x [M, K]) @ dequant(w [N, K])^T + bias in one launch, or 1: too many tokens, take the two above
+// bf16 out [M, N] = fp8(x [M, K]) @ dequant(w [N, K])^T + bias in one launch, or 1: not one of the
+// sizes where that is faster (gemm_fp8.cu), take fp8_quantize and the GEMM
 int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,
                      int64_t w_scales_numel, const void* bias, void* out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream);
 }  // namespace b200q

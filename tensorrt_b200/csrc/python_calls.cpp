@@ -119,8 +119,8 @@ std::optional<Tensor> fp8_linear(const Tensor& x_in, const Tensor& w, const Tens
   c10::cuda::CUDAGuard guard(dev);
   const Tensor x = x_in.contiguous();
   const int64_t n = amax == nullptr ? 0 : amax->numel(), n_scales = n == 1 ? 1 : M;
-  if (cfg.tile_n == 0 && M <= 16) {
-    Tensor out = bf16_like(x, N);
+  Tensor out = bf16_like(x, N);
+  if (cfg.tile_n == 0) {
     const int rc = b200q::fp8_linear_small(x.data_ptr(), dt, f32(amax), n, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),
                                            bias == nullptr ? nullptr : bias->data_ptr(), out.data_ptr(), M, N, K, current_stream());
     if (rc != 1) {
@@ -131,7 +131,6 @@ std::optional<Tensor> fp8_linear(const Tensor& x_in, const Tensor& w, const Tens
   Tensor scratch = at::empty({up16(M * K) + 4 * n_scales}, x.options().dtype(at::kByte));
   auto* codes = static_cast<uint8_t*>(scratch.data_ptr());
   auto* scales = reinterpret_cast<float*>(codes + up16(M * K));
-  Tensor out = bf16_like(x, N);
   const auto st = current_stream();
   if (!taken(b200q::fp8_quantize(x.data_ptr(), dt, M, K, f32(amax), n, codes, scales, st, true), "b200q_fp8_quantize")) return std::nullopt;
   must(b200q_fp8_gemm(codes, scales, n_scales, static_cast<const uint8_t*>(w.data_ptr()), f32(&ws), ws.numel(),

@@ -1,6 +1,6 @@
 """FP8 linear of a few tokens in one launch (the GEMM quantizes its activation): the same bits as the quantize kernel
-followed by the GEMM, for every way of scaling, at the edges of its range (tokens, row length, K slices of a cluster,
-ragged N and K) and just outside it."""
+followed by the GEMM, for every way of scaling, at the edges of its range (activation bytes, tokens, K tiles per CTA,
+weight tiles, ragged N and K) and outside it."""
 import pytest
 import torch
 
@@ -9,7 +9,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (1, 128, 16), (1, 130, 144), (2, 1000, 2064), (7, 257, 1040), (16, 4096, 4096), (16, 8192, 4112),
-                                   (15, 384, 4368), (9, 512, 7280), (1, 1024, 28672), (2, 28672, 32768), (1, 136, 65536), (17, 256, 1024)])
+                                   (15, 384, 4368), (9, 512, 7280), (1, 1024, 28672), (2, 28672, 32768), (1, 136, 65536), (17, 256, 1024),
+                                   (1, 1921, 16), (1, 1920, 16), (8, 4096, 1024), (8, 2049, 512), (9, 4096, 512), (2, 4100, 4096), (2, 4096, 2048),
+                                   (3, 2001, 1360), (5, 2100, 1024), (5, 2100, 1040), (7, 6144, 144), (1, 28672, 512), (1, 28672, 528),
+                                   (1, 10240, 1008), (2, 14336, 1024), (4, 28672, 256), (1, 4096, 4112), (6, 4097, 640)])
 def test_same_bits_as_two_launches(b200, m, n, k, dtype):
     capi = b200.capi
     g = torch.Generator(device="cuda").manual_seed(m * 7 + n + k)
