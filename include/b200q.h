@@ -129,10 +129,10 @@ int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, c
                          uint8_t* codes_out, uint8_t* scales_out, float* global_scale_out,
                          b200q_stream_t stream);
 /* b200q_nvfp4_quantize under the tensor's own abs-max, measured here: the same result as b200q_amax followed by
- * b200q_nvfp4_quantize.  One launch for small tensors, which need no workspace (.._workspace_bytes() is 0).  For
- * others a workspace like that of b200q_amax (first 16 bytes zero before the first use, first 8 zero again afterwards),
- * which carries the abs-max from the first launch to the second: no other call may use it, on any thread, before this
- * one has returned. */
+ * b200q_nvfp4_quantize.  One launch for tensors of up to 256 KB, which need no workspace (.._workspace_bytes() is 0
+ * where that holds for every dtype).  For others (B200Q_ERR_WORKSPACE without) a workspace like that of b200q_amax,
+ * first 16 bytes zero before the first use, first 8 zero again afterwards; it carries the abs-max from the first launch
+ * to the second, so no other call may use it, on any thread, before this one has returned. */
 size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols);
 int b200q_nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out,
                                  uint8_t* scales_out, float* global_scale_out, void* workspace, size_t workspace_bytes,

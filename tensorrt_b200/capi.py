@@ -14,6 +14,7 @@ import torch
 from . import _native
 from ._lib import cfg_ref, check, load
 
+_ERR_WORKSPACE = -5     # B200Q_ERR_WORKSPACE
 _DTYPE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 
@@ -162,12 +163,13 @@ def nvfp4_quantize_dynamic(x: torch.Tensor):
     rows, cols = _rows_cols(x)
     if cols % 16:
         raise ValueError(f"last dimension ({cols}) must be a multiple of the block size 16")
-    if load().b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols):
-        return nvfp4_quantize(x, amax(x))
     codes, scales, g = _nvfp4_out(x.shape, rows, cols, x.device)
     with torch.cuda.device(x.device):
-        check(load().b200q_nvfp4_quantize_dynamic(x.data_ptr(), _dt(x), rows, cols, codes.data_ptr(), scales.data_ptr(), g.data_ptr(), None, 0,
-                                                  _stream(x)), "b200q_nvfp4_quantize_dynamic")
+        rc = load().b200q_nvfp4_quantize_dynamic(x.data_ptr(), _dt(x), rows, cols, codes.data_ptr(), scales.data_ptr(), g.data_ptr(), None, 0,
+                                                 _stream(x))
+    if rc == _ERR_WORKSPACE:
+        return nvfp4_quantize(x, amax(x))
+    check(rc, "b200q_nvfp4_quantize_dynamic")
     return codes, scales, g
 
 

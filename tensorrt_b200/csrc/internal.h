@@ -15,6 +15,7 @@ int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const f
                    float* global_scale_out, b200q_stream_t stream, bool late);
 int nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
                            float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream, bool late);
+size_t nvfp4_dynamic_workspace_bytes(int dtype, int64_t rows, int64_t cols);   // 0: one launch
 // bf16 out [M, N] = fp8(x [M, K]) @ dequant(w [N, K])^T + bias in one launch, or 1: not one of the
 // sizes where that is faster (gemm_fp8.cu), take fp8_quantize and the GEMM
 int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,

@@ -155,7 +155,7 @@ std::optional<Tensor> nvfp4_linear(const Tensor& x_in, const Tensor& w, const Te
   const Tensor x = x_in.contiguous();
   if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 32 != 0) return std::nullopt;
   const int64_t M = x.numel() / K, sf_bytes = static_cast<int64_t>(b200q_nvfp4_scale_bytes(M, K));
-  const int64_t ws_bytes = amax == nullptr ? static_cast<int64_t>(b200q_nvfp4_quantize_dynamic_workspace_bytes(M, K)) : 0;
+  const int64_t ws_bytes = amax == nullptr ? static_cast<int64_t>(b200q::nvfp4_dynamic_workspace_bytes(dt, M, K)) : 0;
   const int64_t code_bytes = up16(M * K / 2);
   Tensor scratch = at::empty({code_bytes + sf_bytes + 16 + ws_bytes}, x.options().dtype(at::kByte));
   auto* codes = static_cast<uint8_t*>(scratch.data_ptr());

@@ -177,12 +177,20 @@ nvfp4_quantize_kernel(const T* __restrict__ x, const float* __restrict__ amax, u
   }
 }
 
-// Quantize of a small tensor under its own abs-max, measured in the same launch: every CTA reads the whole tensor (at
-// most kDynamicMaxElems elements, from L2 after the first) for the maximum and quantizes its share.  A decode step's
-// activation is a few hundred KB at most: three launches in a row (a cleared result, the abs-max, the quantize) cost
-// more than reading it 16 times over.  A thread owns one block; rows take a multiple of four blocks (one scale word),
-// the rows that pad the last 128-row scale tile only clear their words.
-constexpr int64_t kDynamicMaxElems = 1 << 17;
+// Quantize of a small tensor under its own abs-max, measured in the same launch: every CTA that has blocks of its own
+// reads the whole tensor (from L2 after the first) for the maximum and quantizes its share; three launches in a row (a
+// cleared result, the abs-max, the quantize) cost more.  A thread owns one block; rows take a multiple of four blocks (one
+// scale word), the rows that pad the last 128-row scale tile only clear their words.
+// Taken up to 256 KB (8 to 64 CTAs read them, 128 at 16 columns) and 2048 CTAs.  Measured against abs-max and quantize in
+// a graph, 1 to 4096 rows: at most 128 KB 0.43 to 0.80 of their time in 16 bits, 0.53 to 0.69 in fp32; at 256 KB 0.65 to 1.05
+// and 0.60 to 1.00; fp32 of 384 to 512 KB 0.97 to 1.74 (16 x 8192: 8.2 us against 5.2); a single row of 98304, whose
+// padding is 3072 CTAs, 7.9 against 6.9.
+constexpr int64_t kDynamicMaxBytes = 1 << 18, kDynamicMaxCtas = 2048;
+bool dynamic_in_one_launch(int dtype, int64_t rows, int64_t cols) {
+  if (rows <= 0 || cols <= 0) return true;
+  if (rows > kDynamicMaxBytes / (dtype == B200Q_F32 ? 4 : 2) / cols) return false;
+  return (rows + 127) / 128 * 128 * ((cols / 16 + 3) / 4 * 4) <= kDynamicMaxCtas * kThreads;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -236,7 +244,7 @@ nvfp4_quantize_dynamic_kernel(const T* __restrict__ x, uint8_t* __restrict__ cod
 template <typename T>
 int launch_dynamic(const void* x, uint8_t* codes, uint8_t* sf, float* gout, int64_t rows, int64_t cols, cudaStream_t st, bool late) {
   const uint32_t bpr = static_cast<uint32_t>(cols >> 4), col_tiles = (bpr + 3u) >> 2;
-  const uint32_t units = static_cast<uint32_t>((rows + 127) / 128 * 128) * col_tiles * 4u;   // rows <= 8192, bpr <= 8192: < 2^26
+  const uint32_t units = static_cast<uint32_t>((rows + 127) / 128 * 128) * col_tiles * 4u;   // at most kDynamicMaxCtas * kThreads
   launch_pdl(nvfp4_quantize_dynamic_kernel<T>, dim3((units + kThreads - 1) / kThreads), dim3(kThreads), 0, st, static_cast<const T*>(x), codes,
              sf, gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), bpr, col_tiles, units, late);
   return check_launch();
@@ -319,13 +327,17 @@ int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const f
   }
 }
 
+size_t nvfp4_dynamic_workspace_bytes(int dtype, int64_t rows, int64_t cols) {
+  return dynamic_in_one_launch(dtype, rows, cols) ? 0 : b200q_amax_workspace_bytes();
+}
+
 int nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,
                                  float* global_scale_out, void* workspace, size_t workspace_bytes, b200q_stream_t stream, bool late) {
   if (int rc = validate(x, dtype, rows, cols, reinterpret_cast<const float*>(x))) return rc;
   if (rows == 0 || cols == 0) return B200Q_OK;
   if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
   if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
-  const size_t need = b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols);
+  const size_t need = nvfp4_dynamic_workspace_bytes(dtype, rows, cols);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need)) return B200Q_ERR_WORKSPACE;
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -359,7 +371,7 @@ int b200q_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, c
 }
 
 size_t b200q_nvfp4_quantize_dynamic_workspace_bytes(int64_t rows, int64_t cols) {
-  return rows <= 0 || cols <= 0 || rows <= kDynamicMaxElems / cols ? 0 : b200q_amax_workspace_bytes();
+  return nvfp4_dynamic_workspace_bytes(B200Q_F32, rows, cols);     // enough for every type
 }
 
 int b200q_nvfp4_quantize_dynamic(const void* x, int dtype, int64_t rows, int64_t cols, uint8_t* codes_out, uint8_t* scales_out,

@@ -366,6 +366,8 @@ def test_measured_nvfp4_range_survives_a_call_of_another_thread_in_between(b200,
 
         def b200q_nvfp4_quantize_dynamic(self, x, dt, rows, cols, codes, scales, g, ws, ws_bytes, st):
             if real.b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols):
+                if ws is None:
+                    return -5
                 self.measure(x, ws + 8)
                 seen.append((x, memory[ws + 8]))
             return 0
@@ -426,3 +428,17 @@ def test_python_extension_is_built_again_for_another_interpreter(b200, monkeypat
     assert _build.build_torch_shim() == _build.TORCH_LIB
     with pytest.raises(Compiled):
         _build.build_python_calls()
+
+
+@pytest.mark.parametrize("dtype,rows,cols,one_launch", [(2, 128, 1024, True), (2, 128, 1040, False), (1, 16, 8192, True), (0, 16, 4096, True),
+                                                        (0, 16, 4112, False), (0, 128, 1024, False), (2, 1, 65536, True), (2, 1, 65600, False),
+                                                        (2, 2, 65536, True), (0, 1, 65536, True), (2, 8192, 16, True), (2, 0, 64, True)])
+def test_sizes_that_the_nvfp4_quantize_takes_in_one_launch(b200, dtype, rows, cols, one_launch):
+    """Up to 256 KB and 2048 CTAs; beyond that the entry point asks for the workspace before it looks for a device."""
+    from tensorrt_b200 import _lib
+
+    lib = _lib.load()
+    p = (ctypes.addressof(ctypes.create_string_buffer(8192)) + 255) & ~255
+    if not torch.cuda.is_available():      # the pointers are not the device's
+        assert (lib.b200q_nvfp4_quantize_dynamic(p, dtype, rows, cols, p, p, p, None, 0, None) != -5) == one_launch
+    assert one_launch or lib.b200q_nvfp4_quantize_dynamic_workspace_bytes(rows, cols) == lib.b200q_amax_workspace_bytes()
