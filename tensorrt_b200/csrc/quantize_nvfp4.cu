@@ -195,7 +195,7 @@ bool dynamic_in_one_launch(int dtype, int64_t rows, int64_t cols) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 nvfp4_quantize_dynamic_kernel(const T* __restrict__ x, uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, float* __restrict__ gout,
-                              uint32_t rows, uint32_t cols, uint32_t blocks_per_row, uint32_t col_tiles, uint32_t units, bool late) {
+                              uint32_t rows, uint32_t blocks_per_row, uint32_t col_tiles, uint32_t units, bool late) {
   __shared__ float red[kThreads / 32];
   pdl_enter(late);
   const uint32_t unit = blockIdx.x * kThreads + threadIdx.x;
@@ -246,7 +246,7 @@ int launch_dynamic(const void* x, uint8_t* codes, uint8_t* sf, float* gout, int6
   const uint32_t bpr = static_cast<uint32_t>(cols >> 4), col_tiles = (bpr + 3u) >> 2;
   const uint32_t units = static_cast<uint32_t>((rows + 127) / 128 * 128) * col_tiles * 4u;   // at most kDynamicMaxCtas * kThreads
   launch_pdl(nvfp4_quantize_dynamic_kernel<T>, dim3((units + kThreads - 1) / kThreads), dim3(kThreads), 0, st, static_cast<const T*>(x), codes,
-             sf, gout, static_cast<uint32_t>(rows), static_cast<uint32_t>(cols), bpr, col_tiles, units, late);
+             sf, gout, static_cast<uint32_t>(rows), bpr, col_tiles, units, late);
   return check_launch();
 }
 
@@ -311,14 +311,14 @@ int validate(const void* x, int dtype, int64_t rows, int64_t cols, const float* 
 }
 
 }  // namespace
-int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, uint8_t* codes_out,
-                         uint8_t* scales_out, float* global_scale_out, b200q_stream_t stream, bool late) {
+
+int nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t cols, const float* amax, uint8_t* codes_out, uint8_t* scales_out,
+                   float* global_scale_out, b200q_stream_t stream, bool late) {
   if (int rc = validate(x, dtype, rows, cols, amax)) return rc;
   if (rows == 0 || cols == 0) return B200Q_OK;
   if (codes_out == nullptr || scales_out == nullptr) return B200Q_ERR_INVALID;
   if (!aligned(codes_out, 8) || !aligned(scales_out, 16)) return B200Q_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
-  if (rows == 0 || cols == 0) return B200Q_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
     case B200Q_BF16: return launch<__nv_bfloat16, false>(x, amax, codes_out, scales_out, nullptr, global_scale_out, rows, cols, st, ExpandMap{}, late);
