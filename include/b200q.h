@@ -152,8 +152,9 @@ int b200q_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales_swizzled,
  * Last argument of the GEMM entry points and of the peer-memory reductions; NULL = all defaults.
  * Nothing here is process-wide: two callers (threads, stacks, graphs) never see each other's choices.
  *   tile_n          GEMM tile selection.  0 = chosen per problem (default); 128 or 256 = single-CTA
- *                   tiles of 128 x tile_n; 512 = CTA-pair kernels (256 x 256 tiles, cta_group::2; chosen
- *                   automatically when the problem has at least one such tile per SM pair);
+ *                   tiles of 128 x tile_n; 512 = CTA-pair kernels (256 x 256 tiles, cta_group::2).  The
+ *                   choice takes the one whose rounds of tiles over the SMs (SM pairs) cost least; the
+ *                   reduce-scatter forms take pairs from one such tile per SM pair on (NVFP4: never);
  *                   1001 / 1002 / 1004 / 1008 = small-M kernel (weights on the tensor core's M side,
  *                   K split over a cluster of 1 / 2 / 4 / 8 CTAs, partial tiles summed through
  *                   distributed shared memory; chosen automatically for M <= 128, ignored for larger
@@ -412,7 +413,8 @@ int b200q_silu_mul_fp8_quantize(const void* gate_up, uint8_t* codes_out, float* 
                                 b200q_stream_t stream);
 /* The NVFP4 forms under a calibrated tensor amax (one fp32 on the device): the same codes, swizzled block scales
  * (padding rows zero) and global scale as rms_norm of h + delta / silu_mul / expand_heads followed by
- * b200q_nvfp4_quantize, without the bf16 tensor in between.  bf16 in.  add_rms_norm: cols % 16 == 0, cols <= 16384;
+ * b200q_nvfp4_quantize, without the bf16 tensor in between (add_rms_norm with fewer than two rows per SM and at least
+ * 2048 columns: up to the order in which the squares of a row are added).  bf16 in.  add_rms_norm: cols % 16 == 0, cols <= 16384;
  * silu_mul: f % 16 == 0, gate_up 32-byte aligned; expand_heads: head_dim, src_stride, src_col0 multiples of 16, src
  * 32-byte aligned, the slice src_col0 + heads_out / rep * head_dim within src_stride.  global_scale_out may be NULL. */
 int b200q_add_rms_norm_nvfp4_quantize(const void* h, const void* delta, const void* weight, void* h_out, const float* amax,

@@ -116,7 +116,8 @@ rms_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // PARTS > 1: a cluster of PARTS CTAs shares one token (few tokens: a decode step); the slices'
 // sums of squares and maxima meet through distributed shared memory, summed in rank order.
 // NVF4: the normalised row leaves as NVFP4 codes and block scales under a calibrated tensor amax (`nv`) instead of
-// per-token FP8; no row maximum is needed (8192 x 4096 through the ring-fed form below: 63 us, add + norm + quantize 77).  CTAs of the rows that only pad the last 128-row scale tile clear theirs.
+// per-token FP8; no row maximum is needed (8192 x 4096 through the ring-fed form below: 63 us, add + norm + quantize 77).
+// CTAs of the rows that only pad the last 128-row scale tile clear theirs.
 template <int ITEMS, int PARTS, bool NVF4>
 __global__ void __launch_bounds__(kThreads)
 add_norm_quant_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,

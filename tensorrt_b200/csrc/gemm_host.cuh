@@ -308,10 +308,12 @@ int forced_smallm_stages();  // from the environment variable B200Q_SMALLM_STAGE
 // a whole number of rounds, or with few rows, to the finer tiles (333 x 10240 x 8192 FP8: 80 pair tiles on 74 pairs are
 // two rounds, 48.0 us; 120 tiles of 128 x 256 are one, 32.6).  A single round of the small tile is not half of the big one's:
 // both wait for the same K loop.  The percentages are from a sweep of the three kernels over 14 row counts (129 to 4096)
-// and seven weight shapes in each format: the rule takes the fastest kernel or one within 1.6 % of it at all 196
-// points.  The choice by tile counts before it was 10 % slower on average and 2.0 times at worst (NVFP4 4096 x
-// 14336 at 600 to 1000 rows: 48 to 64 pair tiles, 57 to 59 us on 128 x 128 tiles, 29.0 to 29.5 on pairs).  The reduce-scatter epilogue keeps the choice by tile counts that
-// its NVLink overlap was measured with.
+// and seven weight shapes in each format.  Over these 196 points the rule takes 1.003 of the fastest kernel's time on
+// average; at worst 1.09, FP8 with K = 4096 and a single round of either tile, where 128 x 256 would win (4096 x 4096 at 600
+// rows 17.7 us against 16.3; at K = 14336 the pair does, 42.9 against 47.5).  The choice by tile counts before it was 14 %
+// slower on average and 2.2 times at worst (NVFP4 4096 x 14336 at 600 to 1000 rows: 48 to 64 pair tiles, 57 to 59 us on
+// 128 x 128 tiles, 28.7 to 29.3 on pairs).  The reduce-scatter epilogue keeps the choice by tile counts that its NVLink
+// overlap was measured with.
 constexpr int kTile256Fp8 = 110, kTile128Fp8 = 85, kTile256Nv = 145, kTile128Nv = 110;   // per cent of a pair tile
 inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
   const int64_t pair = static_cast<int64_t>((M + kPairM - 1) / kPairM) * ((N + kPairN - 1) / kPairN);

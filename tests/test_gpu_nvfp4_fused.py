@@ -1,6 +1,7 @@
 """Kernels that quantize to NVFP4 what they produce (residual add + RMSNorm, silu(gate) * up, repeated kv heads) under a
 calibrated amax: codes, swizzled scales (padding rows included) and global scale equal the separate kernels' bit for
-bit, at row counts around 128-row scale tiles and at the edges of their launch shapes."""
+bit, at row counts around 128-row scale tiles and at the edges of their launch shapes.  Where the norm splits a row over
+a cluster it adds the squares in another order; codes may then differ as rarely as a bf16 rounding does."""
 import pytest
 import torch
 
@@ -23,10 +24,17 @@ def test_add_rms_norm(b200, rows, cols, with_delta):
     delta = d if with_delta else None
     h_ref = capi.add(h, d) if with_delta else h
     x = capi.rms_norm(h_ref, w)
+    split = rows < 2 * torch.cuda.get_device_properties(0).multi_processor_count and cols >= 2048     # a row on several CTAs
     for amax in (capi.amax(x), capi.amax(x) * 0.25, torch.zeros((), device="cuda")):
         h_new, got = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)
         assert torch.equal(h_new, h_ref)
-        _same(got, capi.nvfp4_quantize(x, amax))
+        ref = capi.nvfp4_quantize(x, amax)
+        if split:
+            # the sum's last bits move rsqrt and the products by up to 2 ulp of fp32, one in 2^14 bf16 roundings at most
+            assert torch.equal(got[2], ref[2])
+            assert all(int((a != b).sum()) <= max(1, b.numel() >> 13) for a, b in zip(got[:2], ref[:2]))
+        else:
+            _same(got, ref)
     assert capi.device_status() == 0
 
 
