@@ -19,6 +19,15 @@
 // core is a few per cent of a decoder layer's arithmetic, so the repeated Q K^T is cheaper than a
 // rescaling scheme whose quantization points would differ from the definition above.
 //
+// What bounds it: the exponentials, two per score at 16 per clock and SM: 1024 clocks per 128 x 128 tile and pass, and
+// two warps per scheduler and CTA reach 0.93 of that rate in a loop of their own.  What it loses beside them is warps
+// that wait for scores.  So a softmax thread takes its 64 scores of a tile into registers and hands the tensor-memory
+// buffer back before it computes (the tensor core fills it under the exponentials); in pass 2 the scores of tile j + 2
+// are issued in front of the product of tile j (wait for scores per tile 819 -> 171 clocks of about 2500); edge tiles
+// have their own copy of the loop; query tiles with the most keys start first.  Order and roundings per row are those
+// of a loop over 32-column pieces.  [4, 32 / 8, 2048, 128] causal: 300 -> 245 us for the call; 74 heads of
+// 4096 x 4096: 960 -> 870 us.
+//
 // One CTA per (batch, head, 128 queries): warp 0 = TMA producer, warp 1 = MMA issue + tensor-memory
 // allocation, warps 2-9 = softmax (two threads per query row, each half of the columns; lane quarter = warp & 3).  K and Q tiles are
 // [rows, D] with D bytes per row (K-major), V is supplied TRANSPOSED per head ([D, keys], produced by
@@ -28,6 +37,8 @@
 #include "tcgen05.cuh"
 
 #include <cuda.h>
+
+#include <type_traits>
 
 namespace b200q {
 namespace gemm {
@@ -45,11 +56,10 @@ constexpr int kTile = 128;                 // queries per CTA, keys per step, pa
 constexpr int kTileBytes = kTile * 128;    // one operand tile: 128 rows x 128 bytes
 // Two CTAs per SM: while one waits for its tensor-core results the other's softmax warps have the issue
 // slots.  Per CTA that leaves 6 operand tiles of shared memory (Q, 2 K stages, 1 V stage, 2 P tiles) and
-// 256 columns of tensor memory: one output accumulator and one score tile.  The score tile is computed
-// and consumed as two halves of 64 keys (two buffers of 64 columns), so that the tensor core fills one
-// half while the softmax warps work on the other.
-constexpr int kKStages = 2, kVStages = 1, kSBufs = 2;
-constexpr int kHalf = kTile / 2;           // keys per score buffer
+// 256 columns of tensor memory.  Columns 0-127 hold a score tile; columns 128-255 a second one in pass 1
+// and the output accumulator in pass 2.
+constexpr int kKStages = 2, kVStages = 1;
+constexpr int kChunk = 32;                 // score columns of one step of a softmax thread
 constexpr int kTmemCols = 256;
 constexpr int kAttSmem = 1024 + kTileBytes * (1 + kKStages + kVStages + 2) + 4096;   // tail: barriers, row statistics
 
@@ -61,6 +71,7 @@ struct AttParams {
   int64_t out_sb, out_sh, out_ss;
   int out_dtype;
   int Hq, Hkv, Sq, Sk, D;
+  int BH, q_tiles;          // B * Hq, tiles of 128 queries
   float softmax_scale;
   int causal;
   int* status;
@@ -73,6 +84,37 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// two fp32 values in one 64-bit register: one issue slot for two fused multiply-adds
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// four fp32 -> four E4M3 bytes in one register
+__device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, float d) {
+  uint32_t r;
+  asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\t"
+      "mov.b32 %0, {lo, hi};\n\t}"
+      : "=r"(r)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
 }
 
 __global__ void __launch_bounds__(kAttThreads, 2)
@@ -91,16 +133,18 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint64_t* v_full = k_empty + kKStages;
   uint64_t* v_empty = v_full + kVStages;
   uint64_t* s_full = v_empty + kVStages;     // score buffers in tensor memory
-  uint64_t* s_empty = s_full + kSBufs;
-  uint64_t* p_full = s_empty + kSBufs;       // 2 probability tiles in shared memory
+  uint64_t* s_empty = s_full + 2;
+  uint64_t* p_full = s_empty + 2;            // 2 probability tiles in shared memory
   uint64_t* p_empty = p_full + 2;
   uint64_t* o_full = p_empty + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 1);
   float2* row_stat = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + 1024);   // [2][kTile] (max, sum) of each column half
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * kTile;
-  const int bh = blockIdx.y;                                  // b * Hq + h
+  // the query tiles with the most keys first: a causal launch then ends on its shortest CTAs
+  const int q_tile = static_cast<int>(blockIdx.x) / p.BH;
+  const int q0 = (p.q_tiles - 1 - q_tile) * kTile;
+  const int bh = static_cast<int>(blockIdx.x) - q_tile * p.BH;   // b * Hq + h
   const int b = bh / p.Hq, h = bh - b * p.Hq;
   const int bhkv = b * p.Hkv + h / (p.Hq / p.Hkv);
   const int shift = p.Sk - p.Sq;                              // causal: key j visible to query i when j <= i + shift
@@ -112,19 +156,22 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     ptx::mbar_init(q_full, 1);
     for (int s = 0; s < kKStages; ++s) ptx::mbar_init(k_full + s, 1), ptx::mbar_init(k_empty + s, 1);
     for (int s = 0; s < kVStages; ++s) ptx::mbar_init(v_full + s, 1), ptx::mbar_init(v_empty + s, 1);
-    for (int s = 0; s < kSBufs; ++s) {
+    for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(s_full + s, 1);
       ptx::mbar_init(s_empty + s, 8);   // one arrival per softmax warp
-    }
-    for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(p_full + s, 8);
       ptx::mbar_init(p_empty + s, 1);
     }
     ptx::mbar_init(o_full, 1);
     ptx::fence_barrier_init();
-    ptx::prefetch_tmap(&tmap_q);
-    ptx::prefetch_tmap(&tmap_k);
     ptx::prefetch_tmap(&tmap_vt);
+    // this thread is the producer: the first tiles are requested in front of the tensor-memory allocation
+    ptx::mbar_arrive_expect_tx(q_full, kTileBytes);
+    ptx::tma_load_3d(sq, &tmap_q, q_full, 0, q0, bh);
+    if (n_tiles > 0) {
+      ptx::mbar_arrive_expect_tx(k_full, kTileBytes);
+      ptx::tma_load_3d(sk, &tmap_k, k_full, 0, 0, bhkv);
+    }
   }
   if (warp == 1) {
     ptx::tmem_alloc<1>(tmem_holder, kTmemCols);
@@ -134,37 +181,40 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tmem_o = tmem_base + kSBufs * kHalf;
+  const uint32_t tmem_o = tmem_base + kTile;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      ptx::mbar_arrive_expect_tx(q_full, kTileBytes);
-      ptx::tma_load_3d(sq, &tmap_q, q_full, 0, q0, bh);
-      int ks = 0, vs = 0;
+      int ks = n_tiles > 0 ? 1 : 0, vs = 0;       // Q and the first K tile are on their way (above)
       uint32_t kph = 0, vph = 0;
       bool ok = true;
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-        for (int j = 0; j < n_tiles; ++j) {
-          if (!ptx::mbar_wait(k_empty + ks, kph ^ 1u)) {
-            att_timeout(p.status, 61);
-            ok = false;
-            break;
-          }
-          ptx::mbar_arrive_expect_tx(k_full + ks, kTileBytes);
-          ptx::tma_load_3d(sk + ks * kTileBytes, &tmap_k, k_full + ks, 0, j * kTile, bhkv);
-          if (++ks == kKStages) ks = 0, kph ^= 1u;
-          if (pass == 1) {
-            if (!ptx::mbar_wait(v_empty + vs, vph ^ 1u)) {
-              att_timeout(p.status, 62);
-              ok = false;
-              break;
-            }
-            ptx::mbar_arrive_expect_tx(v_full + vs, kTileBytes);
-            ptx::tma_load_3d(sv + vs * kTileBytes, &tmap_vt, v_full + vs, j * kTile, 0, bhkv);
-            if (++vs == kVStages) vs = 0, vph ^= 1u;
-          }
+      // the order of the loads is the order in which the MMA thread uses them: pass 1 all K tiles; pass 2 K 0, K 1,
+      // K 2, V 0, K 3, V 1, ...
+      auto load_k = [&](int j) -> bool {
+        if (!ptx::mbar_wait(k_empty + ks, kph ^ 1u)) {
+          att_timeout(p.status, 61);
+          return false;
         }
+        ptx::mbar_arrive_expect_tx(k_full + ks, kTileBytes);
+        ptx::tma_load_3d(sk + ks * kTileBytes, &tmap_k, k_full + ks, 0, j * kTile, bhkv);
+        if (++ks == kKStages) ks = 0, kph ^= 1u;
+        return true;
+      };
+      auto load_v = [&](int j) -> bool {
+        if (!ptx::mbar_wait(v_empty + vs, vph ^ 1u)) {
+          att_timeout(p.status, 62);
+          return false;
+        }
+        ptx::mbar_arrive_expect_tx(v_full + vs, kTileBytes);
+        ptx::tma_load_3d(sv + vs * kTileBytes, &tmap_vt, v_full + vs, j * kTile, 0, bhkv);
+        if (++vs == kVStages) vs = 0, vph ^= 1u;
+        return true;
+      };
+      for (int j = 1; j < n_tiles && ok; ++j) ok = load_k(j);
+      for (int j = 0; j < n_tiles + 2 && ok; ++j) {
+        if (j < n_tiles) ok = load_k(j);
+        if (ok && j >= 2) ok = load_v(j - 2);
       }
       // drain: every load issued above has landed and was consumed before shared memory is released
       for (int s = 0; s < kKStages && ok; ++s) {
@@ -181,45 +231,44 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t idesc = ptx::idesc_f8(kTile, kTile);
+      constexpr uint32_t idesc_s = ptx::idesc_f8(kTile, kTile);
+      const uint32_t idesc_o = ptx::idesc_f8(kTile, p.D);       // only the head's own columns
+      const int kb_scores = (p.D + 31) / 32;                    // 32 bytes of the head dimension per MMA
       const uint32_t q_lo = ptx::desc_lo_sw128(ptx::smem_u32(sq));
       const uint32_t k_lo0 = ptx::desc_lo_sw128(ptx::smem_u32(sk));
       const uint32_t v_lo0 = ptx::desc_lo_sw128(ptx::smem_u32(sv));
       const uint32_t p_lo0 = ptx::desc_lo_sw128(ptx::smem_u32(sp));
-      int ks = 0, vs = 0, sb = 0, pb = 0;
-      uint32_t kph = 0, vph = 0, sph = 0, pph = 0;
+      int ks = 0, vs = 0, pb = 0;
+      uint32_t kph = 0, vph = 0, pph = 0;
+      uint32_t sph0 = 0, sph1 = 0;                              // score buffers: parity of their next use
       bool ok = ptx::mbar_wait(q_full, 0);
       if (!ok) att_timeout(p.status, 65);
-      // S[sb] = Q K^T for the two halves (64 keys each) of the next key tile in ring order
-      constexpr uint32_t idesc_half = ptx::idesc_f8(kTile, kHalf);
-      auto issue_scores = [&]() -> bool {
-        if (!ptx::mbar_wait(k_full + ks, kph)) {
+      // scores of the next key tile in ring order into score buffer `sb`
+      auto issue_scores = [&](int sb) -> bool {
+        const uint32_t sph = sb == 0 ? sph0 : sph1;
+        if (!ptx::mbar_wait(k_full + ks, kph) || !ptx::mbar_wait(s_empty + sb, sph ^ 1u)) {
           att_timeout(p.status, 66);
           return false;
         }
-        for (int hh = 0; hh < 2; ++hh) {
-          if (!ptx::mbar_wait(s_empty + sb, sph ^ 1u)) {
-            att_timeout(p.status, 66);
-            return false;
-          }
-          ptx::tc_fence_after();
-          // keys 64 hh .. 64 hh + 63 of the stage: 64 rows of 128 bytes further on (whole swizzle atoms)
-          const uint32_t k_lo = k_lo0 + ks * (kTileBytes >> 4) + hh * ((kHalf * 128) >> 4);
-#pragma unroll
-          for (int kb = 0; kb < 4; ++kb)
-            ptx::mma_f8<1>(tmem_base + sb * kHalf, ptx::desc_join(q_lo + kb * 2, ptx::kDescHiSw128),
-                           ptx::desc_join(k_lo + kb * 2, ptx::kDescHiSw128), idesc_half, kb > 0 ? 1u : 0u);
-          ptx::tc_commit<1>(s_full + sb);
-          if (++sb == kSBufs) sb = 0, sph ^= 1u;
-        }
+        ptx::tc_fence_after();
+        const uint32_t k_lo = k_lo0 + ks * (kTileBytes >> 4);
+        for (int kb = 0; kb < kb_scores; ++kb)
+          ptx::mma_f8<1>(tmem_base + sb * kTile, ptx::desc_join(q_lo + kb * 2, ptx::kDescHiSw128),
+                         ptx::desc_join(k_lo + kb * 2, ptx::kDescHiSw128), idesc_s, kb > 0 ? 1u : 0u);
+        ptx::tc_commit<1>(s_full + sb);
         ptx::tc_commit<1>(k_empty + ks);
+        if (sb == 0) sph0 ^= 1u;
+        else sph1 ^= 1u;
         if (++ks == kKStages) ks = 0, kph ^= 1u;
         return true;
       };
-      for (int j = 0; j < n_tiles && ok; ++j) ok = issue_scores();         // pass 1: scores only
-      if (ok && n_tiles > 0) ok = issue_scores();                          // pass 2, first tile
+      for (int j = 0; j < n_tiles && ok; ++j) ok = issue_scores(j & 1);    // pass 1: scores only, two buffers
+      // pass 2: the scores of tile j + 2 are issued in front of the product of tile j.  Their buffer is free once every
+      // warp has taken tile j + 1, which it does right after writing its part of P j: the warps wait for scores, nobody
+      // waits for the product yet.
+      for (int j = 0; j < min(2, n_tiles) && ok; ++j) ok = issue_scores(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) ok = issue_scores();                          // scores of tile j + 1 under the softmax of tile j
+        if (j + 2 < n_tiles) ok = issue_scores(0);
         if (!ok) break;
         if (!ptx::mbar_wait(p_full + pb, pph) || !ptx::mbar_wait(v_full + vs, vph)) {
           att_timeout(p.status, 67);
@@ -232,7 +281,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int kb = 0; kb < 4; ++kb)
           ptx::mma_f8<1>(tmem_o, ptx::desc_join(p_lo + kb * 2, ptx::kDescHiSw128), ptx::desc_join(v_lo + kb * 2, ptx::kDescHiSw128),
-                         idesc, (j > 0 || kb > 0) ? 1u : 0u);
+                         idesc_o, (j > 0 || kb > 0) ? 1u : 0u);
         ptx::tc_commit<1>(p_empty + pb);
         ptx::tc_commit<1>(v_empty + vs);
         if (++vs == kVStages) vs = 0, vph ^= 1u;
@@ -243,7 +292,9 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   } else {
     // ------------------------------------------------------------ softmax (warps 2..9): two threads per query row.
     // A warp reaches the 32 tensor-memory lanes of its quarter (warp & 3); the two warps of a quarter split
-    // the columns: of every 64-key score buffer (and of the output) warp set `ch` takes the 32-column chunk ch.
+    // the columns: warp set `ch` takes the 32-column chunks ch and ch + 2 of every score tile (columns 32 ch .. and
+    // 64 + 32 ch ..).  A thread takes both into registers and hands the buffer back before it computes, so the
+    // tensor core fills the next tile under the exponentials of this one.
     const int q = warp & 3;
     const int ch = (warp - 2) >> 2;
     const int r = q * 32 + lane;                  // row inside the tile
@@ -252,66 +303,81 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // scores in the base-2 exponent domain: s2 = acc * c2, c2 = q_scale * k_scale * softmax_scale * log2(e) > 0,
     // so the running maximum is kept on the raw accumulators and the scaling rides in the FMA in front of ex2
     const float c2 = __ldg(p.q_scale) * __ldg(p.k_scale) * p.softmax_scale * 1.4426950408889634f;
+    const uint64_t c2c2 = pack2(c2, c2);
     const int last_key = p.causal ? min(k_end - 1, qi + shift) : k_end - 1;   // keys beyond it are masked for this row
     // key tiles below this index are visible to every row of the CTA in full: no per-element mask there
     const int full_tiles = (p.causal ? max(0, min(k_end, q0 + shift + 1)) : k_end) / kTile;
-    int sb = 0, pb = 0;
-    uint32_t sph = 0, pph = 0;
+    int pb = 0;
+    uint32_t sph0 = 0, sph1 = 0, pph = 0;
     float m = -INFINITY, l = 0.0f;                // raw-accumulator maximum, sum of 2^(s2 - m * c2)
     bool ok = true;
-    // ---- pass 1: running maximum and sum, one half tile (64 keys) per step
-    for (int t = 0; t < 2 * n_tiles && ok; ++t) {
-      if (!ptx::mbar_wait(s_full + sb, sph)) {
-        att_timeout(p.status, 68);
-        ok = false;
-        break;
-      }
+    // scores of key tile j (buffer sb) into v (chunk ch, then chunk ch + 2), masked; false when the wait gave up
+    auto take_scores = [&](auto masked, int j, int sb, uint32_t* v) -> bool {
+      if (!ptx::mbar_wait(s_full + sb, sb == 0 ? sph0 : sph1)) return false;
+      if (sb == 0) sph0 ^= 1u;
+      else sph1 ^= 1u;
       ptx::tc_fence_after();
-      const bool masked = (t >> 1) >= full_tiles;
-      {
-        const int c = ch;
-        uint32_t v[32];
-        ptx::tmem_ld_32x32(tmem_base + lane_addr + sb * kHalf + c * 32, v);
-        ptx::tmem_ld_wait();
-        if (masked) {
-          const int key0 = t * kHalf + c * 32;
+      const uint32_t taddr = tmem_base + lane_addr + sb * kTile + ch * kChunk;
+      ptx::tmem_ld_32x32(taddr, v);
+      ptx::tmem_ld_32x32(taddr + 2 * kChunk, v + kChunk);
+      ptx::tmem_ld_wait();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(s_empty + sb);
+      if constexpr (decltype(masked)::value) {
+        const int visible = last_key - (j * kTile + ch * kChunk);      // index of the last visible column, from the first chunk's start
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (key0 + i > last_key) v[i] = 0xff800000u;   // -inf
+        for (int i = 0; i < kChunk; ++i) {
+          if (i > visible) v[i] = 0xff800000u;   // -inf
+          if (i + 2 * kChunk > visible) v[kChunk + i] = 0xff800000u;
         }
+      }
+      return true;
+    };
+    // ---- pass 1: running maximum and sum
+    auto pass1 = [&](auto masked, int j) -> bool {
+      uint32_t vv[2 * kChunk];
+      if (!take_scores(masked, j, j & 1, vv)) {
+        att_timeout(p.status, 68);
+        return false;
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const uint32_t* v = vv + c * kChunk;
         // four independent chains each for the maximum and the sum: a warp has few neighbours on its scheduler
         // here, so the length of a dependent chain is what it waits for
-        float c0 = __uint_as_float(v[0]), c1 = __uint_as_float(v[1]), c2m = __uint_as_float(v[2]), c3 = __uint_as_float(v[3]);
+        float x0 = __uint_as_float(v[0]), x1 = __uint_as_float(v[1]), x2 = __uint_as_float(v[2]), x3 = __uint_as_float(v[3]);
 #pragma unroll
-        for (int i = 4; i < 32; i += 4) {
-          c0 = fmaxf(c0, __uint_as_float(v[i]));
-          c1 = fmaxf(c1, __uint_as_float(v[i + 1]));
-          c2m = fmaxf(c2m, __uint_as_float(v[i + 2]));
-          c3 = fmaxf(c3, __uint_as_float(v[i + 3]));
+        for (int i = 4; i < kChunk; i += 4) {
+          x0 = fmaxf(x0, __uint_as_float(v[i]));
+          x1 = fmaxf(x1, __uint_as_float(v[i + 1]));
+          x2 = fmaxf(x2, __uint_as_float(v[i + 2]));
+          x3 = fmaxf(x3, __uint_as_float(v[i + 3]));
         }
-        const float cm = fmaxf(fmaxf(c0, c1), fmaxf(c2m, c3));
+        const float cm = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
         if (cm > m) {
           l *= ex2_approx((m - cm) * c2);         // m = -inf: l is 0 and stays 0
           m = cm;
         }
-        if (m > -INFINITY) {
-          const float off = -m * c2;
-          float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
+        // nothing visible yet (m = -inf): offset 0, every exponential of -inf adds 0
+        const float off = m > -INFINITY ? -m * c2 : 0.0f;
+        const uint64_t offoff = pack2(off, off);
+        uint64_t l01 = 0ull, l23 = 0ull;          // pairs of zeros
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            l0 += ex2_approx(fmaf(__uint_as_float(v[i]), c2, off));
-            l1 += ex2_approx(fmaf(__uint_as_float(v[i + 1]), c2, off));
-            l2 += ex2_approx(fmaf(__uint_as_float(v[i + 2]), c2, off));
-            l3 += ex2_approx(fmaf(__uint_as_float(v[i + 3]), c2, off));
-          }
-          l += (l0 + l1) + (l2 + l3);
+        for (int i = 0; i < kChunk; i += 4) {
+          const float2 a = unpack2(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2c2, offoff));
+          const float2 b = unpack2(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c2c2, offoff));
+          l01 = add2(l01, pack2(ex2_approx(a.x), ex2_approx(a.y)));
+          l23 = add2(l23, pack2(ex2_approx(b.x), ex2_approx(b.y)));
         }
+        const float2 s0 = unpack2(l01), s1 = unpack2(l23);
+        l += (s0.x + s0.y) + (s1.x + s1.y);
       }
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(s_empty + sb);
-      if (++sb == kSBufs) sb = 0, sph ^= 1u;
-    }
+      return true;
+    };
+    const int first_edge = min(full_tiles, n_tiles);
+    for (int j = 0; j < first_edge && ok; ++j) ok = pass1(std::false_type{}, j);
+    for (int j = first_edge; j < n_tiles && ok; ++j) ok = pass1(std::true_type{}, j);
     // the two threads of a row each hold the statistics of their columns: merge (every softmax thread gets here)
     row_stat[ch * kTile + r] = make_float2(m, l);
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -326,50 +392,36 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // ---- pass 2: final probabilities, quantized with scale 1/448, written as the A operand of P V:
     // 448 * 2^(s2 - m2) / l = 2^(acc * c2 + off2) with the normaliser folded into the exponent
     const float off2 = l > 0.0f ? -m * c2 + __log2f(kE4M3Max / l) : -INFINITY;
-    for (int t = 0; t < 2 * n_tiles && ok; ++t) {
-      const int hh = t & 1;
-      if (!ptx::mbar_wait(s_full + sb, sph) || (hh == 0 && !ptx::mbar_wait(p_empty + pb, pph ^ 1u))) {
+    const uint64_t off22 = pack2(off2, off2);
+    auto pass2 = [&](auto masked, int j) -> bool {
+      uint32_t v[2 * kChunk];
+      if (!take_scores(masked, j, 0, v) || !ptx::mbar_wait(p_empty + pb, pph ^ 1u)) {
         att_timeout(p.status, 69);
-        ok = false;
-        break;
+        return false;
       }
-      ptx::tc_fence_after();
-      const bool masked = (t >> 1) >= full_tiles;
       uint8_t* prow = sp + pb * kTileBytes + r * 128;
-      {
-        const int c = ch;
-        uint32_t v[32];
-        ptx::tmem_ld_32x32(tmem_base + lane_addr + sb * kHalf + c * 32, v);
-        ptx::tmem_ld_wait();
-        if (masked) {
-          const int key0 = t * kHalf + c * 32;
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (key0 + i > last_key) v[i] = 0xff800000u;   // -inf -> probability 0
-        }
-        uint32_t w[8];
+      for (int g = 0; g < 4; ++g) {               // 16 columns = one 16-byte piece of the operand row
+        uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float pr[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) pr[e] = ex2_approx(fmaf(__uint_as_float(v[4 * i + e]), c2, off2));
-          w[i] = f32x2_to_e4m3x2(pr[0], pr[1]) | (f32x2_to_e4m3x2(pr[2], pr[3]) << 16);
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t* e = v + g * 16 + i * 4;
+          const float2 a = unpack2(fma2(pack2(__uint_as_float(e[0]), __uint_as_float(e[1])), c2c2, off22));
+          const float2 b = unpack2(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22));
+          w[i] = f32x4_to_e4m3x4(ex2_approx(a.x), ex2_approx(a.y), ex2_approx(b.x), ex2_approx(b.y));
         }
         // 128-byte swizzle of the operand layout: the 16-byte piece i of row r lives at piece i ^ (r & 7)
-        const int piece = 2 * (hh * 2 + c);
+        const int piece = 2 * ch + (g & 1) + 4 * (g >> 1);
         *reinterpret_cast<uint4*>(prow + ((piece ^ (r & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(prow + (((piece + 1) ^ (r & 7)) * 16)) = make_uint4(w[4], w[5], w[6], w[7]);
       }
-      if (hh == 1) ptx::fence_proxy_async();      // the tensor core reads this tile through the async proxy
-      ptx::tc_fence_before();
+      ptx::fence_proxy_async();                   // the tensor core reads this tile through the async proxy
       __syncwarp();
-      if (lane == 0) {
-        if (hh == 1) ptx::mbar_arrive(p_full + pb);
-        ptx::mbar_arrive(s_empty + sb);
-      }
-      if (++sb == kSBufs) sb = 0, sph ^= 1u;
-      if (hh == 1 && ++pb == 2) pb = 0, pph ^= 1u;
-    }
+      if (lane == 0) ptx::mbar_arrive(p_full + pb);
+      if (++pb == 2) pb = 0, pph ^= 1u;
+      return true;
+    };
+    for (int j = 0; j < first_edge && ok; ++j) ok = pass2(std::false_type{}, j);
+    for (int j = first_edge; j < n_tiles && ok; ++j) ok = pass2(std::true_type{}, j);
     // ---- output: O * (v_scale / 448) -> out dtype
     if (ok && n_tiles > 0 && !ptx::mbar_wait(o_full, 0)) {
       att_timeout(p.status, 70);
@@ -683,7 +735,11 @@ int b200q_fp8_sdpa_strided(const uint8_t* q_codes, const uint8_t* k_codes, const
   p.D = static_cast<int>(D);
   p.softmax_scale = softmax_scale;
   p.causal = causal ? 1 : 0;
-  const dim3 grid(static_cast<unsigned>((Sq + kTile - 1) / kTile), static_cast<unsigned>(B * Hq));
+  p.BH = static_cast<int>(B * Hq);
+  p.q_tiles = static_cast<int>((Sq + kTile - 1) / kTile);
+  const int64_t ctas = static_cast<int64_t>(p.q_tiles) * p.BH;
+  if (ctas > 0x7fffffffLL) return B200Q_ERR_INVALID;
+  const dim3 grid(static_cast<unsigned>(ctas));
   fp8_sdpa_kernel<<<grid, kAttThreads, kAttSmem, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
   return check_launch();
 }
