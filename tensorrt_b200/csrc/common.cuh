@@ -261,6 +261,41 @@ __device__ __forceinline__ float div_path(float x, float d, float y, float lim) 
   }
 }
 
+// Two fp32 values in a register pair: one issue slot for two operations, each rounded as the scalar one.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// b200q_div_by_shared of a pair of NEGATED numerators nx = (-a, -b): dd = (d, d), ny = (-RN(1/d), -RN(1/d)); gives (a / d, b / d).
+// Negating the numerator beforehand costs nothing where it is computed and keeps every step, the sign of a zero included,
+// that of the scalar form: q0 = (-a)(-y), r = d q0 + (-a), q = r (-y) + q0.
+__device__ __forceinline__ uint64_t div2_by_shared_negated(uint64_t nx, uint64_t dd, uint64_t ny) {
+  const uint64_t q0 = mul2(nx, ny);
+  return fma2(fma2(dd, q0, nx), ny, q0);
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -116,7 +116,7 @@ rms_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // PARTS > 1: a cluster of PARTS CTAs shares one token (few tokens: a decode step); the slices'
 // sums of squares and maxima meet through distributed shared memory, summed in rank order.
 // NVF4: the normalised row leaves as NVFP4 codes and block scales under a calibrated tensor amax (`nv`) instead of
-// per-token FP8; no row maximum is needed (8192 x 4096 through the ring-fed form below: 63 us, add + norm + quantize 77).
+// per-token FP8; no row maximum is needed.
 // CTAs of the rows that only pad the last 128-row scale tile clear theirs.
 template <int ITEMS, int PARTS, bool NVF4>
 __global__ void __launch_bounds__(kThreads)
@@ -229,11 +229,13 @@ add_norm_quant_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* 
   }
 }
 
-// Many-token form of add_norm_quant_kernel: persistent CTAs (two per SM) walk the rows with a stride
+// Form of add_norm_quant_kernel for many long rows that add_norm_quant_warp_kernel does not take (FP8 with a delta and more
+// than 4096 columns, inputs that are not 32-byte aligned): persistent CTAs (two per SM) walk the rows with a stride
 // of the grid, and the rows of h and delta arrive through a ring of shared-memory stages filled by
 // bulk asynchronous copies that one thread issues `stages` rows ahead.  One CTA per row keeps too few
 // bytes in flight to cover the HBM latency (its loads stop while it reduces and stores); here the
-// copies of the next rows run during all of that.  Thread-to-element mapping, arithmetic and
+// copies of the next rows run during all of that.  What is left is the chain of a row, about 2 us with its barriers: rows
+// of 4096 columns and less are bound by it.  Thread-to-element mapping, arithmetic and
 // reduction order are those of add_norm_quant_kernel, so the results are bit-identical.
 constexpr int kStreamStagesMax = 8;
 constexpr int kStreamRingBytes = 96 * 1024;
@@ -364,6 +366,207 @@ add_norm_quant_stream_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfl
     if (b200q_div_fast_ok(scale)) emit(std::true_type{});   // one branch per row, not one select per element
     else emit(std::false_type{});
   }
+}
+
+// Form for many tokens with rows of up to 8192 elements (a multiple of 16, 32-byte aligned): WPR warps (1, 2, 4 for rows of
+// up to 2048, 4096, 8192 elements) hold a row in registers, packed as bf16, four pieces of 16 elements per lane, and reduce
+// it with shuffles and one barrier between those warps.  No CTA-wide barrier stands between loading, reducing and storing,
+// so the rows of an SM stream independently.  What bounds it is issue slots beside HBM: hence bf16 pair additions for
+// h + delta, fp32 pairs for the squares, the products and the quotients (about 10 instructions an element, half of what the
+// scalar form takes).  The residual sum is one bf16 pair addition: it rounds the exact sum once, and an fp32 addition in
+// front of that rounding changes nothing (the sum of two bf16 values with more than 24 bits lies next to the larger one).
+// The squares are added in the order of add_norm_quant_kernel, whose thread t sums groups t, t + 256, ... of 8 elements and
+// whose 8 warps of 32 threads are added by a tree: lane l of a warp here plays threads 2l and 2l + 1 of two of them.
+template <int ITEMS, int WPR, bool HAS_DELTA, bool NVF4>
+__global__ void __launch_bounds__(kThreads, 2)
+add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
+                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out, uint8_t* __restrict__ codes,
+                           float* __restrict__ scales, int64_t rows, int64_t cols, float eps, const Nvfp4Out nv) {
+  constexpr int kSlots = kThreads / 32 / WPR;     // rows per CTA
+  constexpr int VP = 4 / WPR;                     // pairs of warps of the one-CTA form that this warp stands for
+  constexpr int N = ITEMS * VP;                   // pieces of 16 elements per lane
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float part[kSlots][8];
+  __shared__ float part_max[kSlots][WPR];
+  const int lane = threadIdx.x & 31, slot = (threadIdx.x >> 5) / WPR, sub = (threadIdx.x >> 5) % WPR;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * kSlots + slot;
+  const int pieces = static_cast<int>(cols >> 4);
+  if (row >= rows) {                              // the warps of a row leave together
+    if constexpr (NVF4) {
+      if (sub == 0 && row < (rows + 127) / 128 * 128) {
+        uint8_t* sf = nv.sf + (row >> 7) * static_cast<int64_t>(nv.col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+        for (uint32_t c = lane; c < nv.col_tiles; c += 32) *reinterpret_cast<uint32_t*>(sf + c * 512u) = 0u;
+      }
+    }
+    return;
+  }
+  const auto piece_of = [&](int k) { return (sub * VP + k / ITEMS) * 32 + lane + (k % ITEMS) * (kThreads / 2); };
+  const __nv_bfloat16* hr = h + row * cols;
+  U32x8 x[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int p = piece_of(k);
+    if (p < pieces) x[k] = ld_nc_256(hr + p * 16);
+    else x[k] = U32x8{};
+  }
+  if constexpr (HAS_DELTA) {
+    const __nv_bfloat16* dr = delta + row * cols;
+    U32x8 d[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (piece_of(k) < pieces) d[k] = ld_nc_256(dr + piece_of(k) * 16);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if (piece_of(k) < pieces) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const __nv_bfloat162 t = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&x[k].v[j]), *reinterpret_cast<const __nv_bfloat162*>(&d[k].v[j]));
+          x[k].v[j] = *reinterpret_cast<const uint32_t*>(&t);
+        }
+        st_256(h_out + row * cols + piece_of(k) * 16, x[k]);
+      }
+    }
+  }
+  // sums of squares of the even and the odd group of 8 (low and high half of a pair)
+  float sums[8];
+#pragma unroll
+  for (int v = 0; v < VP; ++v) {
+    uint64_t ss = 0ull;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const U32x8& t = x[v * ITEMS + i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t lo = pack2(__uint_as_float(t.v[j] << 16), __uint_as_float(t.v[4 + j] << 16));
+        const uint64_t hi = pack2(__uint_as_float(t.v[j] & 0xffff0000u), __uint_as_float(t.v[4 + j] & 0xffff0000u));
+        ss = fma2(lo, lo, ss);
+        ss = fma2(hi, hi, ss);
+      }
+    }
+    float2 s = unpack2(ss);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    sums[v] = s.x + s.y;                          // lanes 0-15: warp 2 (sub VP + v) of the one-CTA form, lanes 16-31: the next
+  }
+  if constexpr (WPR > 1) {
+    if ((lane & 15) == 0) {
+#pragma unroll
+      for (int v = 0; v < VP; ++v) part[slot][(sub * VP + v) * 2 + (lane >> 4)] = sums[v];
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(32 * WPR) : "memory");
+#pragma unroll
+    for (int v = 0; v < 8; ++v) sums[v] = part[slot][v];
+  } else {
+    float t[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) t[v] = sums[v];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      sums[2 * v] = __shfl_sync(0xffffffffu, t[v], 0);
+      sums[2 * v + 1] = __shfl_sync(0xffffffffu, t[v], 16);
+    }
+  }
+  const float total = ((sums[0] + sums[4]) + (sums[2] + sums[6])) + ((sums[1] + sums[5]) + (sums[3] + sums[7]));
+  const float inv = rsqrtf(total / static_cast<float>(cols) + eps);
+  // the normalised values, negated for the divisions below (the signs cancel there; magnitudes are the same)
+  const uint64_t ninv = pack2(-inv, -inv);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int p = piece_of(k);
+    if (p < pieces) {
+      const uint4* wp = reinterpret_cast<const uint4*>(w + p * 16);
+      const uint4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
+      const uint32_t wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint64_t xv = pack2(__uint_as_float(x[k].v[j] << 16), __uint_as_float(x[k].v[j] & 0xffff0000u));
+        const uint64_t wj = pack2(__uint_as_float(wv[j] << 16), __uint_as_float(wv[j] & 0xffff0000u));
+        const float2 t = unpack2(mul2(mul2(xv, ninv), wj));
+        const __nv_bfloat162 b = __floats2bfloat162_rn(t.x, t.y);
+        x[k].v[j] = *reinterpret_cast<const uint32_t*>(&b);
+      }
+    }
+  }
+  const auto abs_max = [](const U32x8& t) {       // of 16 values; NaN only when all are
+    __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&t.v[0]));
+#pragma unroll
+    for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&t.v[j])));
+    return fmaxf(__low2float(m), __high2float(m));
+  };
+  const auto values = [](const U32x8& t, float* f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      f[2 * j] = __uint_as_float(t.v[j] << 16);
+      f[2 * j + 1] = __uint_as_float(t.v[j] & 0xffff0000u);
+    }
+  };
+  if constexpr (NVF4) {
+    const GlobalScale gs(ld_dependent(nv.amax));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nv.gout != nullptr) *nv.gout = gs.g;
+    uint8_t* sf = nv.sf + (row >> 7) * static_cast<int64_t>(nv.col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int p = piece_of(k);
+      uint32_t sb = 0u;
+      if (p < pieces) {
+        float f[16];
+        uint32_t c[2];
+        values(x[k], f);
+        sb = quantize_negated<16>(f, abs_max(x[k]), gs, c);
+        *reinterpret_cast<uint2*>(nv.codes + row * (cols >> 1) + p * 8) = make_uint2(c[0], c[1]);
+      }
+      uint32_t word = sb << (8 * (p & 3));        // four lanes hold one scale word
+      word |= __shfl_xor_sync(0xffffffffu, word, 1);
+      word |= __shfl_xor_sync(0xffffffffu, word, 2);
+      if ((p & 3) == 0 && p < pieces) *reinterpret_cast<uint32_t*>(sf + static_cast<uint32_t>(p >> 2) * 512u) = word;
+    }
+    return;
+  }
+  float amax = 0.0f;
+#pragma unroll
+  for (int k = 0; k < N; ++k) amax = fmaxf(amax, abs_max(x[k]));   // pieces beyond the row hold zeros
+  amax = warp_max(amax);
+  if constexpr (WPR > 1) {
+    if (lane == 0) part_max[slot][sub] = amax;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(32 * WPR) : "memory");
+#pragma unroll
+    for (int v = 0; v < WPR; ++v) amax = fmaxf(amax, part_max[slot][v]);
+  }
+  const float scale = fp8_scale_from_amax(amax);
+  if (lane == 0 && sub == 0) scales[row] = scale;
+  const float y = b200q_rcp_rn(scale);
+  const uint64_t dd = pack2(scale, scale), ny = pack2(-y, -y);
+  auto emit = [&](auto fast_tag) {
+    constexpr bool kFast = decltype(fast_tag)::value;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int p = piece_of(k);
+      if (p < pieces) {
+        float f[16];
+        values(x[k], f);
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          if constexpr (kFast) {
+            const float2 q = unpack2(div2_by_shared_negated(pack2(f[j], f[j + 1]), dd, ny));
+            f[j] = q.x, f[j + 1] = q.y;
+          } else {
+            f[j] = __fdiv_rn(-f[j], scale), f[j + 1] = __fdiv_rn(-f[j + 1], scale);
+          }
+        }
+        uint4 c;
+        uint32_t* o = &c.x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = f32x2_to_e4m3x2(f[4 * j], f[4 * j + 1]) | (f32x2_to_e4m3x2(f[4 * j + 2], f[4 * j + 3]) << 16);
+        *reinterpret_cast<uint4*>(codes + row * cols + p * 16) = c;
+      }
+    }
+  };
+  if (b200q_div_fast_ok(scale)) emit(std::true_type{});   // one branch per row, not one select per element
+  else emit(std::false_type{});
 }
 
 // act[t, j] = silu(gu[t, j]) * gu[t, F + j], gu is [T, 2F] (gate columns first)
@@ -669,6 +872,17 @@ int grid_for(int64_t work_items) {
   return static_cast<int>(ctas < 1 ? 1 : (ctas > cap ? cap : ctas));
 }
 
+// Whether the rows of add_norm_quant go to warps instead of CTAs.  Measured (us; CTA forms -> warps): 8192 x 4096 with delta
+// 55.5 -> 47.8 FP8 and 60.0 -> 43.3 NVFP4, without 52.6 -> 25.6 and 57.4 -> 28.0; 1200 x 512 7.2 -> 2.7; 300 x 8192 7.8 -> 5.1.
+// Not faster: few short rows (300 x 2048 2.9 -> 3.8, 600 x 4096 NVFP4 6.1 -> 6.2), where a CTA per row has more threads on the
+// device, and many long rows with a delta in FP8 (8192 x 8192 78.7 -> 81.1), which the ring-fed form streams.
+bool warp_rows(int64_t rows, int64_t cols, bool has_delta, bool nvf4) {
+  if (cols % 16 != 0 || cols > 8192) return false;
+  const bool many = rows >= 8 * sm_count();
+  if (cols > 4096 && has_delta && !nvf4 && many) return false;
+  return many || rows * cols >= (cols > 4096 || !nvf4 ? int64_t{1} << 21 : int64_t{3} << 20);
+}
+
 // Launch of the add + RMSNorm + quantize kernels (checked arguments).  NVF4: result into `nv`, else per-token FP8.
 template <bool NVF4>
 int launch_add_norm_quant(const void* h, const void* delta, const void* weight, void* h_out, uint8_t* codes_out, float* scales_out,
@@ -684,7 +898,24 @@ int launch_add_norm_quant(const void* h, const void* delta, const void* weight, 
   if (NVF4) per_part = (per_part + 7) / 8 * 8;
   const int items = static_cast<int>((per_part + kThreads - 1) / kThreads);
   const int64_t grid_rows = NVF4 ? (rows + 127) / 128 * 128 : rows;
-  // many tokens: persistent CTAs fed through a shared-memory ring of rows
+  if (parts == 1 && warp_rows(rows, cols, delta != nullptr, NVF4) && aligned(h, 32) && aligned(delta, 32) && (delta == nullptr || aligned(h_out, 32)) &&
+      (NVF4 ? aligned(nv.codes, 8) : aligned(codes_out, 16))) {
+    const int per_cta = items <= 1 ? 8 : (items <= 2 ? 4 : 2);
+    const dim3 grid(static_cast<unsigned>((grid_rows + per_cta - 1) / per_cta));
+#define B200Q_ANQW(I, W)                                                                                                                   \
+  do {                                                                                                                                     \
+    if (delta != nullptr) launch_pdl(add_norm_quant_warp_kernel<I, W, true, NVF4>, grid, dim3(kThreads), 0, st, hp, dp, wp, op, codes_out, \
+                                     scales_out, rows, cols, eps, nv);                                                                     \
+    else launch_pdl(add_norm_quant_warp_kernel<I, W, false, NVF4>, grid, dim3(kThreads), 0, st, hp, dp, wp, op, codes_out, scales_out,     \
+                    rows, cols, eps, nv);                                                                                                  \
+  } while (0)
+    if (items <= 1) B200Q_ANQW(1, 1);
+    else if (items <= 2) B200Q_ANQW(2, 2);
+    else B200Q_ANQW(4, 4);
+#undef B200Q_ANQW
+    return check_launch();
+  }
+  // many tokens that the warps do not take: persistent CTAs fed through a shared-memory ring of rows
   const int64_t stage_bytes = cols * 2 * (delta != nullptr ? 2 : 1);
   if (parts == 1 && items <= 4 && rows >= 8 * sm_count() && kStreamRingBytes / stage_bytes >= 2) {
     int stages = static_cast<int>(kStreamRingBytes / stage_bytes);

@@ -90,6 +90,41 @@ __device__ __forceinline__ uint32_t quantize_values(const float* f, float a, con
   return sb;
 }
 
+// The same with the block's values negated (nf = -f): the quotients of two values at a time (div2_by_shared_negated).
+template <int N>
+__device__ __forceinline__ uint32_t quantize_negated(const float* nf, float a, const GlobalScale& gs, uint32_t* codes) {
+  float s;
+  if (gs.fast) {
+    s = b200q_div_by_shared(b200q_div_by_shared(a, kE2M1Max, kRcp6), gs.g, gs.yg);
+  } else {
+    s = __fdiv_rn(__fdiv_rn(a, kE2M1Max), gs.g);
+  }
+  const bool clamped = s > kE4M3Max;
+  const uint32_t sb = f32x2_to_e4m3x2(s, 0.0f) & 0xffu;  // saturates to 448
+  const float d = __fmul_rn(e4m3_to_f32(sb), gs.g);
+  float q[N];
+  if (sb != 0u && !clamped && b200q_div_fast_ok(d)) {
+    const float y = b200q_rcp_rn(d);
+    const uint64_t dd = pack2(d, d), ny = pack2(-y, -y);
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float2 t = unpack2(div2_by_shared_negated(pack2(nf[i], nf[i + 1]), dd, ny));
+      q[i] = t.x, q[i + 1] = t.y;
+    }
+  } else if (sb != 0u) {
+    const float lim = __fmul_rn(d, 8.0f);
+#pragma unroll
+    for (int i = 0; i < N; ++i) q[i] = with_sign_of(__fdiv_rn(fminf(fabsf(nf[i]), lim), d), -nf[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N / 8; ++i) codes[i] = 0u;
+    return sb;
+  }
+#pragma unroll
+  for (int i = 0; i < N; i += 8) codes[i / 8] = pack8_e2m1(q[i], q[i + 1], q[i + 2], q[i + 3], q[i + 4], q[i + 5], q[i + 6], q[i + 7]);
+  return sb;
+}
+
 // Quantize one block held in f[16].
 __device__ __forceinline__ uint32_t quantize_block(const float* f, const GlobalScale& gs, uint32_t& c_lo, uint32_t& c_hi,
                                                    float& d_out) {

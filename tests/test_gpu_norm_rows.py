@@ -1,0 +1,46 @@
+"""Residual add + RMSNorm + quantize at the edges of its launch shapes: one, two and four warps per row, the last column
+count of each, rows at the threshold of the form and one past a CTA, bases that are 16-byte but not 32-byte aligned
+(another kernel).  Codes and scales equal the separate kernels' bit for bit: the squares are added in the same order."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("offset", [0, 8])
+@pytest.mark.parametrize("rows,cols", [(1184, 16), (1185, 48), (1187, 2032), (1184, 2048), (1191, 2064), (1185, 4080), (1184, 4096), (1187, 4112),
+                                       (1185, 8192), (300, 8176), (1024, 4096), (2049, 1024)])
+def test_matches_separate_kernels(b200, rows, cols, offset):
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    make = lambda: torch.randn(rows * cols + offset, device="cuda", generator=g).bfloat16()[offset:].view(rows, cols)  # noqa: E731
+    h, d = make(), make()
+    h[3] = 0
+    d[3] = -0.0
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=g)).bfloat16()
+    for delta in (d, None):
+        h_ref = capi.add(h, d) if delta is not None else h
+        x = capi.rms_norm(h_ref, w)
+        h_new, codes, scales = capi.add_rms_norm_fp8_quantize(h, delta, w)
+        c_ref, s_ref = capi.fp8_quantize(x, None)
+        assert torch.equal(h_new, h_ref) and torch.equal(codes, c_ref) and torch.equal(scales.flatten(), s_ref.flatten())
+        for amax in (capi.amax(x), capi.amax(x) * 0.25):
+            h_new, got = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)
+            ref = capi.nvfp4_quantize(x, amax)
+            assert torch.equal(h_new, h_ref) and all(torch.equal(a, b) for a, b in zip(got, ref))
+    assert capi.device_status() == 0
+
+
+def test_rows_that_are_not_finite(b200):
+    capi = b200.capi
+    rows, cols = 1190, 4096
+    h, d = (torch.randn(rows, cols, device="cuda").bfloat16() for _ in range(2))
+    h[0, cols // 2], h[1, 5], d[2, cols - 1] = float("nan"), float("inf"), float("nan")
+    w = torch.ones(cols, device="cuda").bfloat16()
+    x = capi.rms_norm(capi.add(h, d), w)
+    _, codes, scales = capi.add_rms_norm_fp8_quantize(h, d, w)
+    c_ref, s_ref = capi.fp8_quantize(x, None)
+    assert torch.equal(codes, c_ref) and torch.equal(scales.flatten(), s_ref.flatten())
+    amax = torch.tensor(4.0, device="cuda")
+    got, ref = capi.add_rms_norm_nvfp4_quantize(h, d, w, amax)[1], capi.nvfp4_quantize(x, amax)
+    assert all(torch.equal(a, b) for a, b in zip(got, ref))
