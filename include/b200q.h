@@ -220,6 +220,15 @@ int b200q_nvfp4_gemm(const uint8_t* a_codes, const uint8_t* a_scales, const floa
                      const uint8_t* b_codes, const uint8_t* b_scales, const float* b_global,
                      const void* bias, void* out, int64_t M, int64_t N, int64_t K,
                      b200q_stream_t stream, const b200q_cfg* cfg);
+/* NVFP4 gate/up GEMM of a gated MLP with the activation and its static quantizer in the epilogue: B holds F
+ * gate rows, then F up rows (N = 2F, N % 256 == 0); codes_out [M, F/2], scales_out (swizzled, padding rows of the last
+ * 128-row tile zero) and global_scale_out[0] (may be NULL) hold silu(gate) * up under the calibrated abs-max
+ * act_amax[0]: the same bits as b200q_nvfp4_gemm on 256-column tiles, b200q_silu_mul and b200q_nvfp4_quantize, without the
+ * [M, 2F] tensor in between. */
+int b200q_nvfp4_gemm_silu_mul_quantize(const uint8_t* a_codes, const uint8_t* a_scales, const float* a_global,
+                                       const uint8_t* b_codes, const uint8_t* b_scales, const float* b_global,
+                                       const float* act_amax, uint8_t* codes_out, uint8_t* scales_out,
+                                       float* global_scale_out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream);
 
 /* ------------------------------------------------------------------ fused row-parallel linear (GEMM + all-reduce over peer memory)
  * Replaces "row-parallel linear, then tensorrt::fused_nccl_all_reduce" (the reference's

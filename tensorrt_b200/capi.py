@@ -317,6 +317,26 @@ def nvfp4_gemm(a_codes, a_scales, a_global, b_codes, b_scales, b_global, bias=No
     return out
 
 
+def nvfp4_gemm_silu_mul_quantize(a_codes, a_scales, a_global, b_codes, b_scales, b_global, act_amax):
+    """gate/up GEMM (B = F gate rows, then F up rows; F a multiple of 128) with silu(gate) * up and its NVFP4 quantizer
+    under the calibrated abs-max in the epilogue -> NVFP4 operand [.., F] (codes, swizzled scales, global scale), the same
+    bits as `nvfp4_gemm` on 256-column tiles, `silu_mul` and `nvfp4_quantize`."""
+    _need_cuda(a_codes, a_scales, a_global, b_codes, b_scales, b_global, act_amax)
+    a_codes, b_codes = a_codes.contiguous(), b_codes.contiguous()
+    N, half = b_codes.shape
+    if a_codes.shape[-1] != half or N % 256:
+        raise ValueError(f"b must be [2F, {a_codes.shape[-1] * 2}] with F a multiple of 128, got {(N, half * 2)}")
+    M = a_codes.numel() // half
+    a = _scalar_amax(act_amax, a_codes.device)
+    codes, scales, g = _nvfp4_out((*a_codes.shape[:-1], 0), M, N // 2, a_codes.device)
+    with torch.cuda.device(a_codes.device):
+        check(load().b200q_nvfp4_gemm_silu_mul_quantize(a_codes.data_ptr(), a_scales.data_ptr(), a_global.data_ptr(), b_codes.data_ptr(),
+                                                        b_scales.data_ptr(), b_global.data_ptr(), a.data_ptr(), codes.data_ptr(),
+                                                        scales.data_ptr(), g.data_ptr(), M, N, half * 2, _stream(a_codes)),
+              "b200q_nvfp4_gemm_silu_mul_quantize")
+    return codes, scales, g
+
+
 def _need_heads(Hq: int, Hkv: int, D: int) -> None:
     if Hkv <= 0 or Hq % Hkv or D <= 0 or D % 16 or D > 128:
         raise ValueError(f"need Hq % Hkv == 0 and a head dimension that is a multiple of 16 up to 128, got Hq={Hq}, Hkv={Hkv}, D={D}")

@@ -165,13 +165,14 @@ int launch_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, c
 }
 
 // NVFP4 CTA-pair kernel with the scales stored to tensor memory by warps (gemm_kernel_nvf4_pair.cuh).
-inline int launch_nvf4_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st) {
+template <bool SILU = false>
+int launch_nvf4_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st) {
   using C = CfgNvPair;
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gemm_nvf4_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_nvf4_pair_kernel<SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
       return B200Q_ERR_CUDA;
     configured[dev] = true;
   }
@@ -179,8 +180,8 @@ inline int launch_nvf4_pair(const uint8_t* a, const uint8_t* b, Params p, cudaSt
   if (int rc = make_operand_map(&ta, a, p.M, p.k_bytes, 128)) return rc;
   if (int rc = make_operand_map(&tb, b, p.N, p.k_bytes, 128)) return rc;
   if (int rc = make_scale_map(&tsfa, p.sfa, (p.M + 127) / 128, p.sf_col_tiles, 1)) return rc;
-  if (int rc = make_scale_map(&tsfb, p.sfb, (p.N + 127) / 128, p.sf_col_tiles, 2)) return rc;
-  const int tiles = ((p.M + kPairM - 1) / kPairM) * ((p.N + kPairN - 1) / kPairN);
+  if (int rc = make_scale_map(&tsfb, p.sfb, (p.N + 127) / 128, p.sf_col_tiles, SILU ? 1 : 2)) return rc;
+  const int tiles = ((p.M + kPairM - 1) / kPairM) * ((p.N + kPairN - 1) / kPairN);   // SILU: N = 2 F, F / 128 tiles of columns
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   cudaLaunchConfig_t cfg = {};
@@ -195,7 +196,7 @@ inline int launch_nvf4_pair(const uint8_t* a, const uint8_t* b, Params p, cudaSt
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_nvf4_pair_kernel<0>, ta, tb, tsfa, tsfb, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_nvf4_pair_kernel<SILU>, ta, tb, tsfa, tsfb, p) != cudaSuccess) {
     cudaGetLastError();
     return B200Q_ERR_CUDA;
   }

@@ -97,6 +97,7 @@ struct Params {
                            // writes out[M, F] = silu(gate) * up, each linear output rounded to bf16 first
   const float* act_amax;   // quantizing form of the above: static per-tensor abs-max of the activation; `out` then
   float* act_scale_out;    // receives E4M3 codes [M, F] (one byte each) and act_scale_out[0] the scale amax / 448
+  uint8_t* act_sf;         // NVFP4 quantizing form: swizzled block scales; `out` receives packed codes, act_scale_out[0] the global scale
   int sf_copier;           // NVFP4, 1-CTA kernel: 1 = a dedicated warp (warp 6 of 224 threads) issues the tcgen05.cp scale copies
   int* status;             // device status word (0 = ok)
 };

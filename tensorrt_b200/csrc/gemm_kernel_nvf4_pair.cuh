@@ -34,9 +34,17 @@
 //   warpgroup 1: scale warps (lane quarter = warp & 3)
 //   warpgroups 2, 3: epilogue (lane quarter = warp & 3, column half = warpgroup - 2)
 // No TMA multicast; every wait is bounded as in the other kernels.
+//
+// SILU: B holds F gate rows and then F up rows (N = 2 F).  The leader CTA loads 128 gate rows and the peer the up rows of
+// the same columns, so accumulator columns 0-127 / 128-255 of a tile are gate / up pairs; an epilogue thread takes 64 of each,
+// rounds both to bf16 as the plain form stores them, and leaves silu(gate) * up as NVFP4 codes (32 bytes) and one scale word
+// under the calibrated range of the activation: the same bits as GEMM, silu_mul and NVFP4 quantize.  The bf16 [M, 2F]
+// tensor (470 MB at 8192 tokens and F = 14336, written once and read once: 120 us of a 1150 us layer) is not written; the
+// arithmetic runs under the next tile's MMAs, because tensor memory is handed back first.
 #pragma once
 
 #include "gemm_kernel_2cta.cuh"
+#include "nvfp4_block.cuh"
 
 namespace b200q {
 namespace gemm {
@@ -59,8 +67,7 @@ struct CfgNvPair {
   static_assert(kStages >= 4, "pipeline too shallow");
 };
 
-// (a template only so that the definition may live in a header included by several translation units)
-template <int kVariant = 0>
+template <bool SILU>
 __global__ void __launch_bounds__(kNvPairThreads, 1)
 gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                          const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb, const Params p) {
@@ -84,7 +91,7 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta_rank = ptx::cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int m_blocks = (p.M + kPairM - 1) / kPairM, n_blocks = (p.N + kPairN - 1) / kPairN;
+  const int m_blocks = (p.M + kPairM - 1) / kPairM, n_blocks = SILU ? p.silu_f / 128 : (p.N + kPairN - 1) / kPairN;
   const int num_tiles = m_blocks * n_blocks;
   const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
   constexpr int kGroupM = 8;
@@ -141,7 +148,7 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         int mb, nb;
         tile_coord(t, mb, nb);
         const int32_t m0 = mb * kPairM + static_cast<int>(cta_rank) * 128;
-        const int32_t n0 = nb * kPairN + static_cast<int>(cta_rank) * (kPairN / 2);
+        const int32_t n0 = SILU ? nb * 128 + (cta_rank == 0 ? 0 : p.silu_f) : nb * kPairN + static_cast<int>(cta_rank) * (kPairN / 2);
         for (int kt = 0; kt < k_tiles; ++kt) {
           {
             if (!ptx::mbar_wait(sf_empty + entry, sf_phase ^ 1u)) {
@@ -153,7 +160,12 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint8_t* ssfb = ssfa + P::kSfaBytes;
             ptx::mbar_arrive_expect_tx(sf_full + entry, P::kSfEntryBytes);
             ptx::tma_load_3d(ssfa, &tmap_sfa, sf_full + entry, 0, kt * 4, mb * 2 + static_cast<int>(cta_rank));
-            ptx::tma_load_3d(ssfb, &tmap_sfb, sf_full + entry, 0, kt * 4, nb * 2);
+            if constexpr (SILU) {                        // the gate rows' scale tile, then the up rows'
+              ptx::tma_load_3d(ssfb, &tmap_sfb, sf_full + entry, 0, kt * 4, nb);
+              ptx::tma_load_3d(ssfb + 2048, &tmap_sfb, sf_full + entry, 0, kt * 4, p.silu_f / 128 + nb);
+            } else {
+              ptx::tma_load_3d(ssfb, &tmap_sfb, sf_full + entry, 0, kt * 4, nb * 2);
+            }
             if (++entry == C::kSfEntries) entry = 0, sf_phase ^= 1u;
           }
           if (!ptx::mbar_wait(empty_bar + stage, phase ^ 1u)) {
@@ -287,11 +299,13 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     // ------------------------------------------------------------ epilogue (warpgroups 2 and 3, both CTAs)
     ptx::setmaxnreg_inc<184>();
     const int q = warp & 3;                 // tensor-memory lane quarter this warp may read
-    const int half = (warp - 8) >> 2;       // which 128 of the 256 accumulator columns
+    const int half = (warp - 8) >> 2;       // which 128 of the 256 accumulator columns (SILU: which 64 of the gate and up columns)
     uint32_t acc_phase = 0;
     const float gscale = __fmul_rn(__ldg(p.a_scales), __ldg(p.b_scales));
     // 32-byte stores need rows and base on 32-byte boundaries; the entry point asks for a 16-byte aligned output only
     const bool vec32 = (p.N % 16) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0, vec16 = (p.N % 8) == 0;
+    const GlobalScale act_scale(SILU ? __ldg(p.act_amax) : 1.0f);
+    if (SILU && blockIdx.x == 0 && threadIdx.x == 256 && p.act_scale_out != nullptr) *p.act_scale_out = act_scale.g;
     for (int t = pair; t < num_tiles; t += num_pairs) {
       int mb, nb;
       tile_coord(t, mb, nb);
@@ -301,10 +315,10 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
       acc_phase ^= 1u;
       ptx::tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * 128;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * (SILU ? 64 : 128);
       uint32_t r[128];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(taddr + c * 32, r + c * 32);
+      for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(taddr + (SILU ? (c & 1) * 32 + (c >> 1) * 128 : c * 32), r + c * 32);
       ptx::tmem_ld_wait();
       // the accumulator is in registers (the loads have completed): hand tensor memory back before
       // converting and storing; no release needed, nothing this warp wrote is part of the signal
@@ -315,6 +329,43 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         else ptx::mbar_arrive_cluster_relaxed(acc_empty, 0);
       }
       const int row = mb * kPairM + static_cast<int>(cta_rank) * 128 + q * 32 + lane;
+      if constexpr (SILU) {
+        const int col = nb * 128 + half * 64;
+        if (row < (p.M + 127) / 128 * 128) {
+          U32x8 codes = {};
+          uint32_t word = 0u;                     // rows past the last one of a 128-row scale tile: zero scales
+          if (row < p.M) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              uint32_t nw[8];                     // -silu(gate) * up, packed bf16
+              float nf[16];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const __nv_bfloat162 g2 = __floats2bfloat162_rn(__uint_as_float(r[b * 16 + 2 * i]) * gscale, __uint_as_float(r[b * 16 + 2 * i + 1]) * gscale);
+                const __nv_bfloat162 u2 =
+                    __floats2bfloat162_rn(__uint_as_float(r[64 + b * 16 + 2 * i]) * -gscale, __uint_as_float(r[64 + b * 16 + 2 * i + 1]) * -gscale);
+                const __nv_bfloat162 a2 = __floats2bfloat162_rn(silu_mul_f32(__low2float(g2), __low2float(u2)), silu_mul_f32(__high2float(g2), __high2float(u2)));
+                nw[i] = *reinterpret_cast<const uint32_t*>(&a2);
+                nf[2 * i] = __uint_as_float(nw[i] << 16);
+                nf[2 * i + 1] = __uint_as_float(nw[i] & 0xffff0000u);
+              }
+              __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&nw[0]));
+#pragma unroll
+              for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&nw[i])));
+              word |= quantize_negated<16>(nf, fmaxf(__low2float(m), __high2float(m)), act_scale, codes.v + 2 * b) << (8 * b);
+            }
+            uint8_t* crow = reinterpret_cast<uint8_t*>(p.out) + static_cast<int64_t>(row) * (p.silu_f >> 1) + (col >> 1);
+            if (vec32) {
+              st_256(crow, codes);
+            } else {
+              *reinterpret_cast<uint4*>(crow) = make_uint4(codes.v[0], codes.v[1], codes.v[2], codes.v[3]);
+              *reinterpret_cast<uint4*>(crow + 16) = make_uint4(codes.v[4], codes.v[5], codes.v[6], codes.v[7]);
+            }
+          }
+          *reinterpret_cast<uint32_t*>(p.act_sf + swizzled_word_offset(row, col >> 4, p.silu_f >> 6)) = word;
+        }
+        continue;
+      }
       const int col0 = nb * BN + half * 128;
       if (row < p.M) {
         __nv_bfloat16* orow = p.out + static_cast<int64_t>(row) * p.N;
