@@ -101,6 +101,13 @@ __device__ __forceinline__ uint4 ld_nc_128(const void* p) {
   return r;
 }
 
+// The same through L1, for what several warps of an SM read; an ordered load, which stays behind a pdl_wait().
+__device__ __forceinline__ uint4 ld_128(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
 __device__ __forceinline__ void st_256(void* p, const U32x8& r) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r.v[0]), "r"(r.v[1]),
                "r"(r.v[2]), "r"(r.v[3]), "r"(r.v[4]), "r"(r.v[5]), "r"(r.v[6]), "r"(r.v[7])

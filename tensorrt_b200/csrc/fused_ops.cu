@@ -478,8 +478,7 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
   for (int k = 0; k < N; ++k) {
     const int p = piece_of(k);
     if (p < pieces) {
-      const uint4* wp = reinterpret_cast<const uint4*>(w + p * 16);
-      const uint4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
+      const uint4 w0 = ld_128(w + p * 16), w1 = ld_128(w + p * 16 + 8);
       const uint32_t wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
