@@ -79,7 +79,7 @@ int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_n
   const int tiles = static_cast<int>((N + gemm::kSmallWRows - 1) / gemm::kSmallWRows);
   const int k_tiles = static_cast<int>((K + gemm::kBKBytes - 1) / gemm::kBKBytes);
   if (tiles < 16) return 1;
-  const int splits = gemm::smallm_splits(tiles, k_tiles, sm_count(), static_cast<int>(M)), per_cta = (k_tiles + splits - 1) / splits;
+  const int splits = gemm::smallm_most_splits(tiles, k_tiles, sm_count(), static_cast<int>(M)), per_cta = (k_tiles + splits - 1) / splits;
   if (per_cta > gemm::kOwnXTiles || per_cta * M > gemm::kOwnXSlice) return 1;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(out, 16)) return 1;
   if (int rc = check_arch()) return rc;

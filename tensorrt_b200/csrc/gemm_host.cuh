@@ -292,11 +292,42 @@ int launch_smallm_own_x(const uint8_t* b, const Params& p, cudaStream_t st, int 
 // 16 tokens, neutral at 64, slower at 128), so the target there is one and a half CTAs per SM, as long
 // as all CTAs are resident at once: 80 tiles x 4 = 320 CTAs on 296 places cost a second round (10240 x 8192
 // at 1 / 16 tokens: FP8 23.0 / 24.4 us against 17.4 / 18.4 with 2 CTAs per tile, NVFP4 16.2 / 17.6 against 12.4 / 13.2).
-inline int smallm_splits(int n_tiles, int k_tiles, int sms, int tokens) {
+inline int smallm_most_splits(int n_tiles, int k_tiles, int sms, int tokens) {
   const int want = tokens <= 32 ? (sms * 3) / 2 : (sms * 3) / 4;
   int s = 1;
   while (s < 8 && n_tiles * s < want && n_tiles * s * 2 <= 2 * sms && s * 2 <= k_tiles) s <<= 1;
   return s;
+}
+
+// Time of the small-M kernel with clusters of `s` CTAs in ns, good enough to compare cluster sizes: a launch, the K tiles of a
+// CTA, and what the cluster adds (every token's partial sums, twice from eight CTAs); dearer where CTAs share an SM; once more
+// for every further round of clusters.  With a ring that takes the whole SM, 12 clusters of 8 and 33 of 4 were seen resident
+// at once (16 of 8 and 36 of 4 take two rounds: clusters do not cross GPCs).
+inline int64_t smallm_cost(int n_tiles, int k_tiles, int sms, int tokens, int s) {
+  const bool shared_sm = n_tiles * s > sms;
+  const int log2s = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
+  const int resident = shared_sm ? (s == 8 ? 33 : (s == 4 ? 72 : 2 * sms / s)) : (s == 8 ? 12 : (s == 4 ? 33 : sms / s));
+  const int64_t rounds = (n_tiles + resident - 1) / resident, per = (k_tiles + s - 1) / s;
+  const int64_t stream = per * (1800 + 3 * tokens) * (shared_sm ? 13 : 10) / 100;
+  const int64_t reduce = tokens * 3 * log2s * (shared_sm ? 3 : 1) + (s == 8 ? 9 * tokens : 0);
+  return rounds * (4900 + stream) + reduce;
+}
+
+// Fewer CTAs per tile than that where they are cheaper by more than 3 %: short K slices and many tokens (the reduction), and
+// cluster counts just above what is resident.  Measured at 32 weight shapes (1024 x 1024 to 57344 x 8192), 10 token counts
+// and both formats: 1.011 of the best cluster size on average (1.106 without this step, 2.2 times at worst: FP8 2048 x 2048
+// at 16 / 64 / 128 tokens 9.1 / 13.5 / 17.9 us on 8 CTAs, 5.0 / 6.7 / 8.7 on 4; 6144 x 4096 at 128 tokens 16.3 on 4, 12.3 on
+// 2), and nowhere more than 5 % slower than without.
+inline int smallm_splits(int n_tiles, int k_tiles, int sms, int tokens) {
+  const int most = smallm_most_splits(n_tiles, k_tiles, sms, tokens);
+  const int64_t cost = smallm_cost(n_tiles, k_tiles, sms, tokens, most);
+  int best = most;
+  int64_t least = cost * 97 / 100;
+  for (int s = most >> 1; s >= 1; s >>= 1) {
+    const int64_t c = smallm_cost(n_tiles, k_tiles, sms, tokens, s);
+    if (c < least) least = c, best = s;
+  }
+  return best;
 }
 
 bool valid_tile_n(int bn);    // values b200q_cfg::tile_n accepts
