@@ -368,14 +368,108 @@ add_norm_quant_stream_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfl
   }
 }
 
+// ---- add + RMSNorm + quantize on pieces of 16 elements, packed as bf16
+
+// x + delta.  One bf16 pair addition rounds the exact sum once, and an fp32 addition in front of that rounding changes
+// nothing: the sum of two bf16 values that needs more than 24 bits lies next to the larger one.
+__device__ __forceinline__ void piece_add(U32x8& x, const U32x8& d) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const __nv_bfloat162 t = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&x.v[j]), *reinterpret_cast<const __nv_bfloat162*>(&d.v[j]));
+    x.v[j] = *reinterpret_cast<const uint32_t*>(&t);
+  }
+}
+
+// Squares of a piece added to `ss`: its low half takes the first 8 elements, the high half the others, each in order.
+__device__ __forceinline__ uint64_t piece_squares(const U32x8& x, uint64_t ss) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t lo = pack2(__uint_as_float(x.v[j] << 16), __uint_as_float(x.v[4 + j] << 16));
+    const uint64_t hi = pack2(__uint_as_float(x.v[j] & 0xffff0000u), __uint_as_float(x.v[4 + j] & 0xffff0000u));
+    ss = fma2(lo, lo, ss);
+    ss = fma2(hi, hi, ss);
+  }
+  return ss;
+}
+
+// -(x * inv * w) rounded to bf16 (ninv = (-inv, -inv)): negated for the divisions of the quantizers, where the signs cancel.
+__device__ __forceinline__ void piece_norm_negated(U32x8& x, const uint4& w0, const uint4& w1, uint64_t ninv) {
+  const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint64_t xv = pack2(__uint_as_float(x.v[j] << 16), __uint_as_float(x.v[j] & 0xffff0000u));
+    const uint64_t wj = pack2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+    const float2 t = unpack2(mul2(mul2(xv, ninv), wj));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(t.x, t.y);
+    x.v[j] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+}
+
+// abs-max of a piece; NaN only when all its values are
+__device__ __forceinline__ float piece_abs_max(const U32x8& x) {
+  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&x.v[0]));
+#pragma unroll
+  for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&x.v[j])));
+  return fmaxf(__low2float(m), __high2float(m));
+}
+
+__device__ __forceinline__ void piece_values(const U32x8& x, float* f) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    f[2 * j] = __uint_as_float(x.v[j] << 16);
+    f[2 * j + 1] = __uint_as_float(x.v[j] & 0xffff0000u);
+  }
+}
+
+// E4M3 codes of a negated piece under `scale` (dd = (scale, scale), ny = -(1 / scale) twice; FAST: b200q_div_fast_ok(scale)).
+template <bool FAST>
+__device__ __forceinline__ uint4 piece_fp8(const U32x8& x, float scale, uint64_t dd, uint64_t ny) {
+  float f[16];
+  piece_values(x, f);
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) {
+    if constexpr (FAST) {
+      const float2 q = unpack2(div2_by_shared_negated(pack2(f[j], f[j + 1]), dd, ny));
+      f[j] = q.x, f[j + 1] = q.y;
+    } else {
+      f[j] = __fdiv_rn(-f[j], scale), f[j + 1] = __fdiv_rn(-f[j + 1], scale);
+    }
+  }
+  uint4 c;
+  uint32_t* o = &c.x;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[j] = f32x2_to_e4m3x2(f[4 * j], f[4 * j + 1]) | (f32x2_to_e4m3x2(f[4 * j + 2], f[4 * j + 3]) << 16);
+  return c;
+}
+
+// Place of the first scale word of a row.
+__device__ __forceinline__ uint8_t* nvfp4_scale_row(const Nvfp4Out& nv, int64_t row) {
+  return nv.sf + (row >> 7) * static_cast<int64_t>(nv.col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+}
+
+// NVFP4 codes and scale word of negated piece p of a row; all 32 lanes, the warp's pieces in order (p % 4 == lane % 4): four
+// lanes hold one scale word.
+__device__ __forceinline__ void piece_nvfp4_store(const U32x8& x, int p, int pieces, const GlobalScale& gs, uint8_t* code_row, uint8_t* sf_row) {
+  uint32_t sb = 0u;
+  if (p < pieces) {
+    float f[16];
+    uint32_t c[2];
+    piece_values(x, f);
+    sb = quantize_negated<16>(f, piece_abs_max(x), gs, c);
+    *reinterpret_cast<uint2*>(code_row + p * 8) = make_uint2(c[0], c[1]);
+  }
+  uint32_t word = sb << (8 * (p & 3));
+  word |= __shfl_xor_sync(0xffffffffu, word, 1);
+  word |= __shfl_xor_sync(0xffffffffu, word, 2);
+  if ((p & 3) == 0 && p < pieces) *reinterpret_cast<uint32_t*>(sf_row + static_cast<uint32_t>(p >> 2) * 512u) = word;
+}
+
 // Form for many tokens with rows of up to 8192 elements (a multiple of 16, 32-byte aligned): WPR warps (1, 2, 4 for rows of
 // up to 2048, 4096, 8192 elements) hold a row in registers, packed as bf16, four pieces of 16 elements per lane, and reduce
 // it with shuffles and one barrier between those warps.  No CTA-wide barrier stands between loading, reducing and storing,
 // so the rows of an SM stream independently.  What bounds it is issue slots beside HBM: hence bf16 pair additions for
 // h + delta, fp32 pairs for the squares, the products and the quotients (about 10 instructions an element, half of what the
-// scalar form takes).  The residual sum is one bf16 pair addition: it rounds the exact sum once, and an fp32 addition in
-// front of that rounding changes nothing (the sum of two bf16 values with more than 24 bits lies next to the larger one).
-// The squares are added in the order of add_norm_quant_kernel, whose thread t sums groups t, t + 256, ... of 8 elements and
+// scalar form takes).  The squares are added in the order of add_norm_quant_kernel, whose thread t sums groups t, t + 256, ... of 8 elements and
 // whose 8 warps of 32 threads are added by a tree: lane l of a warp here plays threads 2l and 2l + 1 of two of them.
 template <int ITEMS, int WPR, bool HAS_DELTA, bool NVF4>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -395,7 +489,7 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
   if (row >= rows) {                              // the warps of a row leave together
     if constexpr (NVF4) {
       if (sub == 0 && row < (rows + 127) / 128 * 128) {
-        uint8_t* sf = nv.sf + (row >> 7) * static_cast<int64_t>(nv.col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+        uint8_t* sf = nvfp4_scale_row(nv, row);
         for (uint32_t c = lane; c < nv.col_tiles; c += 32) *reinterpret_cast<uint32_t*>(sf + c * 512u) = 0u;
       }
     }
@@ -419,11 +513,7 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       if (piece_of(k) < pieces) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const __nv_bfloat162 t = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&x[k].v[j]), *reinterpret_cast<const __nv_bfloat162*>(&d[k].v[j]));
-          x[k].v[j] = *reinterpret_cast<const uint32_t*>(&t);
-        }
+        piece_add(x[k], d[k]);
         st_256(h_out + row * cols + piece_of(k) * 16, x[k]);
       }
     }
@@ -434,16 +524,7 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
   for (int v = 0; v < VP; ++v) {
     uint64_t ss = 0ull;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      const U32x8& t = x[v * ITEMS + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint64_t lo = pack2(__uint_as_float(t.v[j] << 16), __uint_as_float(t.v[4 + j] << 16));
-        const uint64_t hi = pack2(__uint_as_float(t.v[j] & 0xffff0000u), __uint_as_float(t.v[4 + j] & 0xffff0000u));
-        ss = fma2(lo, lo, ss);
-        ss = fma2(hi, hi, ss);
-      }
-    }
+    for (int i = 0; i < ITEMS; ++i) ss = piece_squares(x[v * ITEMS + i], ss);
     float2 s = unpack2(ss);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) {
@@ -478,56 +559,19 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
   for (int k = 0; k < N; ++k) {
     const int p = piece_of(k);
     if (p < pieces) {
-      const uint4 w0 = ld_128(w + p * 16), w1 = ld_128(w + p * 16 + 8);
-      const uint32_t wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint64_t xv = pack2(__uint_as_float(x[k].v[j] << 16), __uint_as_float(x[k].v[j] & 0xffff0000u));
-        const uint64_t wj = pack2(__uint_as_float(wv[j] << 16), __uint_as_float(wv[j] & 0xffff0000u));
-        const float2 t = unpack2(mul2(mul2(xv, ninv), wj));
-        const __nv_bfloat162 b = __floats2bfloat162_rn(t.x, t.y);
-        x[k].v[j] = *reinterpret_cast<const uint32_t*>(&b);
-      }
+      piece_norm_negated(x[k], ld_128(w + p * 16), ld_128(w + p * 16 + 8), ninv);
     }
   }
-  const auto abs_max = [](const U32x8& t) {       // of 16 values; NaN only when all are
-    __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&t.v[0]));
-#pragma unroll
-    for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&t.v[j])));
-    return fmaxf(__low2float(m), __high2float(m));
-  };
-  const auto values = [](const U32x8& t, float* f) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      f[2 * j] = __uint_as_float(t.v[j] << 16);
-      f[2 * j + 1] = __uint_as_float(t.v[j] & 0xffff0000u);
-    }
-  };
   if constexpr (NVF4) {
     const GlobalScale gs(ld_dependent(nv.amax));
     if (blockIdx.x == 0 && threadIdx.x == 0 && nv.gout != nullptr) *nv.gout = gs.g;
-    uint8_t* sf = nv.sf + (row >> 7) * static_cast<int64_t>(nv.col_tiles) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const int p = piece_of(k);
-      uint32_t sb = 0u;
-      if (p < pieces) {
-        float f[16];
-        uint32_t c[2];
-        values(x[k], f);
-        sb = quantize_negated<16>(f, abs_max(x[k]), gs, c);
-        *reinterpret_cast<uint2*>(nv.codes + row * (cols >> 1) + p * 8) = make_uint2(c[0], c[1]);
-      }
-      uint32_t word = sb << (8 * (p & 3));        // four lanes hold one scale word
-      word |= __shfl_xor_sync(0xffffffffu, word, 1);
-      word |= __shfl_xor_sync(0xffffffffu, word, 2);
-      if ((p & 3) == 0 && p < pieces) *reinterpret_cast<uint32_t*>(sf + static_cast<uint32_t>(p >> 2) * 512u) = word;
-    }
+    for (int k = 0; k < N; ++k) piece_nvfp4_store(x[k], piece_of(k), pieces, gs, nv.codes + row * (cols >> 1), nvfp4_scale_row(nv, row));
     return;
   }
   float amax = 0.0f;
 #pragma unroll
-  for (int k = 0; k < N; ++k) amax = fmaxf(amax, abs_max(x[k]));   // pieces beyond the row hold zeros
+  for (int k = 0; k < N; ++k) amax = fmaxf(amax, piece_abs_max(x[k]));   // pieces beyond the row hold zeros
   amax = warp_max(amax);
   if constexpr (WPR > 1) {
     if (lane == 0) part_max[slot][sub] = amax;
@@ -540,32 +584,77 @@ add_norm_quant_warp_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloa
   const float y = b200q_rcp_rn(scale);
   const uint64_t dd = pack2(scale, scale), ny = pack2(-y, -y);
   auto emit = [&](auto fast_tag) {
-    constexpr bool kFast = decltype(fast_tag)::value;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       const int p = piece_of(k);
-      if (p < pieces) {
-        float f[16];
-        values(x[k], f);
-#pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-          if constexpr (kFast) {
-            const float2 q = unpack2(div2_by_shared_negated(pack2(f[j], f[j + 1]), dd, ny));
-            f[j] = q.x, f[j + 1] = q.y;
-          } else {
-            f[j] = __fdiv_rn(-f[j], scale), f[j + 1] = __fdiv_rn(-f[j + 1], scale);
-          }
-        }
-        uint4 c;
-        uint32_t* o = &c.x;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = f32x2_to_e4m3x2(f[4 * j], f[4 * j + 1]) | (f32x2_to_e4m3x2(f[4 * j + 2], f[4 * j + 3]) << 16);
-        *reinterpret_cast<uint4*>(codes + row * cols + p * 16) = c;
-      }
+      if (p < pieces) *reinterpret_cast<uint4*>(codes + row * cols + p * 16) = piece_fp8<decltype(fast_tag)::value>(x[k], scale, dd, ny);
     }
   };
   if (b200q_div_fast_ok(scale)) emit(std::true_type{});   // one branch per row, not one select per element
   else emit(std::false_type{});
+}
+
+// Form for few tokens (a decode step) with rows of 2048 to 16384 elements (a multiple of 16, 32-byte aligned): one CTA per
+// row with one piece of 16 elements per thread, so that what a launch takes is one round trip to L2 (row, delta and norm
+// weights at once) and two reductions over at most 32 warps.  A cluster of CTAs per row took longer for its barriers than
+// it saved: with delta, FP8 / NVFP4, 64 x 8192 6.4 / 5.3 us there, 3.2 / 3.9 here; 8 x 4096 3.4 / 3.4, 2.1 / 2.3; 128 x 2048 4.2 /
+// 4.0, 2.0 / 2.3.  The squares are added in another order than in the other forms (a piece per thread, then a tree).
+template <bool HAS_DELTA, bool NVF4>
+__global__ void __launch_bounds__(1024, 1)
+add_norm_quant_row_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ delta,
+                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out, uint8_t* __restrict__ codes,
+                          float* __restrict__ scales, int64_t rows, int64_t cols, float eps, const Nvfp4Out nv) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float part[32], part_max[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int64_t row = blockIdx.x;
+  const int pieces = static_cast<int>(cols >> 4), p = threadIdx.x;
+  if constexpr (NVF4) {
+    if (row >= rows) {
+      zero_scale_row(nv.sf, row, nv.col_tiles);
+      return;
+    }
+  }
+  const bool live = p < pieces;
+  U32x8 x{};
+  uint4 w0{}, w1{};
+  if (live) {
+    x = ld_nc_256(h + row * cols + p * 16);
+    U32x8 d;
+    if constexpr (HAS_DELTA) d = ld_nc_256(delta + row * cols + p * 16);
+    w0 = ld_nc_128(w + p * 16), w1 = ld_nc_128(w + p * 16 + 8);
+    if constexpr (HAS_DELTA) {
+      piece_add(x, d);
+      st_256(h_out + row * cols + p * 16, x);
+    }
+  }
+  const float2 s2 = unpack2(piece_squares(x, 0ull));
+  float ss = s2.x + s2.y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (lane == 0) part[warp] = ss;
+  __syncthreads();
+  float total = lane < warps ? part[lane] : 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  const float inv = rsqrtf(total / static_cast<float>(cols) + eps);
+  if (live) piece_norm_negated(x, w0, w1, pack2(-inv, -inv));
+  if constexpr (NVF4) {
+    const GlobalScale gs(ld_dependent(nv.amax));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nv.gout != nullptr) *nv.gout = gs.g;
+    piece_nvfp4_store(x, p, pieces, gs, nv.codes + row * (cols >> 1), nvfp4_scale_row(nv, row));
+    return;
+  }
+  const float mine = warp_max(fmaxf(0.0f, piece_abs_max(x)));
+  if (lane == 0) part_max[warp] = mine;
+  __syncthreads();
+  const float scale = fp8_scale_from_amax(warp_max(lane < warps ? part_max[lane] : 0.0f));
+  if (threadIdx.x == 0) scales[row] = scale;
+  const float y = b200q_rcp_rn(scale);
+  if (live)
+    *reinterpret_cast<uint4*>(codes + row * cols + p * 16) =
+        b200q_div_fast_ok(scale) ? piece_fp8<true>(x, scale, pack2(scale, scale), pack2(-y, -y)) : piece_fp8<false>(x, scale, 0ull, 0ull);
 }
 
 // act[t, j] = silu(gu[t, j]) * gu[t, F + j], gu is [T, 2F] (gate columns first)
@@ -876,7 +965,7 @@ int grid_for(int64_t work_items) {
 // Not faster: few short rows (300 x 2048 2.9 -> 3.8, 600 x 4096 NVFP4 6.1 -> 6.2), where a CTA per row has more threads on the
 // device, and many long rows with a delta in FP8 (8192 x 8192 78.7 -> 81.1), which the ring-fed form streams.
 bool warp_rows(int64_t rows, int64_t cols, bool has_delta, bool nvf4) {
-  if (cols % 16 != 0 || cols > 8192) return false;
+  if (cols > 8192) return false;
   const bool many = rows >= 8 * sm_count();
   if (cols > 4096 && has_delta && !nvf4 && many) return false;
   return many || rows * cols >= (cols > 4096 || !nvf4 ? int64_t{1} << 21 : int64_t{3} << 20);
@@ -897,8 +986,16 @@ int launch_add_norm_quant(const void* h, const void* delta, const void* weight, 
   if (NVF4) per_part = (per_part + 7) / 8 * 8;
   const int items = static_cast<int>((per_part + kThreads - 1) / kThreads);
   const int64_t grid_rows = NVF4 ? (rows + 127) / 128 * 128 : rows;
-  if (parts == 1 && warp_rows(rows, cols, delta != nullptr, NVF4) && aligned(h, 32) && aligned(delta, 32) && (delta == nullptr || aligned(h_out, 32)) &&
-      (NVF4 ? aligned(nv.codes, 8) : aligned(codes_out, 16))) {
+  const bool by_pieces = cols % 16 == 0 && aligned(h, 32) && aligned(delta, 32) && (delta == nullptr || aligned(h_out, 32)) &&
+                         (NVF4 ? aligned(nv.codes, 8) : aligned(codes_out, 16));
+  // (a CTA of 1024 threads starts later than a cluster where there are hardly any rows: 8 x 16384 NVFP4 4.2 us, 4.0)
+  if (by_pieces && parts > 1 && (cols <= 8192 || rows > 16)) {
+    const dim3 grid(static_cast<unsigned>(grid_rows)), block(static_cast<unsigned>((cols / 16 + 31) / 32 * 32));
+    if (delta != nullptr) launch_pdl(add_norm_quant_row_kernel<true, NVF4>, grid, block, 0, st, hp, dp, wp, op, codes_out, scales_out, rows, cols, eps, nv);
+    else launch_pdl(add_norm_quant_row_kernel<false, NVF4>, grid, block, 0, st, hp, dp, wp, op, codes_out, scales_out, rows, cols, eps, nv);
+    return check_launch();
+  }
+  if (by_pieces && parts == 1 && warp_rows(rows, cols, delta != nullptr, NVF4)) {
     const int per_cta = items <= 1 ? 8 : (items <= 2 ? 4 : 2);
     const dim3 grid(static_cast<unsigned>((grid_rows + per_cta - 1) / per_cta));
 #define B200Q_ANQW(I, W)                                                                                                                   \

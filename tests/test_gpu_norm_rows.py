@@ -44,3 +44,28 @@ def test_rows_that_are_not_finite(b200):
     amax = torch.tensor(4.0, device="cuda")
     got, ref = capi.add_rms_norm_nvfp4_quantize(h, d, w, amax)[1], capi.nvfp4_quantize(x, amax)
     assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 2048), (3, 2064), (17, 16384), (33, 10240), (147, 4112), (295, 2048)])
+def test_few_rows_one_piece_per_thread(b200, rows, cols):
+    """A CTA per row adds the squares in an order of its own: the last bits of the sum move rsqrt and the products by up to 2
+    ulp of fp32, which changes one in 2^14 bf16 roundings at most, and with it a code (or, through a row's abs-max, a scale)."""
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    h, d = (torch.randn(rows, cols, device="cuda", generator=g).bfloat16() for _ in range(2))
+    h[rows // 2] = 0
+    d[rows // 2] = -0.0
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=g)).bfloat16()
+    few = lambda a, b: int((a != b).sum()) <= max(1, b.numel() >> 13)  # noqa: E731
+    for delta in (d, None):
+        h_ref = capi.add(h, d) if delta is not None else h
+        x = capi.rms_norm(h_ref, w)
+        h_new, codes, scales = capi.add_rms_norm_fp8_quantize(h, delta, w)
+        c_ref, s_ref = capi.fp8_quantize(x, None)
+        same = scales.flatten() == s_ref.flatten()
+        assert torch.equal(h_new, h_ref) and int((~same).sum()) <= 1 + rows // 64 and few(codes[same], c_ref[same])
+        amax = capi.amax(x)
+        h_new, got = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)
+        ref = capi.nvfp4_quantize(x, amax)
+        assert torch.equal(h_new, h_ref) and torch.equal(got[2], ref[2]) and all(few(a, b) for a, b in zip(got[:2], ref[:2]))
+    assert capi.device_status() == 0
