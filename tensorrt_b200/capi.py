@@ -495,9 +495,9 @@ def _scalar_amax(amax_t, device):
 
 def add_rms_norm_nvfp4_quantize(h: torch.Tensor, delta: torch.Tensor | None, weight: torch.Tensor, amax_t: torch.Tensor, eps: float = 1e-5):
     """-> (h + delta (h itself when delta is None), NVFP4 operand of rms_norm(h + delta) under the calibrated
-    tensor amax): `add`, `rms_norm` and `nvfp4_quantize` in one pass.  The same bits where a row stays in one CTA; with fewer
-    than two rows per SM, rows of 2048 columns and more are split and their squares added in another order (a code differs
-    about as often as a bf16 rounding does: 6 bytes in 16 million).  At most 16384 columns."""
+    tensor amax): `add`, `rms_norm` and `nvfp4_quantize` in one pass.  The same bits, except that with fewer than two rows per
+    SM and 2048 columns or more the squares are added in another order (a code differs about as often as a bf16 rounding
+    does: 6 bytes in 16 million).  At most 16384 columns."""
     _need_cuda(h, delta, weight, amax_t)
     _bf16(h, weight)
     h = h.contiguous()
