@@ -1,5 +1,6 @@
 // FP8 E4M3 x E4M3 GEMM entry point (tcgen05 kind::f8f6f4) and the pieces shared by both
 // quantized GEMMs: the TMA descriptor encoder lookup and the device status word.
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -36,6 +37,34 @@ int* device_status_word() {
     g_status_addr[dev] = static_cast<int*>(p);
   }
   return g_status_addr[dev];
+}
+
+int active_clusters(int size) {
+  static std::atomic<int> known[64][4] = {};               // by device and log2(size); 0 = not asked yet
+  const int sms = sm_count(), i = size == 2 ? 1 : (size == 4 ? 2 : 3);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sms / size;
+  int n = known[dev][i].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  using C = SmallCfg<false>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(size * sms));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(C::smem_bytes(16, C::max_stages(16, kSmemLimit)));
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(size);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(gemm_smallm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_smallm_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = sms / size;                                        // as if no GPC had SMs left over
+  }
+  known[dev][i].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 bool valid_tile_n(int bn) {

@@ -299,14 +299,30 @@ inline int smallm_most_splits(int n_tiles, int k_tiles, int sms, int tokens) {
   return s;
 }
 
+// Clusters of 2, 4 or 8 CTAs, one per SM, that are resident at once on the current device.  A cluster does not cross a GPC, and
+// how many SMs a GPC has differs from part to part, so the occupancy API is asked, once per device.
+int active_clusters(int size);
+
+// Clusters of `s` CTAs of a small-M kernel that are resident at once, two CTAs per SM where `shared_sm`.  Seen as the jump to a
+// second round on a part where the API gives 74, 33 and 15 clusters of 2, 4 and 8 (FP8 at 16 tokens, K 4096): alone 15 of 8
+// (5.98 us, 16 take 10.2) and 33 of 4 (8.1, 34 take 12.3); two CTAs per SM have the places of clusters of half the size: 33 of 8
+// (7.3, 34 take 11.3), 148 of 2 (14.9, 149 take 21.1), and of 4 nearly, 71 (9.4, 72 take 14.1).
+inline int smallm_resident(int s, int sms, bool shared_sm) {
+  if (s == 1) return shared_sm ? 2 * sms : sms;
+  if (!shared_sm) return active_clusters(s);
+  return s == 2 ? sms : (s == 4 ? (active_clusters(2) * 71 + 73) / 74 : active_clusters(4));
+}
+
 // Time of the small-M kernel with clusters of `s` CTAs in ns, good enough to compare cluster sizes: a launch, the K tiles of a
 // CTA, and what the cluster adds (every token's partial sums, twice from eight CTAs); dearer where CTAs share an SM; once more
-// for every further round of clusters.  With a ring that takes the whole SM, 12 clusters of 8 and 33 of 4 were seen resident
-// at once (16 of 8 and 36 of 4 take two rounds: clusters do not cross GPCs).
+// for every further round of clusters.  Clusters of eight count as one round up to four fifths of those that fit: with 13 to 15
+// tiles clusters of four take 0.87 to 0.97 of their time (NVFP4 1920 x 2048 at 8 tokens 4.5 us against 5.1, FP8 1920 x 4096 at 64
+// tokens 7.65 against 8.4; only 1664 x 4096 at one token is 2 % slower).
 inline int64_t smallm_cost(int n_tiles, int k_tiles, int sms, int tokens, int s) {
   const bool shared_sm = n_tiles * s > sms;
   const int log2s = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
-  const int resident = shared_sm ? (s == 8 ? 33 : (s == 4 ? 72 : 2 * sms / s)) : (s == 8 ? 12 : (s == 4 ? 33 : sms / s));
+  int resident = smallm_resident(s, sms, shared_sm);
+  if (s == 8 && !shared_sm) resident = (resident * 4 + 4) / 5;
   const int64_t rounds = (n_tiles + resident - 1) / resident, per = (k_tiles + s - 1) / s;
   const int64_t stream = per * (1800 + 3 * tokens) * (shared_sm ? 13 : 10) / 100;
   const int64_t reduce = tokens * 3 * log2s * (shared_sm ? 3 : 1) + (s == 8 ? 9 * tokens : 0);
@@ -314,10 +330,11 @@ inline int64_t smallm_cost(int n_tiles, int k_tiles, int sms, int tokens, int s)
 }
 
 // Fewer CTAs per tile than that where they are cheaper by more than 3 %: short K slices and many tokens (the reduction), and
-// cluster counts just above what is resident.  Measured at 32 weight shapes (1024 x 1024 to 57344 x 8192), 10 token counts
-// and both formats: 1.011 of the best cluster size on average (1.106 without this step, 2.2 times at worst: FP8 2048 x 2048
+// cluster counts just above what is resident.  Measured at 37 weight shapes (1024 x 1024 to 57344 x 8192), 10 token counts and
+// both formats: 1.011 of the best cluster size's time on average (1.171 without this step, 2.3 times at worst: FP8 2048 x 2048
 // at 16 / 64 / 128 tokens 9.1 / 13.5 / 17.9 us on 8 CTAs, 5.0 / 6.7 / 8.7 on 4; 6144 x 4096 at 128 tokens 16.3 on 4, 12.3 on
-// 2), and nowhere more than 5 % slower than without.
+// 2), and nowhere more than 2 % slower than without.  At worst 1.23 of the best: FP8 5120 x 5120 at 96 tokens 14.8 us on 4
+// CTAs, 12.1 on 2; 4096 x 1024 in both formats 1.08 to 1.21, where 2 CTAs would win at every token count.
 inline int smallm_splits(int n_tiles, int k_tiles, int sms, int tokens) {
   const int most = smallm_most_splits(n_tiles, k_tiles, sms, tokens);
   const int64_t cost = smallm_cost(n_tiles, k_tiles, sms, tokens, most);
