@@ -94,13 +94,15 @@ namespace b200q {
 
 // One launch where every CTA can quantize its slice of the activation while its weights arrive: at most 16 KB of
 // activation (read by every CTA for the abs-max), at most kOwnXTiles K tiles per CTA, at most kOwnXSlice tokens x K tiles,
-// and 16 tiles of weight rows.  Measured against the quantize launch and the GEMM behind it at 1 to 16 tokens, N 1024 to
-// 28672, K 1024 to 65536, bf16, fp16 and fp32, weights rotating through more than L2 where they are that large: at the 152
-// points inside it takes 0.89 of their device time on average (0.57 at N = 2048, where the eight-CTA clusters of the plain
-// GEMM take two rounds; 0.92 elsewhere; at most 1.04 or 0.3 us more, 4 fp32 tokens of 4096 x 1024) and 0.86 of the time of
-// an eager call, which a launch less decides.  Outside, with the same kernel: 4 x 10240 x 4096 16.0 us against 13.3, 1 x
-// 10240 x 8192 27.0 against 19.5, 16 x 4096 x 4096 14.7 against 9.4 (the quantizer's work in every CTA), 1 x 1024 x 1024
-// 5.3 against 4.9 (too few CTAs to gain).
+// and 16 tiles of weight rows.  Clusters as large as they may be, which keeps the slices short, but no more than are resident at
+// once: 34 tiles on clusters of eight and 72 on clusters of four would take two rounds, which the plain GEMM avoids (8 x 4608 x
+// 1024 12.0 us against 6.5; such sizes then take smaller clusters or two launches).  Measured against the quantize launch and the
+// GEMM behind it at 844 points inside (1 to 8 tokens, N 1920 to 28672, K 256 to 8192, bf16 and fp32, weights rotating through more
+// than L2 where they are that large): 0.82 of the time of an eager call, which a launch less decides (at worst 1.09, fp32
+// 1.21).  In a replayed graph 0.91 where the range is given (at worst 1.04); where it is measured 1.02 for bf16 and 1.07 for
+// fp32 (at worst 1.16 and 1.35), whose elements every CTA reads twice.  Outside, with the same kernel: 4 x 10240 x 4096 16.0 us
+// against 12.6, 1 x 10240 x 8192 27.2 against 18.4, 16 x 4096 x 4096 14.7 against 9.0 (the quantizer's work in every CTA), 1 x
+// 1024 x 1024 5.3 against 5.2 (too few CTAs to gain).
 int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,
                      int64_t w_scales_numel, const void* bias, void* out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream) {
   const int64_t width = dtype == B200Q_F32 ? 4 : 2;
@@ -108,7 +110,9 @@ int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_n
   const int tiles = static_cast<int>((N + gemm::kSmallWRows - 1) / gemm::kSmallWRows);
   const int k_tiles = static_cast<int>((K + gemm::kBKBytes - 1) / gemm::kBKBytes);
   if (tiles < 16) return 1;
-  const int splits = gemm::smallm_most_splits(tiles, k_tiles, sm_count(), static_cast<int>(M)), per_cta = (k_tiles + splits - 1) / splits;
+  int splits = gemm::smallm_most_splits(tiles, k_tiles, sm_count(), static_cast<int>(M));
+  while (splits > 1 && tiles > gemm::smallm_resident(splits, sm_count(), true)) splits >>= 1;      // its CTAs share SMs
+  const int per_cta = (k_tiles + splits - 1) / splits;
   if (per_cta > gemm::kOwnXTiles || per_cta * M > gemm::kOwnXSlice) return 1;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(out, 16)) return 1;
   if (int rc = check_arch()) return rc;

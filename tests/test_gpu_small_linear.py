@@ -26,3 +26,17 @@ def test_same_bits_as_two_launches(b200, m, n, k, dtype):
         assert torch.equal(b200.fp8_linear(x, w, ws, b, amax), ref)
     assert torch.equal(b200.fp8_linear(torch.zeros_like(x), w, ws), torch.zeros(m, n, device="cuda", dtype=torch.bfloat16))
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 4224, 1024), (1, 4352, 1024), (8, 4352, 512), (2, 4736, 1536), (4, 9088, 512), (1, 9216, 512), (3, 9472, 512)])
+def test_cluster_counts_around_what_is_resident(b200, m, n, k):
+    """33, 34, 37, 71, 72 and 74 weight tiles: at most as many clusters as are resident at once, else smaller ones (or, where
+    the K slices are then too long, two launches).  The same bits as two launches at any cluster size."""
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    x = torch.randint(-2, 3, (m, k), device="cuda", generator=g).bfloat16()       # sums that are the same in any order
+    w = torch.randint(-2, 3, (n, k), device="cuda", generator=g).float().to(torch.float8_e4m3fn).view(torch.uint8)
+    one = torch.ones((), device="cuda")
+    y = b200.fp8_linear(x, w, one.reshape(1), None, one * 448)
+    assert torch.equal(y, (x.double() @ w.view(torch.float8_e4m3fn).double().t()).bfloat16())
+    assert capi.device_status() == 0
