@@ -39,13 +39,8 @@ int* device_status_word() {
   return g_status_addr[dev];
 }
 
-int active_clusters(int size) {
-  static std::atomic<int> known[64][4] = {};               // by device and log2(size); 0 = not asked yet
-  const int sms = sm_count(), i = size == 2 ? 1 : (size == 4 ? 2 : 3);
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sms / size;
-  int n = known[dev][i].load(std::memory_order_relaxed);
-  if (n > 0) return n;
+namespace {
+int ask_active_clusters(int size, int sms) {
   using C = SmallCfg<false>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(size * sms));
@@ -58,13 +53,26 @@ int active_clusters(int size) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  int n = 0;
   if (cudaFuncSetAttribute(gemm_smallm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&n, gemm_smallm_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
-    n = sms / size;                                        // as if no GPC had SMs left over
+    n = sms > size ? sms / size : 1;                       // as if no GPC had SMs left over
   }
-  known[dev][i].store(n, std::memory_order_relaxed);
   return n;
+}
+}  // namespace
+
+ActiveClusters active_clusters(int sms) {
+  static std::atomic<uint64_t> known[64] = {};             // by device: three counts of 16 bits, 0 = not asked yet
+  int dev = 0;
+  const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+  uint64_t v = keep ? known[dev].load(std::memory_order_relaxed) : 0u;
+  if (v == 0) {
+    for (int size = 8; size >= 2; size >>= 1) v = v << 16 | static_cast<uint64_t>(ask_active_clusters(size, sms));
+    if (keep) known[dev].store(v, std::memory_order_relaxed);
+  }
+  return {sms, static_cast<int>(v & 0xffffu), static_cast<int>(v >> 16 & 0xffffu), static_cast<int>(v >> 32)};
 }
 
 bool valid_tile_n(int bn) {
@@ -110,8 +118,12 @@ int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_n
   const int tiles = static_cast<int>((N + gemm::kSmallWRows - 1) / gemm::kSmallWRows);
   const int k_tiles = static_cast<int>((K + gemm::kBKBytes - 1) / gemm::kBKBytes);
   if (tiles < 16) return 1;
-  int splits = gemm::smallm_most_splits(tiles, k_tiles, sm_count(), static_cast<int>(M));
-  while (splits > 1 && tiles > gemm::smallm_resident(splits, sm_count(), true)) splits >>= 1;      // its CTAs share SMs
+  const int sms = sm_count();
+  int splits = gemm::smallm_most_splits(tiles, k_tiles, sms, static_cast<int>(M));
+  if (splits > 1) {
+    const gemm::ActiveClusters clusters = gemm::active_clusters(sms);
+    while (splits > 1 && tiles > gemm::smallm_resident(splits, clusters, true)) splits >>= 1;      // its CTAs share SMs
+  }
   const int per_cta = (k_tiles + splits - 1) / splits;
   if (per_cta > gemm::kOwnXTiles || per_cta * M > gemm::kOwnXSlice) return 1;
   if (!aligned(x, 16) || !aligned(w, 16) || !aligned(out, 16)) return 1;

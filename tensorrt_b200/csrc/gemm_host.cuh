@@ -300,17 +300,19 @@ inline int smallm_most_splits(int n_tiles, int k_tiles, int sms, int tokens) {
 }
 
 // Clusters of 2, 4 or 8 CTAs, one per SM, that are resident at once on the current device.  A cluster does not cross a GPC, and
-// how many SMs a GPC has differs from part to part, so the occupancy API is asked, once per device.
-int active_clusters(int size);
+// how many SMs a GPC has differs from part to part, so the occupancy API is asked, once per device.  `sms`: SMs of the device.
+struct ActiveClusters {
+  int sms, of2, of4, of8;
+};
+ActiveClusters active_clusters(int sms);
 
 // Clusters of `s` CTAs of a small-M kernel that are resident at once, two CTAs per SM where `shared_sm`.  Seen as the jump to a
 // second round on a part where the API gives 74, 33 and 15 clusters of 2, 4 and 8 (FP8 at 16 tokens, K 4096): alone 15 of 8
 // (5.98 us, 16 take 10.2) and 33 of 4 (8.1, 34 take 12.3); two CTAs per SM have the places of clusters of half the size: 33 of 8
 // (7.3, 34 take 11.3), 148 of 2 (14.9, 149 take 21.1), and of 4 nearly, 71 (9.4, 72 take 14.1).
-inline int smallm_resident(int s, int sms, bool shared_sm) {
-  if (s == 1) return shared_sm ? 2 * sms : sms;
-  if (!shared_sm) return active_clusters(s);
-  return s == 2 ? sms : (s == 4 ? (active_clusters(2) * 71 + 73) / 74 : active_clusters(4));
+inline int smallm_resident(int s, const ActiveClusters& c, bool shared_sm) {
+  if (!shared_sm) return s == 1 ? c.sms : (s == 2 ? c.of2 : (s == 4 ? c.of4 : c.of8));
+  return s == 1 ? 2 * c.sms : (s == 2 ? c.sms : (s == 4 ? (c.of2 * 71 + 73) / 74 : c.of4));
 }
 
 // Time of the small-M kernel with clusters of `s` CTAs in ns, good enough to compare cluster sizes: a launch, the K tiles of a
@@ -318,10 +320,10 @@ inline int smallm_resident(int s, int sms, bool shared_sm) {
 // for every further round of clusters.  Clusters of eight count as one round up to four fifths of those that fit: with 13 to 15
 // tiles clusters of four take 0.87 to 0.97 of their time (NVFP4 1920 x 2048 at 8 tokens 4.5 us against 5.1, FP8 1920 x 4096 at 64
 // tokens 7.65 against 8.4; only 1664 x 4096 at one token is 2 % slower).
-inline int64_t smallm_cost(int n_tiles, int k_tiles, int sms, int tokens, int s) {
-  const bool shared_sm = n_tiles * s > sms;
+inline int64_t smallm_cost(int n_tiles, int k_tiles, const ActiveClusters& c, int tokens, int s) {
+  const bool shared_sm = n_tiles * s > c.sms;
   const int log2s = s == 1 ? 0 : (s == 2 ? 1 : (s == 4 ? 2 : 3));
-  int resident = smallm_resident(s, sms, shared_sm);
+  int resident = smallm_resident(s, c, shared_sm);
   if (s == 8 && !shared_sm) resident = (resident * 4 + 4) / 5;
   const int64_t rounds = (n_tiles + resident - 1) / resident, per = (k_tiles + s - 1) / s;
   const int64_t stream = per * (1800 + 3 * tokens) * (shared_sm ? 13 : 10) / 100;
@@ -337,11 +339,13 @@ inline int64_t smallm_cost(int n_tiles, int k_tiles, int sms, int tokens, int s)
 // CTAs, 12.1 on 2; 4096 x 1024 in both formats 1.08 to 1.21, where 2 CTAs would win at every token count.
 inline int smallm_splits(int n_tiles, int k_tiles, int sms, int tokens) {
   const int most = smallm_most_splits(n_tiles, k_tiles, sms, tokens);
-  const int64_t cost = smallm_cost(n_tiles, k_tiles, sms, tokens, most);
+  if (most == 1) return 1;
+  const ActiveClusters clusters = active_clusters(sms);
+  const int64_t cost = smallm_cost(n_tiles, k_tiles, clusters, tokens, most);
   int best = most;
   int64_t least = cost * 97 / 100;
   for (int s = most >> 1; s >= 1; s >>= 1) {
-    const int64_t c = smallm_cost(n_tiles, k_tiles, sms, tokens, s);
+    const int64_t c = smallm_cost(n_tiles, k_tiles, clusters, tokens, s);
     if (c < least) least = c, best = s;
   }
   return best;
