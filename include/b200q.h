@@ -195,7 +195,7 @@ int b200q_fp8_gemm(const uint8_t* a_codes, const float* a_scales, int64_t a_scal
                    const void* bias, void* out, int64_t M, int64_t N, int64_t K,
                    b200q_stream_t stream, const b200q_cfg* cfg);
 
-/* b200q_fp8_gemm with the gate/up activation fused into its epilogue (producer fusion):
+/* b200q_fp8_gemm with the gate/up activation fused into its epilogue:
  * b holds F gate rows followed by F up rows (N = 2 F, F a multiple of 128; scales and bias indexed the
  * same way), out is [M, F] bf16 = silu(g) * u with g, u the two linear outputs rounded to bf16 first,
  * i.e. the same bits as b200q_fp8_gemm followed by b200q_silu_mul, without the [M, 2 F] round trip
@@ -220,6 +220,9 @@ int b200q_nvfp4_gemm(const uint8_t* a_codes, const uint8_t* a_scales, const floa
                      const uint8_t* b_codes, const uint8_t* b_scales, const float* b_global,
                      const void* bias, void* out, int64_t M, int64_t N, int64_t K,
                      b200q_stream_t stream, const b200q_cfg* cfg);
+/* Tile that b200q_nvfp4_gemm takes for M rows and N columns when cfg does not force one, as a b200q_cfg::tile_n value: 512, 256
+ * or 128; 0 for the kernel of up to 128 rows.  Host only. */
+int b200q_nvfp4_gemm_tile(int64_t M, int64_t N);
 /* NVFP4 gate/up GEMM of a gated MLP with the activation and its static quantizer in the epilogue: B holds F
  * gate rows, then F up rows (N = 2F, N % 256 == 0); codes_out [M, F/2], scales_out (swizzled, padding rows of the last
  * 128-row tile zero) and global_scale_out[0] (may be NULL) hold silu(gate) * up under the calibrated abs-max

@@ -38,6 +38,7 @@ SIGNATURES = {
     "b200q_fp8_gemm_silu_mul": (_c.c_int, [_p, _p, _i64, _p, _p, _i64, _p, _p, _i64, _i64, _i64, _p, _p]),
     "b200q_fp8_gemm_silu_mul_quantize": (_c.c_int, [_p, _p, _i64, _p, _p, _i64, _p, _p, _p, _p, _i64, _i64, _i64, _p, _p]),
     "b200q_nvfp4_gemm": (_c.c_int, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _p, _p]),
+    "b200q_nvfp4_gemm_tile": (_c.c_int, [_i64, _i64]),
     "b200q_nvfp4_gemm_silu_mul_quantize": (_c.c_int, [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _p]),
     "b200q_fp8_gemm_reduce_scatter": (_c.c_int, [_p, _p, _i64, _p, _p, _i64, _p, _i64, _i64, _i64, _p, _p]),
     "b200q_nvfp4_gemm_reduce_scatter": (_c.c_int, [_p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _p, _p]),

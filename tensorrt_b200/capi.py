@@ -317,6 +317,12 @@ def nvfp4_gemm(a_codes, a_scales, a_global, b_codes, b_scales, b_global, bias=No
     return out
 
 
+def nvfp4_gemm_tile(M: int, N: int) -> int:
+    """`tile_n` that `nvfp4_gemm` takes for M rows and N columns here: what `gemm_config` forces, else the library's choice
+    (512 = CTA pair; 0 = the kernel of up to 128 rows)."""
+    return gemm_defaults()[0] or load().b200q_nvfp4_gemm_tile(M, N)
+
+
 def nvfp4_gemm_silu_mul_quantize(a_codes, a_scales, a_global, b_codes, b_scales, b_global, act_amax):
     """gate/up GEMM (B = F gate rows, then F up rows; F a multiple of 128) with silu(gate) * up and its NVFP4 quantizer
     under the calibrated abs-max in the epilogue -> NVFP4 operand [.., F] (codes, swizzled scales, global scale), the same

@@ -33,6 +33,11 @@ int b200q_nvfp4_gemm(const uint8_t* a_codes, const uint8_t* a_scales, const floa
   return gemm::launch<true>(a_codes, b_codes, p, static_cast<cudaStream_t>(stream), cfg);
 }
 
+int b200q_nvfp4_gemm_tile(int64_t M, int64_t N) {
+  if (M <= gemm::kBM || N <= 0 || M > 0x7fffff00LL || N > 0x7fffff00LL) return 0;
+  return gemm::large_tile(static_cast<int>(M), static_cast<int>(N), sm_count(), true, false);
+}
+
 int b200q_nvfp4_gemm_silu_mul_quantize(const uint8_t* a_codes, const uint8_t* a_scales, const float* a_global, const uint8_t* b_codes,
                                        const uint8_t* b_scales, const float* b_global, const float* act_amax, uint8_t* codes_out,
                                        uint8_t* scales_out, float* global_scale_out, int64_t M, int64_t N, int64_t K,

@@ -155,11 +155,14 @@ class CudaBackend:
         return capi.silu_mul_nvfp4_quantize(gate_up, amax)
 
     def gate_up_quantize_static(self, xq, qw, amax):
-        """gate/up GEMM with the activation and its NVFP4 quantizer in the epilogue, or None: up to 128 tokens, where the
-        GEMM streams its weights through the small-M kernel, and F that is not whole tiles.  Measured at 129 to 8192 tokens
-        and five weight shapes: 0.70 to 0.98 of the separate kernels' time (14336 x 4096: 26.1 -> 23.8 us at 129 tokens,
-        80.5 -> 64.5 at 1024, 556 -> 424 at 8192)."""
-        if self.mode != "nvfp4" or not self.fuse_gate_up or xq[0].shape[0] <= 128 or qw[0].shape[0] % 256:
+        """gate/up GEMM with the activation and its NVFP4 quantizer in the epilogue, or None: F that is not whole tiles, and
+        where the plain GEMM would not run on CTA pairs, which the fused form always does (up to 128 tokens, and sizes that
+        finer tiles cover in fewer rounds).  Measured at 129 to 8192 tokens and 15 weight shapes: 0.52 to 0.98 of the separate
+        kernels' time, 0.84 on average (14336 x 4096: 26.1 -> 23.8 us at 129 tokens, 80.5 -> 64.5 at 1024, 556 -> 424 at
+        8192); at the ten points of 209 that this leaves out 1.00 to 1.11 (5120 x 8192 at 257 tokens 33.2 against 36.7)."""
+        if self.mode != "nvfp4" or not self.fuse_gate_up or qw[0].shape[0] % 256:
+            return None
+        if capi.nvfp4_gemm_tile(xq[0].shape[0], qw[0].shape[0]) != 512:
             return None
         return capi.nvfp4_gemm_silu_mul_quantize(*xq, *qw, amax)
 

@@ -124,23 +124,27 @@ def test_fused_add_norm_quantize(b200, cols):
 @pytest.mark.parametrize("cols", [64, 1040, 4096, 8192, 12288])
 @pytest.mark.parametrize("rows", [1184, 2501])
 def test_fused_add_norm_quantize_many_tokens(b200, rows, cols):
-    """From 8 rows per SM on, the kernel is the persistent one fed through a shared-memory ring of rows
-    (where a row fits the ring): bit-identical with the one-CTA-per-row form run on slices of the same
-    input, with and without delta, repeatedly (the ring's barriers start from scratch every launch)."""
+    """From 8 rows per SM on, rows of up to 8192 elements go to warps, or with a delta and more than 4096 elements to the
+    persistent kernel fed through a shared-memory ring of rows: bit-identical with the separate kernels and with slices of
+    the same input, which take other forms, with and without delta, repeatedly (the ring's barriers start from scratch every
+    launch)."""
     capi = b200.capi
     g = torch.Generator().manual_seed(rows + cols)
     h = torch.randn(rows, cols, generator=g).bfloat16().cuda()
     d = (torch.randn(rows, cols, generator=g) * 0.3).bfloat16().cuda()
     w = (1 + 0.1 * torch.randn(cols, generator=g)).bfloat16().cuda()
-    # slices of 300 to 900 rows: one CTA per row there (fewer rows would split a row over a cluster,
-    # which sums the squares in another order)
+    # slices of 300 to 900 rows: one CTA per row, or warps where a slice has 2^21 elements (fewer rows would add the squares
+    # in another order)
     edges = list(range(0, rows - 300, 400)) + [rows]
     for delta in (d, None):
         parts = [capi.add_rms_norm_fp8_quantize(h[a:b].clone(), None if delta is None else delta[a:b], w, 1e-5)
                  for a, b in zip(edges[:-1], edges[1:])]
+        h_ref = h if delta is None else capi.add(h, delta)
+        c_ref, s_ref = capi.fp8_quantize(capi.rms_norm(h_ref, w, 1e-5), None)
         for _ in range(2):
             h_new, codes, scales = capi.add_rms_norm_fp8_quantize(h.clone(), delta, w, 1e-5)
             assert torch.equal(h_new, torch.cat([p[0] for p in parts]))
+            assert torch.equal(h_new, h_ref) and torch.equal(codes, c_ref) and torch.equal(scales.flatten(), s_ref.flatten())
             assert torch.equal(codes, torch.cat([p[1] for p in parts]))
             assert torch.equal(scales, torch.cat([p[2] for p in parts]))
     assert capi.device_status() == 0
@@ -164,6 +168,48 @@ def test_stack_matches_oracle_single_gpu(b200, mode):
     # bf16 intermediates round differently on the two sides; the quantized linears then see
     # slightly different inputs, so the tolerance is looser than for a single GEMM
     assert o.rel_l2(y.float().cpu(), ref.float()) < (2e-2 if mode == "fp8" else 6e-2)
+
+
+@pytest.mark.parametrize("tokens,ffn,fused", [(128, 1024, False), (129, 1024, True), (257, 1024, True), (129, 1088, False), (257, 5120, False),
+                                              (513, 5120, True)])
+def test_calibrated_nvfp4_stack_with_fused_gate_up(b200, tokens, ffn, fused):
+    """Calibrated NVFP4 stack whose gate/up GEMM applies the activation and quantizes (F in whole 128-column tiles, sizes that
+    the plain GEMM runs on CTA pairs): the same bits as without it; elsewhere (few tokens, a ragged F, and 257 x 10240, which
+    128 x 256 tiles cover in one round) it is not called."""
+    from tensorrt_b200.stack import CudaBackend, DecoderStack, StackConfig
+
+    cfg = StackConfig(hidden=512, n_q=8, n_kv=2, head_dim=64, ffn=ffn, layers=2, mode="nvfp4")
+    ws = _weights(cfg, 8)
+    h = torch.randn(tokens, cfg.hidden, generator=torch.Generator().manual_seed(tokens)).bfloat16()
+
+    class Counting(CudaBackend):
+        fused = 0
+
+        def gate_up_quantize_static(self, xq, qw, amax):
+            out = super().gate_up_quantize_static(xq, qw, amax)
+            self.fused += out is not None
+            return out
+
+    outs = []
+    for fuse in (True, False):
+        be = Counting("nvfp4", fuse_gate_up=fuse)
+        stack = DecoderStack(cfg, _to(ws, "cuda"), backend=be)
+        stack.calibrate(h.cuda())
+        assert be.fused == 0
+        outs.append(stack.forward(h.cuda()))
+        assert be.fused == (cfg.layers if fuse and fused else 0)
+    assert torch.equal(*outs)
+    with b200.capi.gemm_config(tile_n=128):              # a forced tile keeps the separate kernels
+        stack = DecoderStack(cfg, _to(ws, "cuda"), backend=Counting("nvfp4"))
+        stack.calibrate(h.cuda())
+        stack.forward(h.cuda())
+        assert stack.backend.fused == 0
+    ref = h
+    for w in ws:
+        ref = o.decoder_layer_ref(ref, w, cfg.n_q, cfg.n_kv, cfg.head_dim, "nvfp4")
+    # the calibration batch is the measured one, so the oracle's measured ranges are the calibrated ones up to bf16 roundings
+    assert o.rel_l2(outs[0].float().cpu(), ref.float()) < 6e-2
+    assert b200.capi.device_status() == 0
 
 
 def test_stack_with_fp8_attention_matches_oracle(b200):
