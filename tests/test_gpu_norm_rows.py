@@ -69,3 +69,53 @@ def test_few_rows_one_piece_per_thread(b200, rows, cols):
         ref = capi.nvfp4_quantize(x, amax)
         assert torch.equal(h_new, h_ref) and torch.equal(got[2], ref[2]) and all(few(a, b) for a, b in zip(got[:2], ref[:2]))
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("with_delta", [True, False])
+@pytest.mark.parametrize("rows,cols", [(5, 4096), (1190, 4096), (1190, 528)])
+def test_nan_beside_values_above_the_range(b200, rows, cols, with_delta):
+    """A NaN norm weight puts one NaN into a block of every row; under a range far below the data the block's scale saturates
+    and the NaN's code is decided there.  Small integers in: the sum of squares is the same in any order, codes are compared
+    bit for bit."""
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    h, d = (torch.randint(-3, 4, (rows, cols), device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = torch.ones(cols, device="cuda").bfloat16()
+    w[5], w[cols - 1] = float("nan"), -float("nan")
+    delta = d if with_delta else None
+    x = capi.rms_norm(capi.add(h, d) if with_delta else h, w)
+    assert bool(x[:, 5].isnan().all())
+    for amax in (0.25, 4.0):
+        amax = torch.tensor(amax, device="cuda")
+        got, ref = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)[1], capi.nvfp4_quantize(x, amax)
+        assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+@pytest.mark.parametrize("rows,cols,offset", [(5, 2064, 8), (200, 8192, 8), (200, 16384, 8), (64, 4096, 8), (80, 12288, 8), (5, 8192, 8),
+                                              (16, 16384, 0), (7, 2048, 0), (64, 8192, 0), (200, 4112, 0)])
+@pytest.mark.parametrize("finite", [True, False])
+def test_few_rows_of_small_integers(b200, rows, cols, offset, finite):
+    """Few rows on clusters of two (one, two and four groups of 8 a thread), four (one, two) and eight CTAs, which take bases 16
+    but not 32 bytes aligned, on clusters of eight with aligned bases, and on a CTA per row.  Small integers: the sum of squares
+    is the same in any order, so codes and scales equal the separate kernels' bit for bit, a range below the data included."""
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    make = lambda: torch.randint(-3, 4, (rows * cols + offset,), device="cuda", generator=g).bfloat16()[offset:].view(rows, cols)  # noqa: E731
+    h, d = make(), make()
+    h[rows // 2] = 0
+    d[rows // 2] = -0.0
+    if not finite:
+        h[0, cols // 2], h[1, 5], d[2, cols - 1] = float("nan"), float("inf"), float("nan")
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=g)).bfloat16()
+    same = lambda a, b: torch.equal(a.flatten().view(torch.uint8), b.flatten().view(torch.uint8))  # noqa: E731
+    for delta in (d, None):
+        h_ref = capi.add(h, d) if delta is not None else h
+        x = capi.rms_norm(h_ref, w)
+        h_new, codes, scales = capi.add_rms_norm_fp8_quantize(h, delta, w)
+        c_ref, s_ref = capi.fp8_quantize(x, None)
+        assert same(h_new, h_ref) and same(codes, c_ref) and same(scales, s_ref)
+        for amax in (4.0, 0.5):
+            amax = torch.tensor(amax, device="cuda")
+            got, ref = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)[1], capi.nvfp4_quantize(x, amax)
+            assert all(torch.equal(a, b) for a, b in zip(got, ref))
+    assert capi.device_status() == 0

@@ -1,7 +1,7 @@
 """Kernels that quantize to NVFP4 what they produce (residual add + RMSNorm, silu(gate) * up, repeated kv heads) under a
 calibrated amax: codes, swizzled scales (padding rows included) and global scale equal the separate kernels' bit for
-bit, at row counts around 128-row scale tiles and at the edges of their launch shapes.  Where the norm splits a row over
-a cluster it adds the squares in another order; codes may then differ as rarely as a bf16 rounding does."""
+bit, at row counts around 128-row scale tiles and at the edges of their launch shapes.  With few long rows the norm adds the
+squares in another order; codes may then differ as rarely as a bf16 rounding does."""
 import pytest
 import torch
 
@@ -24,7 +24,7 @@ def test_add_rms_norm(b200, rows, cols, with_delta):
     delta = d if with_delta else None
     h_ref = capi.add(h, d) if with_delta else h
     x = capi.rms_norm(h_ref, w)
-    split = rows < 2 * torch.cuda.get_device_properties(0).multi_processor_count and cols >= 2048     # a row on several CTAs
+    split = rows < 2 * torch.cuda.get_device_properties(0).multi_processor_count and cols >= 2048     # few long rows
     for amax in (capi.amax(x), capi.amax(x) * 0.25, torch.zeros((), device="cuda")):
         h_new, got = capi.add_rms_norm_nvfp4_quantize(h, delta, w, amax)
         assert torch.equal(h_new, h_ref)
@@ -44,7 +44,7 @@ def _scales_by_row(sf, cols):
     return tiles.permute(0, 3, 2, 1, 4).reshape(-1, tiles.shape[1] * 4)
 
 
-@pytest.mark.parametrize("rows,cols", [(3, 272), (5, 4096), (300, 4096), (1300, 2080)])      # one CTA, a cluster a row, many rows, the ring
+@pytest.mark.parametrize("rows,cols", [(3, 272), (5, 4096), (300, 4096), (1300, 2080)])      # CTAs of 8-element groups, a CTA a row of 16-element pieces, groups again, warps
 def test_add_rms_norm_of_rows_that_are_not_finite(b200, rows, cols):
     """A NaN makes its whole row NaN, an infinity makes its row zeros with one NaN: as the separate kernels store them."""
     capi = b200.capi
