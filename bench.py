@@ -12,10 +12,10 @@ grows (strong scaling).  `value` = tokens/s with activations and weights residen
 the same through `DecoderStack.forward` from pinned host activations with the full bf16 result
 copied back to pinned host memory inside the timed region; decode (batch 64, one token) is
 reported beside it.  On one GPU the line also carries `extras`: quantize GB/s and the full
-quantized-linear GEMM sweep, each entry with its own roofline object (the other two thirds of the
-metric), and the CPU baseline.
+quantized-linear GEMM sweep in a few numbers (the other two thirds of the metric), and the CPU baseline.
 
-One JSON line is printed by rank 0.  `--impl reference` times the CPU restatement of the
+One JSON line is printed by rank 0 on stdout, short enough for a reader that keeps the end of the output only; the same with
+every detail (each kernel and GEMM shape with its own roofline object, parity, time per layer) goes to stderr.  `--impl reference` times the CPU restatement of the
 reference's eager semantics (oracle/) on the host cores for the same metric and workload.
 Other workloads: `nvfp4_stack`, `nvfp4_quantize`, `fp8_quantize`, `fp8_gemm`, `nvfp4_gemm`; `small_cases` launches the
 element-wise and attention kernels twice on small inputs (for profiler captures, nothing timed).
@@ -60,7 +60,7 @@ def main():
                     help="tp_stack: 1 = silu(gate) * up in the epilogue of the gate/up GEMM, 0 = in its own kernel (A/B runs)")
     ap.add_argument("--call-times", type=int, default=0, dest="call_times",
                     help="tp_stack on one GPU: 1 = one extra forward with CUDA events around every library call; "
-                         "per-call totals are added to the line as `call_times`")
+                         "per-call totals go to stderr as `call_times`")
     ap.add_argument("--slabs", type=int, default=1, help="row slabs per row-parallel linear (all-reduce overlap) in tp_stack")
     args = ap.parse_args()
     if args.impl == "reference":

@@ -8,6 +8,7 @@ import json
 import os
 import statistics
 import subprocess
+import sys
 import threading
 import time
 from pathlib import Path
@@ -18,6 +19,8 @@ ROOT = Path(__file__).resolve().parent
 
 ROWS = COLS = 8192                        # the NVFP4 quantize configuration: bf16 [8192, 8192]
 ALG_BYTES_PER_ELEM = 2 + 0.5 + 1.0 / 16  # bf16 read, packed code write, block-scale write
+REQUIRED_KEYS = ("impl", "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline",
+                 "dtype", "data", "config", "clocks", "e2e", "gpu_launches", "roofline", "device_status", "error")
 L2_ROTATION = 4                           # distinct input tensors cycled through (4 x 134 MB > 126 MB L2)
 
 
@@ -95,6 +98,27 @@ def make_input(seed: int, rows: int = ROWS, cols: int = COLS) -> torch.Tensor:
     x = torch.randn(rows, cols, generator=g)
     x[torch.rand(rows, cols, generator=g) < 0.01] *= 50
     return x.bfloat16()
+
+
+def _short(v):
+    if isinstance(v, float):
+        return float(f"{v:.6g}")
+    if isinstance(v, dict):
+        return {k: _short(x) for k, x in v.items()}
+    return [_short(x) for x in v] if isinstance(v, (list, tuple)) else v
+
+
+def print_line(line: dict, details: dict | None = None, limit: int = 2600) -> None:
+    """The result as ONE JSON line on stdout, floats at six digits and short enough (`limit` characters) for a reader that keeps
+    the end of the output only.  `details` (per-shape tables) go to stderr with everything else, at full precision; what would
+    still be too long leaves the line from its end."""
+    if details:
+        print(json.dumps({**line, **details}), file=sys.stderr, flush=True)
+    line = _short(line)
+    optional = [k for k in line if k not in REQUIRED_KEYS]
+    while len(json.dumps(line)) > limit and optional:
+        line.pop(optional.pop())
+    print(json.dumps(line), flush=True)
 
 
 def dist_setup(n_gpus: int):

@@ -133,7 +133,7 @@ def quantize_suite(capi, peaks, min_ms=500.0):
 
         ms, k = time_graphed(lambda: capi.fp8_quantize(rot(), None), 12, min_ms)
         alg = 3.0 * n + 4.0 * rows
-        out[f"fp8_per_token_quantize_{rows}x{cols}"] = {"ms": ms, "launches": k, "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "fp8_rows_kernel<bf16>")}
+        out[f"fp8_per_token_quantize_{rows}x{cols}"] = {"ms": ms, "launches": k, "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "fp8_rows_wide_kernel<bf16>" if cols > 4096 else "fp8_rows_kernel<bf16>")}
         ms, k = time_graphed(lambda: capi.amax(rot()), 12, min_ms)
         out[f"amax_{rows}x{cols}"] = {"ms": ms, "launches": k, "roofline": hbm_roofline(2.0 * n / ms / 1e6, peaks, 2.0 * n, "amax_kernel<bf16>")}
         am = capi.amax(xs[0])
@@ -158,7 +158,7 @@ def glue_suite(capi, peaks, min_ms=300.0, tokens=32768, hidden=8192, ffn=28672):
 
     ms, k = time_device(lambda: capi.silu_mul_fp8_quantize(rot(gu)), min_ms)
     alg = tokens * ffn * (4.0 + 1.0) + 4.0 * tokens
-    out[f"silu_mul_fp8_quantize_{tokens}x{ffn}"] = {"ms": ms, "launches": k, "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "silu_mul_quant_kernel")}
+    out[f"silu_mul_fp8_quantize_{tokens}x{ffn}"] = {"ms": ms, "launches": k, "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "silu_mul_quant_stream_kernel")}
     del gu
     hs = [torch.randn(tokens, hidden, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
     ds = [torch.randn(tokens, hidden, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
@@ -166,7 +166,7 @@ def glue_suite(capi, peaks, min_ms=300.0, tokens=32768, hidden=8192, ffn=28672):
     ms, k = time_device(lambda: capi.add_rms_norm_fp8_quantize(rot(hs), rot(ds), w), min_ms)
     alg = tokens * hidden * (2.0 + 2.0 + 2.0 + 1.0) + 4.0 * tokens      # h, delta in; h, codes out
     out[f"add_rms_norm_fp8_quantize_{tokens}x{hidden}"] = {"ms": ms, "launches": k,
-                                                           "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "add_norm_quant_kernel")}
+                                                           "roofline": hbm_roofline(alg / ms / 1e6, peaks, alg, "add_norm_quant_stream_kernel")}
     return out
 
 
@@ -369,6 +369,27 @@ def extras(capi, peaks, min_ms=500.0):
     return out
 
 
+def summary(ex: dict) -> dict:
+    """`extras` in a few numbers: least and largest GB/s of each quantize kernel and GB/s of the layer's glue; least / median /
+    largest fraction of the roofline and largest TFLOP/s of each GEMM sweep; TFLOP/s of attention and MLP.  Entries that failed
+    (they hold an error) are left out."""
+    ok = lambda d: {k: v for k, v in d.items() if "roofline" in v}  # noqa: E731
+    gbs: dict = {}
+    for k, v in {**ok(ex["quantize"]), **ok(ex["layer_glue"])}.items():
+        name = k.replace("_seed1", "").rsplit("_", 1)[0]             # without the sizes
+        gbs.setdefault(name, []).append(round(v["roofline"]["achieved"]))
+    out: dict = {"GBps": {k: [min(v), max(v)] for k, v in gbs.items()}}
+    for kind in ("fp8_gemm", "nvfp4_gemm"):
+        f = sorted(round(v["roofline"]["frac"], 3) for v in ok(ex[kind]).values())
+        if f:
+            out[kind] = {"shapes": len(f), "frac": [f[0], f[len(f) // 2], f[-1]], "tflops_max": round(max(v["tflops"] for v in ok(ex[kind]).values()))}
+    for kind in ("fp8_attention", "fp8_gated_mlp"):
+        v = ex[kind].get("fused_static", ex[kind])
+        if "tflops" in v:
+            out[kind + "_tflops"] = round(v["tflops"])
+    return out
+
+
 # ----------------------------------------------------------------------------- workloads
 def run_gemm(args, kind):
     from tensorrt_b200 import capi
@@ -390,9 +411,10 @@ def run_gemm(args, kind):
                    "l2": "operand sets rotate so that sets smaller than L2 are not re-read from L2",
                    "timing": "every shape is timed as a CUDA graph of back-to-back launches (host issue time excluded); "
                              "M <= 128: weights declared static per call (b200q_cfg::static_weights)"},
-        "clocks": clocks.summary(), "gpu_launches": head["launches"], "roofline": head["roofline"], "shapes": results,
+        "clocks": clocks.summary(), "gpu_launches": head["launches"], "roofline": head["roofline"],
+        "tflops": {k: round(v["tflops"]) for k, v in results.items() if "tflops" in v},
     }
-    print(json.dumps(line))
+    bc.print_line(line, {"shapes": results})
 
 
 def quantize_e2e(capi, which, slabs=8, steps=10):
@@ -454,7 +476,7 @@ def run_quantize(args, which):
         e2e_ms, h2d, d2h = quantize_e2e(capi, which)
     key = "nvfp4_quantize_8192x8192_seed1" if which == "nvfp4" else "fp8_per_token_quantize_16384x4096"
     head = suite[key]
-    print(json.dumps({
+    bc.print_line({
         "metric": f"{which}_quantize_throughput", "value": head["roofline"]["achieved"], "unit": "GB/s", "n_gpus": 1,
         "steps": head["launches"], "warmup": 3, "ms_per_step": head["ms"], "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -463,7 +485,7 @@ def run_quantize(args, which):
         "e2e": {"value": head["roofline"]["algorithmic_bytes_per_launch"] / e2e_ms / 1e6, "unit": "GB/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "path": "pinned host tensor -> device, quantize, codes + scales -> pinned host, 8 row slabs pipelined on two copy streams"},
-        "kernels": suite}))
+        "GBps": {k: round(v["roofline"]["achieved"]) for k, v in suite.items()}}, {"kernels": suite})
 
 
 def run_small_cases(args):

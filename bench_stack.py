@@ -254,8 +254,9 @@ def call_times(capi, stack, h, mb, sharded):
 
     import tensorrt_b200.stack as st
 
-    names = ("fp8_gemm", "fp8_gemm_silu_mul", "nvfp4_gemm", "add_rms_norm_fp8_quantize", "silu_mul_fp8_quantize", "silu_mul", "rms_norm",
-             "expand_heads", "expand_heads_fp8_quantize", "fp8_quantize", "nvfp4_quantize", "amax", "add")
+    names = ("fp8_gemm", "fp8_gemm_silu_mul", "nvfp4_gemm", "nvfp4_gemm_silu_mul_quantize", "add_rms_norm_fp8_quantize", "add_rms_norm_nvfp4_quantize",
+             "silu_mul_fp8_quantize", "silu_mul_nvfp4_quantize", "silu_mul", "rms_norm", "expand_heads", "expand_heads_fp8_quantize",
+             "expand_heads_nvfp4_quantize", "fp8_quantize", "nvfp4_quantize", "fp8_sdpa_packed", "amax", "add")
     records, saved = [], {}
 
     def wrap(name):
@@ -425,9 +426,9 @@ def run(args):
         if sharded and fused:
             breakdown["collective_stages"] = collective_stage_times(capi, stack, cfg, world, tokens // mb)
     # launches of this library per layer and micro-batch: norm + quantize, QKV GEMM, head expansion + quantize, O GEMM,
-    # norm + quantize, gate/up GEMM (activation in its epilogue), quantize, down GEMM; the token-sharded form replaces
-    # the two norm kernels by a flag exchange + reduce / norm / quantize / gather pair each
-    kernels_per_layer = 10 if (world > 1 and sharded and fused) else 8
+    # norm + quantize, gate/up GEMM (activation in its epilogue; calibrated NVFP4 quantizes there too), quantize, down GEMM;
+    # the token-sharded form replaces the two norm kernels by a flag exchange + reduce / norm / quantize / gather pair each
+    kernels_per_layer = 10 if (world > 1 and sharded and fused) else (7 if cfg.mode == "nvfp4" else 8)
     launches = steps * (cfg.layers * kernels_per_layer * (mb if world > 1 else 1) + 2)
     line = {
         "metric": "tp_decoder_stack_prefill_throughput" if tp else "nvfp4_decoder_stack_prefill_throughput",
@@ -445,35 +446,39 @@ def run(args):
         "gpu_launches": launches,
         "e2e": {"value": tokens * e2e_steps / (e2e_ms * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": h_host.numel() * 2,
                 "d2h_bytes_per_step": y_host.numel() * 2, "steps": e2e_steps, "ms_per_step": e2e_ms / e2e_steps,
-                "path": "pinned host bf16 activations -> device"
-                        + (" of rank 0 -> broadcast to the ranks over NVLink" if world > 1 else "")
-                        + ", DecoderStack.forward, bf16 result -> pinned host" + (" of rank 0" if world > 1 else "")},
+                "path": "pinned host -> device" + (" of rank 0 -> broadcast over NVLink" if world > 1 else "")
+                        + ", DecoderStack.forward, result -> pinned host" + (" of rank 0" if world > 1 else "")},
         "model_tflops": tflops,
         "roofline": {"bound": "tensor", "achieved": tflops / world, "peak": peaks["bf16_tflops_sustained"] * scale, "unit": "TFLOP/s",
                      "frac": tflops / world / (peaks["bf16_tflops_sustained"] * scale),
-                     "peak_source": f"{peaks['source']} sustained cuBLAS bf16 x{int(scale)} per GPU; GEMM flops only, per GPU, "
-                                    "over the whole step (glue and exchange kernels included in the time)",
+                     "peak_source": f"{peaks['source']} sustained cuBLAS bf16 x{int(scale)}; GEMM flops over the whole step",
                      "traffic": None, "kernel": "gemm_pair_kernel<fp8>" if cfg.mode == "fp8" else "gemm_nvf4_pair_kernel",
                      "algorithmic_flops_per_step_per_gpu": flops / world},
     }
+    details = {}
     if getattr(args, "call_times", 0) and world == 1 and phase != "decode":
-        line["call_times"] = call_times(capi, stack, h, mb, sharded)
+        details["call_times"] = call_times(capi, stack, h, mb, sharded)
     if parity is not None:
-        line["parity"] = parity
+        details["parity"] = parity
+        line["parity"] = {k: parity[k] for k in ("rel_l2", "tol", "ok") if k in parity}
     if breakdown is not None:
-        line["per_layer"] = breakdown
+        details["per_layer"] = breakdown
+        line["per_layer"] = {k: breakdown[k] for k in ("ms_per_layer", "gemm_only_ms_per_layer", "limiter")}
     if decode:
-        line["decode"] = decode
+        details["decode"] = decode
+        line["decode"] = {k: decode[k] for k in ("tokens_per_s", "ms_per_step", "batch", "cuda_graph", "frac_of_measured_hbm")}
     if rank == 0 and world == 1 and not args.no_extras:
         value, cores, sample, _ = cpu_extrapolated(cfg, seed, tokens, repeats=7)
-        line["cpu_baseline"] = {"value": value, "unit": "tokens/s", "cores": cores, "kind": "port", "sample": sample + " (extrapolated)"}
+        line["cpu_baseline"] = {"value": value, "unit": "tokens/s", "cores": cores, "kind": "port", "sample": "one layer at 1/8 of its rows, extrapolated"}
+        details["cpu_baseline"] = {**line["cpu_baseline"], "sample": sample + " (extrapolated)"}
         del stack
         torch.cuda.empty_cache()
         import bench_kernels as bk
 
-        line["extras"] = bk.extras(capi, peaks)
+        details["extras"] = bk.extras(capi, peaks)
+        line["extras"] = bk.summary(details["extras"])
     if rank == 0:
-        print(json.dumps(line))
+        bc.print_line(line, details)
     if world > 1:
         import torch.distributed as dist
 
