@@ -36,11 +36,35 @@ def workload_string(cfg, batch, seq):
                else "attention core = causal FP8 SDPA per sequence (Q, K, V quantized per tensor)"))
 
 
-def _config(args):
-    from tensorrt_b200.stack import LLAMA3_8B, LLAMA3_70B
+@dataclasses.dataclass(frozen=True)
+class Shape:
+    """A workload's sizes.  The reference arm takes them from here, so that it loads nothing of the package."""
+    hidden: int
+    n_q: int
+    n_kv: int
+    head_dim: int
+    ffn: int
+    layers: int
+    mode: str
+    attention: str = "identity"
+    seq_len: int = 0
 
+    @property
+    def q_width(self):
+        return self.n_q * self.head_dim
+
+    @property
+    def kv_width(self):
+        return self.n_kv * self.head_dim
+
+
+SHAPES = {"tp_stack": Shape(hidden=8192, n_q=64, n_kv=8, head_dim=128, ffn=28672, layers=80, mode="fp8"),
+          "nvfp4_stack": Shape(hidden=4096, n_q=32, n_kv=8, head_dim=128, ffn=14336, layers=32, mode="nvfp4")}
+
+
+def _config(args):
     tp = args.workload == "tp_stack"
-    cfg = LLAMA3_70B if tp else LLAMA3_8B
+    cfg = SHAPES[args.workload]
     if getattr(args, "layers", 0):
         cfg = dataclasses.replace(cfg, layers=args.layers)   # shortened stack: profiling runs only
     batch, seq = (32, 1024) if tp else (8, 2048)
@@ -301,11 +325,12 @@ def call_times(capi, stack, h, mb, sharded):
 
 def run(args):
     from tensorrt_b200 import capi
-    from tensorrt_b200.stack import DecoderStack, random_layer_weights
+    from tensorrt_b200.stack import DecoderStack, StackConfig, random_layer_weights
 
     rank, world, local = bc.dist_setup(args.gpus)
     dev = torch.device("cuda", local)
     tp, cfg, (batch, seq), seed = _config(args)
+    cfg = StackConfig(**dataclasses.asdict(cfg))
     phase = getattr(args, "phase", "all") if tp else "all"
     if not tp and world > 1:
         raise SystemExit("nvfp4_stack is a single-GPU workload; use tp_stack for --gpus > 1")

@@ -1,5 +1,7 @@
-"""The line that the benchmark prints: one JSON object on stdout, short, with every required key; details on stderr."""
+"""The line that the benchmark prints: one JSON object on stdout, short, with every required key; details on stderr.  The
+reference arm times the oracle and loads nothing of the package."""
 import json
+import subprocess
 import sys
 from pathlib import Path
 
@@ -22,3 +24,23 @@ def test_line_is_short_and_keeps_what_is_required(capsys):
     bc.print_line({"metric": "m", "extras": {"a": 1}})
     out, err = capsys.readouterr()
     assert json.loads(out) == {"metric": "m", "extras": {"a": 1}} and err == ""
+
+
+def test_reference_arm_loads_nothing_of_the_package():
+    code = ("import sys, bench_stack, oracle\n"
+            "class A: workload, layers, attention = 'tp_stack', 0, 'identity'\n"
+            "tp, cfg, (batch, seq), seed = bench_stack._config(A)\n"
+            "assert bench_stack.workload_string(cfg, batch, seq) and cfg.q_width == 8192 and cfg.kv_width == 1024\n"
+            "assert not [m for m in sys.modules if m.startswith('tensorrt_b200')]\n")
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
+
+
+def test_shapes_are_those_of_the_package():
+    import dataclasses
+
+    sys.path.insert(0, str(ROOT))
+    import bench_stack
+    from tensorrt_b200.stack import LLAMA3_8B, LLAMA3_70B, StackConfig
+
+    assert StackConfig(**dataclasses.asdict(bench_stack.SHAPES["tp_stack"])) == LLAMA3_70B
+    assert StackConfig(**dataclasses.asdict(bench_stack.SHAPES["nvfp4_stack"])) == LLAMA3_8B
