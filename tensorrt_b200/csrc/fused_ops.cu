@@ -113,7 +113,8 @@ rms_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 //   scale = max|x| / 448 (0 -> 1);  code = e4m3(x / scale)
 // Same arithmetic and rounding points as add -> rms_norm -> fp8 quantize run one after the
 // other, with 1.75 bytes of traffic per element and step instead of 3.25.
-// PARTS > 1: a cluster of PARTS CTAs shares one token (few tokens: a decode step); the slices'
+// PARTS > 1: a cluster of PARTS CTAs shares one token (few tokens that add_norm_quant_row_kernel does not take: bases that are
+// not 32-byte aligned, columns that are no multiple of 16, and up to 16 rows of more than 8192 columns); the slices'
 // sums of squares and maxima meet through distributed shared memory, summed in rank order.
 // NVF4: the normalised row leaves as NVFP4 codes and block scales under a calibrated tensor amax (`nv`) instead of
 // per-token FP8; no row maximum is needed.

@@ -39,8 +39,8 @@
 // the same columns, so accumulator columns 0-127 / 128-255 of a tile are gate / up pairs; an epilogue thread takes 64 of each,
 // rounds both to bf16 as the plain form stores them, and leaves silu(gate) * up as NVFP4 codes (32 bytes) and one scale word
 // under the calibrated range of the activation: the same bits as GEMM, silu_mul and NVFP4 quantize.  The bf16 [M, 2F]
-// tensor (470 MB at 8192 tokens and F = 14336, written once and read once: 120 us of a 1150 us layer) is not written; the
-// arithmetic runs under the next tile's MMAs, because tensor memory is handed back first.
+// tensor (470 MB at 8192 tokens and F = 14336) is neither written nor read again, and the kernel that read it, 120 us of a 1150 us
+// layer, is gone; the arithmetic runs under the next tile's MMAs, because tensor memory is handed back first.
 #pragma once
 
 #include "gemm_kernel_2cta.cuh"
