@@ -123,9 +123,12 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // CTAs walk the heads in groups (head_group), in a group the query tiles with the most keys first: a causal launch then
   // ends on its shortest CTAs
-  const int head0 = static_cast<int>(blockIdx.x) / (p.group * p.q_tiles) * p.group;
-  const int heads = min(p.group, p.BH - head0);
-  const int place = static_cast<int>(blockIdx.x) - head0 * p.q_tiles;
+  int head0 = 0, heads = p.BH, place = static_cast<int>(blockIdx.x);
+  if (p.group < p.BH) {
+    head0 = place / (p.group * p.q_tiles) * p.group;
+    heads = min(p.group, p.BH - head0);
+    place -= head0 * p.q_tiles;
+  }
   const int q_tile = place / heads;
   const int q0 = (p.q_tiles - 1 - q_tile) * kTile;
   const int bh = head0 + place - q_tile * heads;              // b * Hq + h
