@@ -105,12 +105,12 @@ namespace b200q {
 // and 16 tiles of weight rows.  Clusters as large as they may be, which keeps the slices short, but no more than are resident at
 // once: 34 tiles on clusters of eight and 72 on clusters of four would take two rounds, which the plain GEMM avoids (8 x 4608 x
 // 1024 12.0 us against 6.5; such sizes then take smaller clusters or two launches).  Measured against the quantize launch and the
-// GEMM behind it at 844 points inside (1 to 8 tokens, N 1920 to 28672, K 256 to 8192, bf16 and fp32, weights rotating through more
-// than L2 where they are that large): 0.82 of the time of an eager call, which a launch less decides (at worst 1.09, fp32
-// 1.21).  In a replayed graph 0.91 where the range is given (at worst 1.04); where it is measured 1.02 for bf16 and 1.07 for
-// fp32 (at worst 1.16 and 1.35), whose elements every CTA reads twice.  Outside, with the same kernel: 4 x 10240 x 4096 16.0 us
-// against 12.6, 1 x 10240 x 8192 27.2 against 18.4, 16 x 4096 x 4096 14.7 against 9.0 (the quantizer's work in every CTA), 1 x
-// 1024 x 1024 5.3 against 5.2 (too few CTAs to gain).
+// GEMM behind it at 776 points inside (1 to 8 tokens, N 1920 to 28672, K 256 to 8192, bf16 and fp32, weights rotating through more
+// than L2 where they are that large): 0.78 of the time of an eager call, which a launch less decides (at worst 1.05, fp32
+// 1.18).  In a replayed graph 0.91 where the range is given (at worst 1.04); where it is measured 1.03 for bf16 and 1.08 for
+// fp32 (at worst 1.18 and 1.38), whose elements every CTA reads twice.  Outside, with the same kernel: 4 x 10240 x 4096 16.0 us
+// against 12.6, 1 x 10240 x 8192 27.2 against 18.5, 16 x 4096 x 4096 14.7 against 9.1 (the quantizer's work in every CTA), 1 x
+// 1024 x 1024 5.3 against 5.1 (too few CTAs to gain).
 int fp8_linear_small(const void* x, int dtype, const float* amax, int64_t amax_numel, const uint8_t* w, const float* w_scales,
                      int64_t w_scales_numel, const void* bias, void* out, int64_t M, int64_t N, int64_t K, b200q_stream_t stream) {
   const int64_t width = dtype == B200Q_F32 ? 4 : 2;

@@ -333,7 +333,7 @@ inline int64_t smallm_cost(int n_tiles, int k_tiles, const ActiveClusters& c, in
 
 // Fewer CTAs per tile than that where they are cheaper by more than 3 %: short K slices and many tokens (the reduction), and
 // cluster counts just above what is resident.  Measured at 37 weight shapes (1024 x 1024 to 57344 x 8192), 10 token counts and
-// both formats: 1.011 of the best cluster size's time on average (1.171 without this step, 2.3 times at worst: FP8 2048 x 2048
+// both formats: 1.011 of the best cluster size's time on average (1.170 without this step, 2.3 times at worst: FP8 2048 x 2048
 // at 16 / 64 / 128 tokens 9.1 / 13.5 / 17.9 us on 8 CTAs, 5.0 / 6.7 / 8.7 on 4; 6144 x 4096 at 128 tokens 16.3 on 4, 12.3 on
 // 2), and nowhere more than 2 % slower than without.  At worst 1.23 of the best: FP8 5120 x 5120 at 96 tokens 14.8 us on 4
 // CTAs, 12.1 on 2; 4096 x 1024 in both formats 1.08 to 1.21, where 2 CTAs would win at every token count.
