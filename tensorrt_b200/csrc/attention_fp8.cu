@@ -20,8 +20,11 @@
 // rescaling scheme whose quantization points would differ from the definition above.
 //
 // What bounds it: the exponentials, two per score at 16 per clock and SM: 1024 clocks per 128 x 128 tile and pass, and
-// two warps per scheduler and CTA reach 0.93 of that rate in a loop of their own.  What it loses beside them is warps
-// that wait for scores.  So a softmax thread takes its 64 scores of a tile into registers and hands the tensor-memory
+// two warps per scheduler and CTA reach 0.93 of that rate in a loop of their own.  An eighth of them runs on the FMA pipe instead
+// (ex2_poly2, more exact than the unit).  What it loses beside them is warps that wait for scores: without any arithmetic in the
+// softmax warps the kernel still takes 0.58 of its time, the chain of loads, MMAs and barriers of a tile.  Shared-memory addresses
+// that are compile-time constants shorten that chain (203 -> 190 us at [4, 32 / 8, 2048, 128] causal); a second V stage or a third K
+// stage lengthens it (193), scores in buffers of 64 keys too (223).  So a softmax thread takes its 64 scores of a tile into registers and hands the tensor-memory
 // buffer back before it computes (the tensor core fills it under the exponentials); in pass 2 the scores of tile j + 2
 // are issued in front of the product of tile j (wait for scores per tile 819 -> 171 clocks of about 2500); edge tiles
 // have their own copy of the loop; query tiles with the most keys start first (head_group).  Order and roundings per row are those
@@ -61,7 +64,11 @@ constexpr int kTileBytes = kTile * 128;    // one operand tile: 128 rows x 128 b
 constexpr int kKStages = 2, kVStages = 1;
 constexpr int kChunk = 32;                 // score columns of one step of a softmax thread
 constexpr int kTmemCols = 256;
-constexpr int kAttSmem = 1024 + kTileBytes * (1 + kKStages + kVStages + 2) + 4096;   // tail: barriers, row statistics
+constexpr int kAttSmem = kTileBytes * (1 + kKStages + kVStages + 2) + 512;   // tail: barriers
+// Of the 16 pairs of a chunk, those whose exponentials run on the FMA pipe (ex2_poly2), us of this kernel with 0 / 2 / 3 / 4 of them:
+// [4, 32 / 8, 2048, 128] causal 190 / 180 / 181 / 185; [3, 16, 577 x 1500, 64] 41.8 / 40.0 / 39.5 / 40.5; [8, 32 / 8, 1024, 128] causal
+// 119 / 115 / 117 / 118; [1, 74, 4096, 128] 740 / 703 / 700 / 732.  Beyond four the issue slots bind.
+constexpr int kPolyPairs = 2;
 
 struct AttParams {
   const float* q_scale;     // per-tensor scales (device scalars)
@@ -87,6 +94,43 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// maximum that keeps a NaN
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// 2^x of a pair on the FMA pipe, x < 128: x = n + f with n the nearest integer (Cody and Waite's reduction; the rounding constant
+// 1.5 * 2^23 is raised by 127, so that the low bits of the sum are the biased exponent of 2^n), 2^f by the polynomial of degree 6
+// with constant term 1 of the smallest largest relative error on [-1/2, 1/2] (2.0e-9, from a weighted least-squares exchange).  With
+// the fp32 roundings of Horner's scheme: largest relative error 7.9e-8, root mean square 2.7e-8, mean 9e-10; ex2.approx over the same
+// range [-20, 9]: 1.4e-7, 5.5e-8, -2.4e-8.  Below -126.5 the result is 0; NaN stays NaN.
+__device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
+  constexpr float kRound = 12582912.0f + 127.0f;
+  const auto both = [](float c) { return pack2(c, c); };
+  const float2 a = unpack2(x);
+  x = pack2(max_nan(a.x, -127.0f), max_nan(a.y, -127.0f));
+  const uint64_t t = add2(x, both(kRound));
+  const uint64_t f = add2(x, fma2(t, both(-1.0f), both(kRound)));
+  uint64_t y = fma2(f, both(0x1.41fbbcp-13f), both(0x1.5f3e54p-10f));
+  y = fma2(y, f, both(0x1.3b2d4cp-7f));
+  y = fma2(y, f, both(0x1.c6aee8p-5f));
+  y = fma2(y, f, both(0x1.ebfbdcp-3f));
+  y = fma2(y, f, both(0x1.62e430p-1f));
+  y = fma2(y, f, both(1.0f));
+  const float2 n = unpack2(t);
+  return mul2(y, pack2(__uint_as_float(__float_as_uint(n.x) << 23), __uint_as_float(__float_as_uint(n.y) << 23)));
+}
+
+// 2^x of pair k of a chunk
+__device__ __forceinline__ uint64_t ex2_pair(uint64_t x, int k) {
+  constexpr int kPairs = kChunk / 2;
+  if ((k + 1) * kPolyPairs / kPairs != k * kPolyPairs / kPairs) return ex2_poly2(x);
+  const float2 a = unpack2(x);
+  return pack2(ex2_approx(a.x), ex2_approx(a.y));
+}
+
 // four fp32 -> four E4M3 bytes in one register
 __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, float d) {
   uint32_t r;
@@ -100,8 +144,8 @@ __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, f
 __global__ void __launch_bounds__(kAttThreads, 2)
 fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_vt, const AttParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  // the 128-byte swizzle counts from 1024-byte boundaries; addresses that are constants keep the single-thread roles short
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sq = smem;
   uint8_t* sk = sq + kTileBytes;
   uint8_t* sv = sk + kKStages * kTileBytes;
@@ -118,8 +162,11 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint64_t* p_empty = p_full + 2;
   uint64_t* o_full = p_empty + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 1);
-  float2* row_stat = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + 1024);   // [2][kTile] (max, sum) of each column half
 
+  if ((ptx::smem_u32(smem) & 1023u) != 0) {                   // cannot be: no static shared memory stands in front
+    if (threadIdx.x == 0) att_timeout(p.status, 60);
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // CTAs walk the heads in groups (head_group), in a group the query tiles with the most keys first: a causal launch then
   // ends on its shortest CTAs
@@ -239,9 +286,11 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         ptx::tc_fence_after();
         const uint32_t k_lo = k_lo0 + ks * (kTileBytes >> 4);
-        for (int kb = 0; kb < kb_scores; ++kb)
-          ptx::mma_f8<1>(tmem_base + sb * kTile, ptx::desc_join(q_lo + kb * 2, ptx::kDescHiSw128),
-                         ptx::desc_join(k_lo + kb * 2, ptx::kDescHiSw128), idesc_s, kb > 0 ? 1u : 0u);
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb)
+          if (kb < kb_scores)
+            ptx::mma_f8<1>(tmem_base + sb * kTile, ptx::desc_join(q_lo + kb * 2, ptx::kDescHiSw128),
+                           ptx::desc_join(k_lo + kb * 2, ptx::kDescHiSw128), idesc_s, kb > 0 ? 1u : 0u);
         ptx::tc_commit<1>(s_full + sb);
         ptx::tc_commit<1>(k_empty + ks);
         if (sb == 0) sph0 ^= 1u;
@@ -352,10 +401,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         uint64_t l01 = 0ull, l23 = 0ull;          // pairs of zeros
 #pragma unroll
         for (int i = 0; i < kChunk; i += 4) {
-          const float2 a = unpack2(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2c2, offoff));
-          const float2 b = unpack2(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c2c2, offoff));
-          l01 = add2(l01, pack2(ex2_approx(a.x), ex2_approx(a.y)));
-          l23 = add2(l23, pack2(ex2_approx(b.x), ex2_approx(b.y)));
+          l01 = add2(l01, ex2_pair(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2c2, offoff), i / 2));
+          l23 = add2(l23, ex2_pair(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c2c2, offoff), i / 2 + 1));
         }
         const float2 s0 = unpack2(l01), s1 = unpack2(l23);
         l += (s0.x + s0.y) + (s1.x + s1.y);
@@ -365,11 +412,13 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int first_edge = min(full_tiles, n_tiles);
     for (int j = 0; j < first_edge && ok; ++j) ok = pass1(std::false_type{}, j);
     for (int j = first_edge; j < n_tiles && ok; ++j) ok = pass1(std::true_type{}, j);
-    // the two threads of a row each hold the statistics of their columns: merge (every softmax thread gets here)
-    row_stat[ch * kTile + r] = make_float2(m, l);
+    // The two threads of a row each hold the statistics of their columns: merge (every softmax thread gets here).  They pass them
+    // on through the first probability tile, each in a piece of this row that the other one alone writes later, behind its read.
+    uint8_t* srow = sp + r * 128;
+    *reinterpret_cast<float2*>(srow + (((2 * (ch ^ 1)) ^ (r & 7)) * 16)) = make_float2(m, l);
     asm volatile("bar.sync 1, 256;" ::: "memory");
     {
-      const float2 o = row_stat[(ch ^ 1) * kTile + r];
+      const float2 o = *reinterpret_cast<const float2*>(srow + (((2 * ch) ^ (r & 7)) * 16));
       const float mm = fmaxf(m, o.x);
       const float mine = m > -INFINITY ? l * ex2_approx((m - mm) * c2) : 0.0f;
       const float theirs = o.x > -INFINITY ? o.y * ex2_approx((o.x - mm) * c2) : 0.0f;
@@ -393,9 +442,10 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint32_t* e = v + g * 16 + i * 4;
-          const float2 a = unpack2(fma2(pack2(__uint_as_float(e[0]), __uint_as_float(e[1])), c2c2, off22));
-          const float2 b = unpack2(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22));
-          w[i] = f32x4_to_e4m3x4(ex2_approx(a.x), ex2_approx(a.y), ex2_approx(b.x), ex2_approx(b.y));
+          const int k = (g & 1) * 8 + i * 2;
+          const float2 a = unpack2(ex2_pair(fma2(pack2(__uint_as_float(e[0]), __uint_as_float(e[1])), c2c2, off22), k));
+          const float2 b = unpack2(ex2_pair(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22), k + 1));
+          w[i] = f32x4_to_e4m3x4(a.x, a.y, b.x, b.y);
         }
         // 128-byte swizzle of the operand layout: the 16-byte piece i of row r lives at piece i ^ (r & 7)
         const int piece = 2 * ch + (g & 1) + 4 * (g >> 1);
