@@ -392,6 +392,15 @@ int b200q_fp8_attention_quantize(const void* q, const void* k, const void* v, in
                                  const float* amax_q, const float* amax_k, const float* amax_v, uint8_t* q_codes,
                                  uint8_t* k_codes, uint8_t* vt_codes, float* scales, int64_t B, int64_t Hq, int64_t Hkv,
                                  int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D, b200q_stream_t stream);
+/* The whole of it, q, k, v as for b200q_fp8_attention_quantize and the result of their dtype at out_strides (as for
+ * b200q_fp8_sdpa_strided): one launch for the operands of K and V, which go to `workspace` (16-byte aligned,
+ * b200q_fp8_attention_workspace_bytes), one for the attention, which quantizes its queries itself.  Same bits as those two
+ * calls. */
+size_t b200q_fp8_attention_workspace_bytes(int64_t B, int64_t Hkv, int64_t Sk, int64_t D);
+int b200q_fp8_attention(const void* q, const void* k, const void* v, int dtype, const int64_t* strides, const float* amax_q,
+                        const float* amax_k, const float* amax_v, void* out, const int64_t* out_strides, void* workspace,
+                        size_t workspace_bytes, int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t D,
+                        float softmax_scale, int causal, b200q_stream_t stream);
 /* abs-max of three column ranges of x [rows, c1 + c2 + c3] (dtype, row-major): amax_out[0..2], fp32, exact.  The Q, K
  * and V slices of a QKV projection in one pass.  c1, c2, c3 >= 0, multiples of 16; x 32-byte aligned. */
 int b200q_amax_columns(const void* x, int dtype, int64_t rows, int64_t c1, int64_t c2, int64_t c3, float* amax_out,

@@ -54,6 +54,8 @@ SIGNATURES = {
     "b200q_fp8_quantize_transpose": (_c.c_int, [_p, _c.c_int, _i64, _i64, _i64, _p, _p, _i64, _p, _p]),
     "b200q_fp8_sdpa": (_c.c_int, [_p, _p, _p, _p, _p, _p, _p, _c.c_int, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _c.c_float, _c.c_int, _p]),
     "b200q_fp8_sdpa_strided": (_c.c_int, [_p, _p, _p, _p, _p, _p, _p, _p, _c.c_int, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _c.c_float, _c.c_int, _p]),
+    "b200q_fp8_attention_workspace_bytes": (_c.c_size_t, [_i64, _i64, _i64, _i64]),
+    "b200q_fp8_attention": (_c.c_int, [_p, _p, _p, _c.c_int, _p, _p, _p, _p, _p, _p, _p, _c.c_size_t, _i64, _i64, _i64, _i64, _i64, _i64, _c.c_float, _c.c_int, _p]),
     "b200q_fp8_attention_quantize": (_c.c_int, [_p, _p, _p, _c.c_int, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _p]),
     "b200q_amax_columns": (_c.c_int, [_p, _c.c_int, _i64, _i64, _i64, _i64, _p, _p]),
     "b200q_rms_norm": (_c.c_int, [_p, _p, _p, _i64, _i64, _c.c_float, _p]),

@@ -404,7 +404,8 @@ def _outer_strides(t: torch.Tensor):
 
 def _fp8_sdpa_into(out: torch.Tensor, q, k, v, amax_q, amax_k, amax_v, is_causal: bool, scale) -> torch.Tensor:
     """`fp8_sdpa` of checked inputs of one dtype into `out` (q's shape and dtype; any strides with D contiguous and
-    the others multiples of 8 elements, 32-byte aligned): one launch that quantizes Q, K and V, one of attention."""
+    the others multiples of 8 elements, 32-byte aligned): one launch that quantizes K and V, one of attention, which
+    quantizes Q."""
     import math
 
     q, k, v = _strided_16(q), _strided_16(k), _strided_16(v)
@@ -412,23 +413,16 @@ def _fp8_sdpa_into(out: torch.Tensor, q, k, v, amax_q, amax_k, amax_v, is_causal
     _, Hkv, Sk, _ = k.shape
     dev, dt = q.device, _dt(q)
     aq, ak, av = (a.to(device=dev, dtype=torch.float32).reshape(1) for a in (amax_q, amax_k, amax_v))
-    vt_stride = max((Sk + 15) // 16 * 16, 16)
-    nq, nk, nv = q.numel(), k.numel(), B * Hkv * D * vt_stride
-    # one workspace: Q codes, K codes, transposed V codes (each a multiple of 16 bytes), three scales
-    ws = torch.empty(nq + nk + nv + 16, dtype=torch.uint8, device=dev)
-    base = ws.data_ptr()
-    scales = base + nq + nk + nv
+    lib = load()
+    # K codes, transposed V codes, scales
+    ws = torch.empty(lib.b200q_fp8_attention_workspace_bytes(B, Hkv, Sk, D), dtype=torch.uint8, device=dev)
     strides = (ctypes.c_int64 * 9)(*_outer_strides(q), *_outer_strides(k), *_outer_strides(v))
     out_strides = (ctypes.c_int64 * 3)(*_outer_strides(out))
-    lib = load()
     with torch.cuda.device(dev):
-        st = _stream(q)
-        check(lib.b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr(), ak.data_ptr(), av.data_ptr(),
-                                               base, base + nq, base + nq + nk, scales, B, Hq, Hkv, Sq, Sk, vt_stride, D, st),
-              "b200q_fp8_attention_quantize")
-        check(lib.b200q_fp8_sdpa_strided(base, base + nq, base + nq + nk, scales, scales + 4, scales + 8, out.data_ptr(), out_strides, dt, B, Hq,
-                                         Hkv, Sq, Sk, vt_stride, D, float(scale if scale is not None else 1.0 / math.sqrt(D)),
-                                         1 if is_causal else 0, st), "b200q_fp8_sdpa")
+        check(lib.b200q_fp8_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr(), ak.data_ptr(), av.data_ptr(),
+                                      out.data_ptr(), out_strides, ws.data_ptr(), ws.numel(), B, Hq, Hkv, Sq, Sk, D,
+                                      float(scale if scale is not None else 1.0 / math.sqrt(D)), 1 if is_causal else 0, _stream(q)),
+              "b200q_fp8_sdpa")
     return out
 
 

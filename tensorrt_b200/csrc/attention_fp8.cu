@@ -74,6 +74,9 @@ struct AttParams {
   const float* q_scale;     // per-tensor scales (device scalars)
   const float* k_scale;
   const float* v_scale;
+  const void* q;            // queries that the kernel quantizes itself: [B, Hq, Sq, D] at these strides (elements), under q_amax
+  const float* q_amax;
+  int64_t q_sb, q_sh, q_ss;
   void* out;                // [B, Hq, Sq, D] at these strides (elements, multiples of 8; D contiguous)
   int64_t out_sb, out_sh, out_ss;
   int out_dtype;
@@ -141,6 +144,12 @@ __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, f
   return r;
 }
 
+// QT: type of the queries, uint8_t = E4M3 codes (tmap_q); WIDE: their rows start on 32-byte boundaries.
+// Queries that are not codes yet are quantized here, by the softmax warps while K is on its way and the kernel in front still writes the
+// operands of K and V: each is read by one CTA only, so a pass of its own would write and read their codes for nothing.  Both launches,
+// us, operand pass for all three / this: [4, 32 / 8, 2048, 128] causal 212 / 202; [3, 16, 577 x 1500, 64] 51 / 47.7; [8, 32 / 8, 1024,
+// 128] causal 147 / 137; [8, 12, 200, 128] causal 21.2 / 18.9; [1, 8, 64, 64] 13.1 / 11.2.
+template <typename QT, bool WIDE>
 __global__ void __launch_bounds__(kAttThreads, 2)
 fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_vt, const AttParams p) {
@@ -167,6 +176,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (threadIdx.x == 0) att_timeout(p.status, 60);
     return;
   }
+  constexpr bool kCodes = std::is_same<QT, uint8_t>::value;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // CTAs walk the heads in groups (head_group), in a group the query tiles with the most keys first: a causal launch then
   // ends on its shortest CTAs
@@ -199,9 +209,14 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     ptx::mbar_init(o_full, 1);
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&tmap_vt);
-    // this thread is the producer: the first tiles are requested in front of the tensor-memory allocation
-    ptx::mbar_arrive_expect_tx(q_full, kTileBytes);
-    ptx::tma_load_3d(sq, &tmap_q, q_full, 0, q0, bh);
+    // this thread is the producer: the first tiles are requested in front of the tensor-memory allocation, once the kernel that
+    // writes the operands is complete (it may still run under a programmatic launch)
+    pdl_wait();
+    ptx::fence_proxy_async_all();
+    if constexpr (kCodes) {
+      ptx::mbar_arrive_expect_tx(q_full, kTileBytes);
+      ptx::tma_load_3d(sq, &tmap_q, q_full, 0, q0, bh);
+    }
     if (n_tiles > 0) {
       ptx::mbar_arrive_expect_tx(k_full, kTileBytes);
       ptx::tma_load_3d(sk, &tmap_k, k_full, 0, 0, bhkv);
@@ -210,6 +225,30 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == 1) {
     ptx::tmem_alloc<1>(tmem_holder, kTmemCols);
     ptx::tmem_relinquish<1>();
+  }
+  float q_scale = 0.0f;
+  if constexpr (!kCodes) {
+    if (warp >= 2) {
+      // 128 rows in pieces of 16 elements, 8 to a row, 4 to a thread.  Queries and their range are older than the kernel in front
+      // of this one, so nothing waits for that.
+      const int g = threadIdx.x & 7, row0 = (static_cast<int>(threadIdx.x) - 64) >> 3;
+      const QT* src = static_cast<const QT*>(p.q) + b * p.q_sb + h * p.q_sh + static_cast<int64_t>(q0 + row0) * p.q_ss + g * 16;
+      Raw16<QT, WIDE> raw[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (g * 16 < p.D && q0 + row0 + u * 32 < p.Sq) raw[u].load(src + static_cast<int64_t>(u * 32) * p.q_ss);
+      q_scale = fp8_scale_from_amax(ld_dependent(p.q_amax));
+      const float y = b200q_rcp_rn(q_scale), lim = __fmul_rn(q_scale, 512.0f);
+      const bool fast = b200q_div_fast_ok(q_scale) != 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int row = row0 + u * 32;
+        uint4 c = make_uint4(0u, 0u, 0u, 0u);     // rows past the end, and columns D..: the contraction takes 32 at a time
+        if (g * 16 < p.D && q0 + row < p.Sq) c = e4m3_of_16(raw[u], q_scale, y, lim, fast);
+        *reinterpret_cast<uint4*>(sq + row * 128 + ((g ^ (row & 7)) * 16)) = c;
+      }
+      ptx::fence_proxy_async();                   // the tensor core reads this tile through the async proxy
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -220,7 +259,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int ks = n_tiles > 0 ? 1 : 0, vs = 0;       // Q and the first K tile are on their way (above)
+      int ks = n_tiles > 0 ? 1 : 0, vs = 0;       // the first K tile is on its way (above)
       uint32_t kph = 0, vph = 0;
       bool ok = true;
       // the order of the loads is the order in which the MMA thread uses them: pass 1 all K tiles; pass 2 K 0, K 1,
@@ -275,7 +314,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       int ks = 0, vs = 0, pb = 0;
       uint32_t kph = 0, vph = 0, pph = 0;
       uint32_t sph0 = 0, sph1 = 0;                              // score buffers: parity of their next use
-      bool ok = ptx::mbar_wait(q_full, 0);
+      bool ok = true;
+      if constexpr (kCodes) ok = ptx::mbar_wait(q_full, 0);     // else written in front of the barrier above
       if (!ok) att_timeout(p.status, 65);
       // scores of the next key tile in ring order into score buffer `sb`
       auto issue_scores = [&](int sb) -> bool {
@@ -338,7 +378,9 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     // scores in the base-2 exponent domain: s2 = acc * c2, c2 = q_scale * k_scale * softmax_scale * log2(e) > 0,
     // so the running maximum is kept on the raw accumulators and the scaling rides in the FMA in front of ex2
-    const float c2 = __ldg(p.q_scale) * __ldg(p.k_scale) * p.softmax_scale * 1.4426950408889634f;
+    pdl_wait();                                   // the other scales come from the kernel in front; results are stored behind it
+    if constexpr (kCodes) q_scale = ld_dependent(p.q_scale);
+    const float c2 = q_scale * ld_dependent(p.k_scale) * p.softmax_scale * 1.4426950408889634f;
     const uint64_t c2c2 = pack2(c2, c2);
     const int last_key = p.causal ? min(k_end - 1, qi + shift) : k_end - 1;   // keys beyond it are masked for this row
     // key tiles below this index are visible to every row of the CTA in full: no per-element mask there
@@ -468,7 +510,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // end of the sequence only skip their stores
     if (ok && q0 + q * 32 < p.Sq) {
       ptx::tc_fence_after();
-      const float oscale = n_tiles > 0 ? __ldg(p.v_scale) / kE4M3Max : 0.0f;
+      const float oscale = n_tiles > 0 ? ld_dependent(p.v_scale) / kE4M3Max : 0.0f;
       const int64_t row_off = b * p.out_sb + h * p.out_sh + qi * p.out_ss;
 #pragma unroll 1
       for (int c = 2 * ch; c < 2 * ch + 2; ++c) {
@@ -510,7 +552,9 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 // of a QKV projection is read where it lies.  HBM-bound (3 bytes per 16-bit element); a CTA takes 128 rows of one
 // head, 16 elements per thread and step with four steps of loads in flight.  Before, Q and K went through the
 // row kernels, one CTA per row of D elements (at [4, 32, 2048, 128] 262144 CTAs of which 16 threads had work), and V through a
-// byte-wise transpose: 355 us for the three operands of [4, 32 / 8, 2048, 128] bf16, 42 us here (3.6 TB/s).
+// byte-wise transpose: 355 us for the three operands of [4, 32 / 8, 2048, 128] bf16.  With a division per element and its choice of
+// path inside the loop, 60 % of the issue slots were taken at 36 % of the memory's rate: 42 us; two quotients at a time where a piece
+// lies within the range (e4m3_of_16): 31.6 us (4.8 TB/s), 12.7 for K and V alone (b200q_fp8_attention).
 struct QkvPart {
   const void* x;
   int64_t sb, sh, ss;        // strides of batch, head, row in elements
@@ -524,6 +568,7 @@ struct QkvParts {
   QkvPart part[3];
   int first[3];              // first CTA of each part
   int D;
+  int inv_pieces;            // 65536 / (D / 16), rounded up: t / pieces = t * inv_pieces >> 16 for t < 2048
   int64_t vt_stride;
 };
 
@@ -534,6 +579,7 @@ fp8_attention_quantize_kernel(const __grid_constant__ QkvParts p) {
   const int cta = static_cast<int>(blockIdx.x);
   const int which = cta >= p.first[2] ? 2 : (cta >= p.first[1] ? 1 : 0);
   const QkvPart& part = p.part[which];
+  pdl_launch_dependents();   // the attention kernel behind it may quantize its first queries meanwhile
   if (cta == 0 && threadIdx.x < 3 && p.part[threadIdx.x].scale_out != nullptr)
     *p.part[threadIdx.x].scale_out = fp8_scale_from_amax(__ldg(p.part[threadIdx.x].amax));
   const int local = cta - p.first[which];
@@ -543,7 +589,7 @@ fp8_attention_quantize_kernel(const __grid_constant__ QkvParts p) {
   const T* x = static_cast<const T*>(part.x) + b * part.sb + h * part.sh;
   const float scale = fp8_scale_from_amax(__ldg(part.amax));
   const float y = b200q_rcp_rn(scale);
-  const bool fast = b200q_div_fast_ok(scale);
+  const bool fast = b200q_div_fast_ok(scale) != 0;
   const float lim = __fmul_rn(scale, 512.0f);     // |x| >= 512 * scale saturates to 448 anyway
   const int pieces = p.D >> 4;                    // 16-element pieces of a row
   constexpr int U = sizeof(T) == 4 ? 2 : 4;
@@ -552,25 +598,15 @@ fp8_attention_quantize_kernel(const __grid_constant__ QkvParts p) {
     Raw16<T, WIDE> raw[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int t = t0 + u * 256, row = t / pieces, g = t - row * pieces;
+      const int t = t0 + u * 256, row = t * p.inv_pieces >> 16, g = t - row * pieces;
       if (row < rows) raw[u].load(x + static_cast<int64_t>(r0 + row) * part.ss + g * 16);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int t = t0 + u * 256, row = t / pieces, g = t - row * pieces;
+      const int t = t0 + u * 256, row = t * p.inv_pieces >> 16, g = t - row * pieces;
       uint4 c = make_uint4(0u, 0u, 0u, 0u);
       if (row < rows) {
-        float v[16];
-        raw[u].widen(v);
-        uint32_t* w = &c.x;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float q[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            q[e] = fast ? div_path<kDivClamped>(v[4 * i + e], scale, y, lim) : div_path<kDivTrue>(v[4 * i + e], scale, y, lim);
-          w[i] = f32x2_to_e4m3x2(q[0], q[1]) | (f32x2_to_e4m3x2(q[2], q[3]) << 16);
-        }
+        c = e4m3_of_16(raw[u], scale, y, lim, fast);
         if (which != 2)
           *reinterpret_cast<uint4*>(part.out + (static_cast<int64_t>(head) * part.S + r0 + row) * p.D + g * 16) = c;
       }
@@ -606,6 +642,7 @@ fp8_attention_quantize_kernel(const __grid_constant__ QkvParts p) {
 // `first` and the grid of the parts filled in; 0 CTAs = nothing to do.
 int launch_attention_quantize(QkvParts& p, int B, int dtype, cudaStream_t st) {
   int64_t ctas = 0;
+  p.inv_pieces = 65536 / (p.D / 16) + 1;
   for (int i = 0; i < 3; ++i) {
     p.first[i] = static_cast<int>(ctas);
     // V: the zero columns between S and the row stride are written too
@@ -664,6 +701,92 @@ int head_group(const AttParams& p) {
   const int64_t kv_heads = kv_bytes > 0 ? (int64_t{32} << 20) / kv_bytes : p.BH;
   const int64_t heads = (kv_heads > 1 ? kv_heads : 1) * rep;
   return heads < p.BH ? static_cast<int>(heads) : p.BH;
+}
+
+// Sizes and pointers that both entry points of the attention kernel ask for.
+int check_attention(const void* q, const void* k, const void* v, const void* out, const int64_t* out_strides, int dtype, int64_t B,
+                           int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t D, float softmax_scale) {
+  if (B < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || Sq < 0 || Sk < 0 || D <= 0 || D > 128 || D % 16 != 0) return B200Q_ERR_INVALID;
+  if (B * Hq > 65535 || Sq > 0x7fffffffLL || Sk > 0x7fffffffLL) return B200Q_ERR_INVALID;
+  if (dtype != B200Q_BF16 && dtype != B200Q_F16 && dtype != B200Q_F32) return B200Q_ERR_INVALID;
+  if (!(softmax_scale > 0.0f)) return B200Q_ERR_INVALID;
+  if (B == 0 || Sq == 0) return B200Q_OK;
+  if (q == nullptr || out == nullptr) return B200Q_ERR_INVALID;
+  if (Sk > 0 && (k == nullptr || v == nullptr)) return B200Q_ERR_INVALID;
+  if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(out, 32)) return B200Q_ERR_ALIGN;
+  if (out_strides == nullptr) return B200Q_ERR_INVALID;
+  for (int i = 0; i < 3; ++i)
+    if (out_strides[i] < 0 || out_strides[i] % 8 != 0) return B200Q_ERR_ALIGN;   // 8-element stores
+  return B200Q_OK;
+}
+
+template <typename QT, bool WIDE>
+int launch_sdpa_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
+                          cudaStream_t st) {
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(fp8_sdpa_kernel<QT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return B200Q_ERR_CUDA;
+    configured[dev] = true;
+  }
+  if (behind) {
+    if (launch_pdl(fp8_sdpa_kernel<QT, WIDE>, dim3(ctas), dim3(kAttThreads), kAttSmem, st, tq, tk, tv, p) != cudaSuccess) return B200Q_ERR_CUDA;
+  } else {
+    fp8_sdpa_kernel<QT, WIDE><<<ctas, kAttThreads, kAttSmem, st>>>(tq, tk, tv, p);
+  }
+  return check_launch();
+}
+
+// p: scales, queries (q_amax == nullptr: codes, at `q_codes`) and the result filled in.  `behind`: the kernel that writes the K and
+// V operands was launched directly in front.
+int launch_sdpa(AttParams& p, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* vt_codes, const int64_t* out_strides,
+                       int q_dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D,
+                       float softmax_scale, int causal, bool behind, b200q_stream_t stream) {
+  p.out_sb = out_strides[0];
+  p.out_sh = out_strides[1];
+  p.out_ss = out_strides[2];
+  p.status = gemm::device_status_word();
+  if (p.status == nullptr) return B200Q_ERR_CUDA;
+  const bool codes = p.q_amax == nullptr;
+  CUtensorMap tq, tk, tv;
+  // a zero-length key axis still needs valid maps: the kernel then loads nothing and writes zeros
+  const int64_t sk_map = Sk > 0 ? Sk : 1;
+  const void* any = codes ? static_cast<const void*>(q_codes) : p.q;
+  const void* kbase = Sk > 0 ? static_cast<const void*>(k_codes) : any;
+  const void* vbase = Sk > 0 ? static_cast<const void*>(vt_codes) : any;
+  if (int rc = make_head_map(&tk, kbase, D, sk_map, B * Hkv, D)) return rc;
+  if (int rc = make_head_map(&tv, vbase, Sk > 0 ? Sk : 16, D, B * Hkv, Sk > 0 ? vt_stride : 16)) return rc;
+  if (codes) {
+    if (int rc = make_head_map(&tq, q_codes, D, Sq, B * Hq, D)) return rc;
+  } else {
+    tq = tk;                                     // not read
+  }
+  p.Hq = static_cast<int>(Hq);
+  p.Hkv = static_cast<int>(Hkv);
+  p.Sq = static_cast<int>(Sq);
+  p.Sk = static_cast<int>(Sk);
+  p.D = static_cast<int>(D);
+  p.softmax_scale = softmax_scale;
+  p.causal = causal ? 1 : 0;
+  p.BH = static_cast<int>(B * Hq);
+  p.q_tiles = static_cast<int>((Sq + kTile - 1) / kTile);
+  const int64_t ctas = static_cast<int64_t>(p.q_tiles) * p.BH;
+  if (ctas > 0x7fffffffLL) return B200Q_ERR_INVALID;
+  p.group = head_group(p);
+  const unsigned n = static_cast<unsigned>(ctas);
+  const auto st = static_cast<cudaStream_t>(stream);
+  if (codes) return launch_sdpa_as<uint8_t, true>(tq, tk, tv, p, n, behind, st);
+  const int64_t unit = q_dtype == B200Q_F32 ? 8 : 16;
+  const bool wide = aligned(p.q, 32) && p.q_sb % unit == 0 && p.q_sh % unit == 0 && p.q_ss % unit == 0;
+#define B200Q_SDPA(T) (wide ? launch_sdpa_as<T, true>(tq, tk, tv, p, n, behind, st) : launch_sdpa_as<T, false>(tq, tk, tv, p, n, behind, st))
+  switch (q_dtype) {
+    case B200Q_BF16: return B200Q_SDPA(__nv_bfloat16);
+    case B200Q_F16: return B200Q_SDPA(__half);
+    case B200Q_F32: return B200Q_SDPA(float);
+    default: return B200Q_ERR_INVALID;
+  }
+#undef B200Q_SDPA
 }
 
 }  // namespace
@@ -742,59 +865,60 @@ int b200q_fp8_sdpa_strided(const uint8_t* q_codes, const uint8_t* k_codes, const
                            const float* k_scale, const float* v_scale, void* out, const int64_t* out_strides, int out_dtype, int64_t B,
                            int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t vt_stride, int64_t D, float softmax_scale, int causal,
                            b200q_stream_t stream) {
-  if (B < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || Sq < 0 || Sk < 0 || D <= 0 || D > 128 || D % 16 != 0) return B200Q_ERR_INVALID;
-  if (vt_stride < Sk || vt_stride % 16 != 0 || B * Hq > 65535 || Sq > 0x7fffffffLL || Sk > 0x7fffffffLL) return B200Q_ERR_INVALID;
-  if (out_dtype != B200Q_BF16 && out_dtype != B200Q_F16 && out_dtype != B200Q_F32) return B200Q_ERR_INVALID;
-  if (!(softmax_scale > 0.0f)) return B200Q_ERR_INVALID;
+  if (vt_stride < Sk || vt_stride % 16 != 0) return B200Q_ERR_INVALID;
+  if (int rc = check_attention(q_codes, k_codes, vt_codes, out, out_strides, out_dtype, B, Hq, Hkv, Sq, Sk, D, softmax_scale)) return rc;
   if (B == 0 || Sq == 0) return B200Q_OK;
-  if (q_codes == nullptr || out == nullptr || q_scale == nullptr || k_scale == nullptr || v_scale == nullptr) return B200Q_ERR_INVALID;
-  if (Sk > 0 && (k_codes == nullptr || vt_codes == nullptr)) return B200Q_ERR_INVALID;
-  if (!aligned(q_codes, 16) || !aligned(k_codes, 16) || !aligned(vt_codes, 16) || !aligned(out, 32)) return B200Q_ERR_ALIGN;
-  if (out_strides == nullptr) return B200Q_ERR_INVALID;
-  for (int i = 0; i < 3; ++i)
-    if (out_strides[i] < 0 || out_strides[i] % 8 != 0) return B200Q_ERR_ALIGN;   // 8-element stores
+  if (q_scale == nullptr || k_scale == nullptr || v_scale == nullptr) return B200Q_ERR_INVALID;
   if (int rc = check_arch()) return rc;
   AttParams p{};
-  p.out_sb = out_strides[0];
-  p.out_sh = out_strides[1];
-  p.out_ss = out_strides[2];
-  p.status = gemm::device_status_word();
-  if (p.status == nullptr) return B200Q_ERR_CUDA;
-  static bool configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
-  if (!configured[dev]) {
-    if (cudaFuncSetAttribute(fp8_sdpa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return B200Q_ERR_CUDA;
-    configured[dev] = true;
-  }
-  CUtensorMap tq, tk, tv;
-  // a zero-length key axis still needs valid maps: the kernel then loads nothing and writes zeros
-  const int64_t sk_map = Sk > 0 ? Sk : 1;
-  const void* kbase = Sk > 0 ? static_cast<const void*>(k_codes) : static_cast<const void*>(q_codes);
-  const void* vbase = Sk > 0 ? static_cast<const void*>(vt_codes) : static_cast<const void*>(q_codes);
-  if (int rc = make_head_map(&tq, q_codes, D, Sq, B * Hq, D)) return rc;
-  if (int rc = make_head_map(&tk, kbase, D, sk_map, B * Hkv, D)) return rc;
-  if (int rc = make_head_map(&tv, vbase, Sk > 0 ? Sk : 16, D, B * Hkv, Sk > 0 ? vt_stride : 16)) return rc;
   p.q_scale = q_scale;
   p.k_scale = k_scale;
   p.v_scale = v_scale;
   p.out = out;
   p.out_dtype = out_dtype;
-  p.Hq = static_cast<int>(Hq);
-  p.Hkv = static_cast<int>(Hkv);
-  p.Sq = static_cast<int>(Sq);
-  p.Sk = static_cast<int>(Sk);
-  p.D = static_cast<int>(D);
-  p.softmax_scale = softmax_scale;
-  p.causal = causal ? 1 : 0;
-  p.BH = static_cast<int>(B * Hq);
-  p.q_tiles = static_cast<int>((Sq + kTile - 1) / kTile);
-  const int64_t ctas = static_cast<int64_t>(p.q_tiles) * p.BH;
-  if (ctas > 0x7fffffffLL) return B200Q_ERR_INVALID;
-  p.group = head_group(p);
-  const dim3 grid(static_cast<unsigned>(ctas));
-  fp8_sdpa_kernel<<<grid, kAttThreads, kAttSmem, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
-  return check_launch();
+  return launch_sdpa(p, q_codes, k_codes, vt_codes, out_strides, out_dtype, B, Hq, Hkv, Sq, Sk, vt_stride, D, softmax_scale, causal, false, stream);
+}
+
+static int64_t round16(int64_t n) { return (n + 15) / 16 * 16; }
+
+size_t b200q_fp8_attention_workspace_bytes(int64_t B, int64_t Hkv, int64_t Sk, int64_t D) {
+  if (B <= 0 || Hkv <= 0 || Sk < 0 || D <= 0) return 16;
+  return static_cast<size_t>(B * Hkv * Sk * D + B * Hkv * D * round16(Sk) + 16);   // D is a multiple of 16
+}
+
+int b200q_fp8_attention(const void* q, const void* k, const void* v, int dtype, const int64_t* strides, const float* amax_q,
+                        const float* amax_k, const float* amax_v, void* out, const int64_t* out_strides, void* workspace,
+                        size_t workspace_bytes, int64_t B, int64_t Hq, int64_t Hkv, int64_t Sq, int64_t Sk, int64_t D, float softmax_scale,
+                        int causal, b200q_stream_t stream) {
+  if (int rc = check_attention(q, k, v, out, out_strides, dtype, B, Hq, Hkv, Sq, Sk, D, softmax_scale)) return rc;
+  if (B == 0 || Sq == 0) return B200Q_OK;
+  if (Sq > 0x7fffff00LL || Sk > 0x7fffff00LL || strides == nullptr || amax_q == nullptr || amax_k == nullptr || amax_v == nullptr)
+    return B200Q_ERR_INVALID;
+  if (workspace == nullptr || workspace_bytes < b200q_fp8_attention_workspace_bytes(B, Hkv, Sk, D)) return B200Q_ERR_INVALID;
+  if (int rc = check_strided(q, strides, dtype)) return rc;
+  if (!aligned(workspace, 16)) return B200Q_ERR_ALIGN;
+  const int64_t vt_stride = round16(Sk);
+  auto* k_codes = static_cast<uint8_t*>(workspace);
+  uint8_t* vt_codes = k_codes + B * Hkv * Sk * D;
+  auto* scales = reinterpret_cast<float*>(vt_codes + B * Hkv * D * vt_stride);
+  if (Sk > 0) {
+    if (int rc = b200q_fp8_attention_quantize(nullptr, k, v, dtype, strides, amax_q, amax_k, amax_v, nullptr, k_codes, vt_codes, scales, B, Hq, Hkv,
+                                              0, Sk, vt_stride, D, stream))
+      return rc;
+  } else if (int rc = check_arch()) {
+    return rc;
+  }
+  AttParams p{};
+  p.q = q;
+  p.q_amax = amax_q;
+  p.q_sb = strides[0];
+  p.q_sh = strides[1];
+  p.q_ss = strides[2];
+  p.k_scale = scales + 1;
+  p.v_scale = scales + 2;
+  p.out = out;
+  p.out_dtype = dtype;
+  return launch_sdpa(p, nullptr, k_codes, vt_codes, out_strides, dtype, B, Hq, Hkv, Sq, Sk, vt_stride, D, softmax_scale, causal, Sk > 0, stream);
 }
 
 }  // extern "C"

@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/b200q.h"
 #include "exact_div.h"
 
@@ -301,6 +303,45 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 __device__ __forceinline__ uint64_t div2_by_shared_negated(uint64_t nx, uint64_t dd, uint64_t ny) {
   const uint64_t q0 = mul2(nx, ny);
   return fma2(fma2(dd, q0, nx), ny, q0);
+}
+
+// E4M3 codes of 16 elements under one scale that is given, not measured on them (elements may lie beyond it): y = RN(1 / scale), lim =
+// 512 * scale (saturates anyway), fast = b200q_div_fast_ok(scale).  Where all 16 are within lim, two quotients at a time; the codes are
+// those of div_path element by element.  Overwrites `raw`.
+template <typename T, bool WIDE>
+__device__ __forceinline__ uint4 e4m3_of_16(Raw16<T, WIDE>& raw, float scale, float y, float lim, bool fast) {
+  bool within;                                    // false for a NaN
+  if constexpr (sizeof(T) == 2) {
+    using T2 = std::conditional_t<std::is_same<T, __half>::value, __half2, __nv_bfloat162>;
+    T2 m = __habs2(*reinterpret_cast<const T2*>(&raw.w[0].v[0]));
+#pragma unroll
+    for (int i = 1; i < 8; ++i) m = __hmax2_nan(m, __habs2(*reinterpret_cast<const T2*>(&raw.w[0].v[i])));
+    within = static_cast<float>(m.x) <= lim && static_cast<float>(m.y) <= lim;
+  } else {
+    within = true;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) within = within && fabsf(__uint_as_float(raw.w[i >> 3].v[i & 7])) <= lim;
+  }
+  float q[16];
+  if (fast && within) {
+#pragma unroll
+    for (int i = 0; i < 8 * Raw16<T, WIDE>::kLoads; ++i) raw.w[i >> 3].v[i & 7] ^= sizeof(T) == 2 ? 0x80008000u : 0x80000000u;
+    raw.widen(q);
+    const uint64_t dd = pack2(scale, scale), ny = pack2(-y, -y);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const float2 t = unpack2(div2_by_shared_negated(pack2(q[i], q[i + 1]), dd, ny));
+      q[i] = t.x, q[i + 1] = t.y;
+    }
+  } else {
+    raw.widen(q);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[i] = fast ? div_path<kDivClamped>(q[i], scale, y, lim) : div_path<kDivTrue>(q[i], scale, y, lim);
+  }
+  uint32_t c[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = f32x2_to_e4m3x2(q[4 * i], q[4 * i + 1]) | (f32x2_to_e4m3x2(q[4 * i + 2], q[4 * i + 3]) << 16);
+  return make_uint4(c[0], c[1], c[2], c[3]);
 }
 
 __device__ __forceinline__ float warp_max(float v) {

@@ -257,19 +257,12 @@ std::optional<Tensor> fp8_sdpa(const Tensor& q, const Tensor& k, const Tensor& v
   int64_t strides[9];
   if (!head_strides(q, strides) || !head_strides(k, strides + 3) || !head_strides(v, strides + 6)) return std::nullopt;
   c10::cuda::CUDAGuard guard(dev);
-  const int64_t vt_stride = up16(Sk), nq = q.numel(), nk = k.numel(), nv = B * Hkv * D * vt_stride;
   Tensor out = at::empty(q.sizes(), q.options());
-  Tensor scratch = at::empty({nq + nk + nv + 16}, q.options().dtype(at::kByte));
-  auto* qc = static_cast<uint8_t*>(scratch.data_ptr());
-  uint8_t *kc = qc + nq, *vc = kc + nk;
-  auto* scales = reinterpret_cast<float*>(vc + nv);
-  const auto st = current_stream();
-  if (!taken(b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, f32(&aq), f32(&ak), f32(&av), qc, kc, vc, scales, B,
-                                          Hq, Hkv, Sq, Sk, vt_stride, D, st),
-             "b200q_fp8_attention_quantize"))
-    return std::nullopt;
-  must(b200q_fp8_sdpa(qc, kc, vc, scales, scales + 1, scales + 2, out.data_ptr(), dt, B, Hq, Hkv, Sq, Sk, vt_stride, D, static_cast<float>(scale),
-                      causal ? 1 : 0, st),
+  const int64_t out_strides[3] = {Hq * Sq * D, Sq * D, D};
+  Tensor scratch = at::empty({static_cast<int64_t>(b200q_fp8_attention_workspace_bytes(B, Hkv, Sk, D))}, q.options().dtype(at::kByte));
+  must(b200q_fp8_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, f32(&aq), f32(&ak), f32(&av), out.data_ptr(), out_strides,
+                           scratch.data_ptr(), static_cast<size_t>(scratch.numel()), B, Hq, Hkv, Sq, Sk, D, static_cast<float>(scale),
+                           causal ? 1 : 0, current_stream()),
        "b200q_fp8_sdpa");
   return out;
 }

@@ -447,19 +447,12 @@ Tensor fp8_sdpa_cuda(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in,
   if (out.numel() == 0) return out;
   auto bytes = q.options().dtype(at::kByte);
   Tensor aq = as_f32_cuda(amax_q, q).reshape({1}), ak = as_f32_cuda(amax_k, q).reshape({1}), av = as_f32_cuda(amax_v, q).reshape({1});
-  Tensor qc = at::empty(q.sizes(), bytes), kc = at::empty(k.sizes(), bytes);
-  Tensor scales = at::empty({3}, q.options().dtype(at::kFloat));
-  const int64_t stride = std::max<int64_t>((Sk + 15) / 16 * 16, 16);
-  Tensor vt = at::empty({B, Hkv, D, stride}, bytes);
+  Tensor scratch = at::empty({static_cast<int64_t>(b200q_fp8_attention_workspace_bytes(B, Hkv, Sk, D))}, bytes);
   const int64_t strides[9] = {Hq * Sq * D, Sq * D, D, Hkv * Sk * D, Sk * D, D, Hkv * Sk * D, Sk * D, D};
-  float* sp = scales.data_ptr<float>();
-  check_status(b200q_fp8_attention_quantize(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr<float>(), ak.data_ptr<float>(),
-                                            av.data_ptr<float>(), qc.data_ptr<uint8_t>(), kc.data_ptr<uint8_t>(), vt.data_ptr<uint8_t>(), sp, B,
-                                            Hq, Hkv, Sq, Sk, stride, D, current_stream()),
-               "b200q_fp8_attention_quantize");
   const float sm = scale > 0.0 ? static_cast<float>(scale) : 1.0f / std::sqrt(static_cast<float>(D));
-  check_status(b200q_fp8_sdpa(qc.data_ptr<uint8_t>(), kc.data_ptr<uint8_t>(), vt.data_ptr<uint8_t>(), sp, sp + 1, sp + 2, out.data_ptr(), dt, B,
-                              Hq, Hkv, Sq, Sk, stride, D, sm, is_causal ? 1 : 0, current_stream()),
+  check_status(b200q_fp8_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), dt, strides, aq.data_ptr<float>(), ak.data_ptr<float>(),
+                                   av.data_ptr<float>(), out.data_ptr(), strides, scratch.data_ptr(), static_cast<size_t>(scratch.numel()), B, Hq,
+                                   Hkv, Sq, Sk, D, sm, is_causal ? 1 : 0, current_stream()),
                "b200q_fp8_sdpa");
   return out;
 }
