@@ -157,8 +157,8 @@ int b200q_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales_swizzled,
  *                   reduce-scatter forms take pairs from one such tile per SM pair on (NVFP4: never);
  *                   1001 / 1002 / 1004 / 1008 = small-M kernel (weights on the tensor core's M side,
  *                   K split over a cluster of 1 / 2 / 4 / 8 CTAs, partial tiles summed through
- *                   distributed shared memory; chosen automatically for M <= 128, ignored for larger
- *                   M).  Results do not depend on it beyond fp32 summation order.  Any other value:
+ *                   distributed shared memory; chosen automatically for M <= 128, and above in blocks of
+ *                   up to 256 (NVFP4 128) tokens where tiles would leave SMs idle).  Results do not depend on it beyond fp32 summation order.  Any other value:
  *                   B200Q_ERR_INVALID.
  *   static_weights  promise about the B operand (weights, their scales, the bias) of THIS call:
  *                   non-zero = the work that wrote it has FINISHED on the device (weights quantized at
@@ -220,8 +220,9 @@ int b200q_nvfp4_gemm(const uint8_t* a_codes, const uint8_t* a_scales, const floa
                      const uint8_t* b_codes, const uint8_t* b_scales, const float* b_global,
                      const void* bias, void* out, int64_t M, int64_t N, int64_t K,
                      b200q_stream_t stream, const b200q_cfg* cfg);
-/* Tile that b200q_nvfp4_gemm takes for M rows and N columns when cfg does not force one, as a b200q_cfg::tile_n value: 512, 256
- * or 128; 0 for the kernel of up to 128 rows.  Host only. */
+/* Tile kernel of b200q_nvfp4_gemm for M rows and N columns when cfg does not force one, as a b200q_cfg::tile_n value: 512, 256
+ * or 128; 0 for the kernel of up to 128 rows.  (Where K is long and tiles are few the GEMM splits K over blocks of tokens
+ * instead.)  Host only. */
 int b200q_nvfp4_gemm_tile(int64_t M, int64_t N);
 /* NVFP4 gate/up GEMM of a gated MLP with the activation and its static quantizer in the epilogue: B holds F
  * gate rows, then F up rows (N = 2F, N % 256 == 0); codes_out [M, F/2], scales_out (swizzled, padding rows of the last

@@ -218,9 +218,9 @@ int allow_smem(Kernel* kernel, int bytes, bool* configured) {
 // One launch of a small-M kernel: `tiles` clusters of `splits` CTAs.
 template <typename Kernel>
 int launch_clusters(Kernel* kernel, int tiles, int splits, int smem_bytes, cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tx,
-                    const Params& p, int stages, int bt) {
+                    const Params& p, int stages, int bt, int blocks) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * blocks * splits));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
   cfg.stream = st;
@@ -233,15 +233,26 @@ int launch_clusters(Kernel* kernel, int tiles, int splits, int smem_bytes, cudaS
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, tw, tx, p, splits, stages, bt) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kernel, tw, tx, p, splits, stages, bt, blocks) != cudaSuccess) {
     cudaGetLastError();
     return B200Q_ERR_CUDA;
   }
   return B200Q_OK;
 }
 
-// Small-M kernel (M <= 128): operands swapped, one cluster of `splits` CTAs per tile of 128
-// weight rows.  Up to one CTA per SM the operand ring takes all of shared memory; beyond that
+// Blocks of tokens of the small-M kernel.
+inline int smallm_blocks(int M, bool nvf4) {
+  const int most = nvf4 ? 128 : 256;
+  return M <= 128 ? 1 : (M + most - 1) / most;
+}
+
+// Tokens of a block: a multiple of 16; NVFP4 in several blocks the 128 rows of a scale tile.
+inline int smallm_block_tokens(int M, int blocks, bool nvf4) {
+  return nvf4 && blocks > 1 ? 128 : ((M + blocks - 1) / blocks + 15) / 16 * 16;
+}
+
+// Small-M kernel: operands swapped, one cluster of `splits` CTAs per tile of 128 weight rows and block of tokens (one block of
+// up to 128; above, FP8 blocks of up to 256, NVFP4 of 128).  Up to one CTA per SM the operand ring takes all of shared memory; beyond that
 // the ring is sized so that two CTAs share an SM, which lets one CTA's prologue and cluster
 // reduction overlap the other's weight stream and fits twice as many CTAs into a wave.
 // `stages` > 0 overrides the ring depth.
@@ -250,12 +261,14 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
   using C = SmallCfg<NVF4>;
   static bool configured[64] = {};
   if (int rc = allow_smem(gemm_smallm_kernel<NVF4>, kSmemLimit, configured)) return rc;
-  const int bt = ((p.M + 15) / 16) * 16;
+  const int blocks = smallm_blocks(p.M, NVF4);
+  const int bt = smallm_block_tokens(p.M, blocks, NVF4);
   const int tiles = (p.N + kSmallWRows - 1) / kSmallWRows;
+  if (static_cast<int64_t>(tiles) * blocks * splits > 0x7fffffffLL) return B200Q_ERR_INVALID;
   const int most = C::max_stages(bt, kSmemLimit);
   if (stages <= 0) {
     stages = most;
-    if (tiles * splits > sm_count()) {
+    if (tiles * blocks * splits > sm_count() && C::max_stages(bt, kSmallHalfSmem) >= C::min_stages(bt)) {
       // two CTAs per SM: half of the SM's 228 KiB (1 KiB reserved per CTA) and, for NVFP4,
       // half of the 512 tensor-memory columns (128 accumulator + 32 scale columns per stage)
       stages = C::max_stages(bt, kSmallHalfSmem);
@@ -263,11 +276,11 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
     }
   }
   if (stages > most) stages = most;
-  if (stages < 2) stages = 2;
+  if (stages < C::min_stages(bt)) stages = C::min_stages(bt);
   CUtensorMap tw, tx;
   if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
   if (int rc = make_operand_map(&tx, a, p.M, p.k_bytes, bt)) return rc;
-  return launch_clusters(gemm_smallm_kernel<NVF4>, tiles, splits, C::smem_bytes(bt, stages), st, tw, tx, p, stages, bt);
+  return launch_clusters(gemm_smallm_kernel<NVF4>, tiles, splits, C::smem_bytes(bt, stages), st, tw, tx, p, stages, bt, blocks);
 }
 
 // The small-M kernel that quantizes its activation (FP8; p.x, p.x_amax set; limits kOwnXTiles, kOwnXSlice).
@@ -281,7 +294,7 @@ int launch_smallm_own_x(const uint8_t* b, const Params& p, cudaStream_t st, int 
   if (int rc = allow_smem(gemm_smallm_kernel<false, XT>, kMostBytes, configured)) return rc;
   CUtensorMap tw;
   if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
-  return launch_clusters(gemm_smallm_kernel<false, XT>, (p.N + kSmallWRows - 1) / kSmallWRows, splits, bytes, st, tw, tw, p, stages, 16);
+  return launch_clusters(gemm_smallm_kernel<false, XT>, (p.N + kSmallWRows - 1) / kSmallWRows, splits, bytes, st, tw, tw, p, stages, 16, 1);
 }
 
 // Cluster size of the small-M kernel.  Measured: one SM pulls about 60 bytes per nanosecond
@@ -383,7 +396,44 @@ inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
   return c256 <= c128 ? 256 : 128;
 }
 
-// `cfg->tile_n` (128 / 256 / 512) overrides the choice of `large_tile` (used by tests to cover the instantiations).
+// Above 128 rows: cluster size of the small-M kernel over blocks of tokens, 0 = the tile kernel that `large_tile` takes.  With few
+// weight rows and some hundred tokens the tiles leave SMs idle, each of which walks all of K (4096 x 14336 FP8 at 129 to 512 rows:
+// 64 to 128 tiles of 128 x 128, 112 K tiles of 0.28 us each); blocks of tokens whose K is split over a cluster use them.  Both sides
+// are estimated in ns from a sweep of all kernels over 12 weight shapes and 129 to 1024 rows in each format (180 points, standard
+// deviation 3 to 6 %): the tile kernels as rounds times (start + K tiles), the small-M kernel as K tiles of a CTA, the parked
+// partial tile (every token, more the larger the cluster) and the traffic of all clusters together; only where all clusters are
+// resident at once, one CTA per SM.  Taken where it is 3 % cheaper: 48 of 180 points, nowhere slower than the tile kernel; FP8, us,
+// tile kernel / this: 4096 x 14336 at 129 rows 35.6 / 19.2, at 256 35.6 / 25.2, at 384 36.2 / 26.7; 2048 x 8192 at 256 22.2 / 17.3;
+// 8192 x 28672 at 129 69.2 / 48.6; 4096 x 4096 at 129 14.0 / 11.4; NVFP4 4096 x 14336 at 256 27.4 / 20.0.
+inline int block_splits(int M, int N, int k_tiles, int sms, bool nvf4, int tile) {
+  const int blocks = smallm_blocks(M, nvf4), n_tiles = (N + kSmallWRows - 1) / kSmallWRows;
+  const int64_t clusters = static_cast<int64_t>(n_tiles) * blocks;
+  if (clusters > sms) return 0;
+  const int bm = tile == 512 ? kPairM : kBM, bn = tile == 128 ? 128 : 256, units = tile == 512 ? sms / 2 : sms;
+  const int64_t tiles = static_cast<int64_t>((M + bm - 1) / bm) * ((N + bn - 1) / bn), rounds = (tiles + units - 1) / units;
+  int64_t least;
+  if (nvf4) {
+    least = tile == 512 ? 4490 + rounds * (1840 + 394 * k_tiles)
+                        : (tile == 256 ? 3290 + rounds * (2550 + 684 * k_tiles) : 4480 + rounds * (290 + 484 * k_tiles));
+  } else {
+    least = tile == 512 ? 5000 + rounds * (1770 + 334 * k_tiles)
+                        : (tile == 256 ? 3600 + rounds * (1640 + 391 * k_tiles) : 4100 + rounds * (510 + 289 * k_tiles));
+  }
+  least = least * 97 / 100;
+  const int64_t bt = smallm_block_tokens(M, blocks, nvf4);
+  const ActiveClusters active = active_clusters(sms);
+  int best = 0;
+  for (int s = 1, log2s = 0; s <= 8 && s <= k_tiles; s <<= 1, ++log2s) {
+    if (clusters * s > sms || clusters > smallm_resident(s, active, false)) break;
+    const int64_t per = (k_tiles + s - 1) / s, all = clusters * s * per;
+    const int64_t cost = nvf4 ? 6260 + per * 390 + 620 * log2s + all * 66 / 100
+                              : 3500 + per * (180 + bt * 48 / 100) + bt * (18 + 6 * log2s + (s == 8 ? 4 : 0)) + all * 77 / 100;
+    if (cost < least) least = cost, best = s;
+  }
+  return best;
+}
+
+// `cfg->tile_n` (128 / 256 / 512, 1001 to 1008) overrides the choice of kernel (used by tests to cover the instantiations).
 // M <= 128 goes to the small-M kernel unless a tile width is forced.
 template <bool NVF4>
 int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const b200q_cfg* cfg, const RsTargets* rs = nullptr) {
@@ -393,16 +443,18 @@ int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const 
   p.static_weights = (cfg != nullptr && cfg->static_weights != 0) ? 1 : 0;
   int bn = cfg != nullptr ? cfg->tile_n : 0;
   const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
-  if (rs == nullptr && p.M <= kBM) {
+  const int tile = p.M > kBM || rs != nullptr ? large_tile(p.M, p.N, sm_count(), NVF4, rs != nullptr) : 0;
+  if (rs == nullptr) {
     // small M: weights are streamed once; the swapped-operand cluster kernel handles it
     // (1001 / 1002 / 1004 / 1008 force 1 / 2 / 4 / 8 CTAs per tile)
     int splits = 0;
     if (bn == 1001 || bn == 1002 || bn == 1004 || bn == 1008) splits = bn - 1000;
-    else if (bn == 0) splits = smallm_splits((p.N + kSmallWRows - 1) / kSmallWRows, k_tiles, sm_count(), p.M);
+    else if (bn == 0 && p.M <= kBM) splits = smallm_splits((p.N + kSmallWRows - 1) / kSmallWRows, k_tiles, sm_count(), p.M);
+    else if (bn == 0) splits = block_splits(p.M, p.N, k_tiles, sm_count(), NVF4, tile);
     if (splits >= 1 && splits <= k_tiles) return launch_smallm<NVF4>(a, b, p, st, splits, forced_smallm_stages());
   }
   if (bn >= 1000) bn = 0;
-  if (bn == 0) bn = large_tile(p.M, p.N, sm_count(), NVF4, rs != nullptr);
+  if (bn == 0) bn = tile != 0 ? tile : large_tile(p.M, p.N, sm_count(), NVF4, false);
   // The NVFP4 pair kernel with the scale warps writes local output only; the reduce-scatter epilogue keeps the
   // generic kernels.
   if (bn == 512) {

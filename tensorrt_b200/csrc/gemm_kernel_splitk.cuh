@@ -1,4 +1,4 @@
-// Small-M variant of the quantized GEMM (decode steps, M <= 128 tokens).
+// Small-M variant of the quantized GEMM (decode steps, M <= 128 tokens; some hundred tokens in blocks, see block_splits).
 //
 // With M <= 128 the problem is a stream of weights: it is HBM-bound, the activations are tiny,
 // and there are only N / 128 output tiles.  Two changes against the persistent kernel:
@@ -39,14 +39,21 @@ struct SmallCfg {
   static constexpr int kSfBytes = NVF4 ? 4096 : 0;                   // weight + token scale atoms of one K tile
   static constexpr int kSfCols = NVF4 ? 32 : 0;                      // tensor-memory columns per stage (16 + 16)
   __host__ __device__ static constexpr int stage_bytes(int bt) { return kWBytes + bt * kBKBytes + kSfBytes; }
-  __host__ __device__ static constexpr int smem_bytes(int bt, int stages) { return 1024 + stages * stage_bytes(bt) + kSmallTailBytes; }
-  __host__ __device__ static constexpr int tmem_cols(int stages) {
-    const int need = 128 + stages * kSfCols;
+  __host__ __device__ static constexpr int tail_bytes(int bt) { return kSmallTailBytes + (bt > 128 ? 512 : 0); }   // scales of `bt` tokens
+  __host__ __device__ static constexpr int smem_bytes(int bt, int stages) { return 1024 + stages * stage_bytes(bt) + tail_bytes(bt); }
+  // the partial tile (fp32, `bt` tokens) takes the place of the ring
+  __host__ __device__ static constexpr int min_stages(int bt) {
+    const int s = (bt * kSmallWRows * 4 + stage_bytes(bt) - 1) / stage_bytes(bt);
+    return s < 2 ? 2 : s;
+  }
+  __host__ __device__ static constexpr int acc_cols(int bt) { return bt > 128 ? 256 : 128; }
+  __host__ __device__ static constexpr int tmem_cols(int bt, int stages) {
+    const int need = acc_cols(bt) + stages * kSfCols;
     return need <= 128 ? 128 : (need <= 256 ? 256 : 512);
   }
   // deepest ring that fits `budget` bytes of shared memory and 512 tensor-memory columns
   static int max_stages(int bt, int budget) {
-    int s = (budget - 1024 - kSmallTailBytes) / stage_bytes(bt);
+    int s = (budget - 1024 - tail_bytes(bt)) / stage_bytes(bt);
     if (s > kSmallMaxStages) s = kSmallMaxStages;
     return s;
   }
@@ -61,7 +68,7 @@ __device__ __forceinline__ float4 ld_shared_cluster_v4(uint32_t addr) {
 // Sum tokens [t0, t1) of the S partial tiles of the cluster, scale, add bias, store bf16.
 // partial tile layout: float [token][128 weight rows]; thread item = (token, group of 8 rows).
 template <int S>
-__device__ __forceinline__ void small_reduce_store(uint32_t partial_u32, int t0, int t1, int n_base, const float* xscale,
+__device__ __forceinline__ void small_reduce_store(uint32_t partial_u32, int t0, int t1, int m_base, int n_base, const float* xscale,
                                                    const float* wscale, const float* wbias, const Params& p) {
   const bool vec_ok = (p.N % 8) == 0;
   const int items = (t1 - t0) * 16;
@@ -92,7 +99,7 @@ __device__ __forceinline__ void small_reduce_store(uint32_t partial_u32, int t0,
       w[j] = *reinterpret_cast<uint32_t*>(&h);
     }
     const int n = n_base + g * 8;
-    __nv_bfloat16* dst = p.out + static_cast<int64_t>(tok) * p.N + n;
+    __nv_bfloat16* dst = p.out + static_cast<int64_t>(m_base + tok) * p.N + n;
     if (vec_ok && n + 8 <= p.N) {
       *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
@@ -192,11 +199,12 @@ __device__ __forceinline__ void small_quantize_x(const Params& p, uint8_t* xs, f
 }
 
 // tmap_w: weights [N, k_bytes], box 128 rows; tmap_x: activations [M, k_bytes], box `bt` rows
-// (bt = M rounded up to 16).  `splits` = cluster size, `stages` = depth of the operand ring.
+// (M over `blocks` blocks of tokens, rounded up to 16; NVFP4 in several blocks: 128, the rows of a scale tile).  `splits` = cluster
+// size, `stages` = depth of the operand ring.  One cluster per tile of 128 weight rows and block of tokens.
 template <bool NVF4, typename XT = void>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const Params p,
-                   const int splits, const int stages, const int bt) {
+                   const int splits, const int stages, const int bt, const int blocks) {
   using C = SmallCfg<NVF4>;
   constexpr bool kOwnX = !std::is_void<XT>::value;       // the kernel quantizes the activation itself
   extern __shared__ uint8_t smem_raw[];
@@ -216,14 +224,16 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   uint64_t* sft_full = reinterpret_cast<uint64_t*>(tail + 384);   // NVFP4: a stage's scales are in tensor memory (4 warps)
   float* wscale = reinterpret_cast<float*>(tail + 512);   // [128] dequantization scale of each weight row
   float* wbias = wscale + 128;                            // [128]
-  float* xscale = wbias + 128;                            // [128] dequantization scale of each token
+  float* xscale = wbias + 128;                            // [128, or 256] dequantization scale of each token
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(ptx::cluster_ctarank());
-  const int nb = blockIdx.x / splits;                     // one cluster per tile of 128 weight rows
+  // the clusters of one weight tile are neighbours: the second block of tokens finds its weights in L2
+  const int cluster = blockIdx.x / splits, nb = cluster / blocks, block = cluster - nb * blocks;
   const int n_base = nb * kSmallWRows;
+  const int m_base = block * bt, m_rows = min(bt, p.M - m_base);
   const int kt0 = min(rank * per, k_tiles), kt1 = min(kt0 + per, k_tiles);
-  const uint32_t tmem_cols = static_cast<uint32_t>(C::tmem_cols(stages));
+  const uint32_t tmem_cols = static_cast<uint32_t>(C::tmem_cols(bt, stages));
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -255,7 +265,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // (static_weights), the first ring of weight tiles is requested before waiting for it and only
     // the activation tiles (which it may still be writing) after; otherwise everything waits.
     const uint8_t* sfw_src = NVF4 ? p.sfb + static_cast<int64_t>(nb) * p.sf_col_tiles * 512 : nullptr;
-    const uint8_t* sfx_src = NVF4 ? p.sfa : nullptr;
+    const uint8_t* sfx_src = NVF4 ? p.sfa + static_cast<int64_t>(block) * p.sf_col_tiles * 512 : nullptr;
     auto sf_bytes_of = [&](int kt) -> uint32_t {
       return NVF4 ? static_cast<uint32_t>(min(4, p.sf_col_tiles - kt * 4)) * 512u : 0u;
     };
@@ -269,7 +279,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     auto issue_x = [&](int kt, int stage) {
       if constexpr (kOwnX) return;
       uint8_t* sx = smem + stage * stage_bytes + C::kWBytes;
-      ptx::tma_load_2d(sx, &tmap_x, full_bar + stage, kt * kBKBytes, 0);
+      ptx::tma_load_2d(sx, &tmap_x, full_bar + stage, kt * kBKBytes, m_base);
       if constexpr (NVF4) ptx::bulk_load(sx + x_bytes + 2048, sfx_src + kt * 2048, sf_bytes_of(kt), full_bar + stage);
     };
     const int pre = min(stages, kt1 - kt0);
@@ -363,10 +373,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (p.bias != nullptr) wb = __bfloat162float(p.bias[n]);
       }
       pdl_wait();  // the activation scales come from the kernel before this one
-      if (wrow < p.M && !kOwnX) {
+      if (wrow < m_rows && !kOwnX) {
         if constexpr (NVF4) xs = __fmul_rn(ld_dependent(p.a_scales), ld_dependent(p.b_scales));
-        else xs = ld_dependent(p.a_scales + static_cast<int64_t>(wrow) * p.a_scale_stride);
+        else xs = ld_dependent(p.a_scales + static_cast<int64_t>(m_base + wrow) * p.a_scale_stride);
       }
+      if constexpr (!NVF4 && !kOwnX)
+        if (wrow + 128 < m_rows) xscale[wrow + 128] = ld_dependent(p.a_scales + static_cast<int64_t>(m_base + wrow + 128) * p.a_scale_stride);
       if constexpr (kOwnX) {     // in front of the stores below, which wait for the scales' loads
         small_quantize_x<XT>(p, own_x, xscale, kt0, kt1, threadIdx.x - 64);
         __syncwarp();
@@ -421,7 +433,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
     ptx::tc_fence_after();
 #pragma unroll 1
-    for (int c = 0; c * 32 < p.M; ++c) {
+    for (int c = 0; c * 32 < m_rows; ++c) {
       uint32_t r[32];
       if (have && ok) {
         ptx::tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c * 32, r);
@@ -432,7 +444,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (c * 32 + j < p.M) partial[(c * 32 + j) * kSmallWRows + wrow] = __uint_as_float(r[j]);
+        if (c * 32 + j < m_rows) partial[(c * 32 + j) * kSmallWRows + wrow] = __uint_as_float(r[j]);
     }
   }
 
@@ -445,14 +457,14 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
   if (*failed == 0) {
     // ------------------------------------------------------------ reduce my tokens over the cluster, scale, store
-    const int per_rank = (p.M + splits - 1) / splits;
-    const int t0 = min(rank * per_rank, p.M), t1 = min(t0 + per_rank, p.M);
+    const int per_rank = (m_rows + splits - 1) / splits;
+    const int t0 = min(rank * per_rank, m_rows), t1 = min(t0 + per_rank, m_rows);
     const uint32_t partial_u32 = ptx::smem_u32(smem);
     switch (splits) {
-      case 1: small_reduce_store<1>(partial_u32, t0, t1, n_base, xscale, wscale, wbias, p); break;
-      case 2: small_reduce_store<2>(partial_u32, t0, t1, n_base, xscale, wscale, wbias, p); break;
-      case 4: small_reduce_store<4>(partial_u32, t0, t1, n_base, xscale, wscale, wbias, p); break;
-      default: small_reduce_store<8>(partial_u32, t0, t1, n_base, xscale, wscale, wbias, p); break;
+      case 1: small_reduce_store<1>(partial_u32, t0, t1, m_base, n_base, xscale, wscale, wbias, p); break;
+      case 2: small_reduce_store<2>(partial_u32, t0, t1, m_base, n_base, xscale, wscale, wbias, p); break;
+      case 4: small_reduce_store<4>(partial_u32, t0, t1, m_base, n_base, xscale, wscale, wbias, p); break;
+      default: small_reduce_store<8>(partial_u32, t0, t1, m_base, n_base, xscale, wscale, wbias, p); break;
     }
   }
 
