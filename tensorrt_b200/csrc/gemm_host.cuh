@@ -256,12 +256,12 @@ inline int smallm_block_tokens(int M, int blocks, bool nvf4) {
 // the ring is sized so that two CTAs share an SM, which lets one CTA's prologue and cluster
 // reduction overlap the other's weight stream and fits twice as many CTAs into a wave.
 // `stages` > 0 overrides the ring depth.
-template <bool NVF4>
+template <bool NVF4, bool BLOCKS>
 int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, int splits, int stages) {
   using C = SmallCfg<NVF4>;
   static bool configured[64] = {};
-  if (int rc = allow_smem(gemm_smallm_kernel<NVF4>, kSmemLimit, configured)) return rc;
-  const int blocks = smallm_blocks(p.M, NVF4);
+  if (int rc = allow_smem(gemm_smallm_kernel<NVF4, void, BLOCKS>, kSmemLimit, configured)) return rc;
+  const int blocks = BLOCKS ? smallm_blocks(p.M, NVF4) : 1;
   const int bt = smallm_block_tokens(p.M, blocks, NVF4);
   const int tiles = (p.N + kSmallWRows - 1) / kSmallWRows;
   if (static_cast<int64_t>(tiles) * blocks * splits > 0x7fffffffLL) return B200Q_ERR_INVALID;
@@ -280,7 +280,7 @@ int launch_smallm(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st,
   CUtensorMap tw, tx;
   if (int rc = make_operand_map(&tw, b, p.N, p.k_bytes, kSmallWRows)) return rc;
   if (int rc = make_operand_map(&tx, a, p.M, p.k_bytes, bt)) return rc;
-  return launch_clusters(gemm_smallm_kernel<NVF4>, tiles, splits, C::smem_bytes(bt, stages), st, tw, tx, p, stages, bt, blocks);
+  return launch_clusters(gemm_smallm_kernel<NVF4, void, BLOCKS>, tiles, splits, C::smem_bytes(bt, stages), st, tw, tx, p, stages, bt, blocks);
 }
 
 // The small-M kernel that quantizes its activation (FP8; p.x, p.x_amax set; limits kOwnXTiles, kOwnXSlice).
@@ -451,7 +451,9 @@ int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const 
     if (bn == 1001 || bn == 1002 || bn == 1004 || bn == 1008) splits = bn - 1000;
     else if (bn == 0 && p.M <= kBM) splits = smallm_splits((p.N + kSmallWRows - 1) / kSmallWRows, k_tiles, sm_count(), p.M);
     else if (bn == 0) splits = block_splits(p.M, p.N, k_tiles, sm_count(), NVF4, tile);
-    if (splits >= 1 && splits <= k_tiles) return launch_smallm<NVF4>(a, b, p, st, splits, forced_smallm_stages());
+    if (splits >= 1 && splits <= k_tiles)
+      return p.M <= kBM ? launch_smallm<NVF4, false>(a, b, p, st, splits, forced_smallm_stages())
+                        : launch_smallm<NVF4, true>(a, b, p, st, splits, forced_smallm_stages());
   }
   if (bn >= 1000) bn = 0;
   if (bn == 0) bn = tile != 0 ? tile : large_tile(p.M, p.N, sm_count(), NVF4, false);
