@@ -304,6 +304,7 @@ def call_times(capi, stack, h, mb, sharded):
 
     for n in names:
         wrap(n)
+    native, stack.native_layers = stack.native_layers, False      # one call otherwise
     try:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
@@ -311,6 +312,7 @@ def call_times(capi, stack, h, mb, sharded):
         e1.record()
         torch.cuda.synchronize()
     finally:
+        stack.native_layers = native
         for n, (orig, static) in saved.items():
             setattr(capi, n, orig)
             if static is not None:

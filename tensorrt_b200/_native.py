@@ -1,5 +1,5 @@
-"""Native whole calls (csrc/python_calls.cpp): `fp8_linear`, `nvfp4_linear`, `fp8_gated_mlp`, `fp8_sdpa`.  Each returns
-the result, or None when the call is not the plain case it takes; the caller then goes through `capi`."""
+"""Native whole calls (csrc/python_calls.cpp): `fp8_linear`, `nvfp4_linear`, `fp8_gated_mlp`, `fp8_sdpa`,
+`decoder_stack`.  Each returns the result, or None when the call is not the plain case it takes; the caller then goes through `capi`."""
 from __future__ import annotations
 
 import importlib.machinery
@@ -20,3 +20,4 @@ def _load():
 _calls = _load()
 fp8_linear, nvfp4_linear = _calls.fp8_linear, _calls.nvfp4_linear
 fp8_gated_mlp, fp8_sdpa = _calls.fp8_gated_mlp, _calls.fp8_sdpa
+decoder_stack = _calls.decoder_stack

@@ -1,4 +1,5 @@
-// Whole calls of the Python modules (quantize -> GEMM, the gated MLP, FP8 attention) as one native function each.
+// Whole calls of the Python modules (quantize -> GEMM, the gated MLP, FP8 attention, a forward of the decoder stack) as one
+// native function each.
 //
 // A decode step's linear runs for ten to twenty microseconds on the device; the same steps issued one by one from
 // Python (argument checks, two to six tensors, a ctypes call per kernel) take longer than that on the host.  The
@@ -23,8 +24,10 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <array>
 #include <cmath>
 #include <optional>
+#include <vector>
 
 #include "b200q.h"
 #include "internal.h"
@@ -267,6 +270,166 @@ std::optional<Tensor> fp8_sdpa(const Tensor& q, const Tensor& k, const Tensor& v
   return out;
 }
 
+// ---------------------------------------------------------------- DecoderStack.forward on one rank
+// The layers of stack.py::DecoderLayer.forward with CudaBackend's kernels, step for step: same calls, same bits.  Issued from
+// Python a layer takes 150 to 250 us of host time (nine to eleven calls, two to six tensors each), which is longer than its
+// kernels run below about a thousand tokens: three layers of hidden 2048 over 300 tokens 450 us eager, 203 in a graph.
+struct QuantizedWeight {
+  const Tensor *codes, *scales, *global;   // global: NVFP4
+  int64_t n() const { return codes->size(0); }
+};
+struct StackLayer {
+  const Tensor *norm1, *norm2;
+  QuantizedWeight qkv, o, gate_up, down;
+  const Tensor* amax[4];                   // NVFP4: calibrated ranges of the inputs of qkv, o, gate_up, down
+};
+struct StackShape {
+  int64_t n_q, n_kv, head_dim, seq_len;    // seq_len 0: every kv head repeated in place of attention
+  float eps;
+  bool fp8, fuse_gate_up;
+};
+
+bool weight_of(const QuantizedWeight& w, int64_t n, int64_t k, bool fp8, at::Device dev) {
+  if (!codes_of(*w.codes, dev) || w.codes->size(1) != (fp8 ? k : k / 2) || (n > 0 && w.n() != n)) return false;
+  if (fp8) return f32_of(*w.scales, 1, w.n(), dev);
+  return w.scales->scalar_type() == at::kByte && w.scales->is_contiguous() && w.scales->device() == dev &&
+         w.scales->numel() >= static_cast<int64_t>(b200q_nvfp4_scale_bytes(w.n(), k)) && f32_of(*w.global, 1, 1, dev);
+}
+
+bool norm_of(const Tensor& w, int64_t n, at::Device dev) {
+  return w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.numel() == n && w.device() == dev;
+}
+
+std::optional<Tensor> decoder_stack(const Tensor& h_in, const std::vector<StackLayer>& layers, const StackShape& s) {
+  const auto dev = h_in.device();
+  if (layers.empty() || h_in.dim() != 2 || h_in.scalar_type() != at::kBFloat16 || !h_in.is_contiguous() || h_in.numel() == 0) return std::nullopt;
+  const int64_t T = h_in.size(0), H = h_in.size(1), Q = s.n_q * s.head_dim, KV = s.n_kv * s.head_dim, W = Q + 2 * KV;
+  if (s.n_q <= 0 || s.n_kv <= 0 || s.head_dim <= 0 || s.n_q % s.n_kv != 0 || H % 32 != 0 || H > 16384 || s.head_dim % 16 != 0 || s.head_dim > 128 || Q % 32 != 0)
+    return std::nullopt;
+  if (s.seq_len < 0 || (s.seq_len > 0 && T % s.seq_len != 0)) return std::nullopt;
+  if (reinterpret_cast<uintptr_t>(h_in.data_ptr()) % 32 != 0) return std::nullopt;
+  const int64_t F = layers[0].gate_up.codes->dim() == 2 ? layers[0].gate_up.n() / 2 : 0;
+  if (F <= 0 || F % 32 != 0 || F > 32768) return std::nullopt;
+  for (const StackLayer& l : layers) {
+    if (!norm_of(*l.norm1, H, dev) || !norm_of(*l.norm2, H, dev) || !weight_of(l.qkv, W, H, s.fp8, dev) || !weight_of(l.o, H, Q, s.fp8, dev) ||
+        !weight_of(l.gate_up, 2 * F, H, s.fp8, dev) || !weight_of(l.down, H, F, s.fp8, dev))
+      return std::nullopt;
+    for (const Tensor* a : l.amax)
+      if (!s.fp8 && !f32_of(*a, 1, 1, dev)) return std::nullopt;
+  }
+  c10::cuda::CUDAGuard guard(dev);
+  const auto st = current_stream();
+  b200q_cfg cfg{};
+  cfg.static_weights = 1;                          // complete since the stack's constructor synchronised
+  // the same choices as CudaBackend.gate_up_activation, gate_up_quantize_static and expand_heads_quantize
+  const bool fused = s.fuse_gate_up && 2 * F % 256 == 0 && (s.fp8 ? T >= 256 : b200q_nvfp4_gemm_tile(T, 2 * F) == 512);
+  const bool attention = s.seq_len > 0, expand_quant = !s.fp8 || KV <= 2048;
+  // scratch: an operand (codes, then its scales), what stands between QKV and O or between gate/up and down, the residual stream
+  // twice, the output of a row-parallel linear
+  const int64_t widest = std::max(H, std::max(Q, F));
+  const int64_t code_bytes = up16(s.fp8 ? T * widest : T * widest / 2);
+  const int64_t scale_bytes = up16(s.fp8 ? 4 * T : static_cast<int64_t>(b200q_nvfp4_scale_bytes(T, widest)) + 16);
+  const int64_t ws_bytes = attention ? up16(static_cast<int64_t>(b200q_fp8_attention_workspace_bytes(T / s.seq_len, s.n_kv, s.seq_len, s.head_dim)) + 16) : 0;
+  const bool bf16_heads = attention || !expand_quant;
+  const auto up32 = [](int64_t n) { return (n + 31) / 32 * 32; };
+  const int64_t qkv_bytes = up32(T * W * 2), head_bytes = bf16_heads ? up32(T * Q * 2) : 0;
+  // (NVFP4 with the activation in the GEMM's epilogue: the down projection's operand itself)
+  const int64_t ffn_bytes = !fused ? T * F * 4 : (s.fp8 ? T * F * 2 : code_bytes + scale_bytes);
+  const int64_t mid_bytes = std::max(qkv_bytes + head_bytes + ws_bytes, ffn_bytes);
+  const int64_t row_bytes = up32(T * H * 2);
+  const int64_t o_codes = 3 * row_bytes + up32(mid_bytes), o_scales = o_codes + code_bytes;
+  Tensor scratch = at::empty({o_scales + scale_bytes}, h_in.options().dtype(at::kByte));
+  auto* base = static_cast<uint8_t*>(scratch.data_ptr());
+  uint8_t *rows[2] = {base, base + row_bytes}, *delta = base + 2 * row_bytes, *mid = base + 3 * row_bytes;
+  uint8_t *qkv = mid, *heads = mid + qkv_bytes, *ws = heads + head_bytes;
+  struct Quantized {
+    uint8_t *codes, *sf;
+    float *scales, *global;
+  };
+  const auto operand = [&](uint8_t* c) {           // NVFP4: the global scale behind the block scales
+    uint8_t* sf = c + code_bytes;
+    return Quantized{c, sf, reinterpret_cast<float*>(sf), reinterpret_cast<float*>(sf + scale_bytes - 16)};
+  };
+  const Quantized x = operand(base + o_codes), act = operand(mid);
+  Tensor out = at::empty(h_in.sizes(), h_in.options());
+  const auto gemm = [&](const Quantized& a, const QuantizedWeight& w, int64_t k, void* y) {
+    const auto* c = static_cast<const uint8_t*>(w.codes->data_ptr());
+    if (s.fp8)
+      must(b200q_fp8_gemm(a.codes, a.scales, T, c, f32(w.scales), w.scales->numel(), nullptr, y, T, w.n(), k, st, &cfg), "b200q_fp8_gemm");
+    else
+      must(b200q_nvfp4_gemm(a.codes, a.sf, a.global, c, static_cast<const uint8_t*>(w.scales->data_ptr()), f32(w.global), nullptr, y, T, w.n(), k, st, &cfg),
+           "b200q_nvfp4_gemm");
+  };
+  const auto quantize = [&](const void* y, int64_t k, const Tensor* amax) {
+    if (s.fp8) must(b200q_fp8_quantize(y, B200Q_BF16, T, k, nullptr, 0, x.codes, x.scales, st), "b200q_fp8_quantize");
+    else must(b200q_nvfp4_quantize(y, B200Q_BF16, T, k, f32(amax), x.codes, x.sf, x.global, st), "b200q_nvfp4_quantize");
+  };
+  const void* h = h_in.data_ptr();
+  const void* d = nullptr;
+  int turn = 0;
+  bool first = true;
+  const auto norm = [&](const Tensor* w, const Tensor* amax) -> bool {
+    void* h_out = d == nullptr ? const_cast<void*>(h) : rows[turn];
+    const int rc = s.fp8 ? b200q_add_rms_norm_fp8_quantize(h, d, w->data_ptr(), h_out, x.codes, x.scales, T, H, s.eps, st)
+                         : b200q_add_rms_norm_nvfp4_quantize(h, d, w->data_ptr(), h_out, f32(amax), x.codes, x.sf, x.global, T, H, s.eps, st);
+    const char* what = s.fp8 ? "b200q_add_rms_norm_fp8_quantize" : "b200q_add_rms_norm_nvfp4_quantize";
+    if (first && !taken(rc, what)) return false;
+    must(rc, what);
+    first = false;
+    if (d != nullptr) h = h_out, turn ^= 1;
+    return true;
+  };
+  for (const StackLayer& l : layers) {
+    if (!norm(l.norm1, l.amax[0])) return std::nullopt;
+    gemm(x, l.qkv, H, qkv);
+    if (attention) {
+      const int64_t B = T / s.seq_len, S = s.seq_len;
+      const auto many = [](int64_t n, int64_t stride) { return n > 1 ? stride : int64_t{0}; };
+      const int64_t in[3] = {many(B, S * W), 0, many(S, W)};
+      const int64_t strides[9] = {in[0], many(s.n_q, s.head_dim), in[2], in[0], many(s.n_kv, s.head_dim), in[2],
+                                  in[0], many(s.n_kv, s.head_dim), in[2]};
+      const int64_t out_strides[3] = {many(B, S * Q), many(s.n_q, s.head_dim), many(S, Q)};
+      auto* amax = reinterpret_cast<float*>(ws + ws_bytes - 16);
+      must(b200q_amax_columns(qkv, B200Q_BF16, T, Q, KV, KV, amax, st), "b200q_amax_columns");
+      must(b200q_fp8_attention(qkv, qkv + Q * 2, qkv + (Q + KV) * 2, B200Q_BF16, strides, amax, amax + 1, amax + 2, heads, out_strides, ws,
+                               static_cast<size_t>(ws_bytes - 16), B, s.n_q, s.n_kv, S, S, s.head_dim,
+                               static_cast<float>(1.0 / std::sqrt(static_cast<double>(s.head_dim))), 1, st),
+           "b200q_fp8_sdpa");
+      quantize(heads, Q, l.amax[1]);
+    } else {
+      const int rep = static_cast<int>(s.n_q / s.n_kv), n_q = static_cast<int>(s.n_q), hd = static_cast<int>(s.head_dim);
+      if (!s.fp8) {
+        must(b200q_expand_heads_nvfp4_quantize(qkv, W, Q + KV, f32(l.amax[1]), x.codes, x.sf, x.global, T, n_q, rep, hd, st), "b200q_expand_heads_nvfp4_quantize");
+      } else if (expand_quant) {
+        must(b200q_expand_heads_fp8_quantize(qkv, W, Q + KV, x.codes, x.scales, T, n_q, rep, hd, st), "b200q_expand_heads_fp8_quantize");
+      } else {
+        must(b200q_expand_heads(qkv, W, Q + KV, heads, T, n_q, rep, hd, st), "b200q_expand_heads");
+        quantize(heads, Q, nullptr);
+      }
+    }
+    gemm(x, l.o, Q, delta);
+    d = delta;
+    norm(l.norm2, l.amax[2]);
+    const auto* gu = static_cast<const uint8_t*>(l.gate_up.codes->data_ptr());
+    if (s.fp8 && fused) {
+      must(b200q_fp8_gemm_silu_mul(x.codes, x.scales, T, gu, f32(l.gate_up.scales), l.gate_up.scales->numel(), nullptr, mid, T, 2 * F, H, st, nullptr),
+           "b200q_fp8_gemm_silu_mul");
+      quantize(mid, F, nullptr);
+    } else if (fused) {
+      must(b200q_nvfp4_gemm_silu_mul_quantize(x.codes, x.sf, x.global, gu, static_cast<const uint8_t*>(l.gate_up.scales->data_ptr()),
+                                              f32(l.gate_up.global), f32(l.amax[3]), act.codes, act.sf, act.global, T, 2 * F, H, st),
+           "b200q_nvfp4_gemm_silu_mul_quantize");
+    } else {
+      gemm(x, l.gate_up, H, mid);
+      if (s.fp8) must(b200q_silu_mul_fp8_quantize(mid, x.codes, x.scales, T, F, st), "b200q_silu_mul_fp8_quantize");
+      else must(b200q_silu_mul_nvfp4_quantize(mid, f32(l.amax[3]), x.codes, x.sf, x.global, T, F, st), "b200q_silu_mul_nvfp4_quantize");
+    }
+    gemm(fused && !s.fp8 ? act : x, l.down, F, delta);
+  }
+  must(b200q_add(h, delta, out.data_ptr(), T * H, st), "b200q_add");
+  return out;
+}
+
 // ---------------------------------------------------------------- Python side
 // Runs `fn` without the GIL (allocations and launches) and hands its result over; None = not taken.
 template <typename F>
@@ -356,6 +519,43 @@ PyObject* py_fp8_sdpa(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// One layer as a tuple of tensors: norm1, norm2, then codes and scales (NVFP4: and global scale) of qkv, o, gate/up and down,
+// NVFP4: then the four ranges.
+bool read_layer(PyObject* t, bool fp8, StackLayer& l) {
+  const Py_ssize_t n = fp8 ? 10 : 18;
+  if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != n) return false;
+  std::array<const Tensor*, 18> a{};
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* o = PyTuple_GET_ITEM(t, i);
+    if (!plain(o)) return false;
+    a[i] = &THPVariable_Unpack(o);
+  }
+  l = StackLayer{};
+  l.norm1 = a[0], l.norm2 = a[1];
+  int i = 2;
+  for (QuantizedWeight* w : {&l.qkv, &l.o, &l.gate_up, &l.down}) {
+    w->codes = a[i++], w->scales = a[i++];
+    if (!fp8) w->global = a[i++];
+  }
+  if (!fp8)
+    for (int k = 0; k < 4; ++k) l.amax[k] = a[i++];
+  return true;
+}
+
+PyObject* py_decoder_stack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_VALUE(n == 9 && PyList_Check(a[1]), "decoder_stack: 9 arguments expected, the second a list");
+  StackShape s{PyLong_AsLongLong(a[2]), PyLong_AsLongLong(a[3]), PyLong_AsLongLong(a[4]), PyLong_AsLongLong(a[5]),
+               static_cast<float>(PyFloat_AsDouble(a[6])), PyObject_IsTrue(a[7]) == 1, PyObject_IsTrue(a[8]) == 1};
+  if (PyErr_Occurred()) return nullptr;
+  if (!plain(a[0]) || modes_active()) Py_RETURN_NONE;
+  std::vector<StackLayer> layers(static_cast<size_t>(PyList_GET_SIZE(a[1])));
+  for (size_t i = 0; i < layers.size(); ++i)
+    if (!read_layer(PyList_GET_ITEM(a[1], static_cast<Py_ssize_t>(i)), s.fp8, layers[i])) Py_RETURN_NONE;
+  return finish([&] { return decoder_stack(THPVariable_Unpack(a[0]), layers, s); });
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
     {"fp8_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fp8_linear)), METH_FASTCALL,
      "x, w_codes, w_scales, bias, x_amax, tile_n -> bf16 tensor, or None: take the general path"},
@@ -365,6 +565,8 @@ PyMethodDef methods[] = {
      "x, gu_codes, gu_scales, down_codes, down_scales, input_amax, act_amax, tile_n -> bf16 tensor or None"},
     {"fp8_sdpa", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_fp8_sdpa)), METH_FASTCALL,
      "q, k, v, amax_q, amax_k, amax_v, is_causal, scale -> tensor like q or None"},
+    {"decoder_stack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_decoder_stack)), METH_FASTCALL,
+     "h, layers, n_q, n_kv, head_dim, seq_len, eps, fp8, fuse_gate_up -> tensor like h or None"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "b200q_native", "Whole calls of the b200q modules", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -306,11 +306,23 @@ class DecoderLayer:
         self.wo = backend.prepare_weight(weights["wo"])
         self.wgu = backend.prepare_weight(weights["wgu"])
         self.wdown = backend.prepare_weight(weights["wdown"])
-        self.row_parallel = row_parallel or (lambda x, qw, amax=None: backend.linear(x, qw, amax))
+        self._local_linear = lambda x, qw, amax=None: backend.linear(x, qw, amax)
+        self.row_parallel = row_parallel or self._local_linear
         # Calibrated activation amax per linear input (the `amax` operand of the quantize op is a
         # constant after calibration in the reference flow); filled by a calibration pass.
         self.amax: dict = {}
         self.calibrating = False
+
+    def plain(self) -> bool:
+        """Nothing replaced or switched on that `DecoderStack._native_forward` does not know of."""
+        return (type(self) is DecoderLayer and self.row_parallel is self._local_linear and self.world == 1 and not self.calibrating and
+                not {"forward", "_attention", "_ffn_act"} & self.__dict__.keys() and
+                (self.cfg.mode == "fp8" or self.amax.keys() >= {"qkv", "o", "gate_up", "down"}))
+
+    def tensors(self) -> tuple:
+        """Weights and calibrated ranges in the order of `_native.decoder_stack`."""
+        ranges = () if self.cfg.mode == "fp8" else tuple(self.amax[n] for n in ("qkv", "o", "gate_up", "down"))
+        return (self.norm1, self.norm2, *self.wqkv, *self.wo, *self.wgu, *self.wdown, *ranges)
 
     def _amax(self, name: str, x):
         if isinstance(x, tuple):
@@ -434,6 +446,7 @@ class DecoderStack:
         self._comm = None
         self._fused = None
         self._pull = None
+        self.native_layers = True                # one rank: a forward is one native call where it is the plain case
         self.check_status = True                 # forward() polls the device status word on the fused TP path
         self.backend = backend or CudaBackend(cfg.mode)
         reduce = AllReduce(group) if world > 1 else None
@@ -501,12 +514,34 @@ class DecoderStack:
 
     def _micro_batch(self, h: torch.Tensor, sharded: bool) -> torch.Tensor:
         """All layers over one batch of tokens on the current stream."""
+        out = self._native_forward(h)
+        if out is not None:
+            return out
         if sharded is True:
             if self._fused is not None and self._fused.usable(h.shape[0]):
                 return self._walk_fused_sharded(h).clone()
             sharded = False
         sharded = bool(sharded)
         return self._finish(*self._walk(self._enter(h, sharded), None, sharded), sharded)
+
+    def _native_forward(self, h: torch.Tensor):
+        """The layers of `DecoderLayer.forward` as one native call (the same kernels in the same order, the same bits), or None
+        where that does not take them: several ranks, another backend or layer class, a replaced method, a forced GEMM tile, a
+        calibrating pass, NVFP4 without calibrated ranges, tokens that are not whole sequences."""
+        cfg, be = self.cfg, self.backend
+        if not self.native_layers or self.world != 1 or type(be) is not CudaBackend or be.__dict__.keys() != {"mode", "fuse_gate_up"} or not h.is_cuda:
+            return None
+        if be.mode != cfg.mode or capi.gemm_defaults() != (0, True) or not all(l.plain() for l in self.layers):
+            return None
+        seq_len = cfg.seq_len if cfg.attention == "fp8_sdpa" else 0
+        if seq_len and h.shape[0] % seq_len:
+            if h.shape[0] >= seq_len:
+                return None
+            seq_len = 0                          # fewer tokens than a sequence: as DecoderLayer._attention
+        from . import _native
+
+        return _native.decoder_stack(h, [l.tensors() for l in self.layers], cfg.n_q, cfg.n_kv, cfg.head_dim, seq_len, cfg.eps, cfg.mode == "fp8",
+                                     bool(be.fuse_gate_up))
 
     def _walk_pull(self, h: torch.Tensor) -> torch.Tensor:
         """A few tokens (decode): replicated residual stream, every row-parallel linear ends in the
