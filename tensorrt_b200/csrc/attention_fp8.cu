@@ -262,8 +262,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       int ks = n_tiles > 0 ? 1 : 0, vs = 0;       // the first K tile is on its way (above)
       uint32_t kph = 0, vph = 0;
       bool ok = true;
-      // the order of the loads is the order in which the MMA thread uses them: pass 1 all K tiles; pass 2 K 0, K 1,
-      // K 2, V 0, K 3, V 1, ...
+      // the order of the loads is the order in which the MMA thread uses them: pass 1 all K tiles; pass 2, which begins with
+      // the last key tile and needs no scores for it, K 0, K 1, V last, K 2, V 0, K 3, V 1, ...
       auto load_k = [&](int j) -> bool {
         if (!ptx::mbar_wait(k_empty + ks, kph ^ 1u)) {
           att_timeout(p.status, 61);
@@ -285,9 +285,9 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         return true;
       };
       for (int j = 1; j < n_tiles && ok; ++j) ok = load_k(j);
-      for (int j = 0; j < n_tiles + 2 && ok; ++j) {
-        if (j < n_tiles) ok = load_k(j);
-        if (ok && j >= 2) ok = load_v(j - 2);
+      for (int i = 1; i < n_tiles + 2 && ok; ++i) {
+        if (i < n_tiles) ok = load_k(i - 1);
+        if (ok && i >= 2) ok = load_v(i == 2 ? n_tiles - 1 : i - 3);
       }
       // drain: every load issued above has landed and was consumed before shared memory is released
       for (int s = 0; s < kKStages && ok; ++s) {
@@ -339,10 +339,10 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         return true;
       };
       for (int j = 0; j < n_tiles && ok; ++j) ok = issue_scores(j & 1);    // pass 1: scores only, two buffers
-      // pass 2: the scores of tile j + 2 are issued in front of the product of tile j.  Their buffer is free once every
-      // warp has taken tile j + 1, which it does right after writing its part of P j: the warps wait for scores, nobody
-      // waits for the product yet.
-      for (int j = 0; j < min(2, n_tiles) && ok; ++j) ok = issue_scores(0);
+      // pass 2, the last key tile (no scores) and then 0, 1, ..: the scores of the tile after next are issued in front of the
+      // product of a tile.  Their buffer is free once every warp has taken the next tile, which it does right after writing its
+      // part of P: the warps wait for scores, nobody waits for the product yet.
+      if (n_tiles > 1 && ok) ok = issue_scores(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (j + 2 < n_tiles) ok = issue_scores(0);
         if (!ok) break;
@@ -451,14 +451,53 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       return true;
     };
-    const int first_edge = min(full_tiles, n_tiles);
+    // The last key tile keeps its exponentials: pass 2 begins with them and scales them, so that this tile's scores are computed and
+    // raised once.  One maximum over both chunks, so that they all have one reference.
+    uint32_t e[2 * kChunk];
+    auto pass1_last = [&]() -> bool {
+      if (!take_scores(std::true_type{}, n_tiles - 1, (n_tiles - 1) & 1, e)) {
+        att_timeout(p.status, 68);
+        return false;
+      }
+      float x0 = __uint_as_float(e[0]), x1 = __uint_as_float(e[1]), x2 = __uint_as_float(e[2]), x3 = __uint_as_float(e[3]);
+#pragma unroll
+      for (int i = 4; i < 2 * kChunk; i += 4) {
+        x0 = fmaxf(x0, __uint_as_float(e[i]));
+        x1 = fmaxf(x1, __uint_as_float(e[i + 1]));
+        x2 = fmaxf(x2, __uint_as_float(e[i + 2]));
+        x3 = fmaxf(x3, __uint_as_float(e[i + 3]));
+      }
+      const float cm = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
+      if (cm > m) {
+        l *= ex2_approx((m - cm) * c2);
+        m = cm;
+      }
+      const float off = m > -INFINITY ? -m * c2 : 0.0f;
+      const uint64_t offoff = pack2(off, off);
+      uint64_t l01 = 0ull, l23 = 0ull;
+#pragma unroll
+      for (int i = 0; i < 2 * kChunk; i += 4) {
+        const uint64_t a = ex2_pair(fma2(pack2(__uint_as_float(e[i]), __uint_as_float(e[i + 1])), c2c2, offoff), (i / 2) & 15);
+        const uint64_t b = ex2_pair(fma2(pack2(__uint_as_float(e[i + 2]), __uint_as_float(e[i + 3])), c2c2, offoff), (i / 2 + 1) & 15);
+        l01 = add2(l01, a);
+        l23 = add2(l23, b);
+        const float2 ua = unpack2(a), ub = unpack2(b);
+        e[i] = __float_as_uint(ua.x), e[i + 1] = __float_as_uint(ua.y), e[i + 2] = __float_as_uint(ub.x), e[i + 3] = __float_as_uint(ub.y);
+      }
+      const float2 s0 = unpack2(l01), s1 = unpack2(l23);
+      l += (s0.x + s0.y) + (s1.x + s1.y);
+      return true;
+    };
+    const int rest = n_tiles - 1, first_edge = min(full_tiles, rest);
     for (int j = 0; j < first_edge && ok; ++j) ok = pass1(std::false_type{}, j);
-    for (int j = first_edge; j < n_tiles && ok; ++j) ok = pass1(std::true_type{}, j);
+    for (int j = max(first_edge, 0); j < rest && ok; ++j) ok = pass1(std::true_type{}, j);
+    if (n_tiles > 0 && ok) ok = pass1_last();
     // The two threads of a row each hold the statistics of their columns: merge (every softmax thread gets here).  They pass them
     // on through the first probability tile, each in a piece of this row that the other one alone writes later, behind its read.
     uint8_t* srow = sp + r * 128;
     *reinterpret_cast<float2*>(srow + (((2 * (ch ^ 1)) ^ (r & 7)) * 16)) = make_float2(m, l);
     asm volatile("bar.sync 1, 256;" ::: "memory");
+    const float m_own = m;
     {
       const float2 o = *reinterpret_cast<const float2*>(srow + (((2 * ch) ^ (r & 7)) * 16));
       const float mm = fmaxf(m, o.x);
@@ -471,6 +510,34 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // 448 * 2^(s2 - m2) / l = 2^(acc * c2 + off2) with the normaliser folded into the exponent
     const float off2 = l > 0.0f ? -m * c2 + __log2f(kE4M3Max / l) : -INFINITY;
     const uint64_t off22 = pack2(off2, off2);
+    // 16 columns = one 16-byte piece of the operand row; 128-byte swizzle: the piece i of row r lives at piece i ^ (r & 7)
+    auto put_piece = [&](uint8_t* prow, int g, const uint32_t* w) {
+      const int piece = 2 * ch + (g & 1) + 4 * (g >> 1);
+      *reinterpret_cast<uint4*>(prow + ((piece ^ (r & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+    };
+    auto tile_written = [&]() {
+      ptx::fence_proxy_async();                   // the tensor core reads this tile through the async proxy
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(p_full + pb);
+      if (++pb == 2) pb = 0, pph ^= 1u;
+    };
+    if (n_tiles > 0 && ok) {                      // the last key tile: 448 * e / l, e referred from this thread's maximum to the row's
+      const float f = l > 0.0f ? kE4M3Max / l * ex2_approx((m_own - m) * c2) : 0.0f;
+      const uint64_t ff = pack2(f, f);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t* t = e + g * 16 + i * 4;
+          const float2 a = unpack2(mul2(pack2(__uint_as_float(t[0]), __uint_as_float(t[1])), ff));
+          const float2 b = unpack2(mul2(pack2(__uint_as_float(t[2]), __uint_as_float(t[3])), ff));
+          w[i] = f32x4_to_e4m3x4(a.x, a.y, b.x, b.y);
+        }
+        put_piece(sp + r * 128, g, w);
+      }
+      tile_written();
+    }
     auto pass2 = [&](auto masked, int j) -> bool {
       uint32_t v[2 * kChunk];
       if (!take_scores(masked, j, 0, v) || !ptx::mbar_wait(p_empty + pb, pph ^ 1u)) {
@@ -489,18 +556,13 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const float2 b = unpack2(ex2_pair(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22), k + 1));
           w[i] = f32x4_to_e4m3x4(a.x, a.y, b.x, b.y);
         }
-        // 128-byte swizzle of the operand layout: the 16-byte piece i of row r lives at piece i ^ (r & 7)
-        const int piece = 2 * ch + (g & 1) + 4 * (g >> 1);
-        *reinterpret_cast<uint4*>(prow + ((piece ^ (r & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+        put_piece(prow, g, w);
       }
-      ptx::fence_proxy_async();                   // the tensor core reads this tile through the async proxy
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(p_full + pb);
-      if (++pb == 2) pb = 0, pph ^= 1u;
+      tile_written();
       return true;
     };
     for (int j = 0; j < first_edge && ok; ++j) ok = pass2(std::false_type{}, j);
-    for (int j = first_edge; j < n_tiles && ok; ++j) ok = pass2(std::true_type{}, j);
+    for (int j = max(first_edge, 0); j < rest && ok; ++j) ok = pass2(std::true_type{}, j);
     // ---- output: O * (v_scale / 448) -> out dtype
     if (ok && n_tiles > 0 && !ptx::mbar_wait(o_full, 0)) {
       att_timeout(p.status, 70);
