@@ -152,7 +152,8 @@ int b200q_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales_swizzled,
  * Last argument of the GEMM entry points and of the peer-memory reductions; NULL = all defaults.
  * Nothing here is process-wide: two callers (threads, stacks, graphs) never see each other's choices.
  *   tile_n          GEMM tile selection.  0 = chosen per problem (default); 128 or 256 = single-CTA
- *                   tiles of 128 x tile_n; 512 = CTA-pair kernels (256 x 256 tiles, cta_group::2).  The
+ *                   tiles of 128 x tile_n; 512 = CTA-pair kernels (256 x 256 tiles, cta_group::2), 448 = the
+ *                   same with 256 x 192 tiles (FP8; NVFP4: as 512).  The
  *                   choice takes the one whose rounds of tiles over the SMs (SM pairs) cost least; the
  *                   reduce-scatter forms take pairs from one such tile per SM pair on (NVFP4: never);
  *                   1001 / 1002 / 1004 / 1008 = small-M kernel (weights on the tensor core's M side,

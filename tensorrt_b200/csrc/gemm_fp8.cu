@@ -76,7 +76,7 @@ ActiveClusters active_clusters(int sms) {
 }
 
 bool valid_tile_n(int bn) {
-  return bn == 0 || bn == 128 || bn == 256 || bn == 512 || bn == 1001 || bn == 1002 || bn == 1004 || bn == 1008;
+  return bn == 0 || bn == 128 || bn == 256 || bn == 448 || bn == 512 || bn == 1001 || bn == 1002 || bn == 1004 || bn == 1008;
 }
 
 int sf_copier_enabled() {

@@ -108,21 +108,21 @@ inline int make_scale_map(CUtensorMap* map, const void* base, int64_t row_tiles,
 }
 
 // CTA-pair kernel: clusters of two CTAs, one cluster per 256 x 256 output tile.
-template <bool NVF4, int SILU = 0>
+template <bool NVF4, int SILU = 0, int BN = kPairN>
 int launch_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const RsTargets* rs = nullptr) {
-  using C = Cfg2<NVF4>;
+  using C = Cfg2<NVF4, BN>;
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<NVF4, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_pair_kernel<NVF4, SILU, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
       return B200Q_ERR_CUDA;
     configured[dev] = true;
   }
   CUtensorMap ta, tb, tsfa, tsfb;
   OutMaps tout = {};
   if (int rc = make_operand_map(&ta, a, p.M, p.k_bytes, 128)) return rc;
-  if (int rc = make_operand_map(&tb, b, p.N, p.k_bytes, kPairN / 2)) return rc;
+  if (int rc = make_operand_map(&tb, b, p.N, p.k_bytes, BN / 2)) return rc;
   if constexpr (SILU == 2) {
     // E4M3 codes [M, F] leave through plain stores: no output map
     p.tma_store = 0;
@@ -142,7 +142,7 @@ int launch_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, c
     tsfa = ta;
     tsfb = ta;
   }
-  const int tiles = ((p.M + kPairM - 1) / kPairM) * (SILU ? (p.silu_f + kPairN / 2 - 1) / (kPairN / 2) : (p.N + kPairN - 1) / kPairN);
+  const int tiles = ((p.M + kPairM - 1) / kPairM) * (SILU ? (p.silu_f + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   cudaLaunchConfig_t cfg = {};
@@ -157,7 +157,7 @@ int launch_pair(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, c
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NVF4, SILU>, ta, tb, tout, tsfa, tsfb, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NVF4, SILU, BN>, ta, tb, tout, tsfa, tsfb, p) != cudaSuccess) {
     cudaGetLastError();
     return B200Q_ERR_CUDA;
   }
@@ -368,7 +368,7 @@ bool valid_tile_n(int bn);    // values b200q_cfg::tile_n accepts
 int sf_copier_enabled();     // environment variable B200Q_SF_COPIER (default in gemm_fp8.cu)
 int forced_smallm_stages();  // from the environment variable B200Q_SMALLM_STAGES (0 when unset)
 
-// Kernel of a problem with more than 128 rows: 512 = CTA pair with 256 x 256 tiles, 256 / 128 = one CTA with 128 x 256 /
+// Kernel of a problem with more than 128 rows: 512 / 448 = CTA pair with 256 x 256 / 256 x 192 tiles, 256 / 128 = one CTA with 128 x 256 /
 // 128 x 128 tiles.  A launch takes as long as its rounds: tiles over SMs (SM pairs), rounded up, times the time of one
 // tile, in units of a pair's 256 x 256 tile.  Large problems (many rounds) go to the pair kernels; a problem just above
 // a whole number of rounds, or with few rows, to the finer tiles (333 x 10240 x 8192 FP8: 80 pair tiles on 74 pairs are
@@ -380,7 +380,11 @@ int forced_smallm_stages();  // from the environment variable B200Q_SMALLM_STAGE
 // slower on average and 2.2 times at worst (NVFP4 4096 x 14336 at 600 to 1000 rows: 48 to 64 pair tiles, 57 to 59 us on
 // 128 x 128 tiles, 28.7 to 29.3 on pairs).  The reduce-scatter epilogue keeps the choice by tile counts that its NVLink
 // overlap was measured with.
-constexpr int kTile256Fp8 = 110, kTile128Fp8 = 85, kTile256Nv = 145, kTile128Nv = 110;   // per cent of a pair tile
+// FP8 pairs also take tiles of 256 x 192, 0.88 of the time of the wide ones: where rounds of those are cheaper, 0.99 of the time
+// on average over 295 points (18 weight shapes, 129 to 6000 rows), 0.88 at best and nowhere more: 10240 x 8192 at 200 rows 30.6 ->
+// 27.4 us, at 512 49.9 -> 44.9; 20480 x 5120 at 256 38.2 -> 33.8; 8192 x 28672 at 600 168.8 -> 148.2.  (Tiles of 256 x 128, 0.83,
+// are never the best by more than 1 %.)
+constexpr int kTile256Fp8 = 110, kTile128Fp8 = 85, kTile192Pair = 90, kTile256Nv = 145, kTile128Nv = 110;   // per cent of a pair tile
 inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
   const int64_t pair = static_cast<int64_t>((M + kPairM - 1) / kPairM) * ((N + kPairN - 1) / kPairN);
   const int64_t t256 = static_cast<int64_t>((M + kBM - 1) / kBM) * ((N + 255) / 256);
@@ -392,6 +396,10 @@ inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
   const auto cost = [](int64_t tiles, int units, int each) { return (tiles + units - 1) / units * each; };
   const int64_t c512 = cost(pair, sms / 2, 100), c256 = cost(t256, sms, nvf4 ? kTile256Nv : kTile256Fp8),
                 c128 = cost(t128, sms, nvf4 ? kTile128Nv : kTile128Fp8);
+  if (!nvf4) {
+    const int64_t pair192 = static_cast<int64_t>((M + kPairM - 1) / kPairM) * ((N + 191) / 192), c448 = cost(pair192, sms / 2, kTile192Pair);
+    if (c448 < c512 && c448 < c256 && c448 < c128) return 448;
+  }
   if (c512 <= c256 && c512 <= c128) return 512;
   return c256 <= c128 ? 256 : 128;
 }
@@ -409,15 +417,17 @@ inline int block_splits(int M, int N, int k_tiles, int sms, bool nvf4, int tile)
   const int blocks = smallm_blocks(M, nvf4), n_tiles = (N + kSmallWRows - 1) / kSmallWRows;
   const int64_t clusters = static_cast<int64_t>(n_tiles) * blocks;
   if (clusters > sms) return 0;
-  const int bm = tile == 512 ? kPairM : kBM, bn = tile == 128 ? 128 : 256, units = tile == 512 ? sms / 2 : sms;
+  const bool pairs = tile == 512 || tile == 448;
+  const int bm = pairs ? kPairM : kBM, bn = tile == 128 ? 128 : (tile == 448 ? 192 : 256), units = pairs ? sms / 2 : sms;
   const int64_t tiles = static_cast<int64_t>((M + bm - 1) / bm) * ((N + bn - 1) / bn), rounds = (tiles + units - 1) / units;
   int64_t least;
   if (nvf4) {
     least = tile == 512 ? 4490 + rounds * (1840 + 394 * k_tiles)
                         : (tile == 256 ? 3290 + rounds * (2550 + 684 * k_tiles) : 4480 + rounds * (290 + 484 * k_tiles));
   } else {
-    least = tile == 512 ? 5000 + rounds * (1770 + 334 * k_tiles)
-                        : (tile == 256 ? 3600 + rounds * (1640 + 391 * k_tiles) : 4100 + rounds * (510 + 289 * k_tiles));
+    least = tile == 512   ? 5000 + rounds * (1770 + 334 * k_tiles)
+            : tile == 448 ? 5000 + rounds * (1300 + 300 * k_tiles)
+                          : (tile == 256 ? 3600 + rounds * (1640 + 391 * k_tiles) : 4100 + rounds * (510 + 289 * k_tiles));
   }
   least = least * 97 / 100;
   const int64_t bt = smallm_block_tokens(M, blocks, nvf4);
@@ -433,7 +443,7 @@ inline int block_splits(int M, int N, int k_tiles, int sms, bool nvf4, int tile)
   return best;
 }
 
-// `cfg->tile_n` (128 / 256 / 512, 1001 to 1008) overrides the choice of kernel (used by tests to cover the instantiations).
+// `cfg->tile_n` (128 / 256 / 448 / 512, 1001 to 1008) overrides the choice of kernel (used by tests to cover the instantiations).
 // M <= 128 goes to the small-M kernel unless a tile width is forced.
 template <bool NVF4>
 int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const b200q_cfg* cfg, const RsTargets* rs = nullptr) {
@@ -459,7 +469,10 @@ int launch(const uint8_t* a, const uint8_t* b, Params p, cudaStream_t st, const 
   if (bn == 0) bn = tile != 0 ? tile : large_tile(p.M, p.N, sm_count(), NVF4, false);
   // The NVFP4 pair kernel with the scale warps writes local output only; the reduce-scatter epilogue keeps the
   // generic kernels.
-  if (bn == 512) {
+  if constexpr (!NVF4) {
+    if (bn == 448) return launch_pair<false, 0, 192>(a, b, p, st, rs);
+  }
+  if (bn == 512 || bn == 448) {
     if constexpr (NVF4) {
       if (rs == nullptr) return launch_nvf4_pair(a, b, p, st);
       return launch_pair<NVF4>(a, b, p, st, rs);

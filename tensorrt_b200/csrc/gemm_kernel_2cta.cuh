@@ -29,17 +29,19 @@ namespace gemm {
 constexpr int kPairM = 256;
 constexpr int kPairN = 256;
 
-template <bool NVF4>
+// BN: columns of a tile, 256, or 192 (FP8) where those cost fewer rounds (large_tile): whole 64-column output panels, BN / 2 rows of
+// B per CTA.
+template <bool NVF4, int BN = kPairN>
 struct Cfg2 {
   static constexpr int kABytes = 128 * kBKBytes;                    // this CTA's 128 rows of A
-  static constexpr int kBBytes = (kPairN / 2) * kBKBytes;           // this CTA's 128 rows of B
+  static constexpr int kBBytes = (BN / 2) * kBKBytes;               // this CTA's half of B's rows
   static constexpr int kSfaBytes = NVF4 ? 2048 : 0;
   static constexpr int kSfbBytes = NVF4 ? 4096 : 0;                 // scales of all 256 B rows
   static constexpr int kStageBytes = kABytes + kBBytes + kSfaBytes + kSfbBytes;
   static constexpr int kAccStages = NVF4 ? 1 : 2;
   static constexpr int kSfCols = NVF4 ? 48 : 0;
   static constexpr int kTailBytes = 2048;
-  static constexpr int kEpiBytes = 2 * 2 * kPairN * 4;
+  static constexpr int kEpiBytes = 2 * 2 * BN * 4;
   static constexpr int kPanelBytes = 32 * 128;
   static constexpr int kFixed = 1024 + kTailBytes + kEpiBytes;
   static constexpr int kStages2 = (kSmemLimit - kFixed - 4 * 2 * kPanelBytes) / kStageBytes;
@@ -47,10 +49,10 @@ struct Cfg2 {
   static constexpr int kEpiBufs = (kStages2 >= 5 || kStages2 == kStages1) ? 2 : 1;
   static constexpr int kStoreBytes = 4 * kEpiBufs * kPanelBytes;
   static constexpr int kStagesRaw = kEpiBufs == 2 ? kStages2 : kStages1;
-  static constexpr int kStagesCap = NVF4 ? (512 - kAccStages * kPairN) / 48 : 8;   // tensor-memory columns for scales
+  static constexpr int kStagesCap = NVF4 ? (512 - kAccStages * BN) / 48 : 8;   // tensor-memory columns for scales
   static constexpr int kStages = kStagesRaw > kStagesCap ? kStagesCap : kStagesRaw;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStoreBytes + kEpiBytes + kTailBytes;
-  static constexpr int kColsNeeded = kAccStages * kPairN + kStages * kSfCols;
+  static constexpr int kColsNeeded = kAccStages * BN + kStages * kSfCols;
   static constexpr int kTmemCols = 512;
   static_assert(kStages >= 3, "pipeline too shallow");
   static_assert(kColsNeeded <= 512, "tensor memory overflow");
@@ -60,13 +62,13 @@ struct Cfg2 {
 // (loaded by the peer, F rows further on), so accumulator columns 0..127 / 128..255 are a gate / up pair
 // and the epilogue writes silu(gate) * up into out[M, F] (Params::silu_f = F): SILU = 1 as bf16, SILU = 2 as E4M3
 // codes at the static per-tensor scale Params::act_amax / 448.
-template <bool NVF4, int SILU = 0>
+template <bool NVF4, int SILU = 0, int BN = kPairN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ OutMaps tmap_out, const __grid_constant__ CUtensorMap tmap_sfa,
                  const __grid_constant__ CUtensorMap tmap_sfb, const Params p) {
-  using C = Cfg2<NVF4>;
-  constexpr int BN = kPairN;
+  static_assert(BN == kPairN || (!NVF4 && SILU == 0 && BN % 64 == 0), "narrow tiles: plain FP8 only");
+  using C = Cfg2<NVF4, BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* store_stage = smem + C::kStages * C::kStageBytes;
@@ -82,7 +84,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t cta_rank = ptx::cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int m_blocks = (p.M + kPairM - 1) / kPairM;
-  const int n_blocks = SILU ? (p.silu_f + kPairN / 2 - 1) / (kPairN / 2) : (p.N + kPairN - 1) / kPairN;
+  const int n_blocks = SILU ? (p.silu_f + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;
   const int num_tiles = m_blocks * n_blocks;
   const int k_tiles = (p.k_bytes + kBKBytes - 1) / kBKBytes;
   constexpr int kGroupM = 8;
@@ -129,8 +131,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         int mb, nb;
         tile_coord(t, mb, nb);
         const int32_t m0 = mb * kPairM + static_cast<int>(cta_rank) * 128;
-        const int32_t n0 = SILU ? nb * (kPairN / 2) + static_cast<int>(cta_rank) * p.silu_f
-                                : nb * kPairN + static_cast<int>(cta_rank) * (kPairN / 2);
+        const int32_t n0 = SILU ? nb * (BN / 2) + static_cast<int>(cta_rank) * p.silu_f : nb * BN + static_cast<int>(cta_rank) * (BN / 2);
         for (int kt = 0; kt < k_tiles; ++kt) {
           if (!ptx::mbar_wait(empty_bar + stage, phase ^ 1u)) {
             raise_timeout(p.status, 11);
