@@ -268,10 +268,11 @@ int launch_rows_items(const T* x, const float* amax, uint8_t* codes, T* fake, fl
   if constexpr (sizeof(T) == 2) {
     // Measured, groups -> pieces, us: 8192 x 14336 measured range 70.4 -> 51.9, 8191 x 5120 25.6 -> 20.0 (fake-quantize 31.6 -> 26.5),
     // 4096 x 2048 7.5 -> 5.8, 4096 x 16384 39.7 -> 30.1.  Not faster, and left as they are: a few hundred rows (333 x 8192 2.9 ->
-    // 3.3) and one piece for nearly every of 256 threads (8192 x 4096 18.5 -> 19.9, 8192 x 3584 17.8 -> 18.3).  Between, 2049 to
-    // 3072 columns would gain as well and are not taken yet (8192 x 2560 16.6 -> 12.5, 8192 x 3072 17.0 -> 14.6; 3328 even).  With the
-    // range given one point of 21 is slower, 4096 x 8192 16.3 -> 16.7.
-    if (rows >= 4 * sm_count() && cols % 16 == 0 && (cols <= 2048 || (cols > 4096 && cols <= 16384)) && aligned(x, 32) &&
+    // 3.3) and one piece for nearly every of 256 threads (8192 x 4096 18.5 -> 19.9, 8192 x 3584 17.8 -> 18.3).  From 2049 to
+    // 3072 columns, measured range / given range / fake-quantize: 8192 x 2560 15.2 -> 11.0 / 18.0 -> 13.2 / 20.5 -> 15.5, 8192 x 3072 16.6 ->
+    // 12.7 / 18.8 -> 15.5 / 21.6 -> 18.4, 4096 x 2304 8.0 -> 6.6 / 9.6 -> 7.5 / 10.8 -> 8.5, 600 x 2560 5.8 -> 5.4 / even / 5.4 -> 4.1; 3328 even.
+    // With the range given one point of 21 is slower, 4096 x 8192 16.3 -> 16.7.
+    if (rows >= 4 * sm_count() && cols % 16 == 0 && (cols <= 3072 || (cols > 4096 && cols <= 16384)) && aligned(x, 32) &&
         (OUT == Out::Codes ? aligned(codes, 16) : aligned(fake, 32))) {
       const int pieces = static_cast<int>(cols >> 4), n = (pieces + kRowThreads - 1) / kRowThreads;
       const dim3 threads(static_cast<unsigned>(((pieces + n - 1) / n + 31) / 32 * 32));
