@@ -29,7 +29,7 @@
 // are issued in front of the product of tile j (wait for scores per tile 819 -> 171 clocks of about 2500); edge tiles
 // have their own copy of the loop; query tiles with the most keys start first (head_group).  Order and roundings per row are those
 // of a loop over 32-column pieces.  [4, 32 / 8, 2048, 128] causal: 300 -> 245 us for the call, 199 with the exponentials on both pipes,
-// constant addresses, queries quantized here and the last tile raised once.
+// constant addresses, queries quantized here and the last tile raised once (bf16 results, see FREE).
 //
 // One CTA per (batch, head, 128 queries): warp 0 = TMA producer, warp 1 = MMA issue + tensor-memory
 // allocation, warps 2-9 = softmax (two threads per query row, each half of the columns; lane quarter = warp & 3).  K and Q tiles are
@@ -127,9 +127,10 @@ __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
 }
 
 // 2^x of pair k of a chunk
+template <bool BOTH_PIPES>
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t x, int k) {
   constexpr int kPairs = kChunk / 2;
-  if ((k + 1) * kPolyPairs / kPairs != k * kPolyPairs / kPairs) return ex2_poly2(x);
+  if (BOTH_PIPES && (k + 1) * kPolyPairs / kPairs != k * kPolyPairs / kPairs) return ex2_poly2(x);
   const float2 a = unpack2(x);
   return pack2(ex2_approx(a.x), ex2_approx(a.y));
 }
@@ -149,7 +150,10 @@ __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, f
 // operands of K and V: each is read by one CTA only, so a pass of its own would write and read their codes for nothing.  Both launches,
 // us, operand pass for all three / this: [4, 32 / 8, 2048, 128] causal 212 / 202; [3, 16, 577 x 1500, 64] 51 / 47.7; [8, 32 / 8, 1024,
 // 128] causal 147 / 137; [8, 12, 200, 128] causal 21.2 / 18.9; [1, 8, 64, 64] 13.1 / 11.2.
-template <typename QT, bool WIDE>
+// FREE: results of 8 significant bits (bf16).  There an eighth of the exponentials runs on the FMA pipe and the last key tile keeps its
+// own; both move a probability that lies within about 1e-7 of a rounding boundary to the next code, which a bf16 result of many
+// keys does not show.  Results of 11 and more bits (fp16, fp32) keep every operation and its order: the same bits as before.
+template <typename QT, bool WIDE, bool FREE>
 __global__ void __launch_bounds__(kAttThreads, 2)
 fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_vt, const AttParams p) {
@@ -285,9 +289,10 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         return true;
       };
       for (int j = 1; j < n_tiles && ok; ++j) ok = load_k(j);
-      for (int i = 1; i < n_tiles + 2 && ok; ++i) {
-        if (i < n_tiles) ok = load_k(i - 1);
-        if (ok && i >= 2) ok = load_v(i == 2 ? n_tiles - 1 : i - 3);
+      // (FREE; otherwise from the first tile on: K 0, K 1, K 2, V 0, ...)
+      for (int i = FREE ? 1 : 0; i < n_tiles + 2 && ok; ++i) {
+        if (i < n_tiles) ok = load_k(FREE ? i - 1 : i);
+        if (ok && i >= 2) ok = load_v(!FREE ? i - 2 : (i == 2 ? n_tiles - 1 : i - 3));
       }
       // drain: every load issued above has landed and was consumed before shared memory is released
       for (int s = 0; s < kKStages && ok; ++s) {
@@ -342,7 +347,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // pass 2, the last key tile (no scores) and then 0, 1, ..: the scores of the tile after next are issued in front of the
       // product of a tile.  Their buffer is free once every warp has taken the next tile, which it does right after writing its
       // part of P: the warps wait for scores, nobody waits for the product yet.
-      if (n_tiles > 1 && ok) ok = issue_scores(0);
+      // (Without FREE tile 0 is the first and has scores as well.)
+      for (int j = FREE ? 1 : 0; j < min(2, n_tiles) && ok; ++j) ok = issue_scores(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (j + 2 < n_tiles) ok = issue_scores(0);
         if (!ok) break;
@@ -443,8 +449,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         uint64_t l01 = 0ull, l23 = 0ull;          // pairs of zeros
 #pragma unroll
         for (int i = 0; i < kChunk; i += 4) {
-          l01 = add2(l01, ex2_pair(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2c2, offoff), i / 2));
-          l23 = add2(l23, ex2_pair(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c2c2, offoff), i / 2 + 1));
+          l01 = add2(l01, ex2_pair<FREE>(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2c2, offoff), i / 2));
+          l23 = add2(l23, ex2_pair<FREE>(fma2(pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), c2c2, offoff), i / 2 + 1));
         }
         const float2 s0 = unpack2(l01), s1 = unpack2(l23);
         l += (s0.x + s0.y) + (s1.x + s1.y);
@@ -480,8 +486,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint64_t l01 = 0ull, l23 = 0ull;
 #pragma unroll
       for (int i = 0; i < 2 * kChunk; i += 4) {
-        const uint64_t a = ex2_pair(fma2(pack2(__uint_as_float(e[i]), __uint_as_float(e[i + 1])), c2c2, offoff), (i / 2) & 15);
-        const uint64_t b = ex2_pair(fma2(pack2(__uint_as_float(e[i + 2]), __uint_as_float(e[i + 3])), c2c2, offoff), (i / 2 + 1) & 15);
+        const uint64_t a = ex2_pair<FREE>(fma2(pack2(__uint_as_float(e[i]), __uint_as_float(e[i + 1])), c2c2, offoff), (i / 2) & 15);
+        const uint64_t b = ex2_pair<FREE>(fma2(pack2(__uint_as_float(e[i + 2]), __uint_as_float(e[i + 3])), c2c2, offoff), (i / 2 + 1) & 15);
         l01 = add2(l01, a);
         l23 = add2(l23, b);
         const float2 ua = unpack2(a), ub = unpack2(b);
@@ -491,10 +497,10 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       l += (s0.x + s0.y) + (s1.x + s1.y);
       return true;
     };
-    const int rest = n_tiles - 1, first_edge = min(full_tiles, rest);
+    const int rest = FREE ? n_tiles - 1 : n_tiles, first_edge = min(full_tiles, rest);
     for (int j = 0; j < first_edge && ok; ++j) ok = pass1(std::false_type{}, j);
     for (int j = max(first_edge, 0); j < rest && ok; ++j) ok = pass1(std::true_type{}, j);
-    if (n_tiles > 0 && ok) ok = pass1_last();
+    if (FREE && n_tiles > 0 && ok) ok = pass1_last();
     // The two threads of a row each hold the statistics of their columns: merge (every softmax thread gets here).  They pass them
     // on through the first probability tile, each in a piece of this row that the other one alone writes later, behind its read.
     uint8_t* srow = sp + r * 128;
@@ -524,7 +530,7 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (lane == 0) ptx::mbar_arrive(p_full + pb);
       if (++pb == 2) pb = 0, pph ^= 1u;
     };
-    if (n_tiles > 0 && ok) {                      // the last key tile: 448 * e / l, e referred from this thread's maximum to the row's
+    if (FREE && n_tiles > 0 && ok) {              // the last key tile: 448 * e / l, e referred from this thread's maximum to the row's
       const float f = l > 0.0f ? kE4M3Max / l * ex2_approx((m_own - m) * c2) : 0.0f;
       const uint64_t ff = pack2(f, f);
 #pragma unroll
@@ -555,8 +561,8 @@ fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int i = 0; i < 4; ++i) {
           const uint32_t* e = v + g * 16 + i * 4;
           const int k = (g & 1) * 8 + i * 2;
-          const float2 a = unpack2(ex2_pair(fma2(pack2(__uint_as_float(e[0]), __uint_as_float(e[1])), c2c2, off22), k));
-          const float2 b = unpack2(ex2_pair(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22), k + 1));
+          const float2 a = unpack2(ex2_pair<FREE>(fma2(pack2(__uint_as_float(e[0]), __uint_as_float(e[1])), c2c2, off22), k));
+          const float2 b = unpack2(ex2_pair<FREE>(fma2(pack2(__uint_as_float(e[2]), __uint_as_float(e[3])), c2c2, off22), k + 1));
           w[i] = f32x4_to_e4m3x4(a.x, a.y, b.x, b.y);
         }
         put_piece(prow, g, w);
@@ -785,22 +791,29 @@ int check_attention(const void* q, const void* k, const void* v, const void* out
   return B200Q_OK;
 }
 
-template <typename QT, bool WIDE>
-int launch_sdpa_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
+template <typename QT, bool WIDE, bool FREE>
+int launch_sdpa_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
                           cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(fp8_sdpa_kernel<QT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return B200Q_ERR_CUDA;
+    if (cudaFuncSetAttribute(fp8_sdpa_kernel<QT, WIDE, FREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return B200Q_ERR_CUDA;
     configured[dev] = true;
   }
   if (behind) {
-    if (launch_pdl(fp8_sdpa_kernel<QT, WIDE>, dim3(ctas), dim3(kAttThreads), kAttSmem, st, tq, tk, tv, p) != cudaSuccess) return B200Q_ERR_CUDA;
+    if (launch_pdl(fp8_sdpa_kernel<QT, WIDE, FREE>, dim3(ctas), dim3(kAttThreads), kAttSmem, st, tq, tk, tv, p) != cudaSuccess) return B200Q_ERR_CUDA;
   } else {
-    fp8_sdpa_kernel<QT, WIDE><<<ctas, kAttThreads, kAttSmem, st>>>(tq, tk, tv, p);
+    fp8_sdpa_kernel<QT, WIDE, FREE><<<ctas, kAttThreads, kAttSmem, st>>>(tq, tk, tv, p);
   }
   return check_launch();
+}
+
+template <typename QT, bool WIDE>
+int launch_sdpa_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
+                   cudaStream_t st) {
+  return p.out_dtype == B200Q_BF16 ? launch_sdpa_form<QT, WIDE, true>(tq, tk, tv, p, ctas, behind, st)
+                                   : launch_sdpa_form<QT, WIDE, false>(tq, tk, tv, p, ctas, behind, st);
 }
 
 // p: scales, queries (q_amax == nullptr: codes, at `q_codes`) and the result filled in.  `behind`: the kernel that writes the K and
