@@ -765,10 +765,9 @@ constexpr int kSiluStages = 6;                                // 6 x 16 KB
 template <int CHUNKS, bool GATED>
 __global__ void __launch_bounds__(kThreads, 2)
 silu_mul_quant_stream_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ codes, float* __restrict__ scales, int rows,
-                             int f, int* __restrict__ status) {
+                             int f, int* __restrict__ status, bool late) {
   constexpr int kStageBytes = (GATED ? 2 : 1) * kSiluChunkBytes;
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_enter(late);
   extern __shared__ __align__(128) unsigned char ring[];
   __shared__ uint64_t full[kSiluStages];
   __shared__ float red[kThreads / 32];
@@ -1085,7 +1084,7 @@ int check_add_norm(const void* h, const void* delta, const void* weight, const v
 // Dynamic per-token FP8 quantize of many long bf16 rows through the ring-fed persistent kernel
 // (silu_mul_quant_stream_kernel<.., false>).  Returns 1 when the shape does not qualify (the caller
 // then takes its one-CTA-per-row kernels), else the launch status.
-int launch_fp8_rows_stream(const __nv_bfloat16* x, uint8_t* codes, float* scales, int64_t rows, int64_t cols, cudaStream_t st) {
+int launch_fp8_rows_stream(const __nv_bfloat16* x, uint8_t* codes, float* scales, int64_t rows, int64_t cols, cudaStream_t st, bool late) {
   static const bool enabled = [] {
     const char* e = std::getenv("B200Q_ROWS_STREAM");   // 0 = always one CTA per row (A/B measurements)
     return e == nullptr || e[0] != '0';
@@ -1105,7 +1104,7 @@ int launch_fp8_rows_stream(const __nv_bfloat16* x, uint8_t* codes, float* scales
 #define B200Q_ROWS_STREAM(C)                                                                                                 \
   do {                                                                                                                        \
     cudaFuncSetAttribute(silu_mul_quant_stream_kernel<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
-    launch_pdl(silu_mul_quant_stream_kernel<C, false>, grid, dim3(kThreads), smem, st, x, codes, scales, r32, f32, status);           \
+    launch_pdl(silu_mul_quant_stream_kernel<C, false>, grid, dim3(kThreads), smem, st, x, codes, scales, r32, f32, status, late);     \
   } while (0)
   if (nch <= 2) B200Q_ROWS_STREAM(2);
   else if (nch <= 4) B200Q_ROWS_STREAM(4);
@@ -1135,7 +1134,7 @@ int silu_mul_fp8_quantize(const void* gate_up, uint8_t* codes_out, float* scales
 #define B200Q_SILUS(C)                                                                                              \
   do {                                                                                                               \
     cudaFuncSetAttribute(silu_mul_quant_stream_kernel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
-    launch_pdl(silu_mul_quant_stream_kernel<C, true>, grid, dim3(kThreads), smem, st, gp, codes_out, scales_out, r32, f32, status);   \
+    launch_pdl(silu_mul_quant_stream_kernel<C, true>, grid, dim3(kThreads), smem, st, gp, codes_out, scales_out, r32, f32, status, late); \
   } while (0)
     if (nch <= 2) B200Q_SILUS(2);
     else if (nch <= 4) B200Q_SILUS(4);
