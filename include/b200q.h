@@ -158,8 +158,9 @@ int b200q_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales_swizzled,
  *                   reduce-scatter forms take pairs from one such tile per SM pair on (NVFP4: never);
  *                   1001 / 1002 / 1004 / 1008 = small-M kernel (weights on the tensor core's M side,
  *                   K split over a cluster of 1 / 2 / 4 / 8 CTAs, partial tiles summed through
- *                   distributed shared memory; chosen automatically for M <= 128, and above in blocks of
- *                   up to 256 (NVFP4 128) tokens where tiles would leave SMs idle).  Results do not depend on it beyond fp32 summation order.  Any other value:
+ *                   distributed shared memory; chosen automatically for M <= 128, ignored for larger M,
+ *                   where it is chosen in blocks of up to 256 (NVFP4 128) tokens if tiles would leave SMs
+ *                   idle).  Results do not depend on it beyond fp32 summation order.  Any other value:
  *                   B200Q_ERR_INVALID.
  *   static_weights  promise about the B operand (weights, their scales, the bias) of THIS call:
  *                   non-zero = the work that wrote it has FINISHED on the device (weights quantized at

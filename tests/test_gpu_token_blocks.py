@@ -1,34 +1,39 @@
 """The GEMM above 128 rows as blocks of tokens with K split over clusters: sizes around the block limits (256 tokens FP8, 128 NVFP4),
-ragged weight rows and K, a bias, every cluster size forced and the library's choice.  Operands are small integers, so that every
+ragged weight rows and K, a bias, and every cluster size that the library chooses.  Operands are small integers, so that every
 order of summation gives the same fp32 value and the result is compared bit for bit."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(129, 1024, 1024), (144, 1001, 528), (255, 256, 4096), (256, 4096, 2048), (257, 2048, 1040), (333, 136, 8192), (512, 1024, 2048), (513, 264, 1024),
-         (700, 128, 4096)]
+# on 148 SMs: tiles, then clusters of 1, 2, 4 and 8
+FP8_SIZES = [(129, 1024, 1024), (144, 1001, 528), (255, 256, 4096), (256, 4096, 2048), (257, 2048, 1040), (512, 1024, 2048), (513, 264, 1024),
+             (257, 8190, 528),
+             (129, 6150, 4096), (513, 1530, 14336),
+             (144, 520, 2064), (257, 1001, 8192), (700, 128, 4096),
+             (129, 130, 8192), (333, 136, 8192), (255, 512, 14336), (1200, 264, 28672)]
+# tiles, then clusters of 2, 4 and 8
+NVFP4_SIZES = [(129, 1024, 1024),
+               (144, 4090, 2080), (384, 2048, 2048),
+               (257, 256, 2080), (256, 1001, 4096),
+               (129, 520, 14336), (500, 136, 8192)]
 
 
-@pytest.mark.parametrize("force", [0, 1001, 1002, 1004, 1008])
-@pytest.mark.parametrize("M,N,K", SIZES)
-def test_fp8(b200, M, N, K, force):
+@pytest.mark.parametrize("M,N,K", FP8_SIZES)
+def test_fp8(b200, M, N, K):
     capi = b200.capi
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     ints = lambda *shape: torch.randint(-2, 3, shape, device="cuda", generator=g).float()  # noqa: E731
     x, w, bias = ints(M, K), ints(N, K), ints(N).bfloat16()
     xs = 2.0 ** torch.randint(-2, 3, (M,), device="cuda", generator=g).float()             # a scale per token tells the rows apart
     to_codes = lambda t: t.to(torch.float8_e4m3fn).view(torch.uint8)  # noqa: E731
-    if force > 1000 and (K + 127) // 128 < force - 1000:
-        force = 0
-    y = capi.fp8_gemm(to_codes(x), xs, to_codes(w), torch.ones(N, device="cuda"), bias, tile_n=force)
+    y = capi.fp8_gemm(to_codes(x), xs, to_codes(w), torch.ones(N, device="cuda"), bias)
     ref = ((x.double() @ w.double().t()) * xs.double()[:, None] + bias.double()).float().bfloat16()
     assert torch.equal(y, ref) and capi.device_status() == 0
 
 
-@pytest.mark.parametrize("force", [0, 1001, 1002, 1004, 1008])
-@pytest.mark.parametrize("M,N,K", [(129, 1024, 1024), (256, 1001, 4096), (257, 256, 2080), (384, 2048, 2048), (500, 136, 8192)])
-def test_nvfp4(b200, M, N, K, force):
+@pytest.mark.parametrize("M,N,K", NVFP4_SIZES)
+def test_nvfp4(b200, M, N, K):
     capi = b200.capi
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     values = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], device="cuda")
@@ -41,8 +46,17 @@ def test_nvfp4(b200, M, N, K, force):
         ref = values[codes & 7] * torch.where(codes >= 8, -1.0, 1.0) * block
         return ((codes[:, 0::2] | (codes[:, 1::2] << 4)).to(torch.uint8), swizzle_scales(sf).cuda(), torch.ones(1, device="cuda")), ref
 
-    if force > 1000 and (K // 2 + 127) // 128 < force - 1000:
-        force = 0
     (xq, x), (wq, w) = operand(M), operand(N)
-    y = capi.nvfp4_gemm(*xq, *wq, tile_n=force)
+    y = capi.nvfp4_gemm(*xq, *wq)
     assert torch.equal(y, (x.double() @ w.double().t()).float().bfloat16()) and capi.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(512, 2048, 8192), (1500, 1024, 8192), (129, 6150, 4096)])
+@pytest.mark.parametrize("force", [1001, 1002, 1004, 1008])
+def test_forced_cluster_size_is_for_128_rows(b200, M, N, K, force):
+    """Above 128 rows it is ignored: the bits of the library's own choice (other kernels sum K in another order)."""
+    capi = b200.capi
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    ops = (*capi.fp8_quantize(x), *capi.fp8_quantize(w))
+    assert torch.equal(capi.fp8_gemm(*ops, tile_n=force), capi.fp8_gemm(*ops)) and capi.device_status() == 0
