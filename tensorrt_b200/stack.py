@@ -313,11 +313,12 @@ class DecoderLayer:
         self.amax: dict = {}
         self.calibrating = False
 
-    def plain(self) -> bool:
-        """Nothing replaced or switched on that `DecoderStack._native_forward` does not know of."""
-        return (type(self) is DecoderLayer and self.row_parallel is self._local_linear and self.world == 1 and not self.calibrating and
-                not {"forward", "_attention", "_ffn_act"} & self.__dict__.keys() and
-                (self.cfg.mode == "fp8" or self.amax.keys() >= {"qkv", "o", "gate_up", "down"}))
+    def plain(self, cfg: StackConfig, backend) -> bool:
+        """A layer of that configuration and backend, with nothing replaced or switched on that `DecoderStack._native_forward`
+        does not know of."""
+        return (type(self) is DecoderLayer and self.cfg is cfg and self.backend is backend and self.row_parallel is self._local_linear and
+                self.world == 1 and not self.calibrating and self.__dict__.keys().isdisjoint(_NATIVE_METHODS[DecoderLayer]) and
+                (cfg.mode == "fp8" or self.amax.keys() >= {"qkv", "o", "gate_up", "down"}))
 
     def tensors(self) -> tuple:
         """Weights and calibrated ranges in the order of `_native.decoder_stack`."""
@@ -526,12 +527,16 @@ class DecoderStack:
 
     def _native_forward(self, h: torch.Tensor):
         """The layers of `DecoderLayer.forward` as one native call (the same kernels in the same order, the same bits), or None
-        where that does not take them: several ranks, another backend or layer class, a replaced method, a forced GEMM tile, a
-        calibrating pass, NVFP4 without calibrated ranges, tokens that are not whole sequences."""
+        where that does not take them: several ranks, another backend or layer class, a method replaced on the stack, a layer,
+        the backend or their classes, a layer with a configuration or backend of its own, a forced GEMM tile, a calibrating pass,
+        NVFP4 without calibrated ranges, tokens that are not whole sequences."""
         cfg, be = self.cfg, self.backend
         if not self.native_layers or self.world != 1 or type(be) is not CudaBackend or be.__dict__.keys() != {"mode", "fuse_gate_up"} or not h.is_cuda:
             return None
-        if be.mode != cfg.mode or capi.gemm_defaults() != (0, True) or not all(l.plain() for l in self.layers):
+        if not self.__dict__.keys().isdisjoint(_NATIVE_METHODS[DecoderStack]) or not (
+                _as_defined(type(self), DecoderStack) and _as_defined(DecoderLayer, DecoderLayer) and _as_defined(CudaBackend, CudaBackend)):
+            return None
+        if be.mode != cfg.mode or capi.gemm_defaults() != (0, True) or not all(l.plain(cfg, be) for l in self.layers):
             return None
         seq_len = cfg.seq_len if cfg.attention == "fp8_sdpa" else 0
         if seq_len and h.shape[0] % seq_len:
@@ -647,6 +652,18 @@ class DecoderStack:
         finally:
             for layer in self.layers:
                 layer.calibrating = False
+
+
+# What a forward on one rank runs besides the kernels, as defined above: the native call stands for exactly this.
+_NATIVE_METHODS = {cls: {n: getattr(cls, n) for n in names} for cls, names in (
+    (DecoderStack, ("_enter", "_walk", "_finish")),
+    (DecoderLayer, ("forward", "_attention", "_ffn_act", "_amax", "_norm_amax", "_static_amax")),
+    (CudaBackend, tuple(n for n in vars(CudaBackend) if not n.startswith("__"))))}
+
+
+def _as_defined(cls, base) -> bool:
+    """No method that a forward on one rank runs is replaced in `cls`, `base` or a class derived from it."""
+    return all(getattr(cls, n) is f for n, f in _NATIVE_METHODS[base].items())
 
 
 def random_layer_weights(cfg: StackConfig, seed: int, device="cuda", dtype=torch.bfloat16):

@@ -69,3 +69,63 @@ def test_what_goes_call_by_call(b200):
         stack.forward(torch.randn(100, 256, device="cuda").bfloat16())      # no whole sequences
     with pytest.raises(ValueError):
         stack.forward(torch.randn(64, 256, device="cuda"))                  # fp32
+
+
+def _other_backend(stack):
+    from tensorrt_b200.stack import CudaBackend
+    stack.layers[1].backend = CudaBackend("nvfp4", fuse_gate_up=False)
+
+
+def _other_config(stack):
+    import dataclasses
+    stack.layers[0].cfg = dataclasses.replace(stack.cfg, eps=0.5)
+
+
+REPLACED = {
+    "a layer's backend": _other_backend, "a layer's configuration": _other_config,
+    **{f"a layer's {n}": (lambda n: lambda stack: setattr(stack.layers[1], n, getattr(stack.layers[1], n)))(n)
+       for n in ("forward", "_attention", "_ffn_act", "_amax", "_norm_amax", "_static_amax")},
+    **{f"the stack's {n}": (lambda n: lambda stack: setattr(stack, n, getattr(stack, n)))(n) for n in ("_enter", "_walk", "_finish")}}
+
+
+@pytest.mark.parametrize("what", REPLACED)
+def test_replaced_on_an_object(b200, what):
+    stack = _stack(b200, "nvfp4", 4, 2, 64, 768, 2, 0, True)
+    h = torch.randn(32, 256, device="cuda").bfloat16()
+    with b200.capi.gemm_config(static_weights=True):
+        assert stack._native_forward(h) is not None
+        REPLACED[what](stack)
+        assert stack._native_forward(h) is None
+
+
+@pytest.mark.parametrize("owner,name", [("DecoderStack", "_walk"), ("DecoderLayer", "forward"), ("DecoderLayer", "_amax"), ("CudaBackend", "matmul"),
+                                        ("CudaBackend", "add")])
+def test_replaced_in_a_class(b200, monkeypatch, owner, name):
+    from tensorrt_b200 import stack as module
+
+    stack = _stack(b200, "fp8", 4, 2, 64, 768, 1, 0, False)
+    h = torch.randn(32, 256, device="cuda").bfloat16()
+    cls = getattr(module, owner)
+    orig = getattr(cls, name)
+    wrapped = lambda *a, **k: orig(*a, **k)  # noqa: E731
+    monkeypatch.setattr(cls, name, staticmethod(wrapped) if name == "add" else wrapped)
+    with b200.capi.gemm_config(static_weights=True):
+        assert stack._native_forward(h) is None
+
+
+def test_subclass_of_the_stack(b200):
+    from tensorrt_b200.stack import DecoderStack, StackConfig, random_layer_weights
+
+    class Doubled(DecoderStack):
+        def _finish(self, h, delta, sharded):
+            return super()._finish(h, delta, sharded) * 2
+
+    class Plain(DecoderStack):
+        pass
+
+    cfg = StackConfig(hidden=256, n_q=4, n_kv=2, head_dim=64, ffn=768, layers=1)
+    h = torch.randn(32, 256, device="cuda").bfloat16()
+    out = [cls(cfg, random_layer_weights(cfg, 3)).forward(h) for cls in (DecoderStack, Plain, Doubled)]
+    assert torch.equal(out[1], out[0]) and torch.equal(out[2], out[0] * 2)
+    with b200.capi.gemm_config(static_weights=True):
+        assert Plain(cfg, random_layer_weights(cfg, 3))._native_forward(h) is not None
