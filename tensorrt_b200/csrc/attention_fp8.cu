@@ -809,13 +809,6 @@ int launch_sdpa_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
   return check_launch();
 }
 
-template <typename QT, bool WIDE>
-int launch_sdpa_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
-                   cudaStream_t st) {
-  return p.out_dtype == B200Q_BF16 ? launch_sdpa_form<QT, WIDE, true>(tq, tk, tv, p, ctas, behind, st)
-                                   : launch_sdpa_form<QT, WIDE, false>(tq, tk, tv, p, ctas, behind, st);
-}
-
 // p: scales, queries (q_amax == nullptr: codes, at `q_codes`) and the result filled in.  `behind`: the kernel that writes the K and
 // V operands was launched directly in front.
 int launch_sdpa(AttParams& p, const uint8_t* q_codes, const uint8_t* k_codes, const uint8_t* vt_codes, const int64_t* out_strides,
@@ -854,14 +847,17 @@ int launch_sdpa(AttParams& p, const uint8_t* q_codes, const uint8_t* k_codes, co
   p.group = head_group(p);
   const unsigned n = static_cast<unsigned>(ctas);
   const auto st = static_cast<cudaStream_t>(stream);
-  if (codes) return launch_sdpa_as<uint8_t, true>(tq, tk, tv, p, n, behind, st);
+  if (codes)
+    return p.out_dtype == B200Q_BF16 ? launch_sdpa_form<uint8_t, true, true>(tq, tk, tv, p, n, behind, st)
+                                     : launch_sdpa_form<uint8_t, true, false>(tq, tk, tv, p, n, behind, st);
   const int64_t unit = q_dtype == B200Q_F32 ? 8 : 16;
   const bool wide = aligned(p.q, 32) && p.q_sb % unit == 0 && p.q_sh % unit == 0 && p.q_ss % unit == 0;
-#define B200Q_SDPA(T) (wide ? launch_sdpa_as<T, true>(tq, tk, tv, p, n, behind, st) : launch_sdpa_as<T, false>(tq, tk, tv, p, n, behind, st))
+  // queries and result have one type here
+#define B200Q_SDPA(T, FREE) (wide ? launch_sdpa_form<T, true, FREE>(tq, tk, tv, p, n, behind, st) : launch_sdpa_form<T, false, FREE>(tq, tk, tv, p, n, behind, st))
   switch (q_dtype) {
-    case B200Q_BF16: return B200Q_SDPA(__nv_bfloat16);
-    case B200Q_F16: return B200Q_SDPA(__half);
-    case B200Q_F32: return B200Q_SDPA(float);
+    case B200Q_BF16: return B200Q_SDPA(__nv_bfloat16, true);
+    case B200Q_F16: return B200Q_SDPA(__half, false);
+    case B200Q_F32: return B200Q_SDPA(float, false);
     default: return B200Q_ERR_INVALID;
   }
 #undef B200Q_SDPA
