@@ -28,8 +28,9 @@
 // buffer back before it computes (the tensor core fills it under the exponentials); in pass 2 the scores of tile j + 2
 // are issued in front of the product of tile j (wait for scores per tile 819 -> 171 clocks of about 2500); edge tiles
 // have their own copy of the loop; query tiles with the most keys start first (head_group).  Order and roundings per row are those
-// of a loop over 32-column pieces.  [4, 32 / 8, 2048, 128] causal: 300 -> 245 us for the call, 199 with the exponentials on both pipes,
-// constant addresses, queries quantized here and the last tile raised once (bf16 results, see FREE).
+// of a loop over 32-column pieces for fp16 and fp32 results; bf16 results see FREE.  [4, 32 / 8, 2048, 128] causal, the whole call in
+// turn with others: 300 -> 246 us, 208 with the exponentials on both pipes, constant addresses, queries quantized here and the last
+// tile raised once.
 //
 // One CTA per (batch, head, 128 queries): warp 0 = TMA producer, warp 1 = MMA issue + tensor-memory
 // allocation, warps 2-9 = softmax (two threads per query row, each half of the columns; lane quarter = warp & 3).  K and Q tiles are
@@ -150,9 +151,14 @@ __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, f
 // operands of K and V: each is read by one CTA only, so a pass of its own would write and read their codes for nothing.  Both launches,
 // us, operand pass for all three / this: [4, 32 / 8, 2048, 128] causal 212 / 202; [3, 16, 577 x 1500, 64] 51 / 47.7; [8, 32 / 8, 1024,
 // 128] causal 147 / 137; [8, 12, 200, 128] causal 21.2 / 18.9; [1, 8, 64, 64] 13.1 / 11.2.
-// FREE: results of 8 significant bits (bf16).  There an eighth of the exponentials runs on the FMA pipe and the last key tile keeps its
-// own; both move a probability that lies within about 1e-7 of a rounding boundary to the next code, which a bf16 result of many
-// keys does not show.  Results of 11 and more bits (fp16, fp32) keep every operation and its order: the same bits as before.
+// FREE: bf16 results.  There an eighth of the exponentials runs on the FMA pipe and the last key tile keeps its own.  Neither holds
+// anything in fewer bits, but both change roundings, and a probability as near to a boundary of E4M3 as fp32 resolves it may take the
+// code on the other side.  How near, in both forms and for rows of up to 200 keys: within 2^-24 ln 2 (8 s + 16) + 2^-21 of it, s the
+// row's largest score in powers of two; a few of 100 000 probabilities.  (Distance to 64 bits at [4, 32 / 8, 2048, 128] causal
+// 1.678e-3 -> 1.656e-3.)  Such a probability changes by one step, at most an eighth.  In a row of few keys that is several steps of a
+// bf16 result; in rows of many, single values moved by up to 0.12 against the other form, 3.5e-4 of the norm.  The line lies at the
+// type because the same change is eight times as many steps of an fp16 result, which callers compare to 1e-3: fp16 and fp32 keep every
+// operation and its order.
 template <typename QT, bool WIDE, bool FREE>
 __global__ void __launch_bounds__(kAttThreads, 2)
 fp8_sdpa_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
