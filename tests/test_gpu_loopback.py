@@ -108,7 +108,8 @@ def _gemm_to_owners(capi, rk, xs, ws, mode, tile):
 
 
 CASES = [(2, 512, 512, 1024, 128), (2, 1024, 768, 2048, 256), (2, 2048, 2560, 1024, 512), (4, 1024, 512, 2048, 0),
-         (4, 2048, 2560, 2048, 512), (8, 2048, 256, 4096, 128), (8, 4096, 1280, 4096, 512)]
+         (4, 2048, 2560, 2048, 512), (8, 2048, 256, 4096, 128), (8, 4096, 1280, 4096, 512),
+         (2, 512, 520, 1024, 448), (4, 2048, 2560, 2048, 448)]
 
 
 @pytest.mark.parametrize("world,M,N,K,tile", CASES)
