@@ -66,6 +66,8 @@ constexpr int kKStages = 2, kVStages = 1;
 constexpr int kChunk = 32;                 // score columns of one step of a softmax thread
 constexpr int kTmemCols = 256;
 constexpr int kAttSmem = kTileBytes * (1 + kKStages + kVStages + 2) + 512;   // tail: barriers
+constexpr int kAttSmemAlone = 114 * 1024;  // with the 1 KB that each CTA costs, more than half of an SM's 228 KB
+static_assert(kAttSmemAlone >= kAttSmem, "");
 // Of the 16 pairs of a chunk, those whose exponentials run on the FMA pipe (ex2_poly2), us of this kernel with 0 / 2 / 3 / 4 of them:
 // [4, 32 / 8, 2048, 128] causal 190 / 180 / 181 / 185; [3, 16, 577 x 1500, 64] 41.8 / 40.0 / 39.5 / 40.5; [8, 32 / 8, 1024, 128] causal
 // 119 / 115 / 117 / 118; [1, 74, 4096, 128] 740 / 703 / 700 / 732.  Beyond four the issue slots bind.
@@ -797,20 +799,31 @@ int check_attention(const void* q, const void* k, const void* v, const void* out
   return B200Q_OK;
 }
 
+// Under a programmatic launch CTAs are placed while the kernel in front still holds SMs: two on an SM that is free, none on one that is
+// free a little later.  With no more CTAs than SMs each therefore asks for so much shared memory that it has its SM alone.  With up to
+// two per SM and causal, where the longest query tiles start first so as to share an SM with short ones, the launch is a plain one.
+// Otherwise the fullest SM has two either way, and calls of up to five key tiles gain more from the early start.  Whole calls in a
+// graph, us, three operands and a plain launch / programmatic as it comes / this rule: bf16 [1, 4, 4096, 128] 72.7 / 93.7 / 58.6, [1, 16 / 4,
+// 909, 64] 24.4 / 28.1 / 20.3; causal [1, 16 / 4, 2048, 128] 46.4 / 50.0 / 39.5, fp16 [1, 15 / 5, 1300, 128] 32.2 / 36.8 / 28.4.  Over 900
+// shapes never slower than the first (0.96 at most; programmatic as it comes 1.55), up to 1.08 of the second where that happens to
+// spread ([4, 5, 1000, 64] causal 26.9 / 21.4 / 22.8).
 template <typename QT, bool WIDE, bool FREE>
 int launch_sdpa_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttParams& p, unsigned ctas, bool behind,
                           cudaStream_t st) {
+  const unsigned sms = static_cast<unsigned>(sm_count());
+  const int smem = behind && ctas <= sms ? kAttSmemAlone : kAttSmem;
+  if (ctas > sms && ctas <= 2 * sms && p.causal && p.Sk > 5 * kTile) behind = false;
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return B200Q_ERR_CUDA;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(fp8_sdpa_kernel<QT, WIDE, FREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmem) != cudaSuccess) return B200Q_ERR_CUDA;
+    if (cudaFuncSetAttribute(fp8_sdpa_kernel<QT, WIDE, FREE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttSmemAlone) != cudaSuccess) return B200Q_ERR_CUDA;
     configured[dev] = true;
   }
   if (behind) {
-    if (launch_pdl(fp8_sdpa_kernel<QT, WIDE, FREE>, dim3(ctas), dim3(kAttThreads), kAttSmem, st, tq, tk, tv, p) != cudaSuccess) return B200Q_ERR_CUDA;
+    if (launch_pdl(fp8_sdpa_kernel<QT, WIDE, FREE>, dim3(ctas), dim3(kAttThreads), smem, st, tq, tk, tv, p) != cudaSuccess) return B200Q_ERR_CUDA;
   } else {
-    fp8_sdpa_kernel<QT, WIDE, FREE><<<ctas, kAttThreads, kAttSmem, st>>>(tq, tk, tv, p);
+    fp8_sdpa_kernel<QT, WIDE, FREE><<<ctas, kAttThreads, smem, st>>>(tq, tk, tv, p);
   }
   return check_launch();
 }

@@ -63,3 +63,18 @@ def test_values_that_are_not_finite(b200, scale, dtype):
     am = [torch.full((1,), a, device="cuda") for a in (2.0 * scale, 2.0, 2.0)]
     ref, out = _both(q, k, v, am, 0)
     assert torch.equal(ref.view(torch.int32 if dtype == torch.float32 else torch.int16), out.view(torch.int32 if dtype == torch.float32 else torch.int16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("keys", [640, 700])              # five key tiles, and more
+@pytest.mark.parametrize("ctas", ["sms - 1", "sms", "sms + 1", "2 * sms", "2 * sms + 1"])
+def test_ways_of_launching(b200, ctas, keys):
+    """One CTA per SM, a plain and a programmatic launch, by the number of CTAs and the length of the key axis: the same bits."""
+    heads = eval(ctas, {"sms": torch.cuda.get_device_properties(0).multi_processor_count})
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    q, k, v = (torch.randn(1, heads, s, 64, device="cuda", generator=g).bfloat16() for s in (100, keys, keys))
+    am = [t.float().abs().max().reshape(1) for t in (q, k, v)]
+    for causal in (0, 1):
+        ref, out = _both(q, k, v, am, causal)
+        assert torch.equal(ref, out)
+    assert b200.capi.device_status() == 0
