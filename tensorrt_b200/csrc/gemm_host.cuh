@@ -3,6 +3,8 @@
 
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "gemm_kernel_2cta.cuh"
 #include "gemm_kernel_nvf4_pair.cuh"
 #include "gemm_kernel_splitk.cuh"
@@ -410,9 +412,14 @@ inline int large_tile(int M, int N, int sms, bool nvf4, bool rs) {
 // are estimated in ns from a sweep of all kernels over 12 weight shapes and 129 to 1024 rows in each format (180 points, standard
 // deviation 3 to 6 %): the tile kernels as rounds times (start + K tiles), the small-M kernel as K tiles of a CTA, the parked
 // partial tile (every token, more the larger the cluster) and the traffic of all clusters together; only where all clusters are
-// resident at once, one CTA per SM.  Taken where it is 3 % cheaper: 48 of 180 points, nowhere slower than the tile kernel; FP8, us,
-// tile kernel / this: 4096 x 14336 at 129 rows 35.6 / 19.2, at 256 35.6 / 25.2, at 384 36.2 / 26.7; 2048 x 8192 at 256 22.2 / 17.3;
-// 8192 x 28672 at 129 69.2 / 48.6; 4096 x 4096 at 129 14.0 / 11.4; NVFP4 4096 x 14336 at 256 27.4 / 20.0.
+// resident at once, one CTA per SM (asked of the kernel for one block, which fills an SM as well).  Taken where it is cheaper by 3 %
+// and by 1 us (NVFP4 1.6): a launch of clusters behind a quantize kernel costs more than one of tiles.  Whole calls in a graph, 1530
+// sizes where this holds (129 to 4000 rows): FP8 0.75 of the time on average, 2 of 808 slower by 2.5 to 2.8 %; NVFP4 0.83, none of 722
+// by more than 1 %.  With 3 % alone, 73 more FP8 sizes, 0.90 to 1.08 of the time, and 370 more NVFP4 sizes, 0.89 to 1.12.  It leaves
+// points behind: FP8 4096 x 4096 at 333 rows 14.3 us on tiles, 13.3 on clusters of two.  FP8, the GEMM alone, us, tile kernel / this:
+// 4096 x 14336 at 129 rows 35.6 / 19.2, at 256 35.6 / 25.2, at 384 36.2 / 26.7; 2048 x 8192 at 256 22.2 / 17.3; 8192 x 28672 at 129 69.2
+// / 48.6; 4096 x 4096 at 129 14.0 / 11.4; NVFP4 4096 x 14336 at 256 27.4 / 20.0.
+constexpr int64_t kBlocksGainFp8 = 1000, kBlocksGainNv = 1600;   // ns
 inline int block_splits(int M, int N, int k_tiles, int sms, bool nvf4, int tile) {
   const int blocks = smallm_blocks(M, nvf4), n_tiles = (N + kSmallWRows - 1) / kSmallWRows;
   const int64_t clusters = static_cast<int64_t>(n_tiles) * blocks;
@@ -429,7 +436,7 @@ inline int block_splits(int M, int N, int k_tiles, int sms, bool nvf4, int tile)
             : tile == 448 ? 5000 + rounds * (1300 + 300 * k_tiles)
                           : (tile == 256 ? 3600 + rounds * (1640 + 391 * k_tiles) : 4100 + rounds * (510 + 289 * k_tiles));
   }
-  least = least * 97 / 100;
+  least = std::min(least * 97 / 100, least - (nvf4 ? kBlocksGainNv : kBlocksGainFp8));
   const int64_t bt = smallm_block_tokens(M, blocks, nvf4);
   const ActiveClusters active = active_clusters(sms);
   int best = 0;

@@ -8,15 +8,16 @@ pytestmark = pytest.mark.gpu
 
 # on 148 SMs: tiles, then clusters of 1, 2, 4 and 8
 FP8_SIZES = [(129, 1024, 1024), (144, 1001, 528), (255, 256, 4096), (256, 4096, 2048), (257, 2048, 1040), (512, 1024, 2048), (513, 264, 1024),
-             (257, 8190, 528),
+             (257, 8190, 528), (144, 520, 2064), (700, 128, 4096),
+             (647, 6266, 3088),
              (129, 6150, 4096), (513, 1530, 14336),
-             (144, 520, 2064), (257, 1001, 8192), (700, 128, 4096),
+             (144, 520, 4112), (257, 1001, 8192),
              (129, 130, 8192), (333, 136, 8192), (255, 512, 14336), (1200, 264, 28672)]
 # tiles, then clusters of 2, 4 and 8
-NVFP4_SIZES = [(129, 1024, 1024),
-               (144, 4090, 2080), (384, 2048, 2048),
-               (257, 256, 2080), (256, 1001, 4096),
-               (129, 520, 14336), (500, 136, 8192)]
+NVFP4_SIZES = [(129, 1024, 1024), (144, 4090, 2080), (384, 2048, 2048), (257, 256, 2080),
+               (144, 4090, 4128), (384, 2048, 8192),
+               (256, 1001, 4096),
+               (129, 520, 14336), (500, 136, 8192), (257, 256, 6176)]
 
 
 @pytest.mark.parametrize("M,N,K", FP8_SIZES)
