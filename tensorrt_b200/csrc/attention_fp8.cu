@@ -19,7 +19,8 @@
 // core is a few per cent of a decoder layer's arithmetic, so the repeated Q K^T is cheaper than a
 // rescaling scheme whose quantization points would differ from the definition above.
 //
-// What bounds it: the exponentials, two per score at 16 per clock and SM: 1024 clocks per 128 x 128 tile and pass, and
+// What bounds it: the chain of a key tile, and beside it (special-function pipe 62 % and issue slots 55 % of active cycles at
+// [4, 32 / 8, 2048, 128] causal) the exponentials, two per score at 16 per clock and SM: 1024 clocks per 128 x 128 tile and pass, and
 // two warps per scheduler and CTA reach 0.93 of that rate in a loop of their own.  An eighth of them runs on the FMA pipe instead
 // (ex2_poly2, more exact than the unit).  What it loses beside them is warps that wait for scores: without any arithmetic in the
 // softmax warps the kernel still takes 0.58 of its time, the chain of loads, MMAs and barriers of a tile.  Shared-memory addresses
