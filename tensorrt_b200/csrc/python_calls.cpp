@@ -5,9 +5,9 @@
 // Python (argument checks, two to six tensors, a ctypes call per kernel) take longer than that on the host.  The
 // functions here issue the same b200q_* calls on the current stream with the scratch of a call in one allocation.
 //
-// Every GEMM here stands directly behind a kernel that quantizes its activation and lets its dependents go late
-// (common.cuh::pdl_enter), so it may request weight tiles before that kernel ends: static_weights without a promise
-// from the caller.
+// The GEMMs of the linears and the MLP stand directly behind a kernel that quantizes their activation and lets its dependents
+// go late (common.cuh::pdl_enter; tests/test_late_quantizers.py), so they may request weight tiles before that kernel ends:
+// static_weights without a promise from the caller.  Those of the stack rest on its constructor, which waits for its weights.
 //
 // They take the plain case only (strided CUDA tensors of the exact Python type, matching sizes, fp32 scales, no
 // dispatch or function mode active) and return None for anything else, before anything is launched: the caller then
